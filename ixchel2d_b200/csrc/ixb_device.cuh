@@ -2,8 +2,8 @@
 // line solvers of the SIMPLE hot path.
 //
 // Layout in HBM: every 2-D field (u, v, p, T, p', the *_ant copies, au, av,
-// b_o, Resu, sources) is one array of (nj+2) rows x LD doubles, LD = mi+1
-// rounded up to 32 elements (256 B), with Fortran index (ii,jj) at
+// b_o, Resu, sources) is one array of (nj+2) rows x LD doubles, LD >= mi+1
+// with LD = 4 modulo 16 (ixb_create), with Fortran index (ii,jj) at
 // (jj-1)*LD + (ii-1).  Adjacent ii are adjacent in memory, so x-lines are
 // contiguous and the y-lines of a tile of adjacent ii are read as coalesced
 // row segments.  1-D metrics are 1-based arrays (element 0 unused).
