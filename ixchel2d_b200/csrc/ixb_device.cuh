@@ -644,13 +644,6 @@ __device__ void thomas_pcr_warp(R* sa, R* sb, R* sc, R* sd, int m, int mp) {
 }
 
 
-// Reduced system of a partitioned line solve: the first and last rows of G
-// chunks, each with unit diagonal, coupled to the neighbouring chunks' end
-// rows (row 2k: eA x_{2k-1} + x_{2k} + eC x_{2k+1} = eD; row 2k+1 likewise
-// with oA, oC, oD).  Solved by parallel cyclic reduction over log2(2G) steps
-// in shared memory `red` (12 G elements, two buffers of a | c | d); thread
-// k supplies rows 2k, 2k+1 and receives their solutions x0, xl.  Called by
-// all threads of the CTA (it holds barriers); `active` false: barriers only.
 // Barrier of the G threads that solve one line when a CTA holds TL lines of
 // whole warps (a named barrier per line, so lines do not wait for each
 // other), else of the whole CTA.
@@ -663,40 +656,157 @@ __device__ __forceinline__ void line_sync() {
   }
 }
 
-template <class R, int G, int TL = 1>
-__device__ __forceinline__ void reduced_pcr(R* red, int k, bool active, R eA, R eC, R eD, R oA, R oC, R oD, R& x0,
-                                            R& xl) {
-  R* cur = red;
-  R* nxt = red + 6 * G;
-  if (active) {
-    cur[2 * k] = eA; cur[2 * G + 2 * k] = eC; cur[4 * G + 2 * k] = eD;
-    cur[2 * k + 1] = oA; cur[2 * G + 2 * k + 1] = oC; cur[4 * G + 2 * k + 1] = oD;
-  }
-  line_sync<G, TL>();
-#pragma unroll 1
-  for (int s = 1; s < 2 * G; s <<= 1) {
-    if (active) {
-      const R* Ac = cur; const R* Cc = cur + 2 * G; const R* Dc = cur + 4 * G;
-      R* An = nxt; R* Cn = nxt + 2 * G; R* Dn = nxt + 4 * G;
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const int i = k + q * G;
-        const R ai = Ac[i], ci = Cc[i], di = Dc[i];
-        R alo = R(0), clo = R(0), dlo = R(0), ahi = R(0), chi = R(0), dhi = R(0);
-        if (i - s >= 0) { alo = Ac[i - s]; clo = Cc[i - s]; dlo = Dc[i - s]; }
-        if (i + s < 2 * G) { ahi = Ac[i + s]; chi = Cc[i + s]; dhi = Dc[i + s]; }
-        const R r = fast_rcp(fmaT(-ci, ahi, fmaT(-ai, clo, R(1))));
-        An[i] = -ai * alo * r;
-        Cn[i] = -ci * chi * r;
-        Dn[i] = fmaT(-ci, dhi, fmaT(-ai, dlo, di)) * r;
-      }
-    }
-    line_sync<G, TL>();
-    R* t = cur; cur = nxt; nxt = t;
-  }
-  x0 = cur[4 * G + 2 * k];
-  xl = cur[4 * G + 2 * k + 1];
+// One parallel-cyclic-reduction step of a row with unit diagonal,
+// x + A x_lo + C x_hi = D, against its two neighbours' rows.
+template <class R>
+__device__ __forceinline__ void pcr_row(R& A, R& C, R& D, R lA, R lC, R lD, R hA, R hC, R hD) {
+  const R r = fast_rcp(fmaT(-C, hA, fmaT(-A, lC, R(1))));
+  const R nA = -A * lA * r, nC = -C * hC * r, nD = fmaT(-C, hD, fmaT(-A, lD, D)) * r;
+  A = nA; C = nC; D = nD;
 }
+
+// Reduced system of a partitioned line solve: the first and last rows of G
+// chunks, each with unit diagonal, coupled to the neighbouring chunks' end
+// rows (row 2k: eA x_{2k-1} + x_{2k} + eC x_{2k+1} = eD; row 2k+1 likewise
+// with oA, oC, oD).  Thread k of a line supplies rows 2k, 2k+1 and receives
+// their solutions x0, xl by parallel cyclic reduction over shared memory.
+//
+// The solve is bound by shared-memory bandwidth (nothing else in it comes
+// close), so a thread keeps its own rows in registers and exchanges only
+// what its neighbours read.  The first step (row distance 1) couples even
+// and odd rows; every later one couples rows of one parity at distance h in
+// k, i.e. two independent systems of G rows.
+//  * HALF: only the odd (last) rows are reduced further and the even ones
+//    follow by substitution: 9 shared-memory words per step and thread.
+//  * otherwise both parities: 18 words, the operations of a plain 2G-row
+//    cyclic reduction in its order (binary32 p' lines are solved outright,
+//    so the form whose rounding they had is kept).
+// The textbook form (rows re-read every step) moved 24 words.
+//
+// N elements per array in `red` (9N used with HALF, else 12N); the rows of
+// neighbouring chunks are TS elements apart.  All threads of the line(s)
+// call `sync`, which orders shared memory between them; `active` false:
+// barriers only.
+template <class R, bool HALF, class Sync>
+__device__ __forceinline__ void reduced_pcr(R* red, const int N, const int TS, const int G, const int pos,
+                                            const int k, const bool active, R eA, R eC, R eD, R oA, R oC, R oD,
+                                            R& x0, R& xl, Sync sync) {
+  const bool lo1 = active && k > 0, hi1 = active && k + 1 < G;
+  if constexpr (HALF) {
+    if (active) { red[pos] = eA; red[N + pos] = eC; red[2 * N + pos] = eD; }
+    sync();
+    R hA = R(0), hC = R(0), hD = R(0);
+    if (hi1) { hA = red[pos + TS]; hC = red[N + pos + TS]; hD = red[2 * N + pos + TS]; }
+    pcr_row(oA, oC, oD, eA, eC, eD, hA, hC, hD);
+    R* cur = red + 3 * N;
+    R* nxt = red + 6 * N;
+#pragma unroll 1
+    for (int h = 1; h < G; h <<= 1) {
+      if (active) { cur[pos] = oA; cur[N + pos] = oC; cur[2 * N + pos] = oD; }
+      sync();
+      R lA = R(0), lC = R(0), lD = R(0);
+      hA = hC = hD = R(0);
+      if (active && k >= h) {
+        const int q = pos - h * TS;
+        lA = cur[q]; lC = cur[N + q]; lD = cur[2 * N + q];
+      }
+      if (active && k + h < G) {
+        const int q = pos + h * TS;
+        hA = cur[q]; hC = cur[N + q]; hD = cur[2 * N + q];
+      }
+      pcr_row(oA, oC, oD, lA, lC, lD, hA, hC, hD);
+      R* t = cur; cur = nxt; nxt = t;
+    }
+    xl = oD;
+    if (active) cur[pos] = xl;
+    sync();
+    const R xm = lo1 ? cur[pos - TS] : R(0);
+    x0 = fmaT(-eC, xl, fmaT(-eA, xm, eD));
+  } else {
+    R* cur = red;
+    R* nxt = red + 6 * N;
+    if (active) {
+      cur[pos] = eA; cur[N + pos] = eC; cur[2 * N + pos] = eD;
+      cur[3 * N + pos] = oA; cur[4 * N + pos] = oC; cur[5 * N + pos] = oD;
+    }
+    sync();
+    {
+      R lA = R(0), lC = R(0), lD = R(0), hA = R(0), hC = R(0), hD = R(0);
+      if (lo1) { lA = cur[3 * N + pos - TS]; lC = cur[4 * N + pos - TS]; lD = cur[5 * N + pos - TS]; }
+      if (hi1) { hA = cur[pos + TS]; hC = cur[N + pos + TS]; hD = cur[2 * N + pos + TS]; }
+      const R e0A = eA, e0C = eC, e0D = eD;
+      pcr_row(eA, eC, eD, lA, lC, lD, oA, oC, oD);
+      pcr_row(oA, oC, oD, e0A, e0C, e0D, hA, hC, hD);
+    }
+#pragma unroll 1
+    for (int h = 1; h < G; h <<= 1) {
+      R* t = cur; cur = nxt; nxt = t;
+      if (active) {
+        cur[pos] = eA; cur[N + pos] = eC; cur[2 * N + pos] = eD;
+        cur[3 * N + pos] = oA; cur[4 * N + pos] = oC; cur[5 * N + pos] = oD;
+      }
+      sync();
+      R lA = R(0), lC = R(0), lD = R(0), hA = R(0), hC = R(0), hD = R(0);
+      R mA = R(0), mC = R(0), mD = R(0), gA = R(0), gC = R(0), gD = R(0);
+      if (active && k >= h) {
+        const int q = pos - h * TS;
+        lA = cur[q]; lC = cur[N + q]; lD = cur[2 * N + q];
+        mA = cur[3 * N + q]; mC = cur[4 * N + q]; mD = cur[5 * N + q];
+      }
+      if (active && k + h < G) {
+        const int q = pos + h * TS;
+        hA = cur[q]; hC = cur[N + q]; hD = cur[2 * N + q];
+        gA = cur[3 * N + q]; gC = cur[4 * N + q]; gD = cur[5 * N + q];
+      }
+      pcr_row(eA, eC, eD, lA, lC, lD, hA, hC, hD);
+      pcr_row(oA, oC, oD, mA, mC, mD, gA, gC, gD);
+    }
+    x0 = eD;
+    xl = oD;
+  }
+}
+
+// One chunk of M >= 3 rows in registers, eliminated to its first and last
+// rows (modified Thomas) and back-substituted once their solutions are
+// known; the operations of chunk_solve in its order.
+template <class R, int M>
+struct Chunk {
+  R a[M], b[M], c[M], d[M];
+  R eA, eC, eD, oA, oC, oD;
+  __device__ __forceinline__ void eliminate() {
+    const R inv = fast_rcp(b[1]);
+    R ap = a[1] * inv, cp = c[1] * inv, dp = d[1] * inv;
+    a[1] = ap; c[1] = cp; d[1] = dp;
+#pragma unroll
+    for (int i = 2; i < M; ++i) {
+      const R ai = a[i];
+      const R r = fast_rcp(fmaT(-ai, cp, b[i]));
+      ap = -ai * ap * r;
+      dp = fmaT(-ai, dp, d[i]) * r;
+      cp = c[i] * r;
+      a[i] = ap; c[i] = cp; d[i] = dp;
+    }
+    R an = a[M - 2], cn = c[M - 2], dn = d[M - 2];
+#pragma unroll
+    for (int i = M - 3; i >= 1; --i) {
+      const R ci = c[i];
+      dn = fmaT(-ci, dn, d[i]);
+      an = fmaT(-ci, an, a[i]);
+      cn = -ci * cn;
+      a[i] = an; c[i] = cn; d[i] = dn;
+    }
+    const R r0 = fast_rcp(fmaT(-c[0], an, b[0]));
+    eA = a[0] * r0; eC = -c[0] * cn * r0; eD = fmaT(-c[0], dn, d[0]) * r0;
+    oA = ap; oC = cp; oD = dp;
+  }
+  // the solution replaces d
+  __device__ __forceinline__ void substitute(R x0, R xl) {
+    d[0] = x0;
+#pragma unroll
+    for (int i = 1; i < M - 1; ++i) d[i] = fmaT(-c[i], xl, fmaT(-a[i], x0, d[i]));
+    d[M - 1] = xl;
+  }
+};
 
 // Partitioned line solve of the TL lines staged in shared memory, G threads
 // per line (thread t: line t / G, chunk k = t % G, rows k*m .. k*m+m-1 at
@@ -711,14 +821,34 @@ __device__ __forceinline__ void reduced_pcr(R* red, int k, bool active, R eA, R 
 // Reciprocals use fast_rcp (two Newton steps).  The solution replaces the
 // right-hand side.  Called by all TL*G threads;
 // threads of lines with `active` false only take part in the barriers.
-template <class R, int G, int TL = 1>
+template <class R, int G, int TL = 1, int M = 0>
 __device__ __forceinline__ void chunk_solve(R* line, int m, int mp, bool active, int rs) {
   const int k = threadIdx.x % G;
+  constexpr bool HALF = sizeof(R) == 8;
   R* a = line + k * mp;
   R* b = a + (size_t)G * mp;
   R* c = b + (size_t)G * mp;
   R* d = c + (size_t)G * mp;
   R* red = line + (size_t)4 * G * mp;
+  if constexpr (M > 0) {
+    // the chunk in registers; shared memory only for the reduced system
+    Chunk<R, M> ch;
+#pragma unroll
+    for (int i = 0; i < M; ++i) {
+      ch.a[i] = R(0); ch.b[i] = R(1); ch.c[i] = R(0); ch.d[i] = R(0);
+      if (active) { ch.a[i] = a[i]; ch.b[i] = b[i]; ch.c[i] = c[i]; ch.d[i] = d[i]; }
+    }
+    ch.eliminate();
+    R x0, xl;
+    reduced_pcr<R, HALF>(red, G, 1, G, k, k, active, ch.eA, ch.eC, ch.eD, ch.oA, ch.oC, ch.oD, x0, xl,
+                         [] { line_sync<G, TL>(); });
+    if (active) {
+      ch.substitute(x0, xl);
+#pragma unroll
+      for (int i = 0; i < M; ++i) d[i] = ch.d[i];
+    }
+    return;
+  }
   constexpr int M2 = warp_chunk(G);
   constexpr int M2P = M2 | 1;
   R eA = R(0), eC = R(0), eD = R(0), oA = R(0), oC = R(0), oD = R(0);
@@ -752,7 +882,7 @@ __device__ __forceinline__ void chunk_solve(R* line, int m, int mp, bool active,
   }
   R x0, xl;
   if (rs == RS_PCR) {
-    reduced_pcr<R, G, TL>(red, k, active, eA, eC, eD, oA, oC, oD, x0, xl);
+    reduced_pcr<R, HALF>(red, G, 1, G, k, k, active, eA, eC, eD, oA, oC, oD, x0, xl, [] { line_sync<G, TL>(); });
   } else {
     // reduced system in the warp solver's [32][M2P] chunk layout
     constexpr int ARR2 = 32 * M2P;

@@ -280,14 +280,7 @@ __device__ __forceinline__ void fused_assemble(typename SweepTypes<SOLVER, EQ>::
     const int idx = threadIdx.x + it * NT;
     int l, r;
     if (X) { l = TL == 1 ? 0 : idx / npad; r = idx - l * npad; }
-    else if (M > 0) {
-      // y-lines with a compile-time chunk: each thread assembles the M
-      // consecutive rows of its own chunk, so neighbouring rows' stencil
-      // loads (row jj+1 of one cell is row jj of the next) repeat within
-      // the thread and the compiler may keep them in registers
-      l = threadIdx.x % TL;
-      r = (threadIdx.x / TL) * M + it;
-    } else { l = idx % TL; r = idx / TL; }
+    else { l = idx % TL; r = idx / TL; }
     const int L = L0 + l;
     const bool valid = L >= line_lo && L <= line_hi && r < n;
     // padding rows and unsolved lines: identity rows, nothing to assemble
@@ -302,6 +295,58 @@ __device__ __forceinline__ void fused_assemble(typename SweepTypes<SOLVER, EQ>::
     sm[off + 3 * arr] = S(row.d);
   }
 }
+
+// y-lines with a compile-time chunk of M rows: thread t holds chunk t / TL of
+// line L0 + t % TL from assembly to solution in registers (a warp's field
+// accesses span TL adjacent ii), and shared memory only carries the reduced
+// system.  Returns this thread's share of ||new - prev||^2, as solve_lines.
+template <int EQ, int SOLVER, int TL, int G, int M>
+__device__ __forceinline__ double fused_y_lines(typename SweepTypes<SOLVER, EQ>::S* red, const Geo<double>& G_,
+                                                const SweepIO<double>& io, const SolveIO& so, const int n,
+                                                const int line_lo, const int line_hi, const int nfull, const int L0) {
+  using ST = SweepTypes<SOLVER, EQ>;
+  using S = typename ST::S;
+  const int l = threadIdx.x % TL, k = threadIdx.x / TL, L = L0 + l;
+  const bool active = L >= line_lo && L <= line_hi;
+  Chunk<S, M> ch;
+  double acc_bo = 0.0;
+#pragma unroll
+  for (int it = 0; it < M; ++it) {
+    const int r = k * M + it;
+    const Row<double> row = active && r < n
+                                ? staged_row<EQ, SOLVER>(G_, io, L, r, n, line_lo, line_hi, true, acc_bo)
+                                : Row<double>{0.0, 1.0, 0.0, 0.0};
+    ch.a[it] = S(row.a); ch.b[it] = S(row.b); ch.c[it] = S(row.c); ch.d[it] = S(row.d);
+  }
+  ch.eliminate();
+  S x0, xl;
+  reduced_pcr<S, sizeof(S) == 8>(red, TL * G, TL, G, threadIdx.x, k, active, ch.eA, ch.eC, ch.eD, ch.oA, ch.oC,
+                                 ch.oD, x0, xl, [] { __syncthreads(); });
+  ch.substitute(x0, xl);
+  double acc = 0.0;
+#pragma unroll
+  for (int it = 0; it < M; ++it) {
+    const int r = k * M + it;
+    if (r >= n || L > nfull) continue;
+    const int g = r * so.LD + (L - 1);
+    double x;
+    if (active) {
+      x = ST::DC ? so.in[g] + double(ch.d[it]) : double(ch.d[it]);
+      if (r >= 1 && r <= n - 2) {
+        const double dv = x - (so.prev ? so.prev[g] : 0.0);
+        acc += dv * dv;
+      }
+    } else {
+      x = so.in[g];
+    }
+    so.out[g] = x;
+  }
+  return acc;
+}
+
+// shared memory of fused_y_lines: the reduced system of TL lines
+template <class S, int TL, int G>
+constexpr size_t fused_y_smem() { return (size_t)(sizeof(S) == 8 ? 9 : 12) * TL * G * sizeof(S); }
 
 // u residual (residuo_u) of row jj = L0 of a fused T-x sweep (one line per
 // CTA): cells ii = 2..mi-1, m per thread (G*m >= mi+1 rows of the line);
@@ -345,11 +390,15 @@ __global__ void __launch_bounds__(TL * G, TL > 1 ? 1 : (G >= 512 ? 2 : 3))
   const int m = M > 0 ? M : so.m;
   const int mp = M > 0 ? (M | 1) : so.mp;
   const int L0 = 1 + blockIdx.x * TL;
-  double acc_bo = 0.0;
-  fused_assemble<EQ, SOLVER, TL, G, M>(sm, G_, io, m, mp, n, line_lo, line_hi, L0, acc_bo);
-  __syncthreads();
-  const double acc = solve_lines<S, EqIsX<EQ>::value, ST::DC, SOLVER == IXB_SOLVER_EXACT, TL, G, M>(
-      sm, so, n, line_lo, line_hi, nfull, L0);
+  double acc_bo = 0.0, acc;
+  if constexpr (!EqIsX<EQ>::value && M > 0) {
+    acc = fused_y_lines<EQ, SOLVER, TL, G, M>(sm, G_, io, so, n, line_lo, line_hi, nfull, L0);
+  } else {
+    fused_assemble<EQ, SOLVER, TL, G, M>(sm, G_, io, m, mp, n, line_lo, line_hi, L0, acc_bo);
+    __syncthreads();
+    acc = solve_lines<S, EqIsX<EQ>::value, ST::DC, SOLVER == IXB_SOLVER_EXACT, TL, G, M>(sm, so, n, line_lo, line_hi,
+                                                                                        nfull, L0);
+  }
   if constexpr (EQ == EQ_TX) {
     if (so.res.resu) {
       // u residual of row jj = L0, whose T this CTA has just written (evaluating it before the
@@ -454,11 +503,16 @@ template <int EQ, int SOLVER>
 cudaError_t fused_launch(const SweepShape& s, const Geo<double>& G, const SweepIO<double>& io, const SolveIO& so,
                          cudaStream_t st) {
   constexpr bool EXACT = SOLVER == IXB_SOLVER_EXACT;
+  using S = typename SweepTypes<SOLVER, EQ>::S;
 #define IXB_FUSED_(TL_, G_)                                                                     \
   if (s.tl == TL_ && s.g == G_) {                                                               \
-    if (!EXACT && s.m == 3) return fused_go<fused_sweep_kernel<EQ, SOLVER, TL_, G_, 3>>(s, G, io, so, st); \
-    if constexpr (!EqIsX<EQ>::value && !EXACT)                                                  \
-      if (s.m == 5) return fused_go<fused_sweep_kernel<EQ, SOLVER, TL_, G_, 5>>(s, G, io, so, st); \
+    if constexpr (!EXACT) {                                                                     \
+      SweepShape r = s;                                                                         \
+      if constexpr (!EqIsX<EQ>::value) r.smem = fused_y_smem<S, TL_, G_>();                     \
+      if (s.m == 3) return fused_go<fused_sweep_kernel<EQ, SOLVER, TL_, G_, 3>>(r, G, io, so, st); \
+      if constexpr (!EqIsX<EQ>::value)                                                          \
+        if (s.m == 5) return fused_go<fused_sweep_kernel<EQ, SOLVER, TL_, G_, 5>>(r, G, io, so, st); \
+    }                                                                                           \
     return fused_go<fused_sweep_kernel<EQ, SOLVER, TL_, G_, 0>>(s, G, io, so, st);                \
   }
   if constexpr (EqIsX<EQ>::value) {

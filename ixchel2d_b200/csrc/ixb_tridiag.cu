@@ -283,7 +283,8 @@ __global__ void __launch_bounds__(kStreamT, 1) tri_stream_kernel(const R* __rest
     const R r0 = fast_rcp(fmaT(-rc[0], an, rb[0]));
     const R eA = ra[0] * r0, eC = -rc[0] * cn * r0, eD = fmaT(-rc[0], dn, rd[0]) * r0;
     R x0, xl;
-    reduced_pcr<R, kStreamT>(red, tid, true, eA, eC, eD, ap, cp, dp, x0, xl);
+    reduced_pcr<R, true>(red, kStreamT, 1, kStreamT, tid, tid, true, eA, eC, eD, ap, cp, dp, x0, xl,
+                         [] { __syncthreads(); });
     // the previous solution must have left xbuf before it is overwritten
     if (tid == 0) bulk_store_wait_read();
     __syncthreads();
