@@ -542,107 +542,10 @@ __device__ void thomas_exact(R* sa, R* sb, R* sc, R* sd, int n, int m, int mp) {
   }
 }
 
-// Reduced-system solvers of the partitioned line solve
-enum ReducedSolve { RS_PCR = 0, RS_WARP = 1 };
-
-__host__ __device__ constexpr int warp_chunk(int G) { return (2 * G + 31) / 32 < 3 ? 3 : (2 * G + 31) / 32; }
-
 // Shared-memory footprint (elements) of one line: the four row arrays of G
-// chunks (pitch mp), plus the reduced system: for RS_PCR two buffers of the
-// 2G normalised rows (a, c, d), for RS_WARP four [32][m2|1] arrays; room
-// for the larger of the two.
-__host__ __device__ constexpr size_t line_smem_elems(int G, int mp) {
-  return (size_t)4 * G * mp +
-         ((size_t)12 * G > (size_t)4 * 32 * (warp_chunk(G) | 1) ? (size_t)12 * G : (size_t)4 * 32 * (warp_chunk(G) | 1));
-}
-
-template <class R>
-__device__ __forceinline__ R shfl_up_r(R x, int d) { return __shfl_up_sync(0xffffffffu, x, d); }
-template <class R>
-__device__ __forceinline__ R shfl_dn_r(R x, int d) { return __shfl_down_sync(0xffffffffu, x, d); }
-
-// One warp solves one system staged as [32][mp] chunks of m >= 3 rows:
-// every lane eliminates its chunk down to two rows coupled to the
-// neighbouring chunks (forward and backward "modified Thomas" sweeps), the
-// warp solves the 64-row reduced system by parallel cyclic reduction with
-// register shuffles, and every lane back-substitutes its chunk.  (Thomas-PCR
-// hybrid of Laszlo, Giles and Appleyard, ACM TOMS 42(4) 2016.)  Must be
-// called by all 32 lanes.
-template <class R>
-__device__ void thomas_pcr_warp(R* sa, R* sb, R* sc, R* sd, int m, int mp) {
-  const int lane = threadIdx.x & 31;
-  R* a = sa + lane * mp;
-  R* b = sb + lane * mp;
-  R* c = sc + lane * mp;
-  R* d = sd + lane * mp;
-  // forward: rows 1..m-1 -> x_k + a'_k x_0 + c'_k x_{k+1} = d'_k
-  const R a0 = a[0], b0 = b[0], c0 = c[0], d0 = d[0];
-  R inv = R(1) / b[1];
-  R ap = a[1] * inv, cp = c[1] * inv, dp = d[1] * inv;
-  a[1] = ap; c[1] = cp; d[1] = dp;
-  for (int k = 2; k < m; ++k) {
-    const R ak = a[k];
-    const R r = R(1) / (b[k] - ak * cp);
-    ap = -ak * ap * r;
-    dp = (d[k] - ak * dp) * r;
-    cp = c[k] * r;
-    a[k] = ap; c[k] = cp; d[k] = dp;
-  }
-  // reduced row 2*lane+1 (chunk's last row): x_{m-1} + ap x_0 + cp x_m = dp
-  R oA = ap, oB = R(1), oC = cp, oD = dp;
-  // backward: rows m-3..1 -> x_k + a''_k x_0 + c''_k x_{m-1} = d''_k
-  R an = a[m - 2], cn = c[m - 2], dn = d[m - 2];
-  for (int k = m - 3; k >= 1; --k) {
-    const R ck = c[k];
-    dn = d[k] - ck * dn;
-    an = a[k] - ck * an;
-    cn = -ck * cn;
-    a[k] = an; c[k] = cn; d[k] = dn;
-  }
-  // reduced row 2*lane (chunk's first row): x_0 + A x_{-1} + C x_{m-1} = D
-  const R r0 = R(1) / (b0 - c0 * an);
-  R eA = a0 * r0, eB = R(1), eC = -c0 * cn * r0, eD = (d0 - c0 * dn) * r0;
-
-  // PCR on the 64 interleaved rows (even = first rows, odd = last rows)
-  {  // stride 1: even row needs odd of lane-1 and own odd; odd needs own even and even of lane+1
-    R lA = shfl_up_r(oA, 1), lB = shfl_up_r(oB, 1), lC = shfl_up_r(oC, 1), lD = shfl_up_r(oD, 1);
-    R hA = shfl_dn_r(eA, 1), hB = shfl_dn_r(eB, 1), hC = shfl_dn_r(eC, 1), hD = shfl_dn_r(eD, 1);
-    if (lane == 0) { lA = R(0); lB = R(1); lC = R(0); lD = R(0); }
-    if (lane == 31) { hA = R(0); hB = R(1); hC = R(0); hD = R(0); }
-    const R k1e = eA / lB, k2e = eC / oB;
-    const R k1o = oA / eB, k2o = oC / hB;
-    const R nEA = -lA * k1e, nEB = eB - lC * k1e - oA * k2e, nEC = -oC * k2e, nED = eD - lD * k1e - oD * k2e;
-    const R nOA = -eA * k1o, nOB = oB - eC * k1o - hA * k2o, nOC = -hC * k2o, nOD = oD - eD * k1o - hD * k2o;
-    eA = nEA; eB = nEB; eC = nEC; eD = nED;
-    oA = nOA; oB = nOB; oC = nOC; oD = nOD;
-  }
-#pragma unroll
-  for (int dl = 1; dl < 32; dl <<= 1) {  // row stride 2*dl: same-parity rows of lanes +-dl
-    R lEA = shfl_up_r(eA, dl), lEB = shfl_up_r(eB, dl), lEC = shfl_up_r(eC, dl), lED = shfl_up_r(eD, dl);
-    R hEA = shfl_dn_r(eA, dl), hEB = shfl_dn_r(eB, dl), hEC = shfl_dn_r(eC, dl), hED = shfl_dn_r(eD, dl);
-    R lOA = shfl_up_r(oA, dl), lOB = shfl_up_r(oB, dl), lOC = shfl_up_r(oC, dl), lOD = shfl_up_r(oD, dl);
-    R hOA = shfl_dn_r(oA, dl), hOB = shfl_dn_r(oB, dl), hOC = shfl_dn_r(oC, dl), hOD = shfl_dn_r(oD, dl);
-    if (lane < dl) { lEA = R(0); lEB = R(1); lEC = R(0); lED = R(0); lOA = R(0); lOB = R(1); lOC = R(0); lOD = R(0); }
-    if (lane + dl > 31) { hEA = R(0); hEB = R(1); hEC = R(0); hED = R(0); hOA = R(0); hOB = R(1); hOC = R(0); hOD = R(0); }
-    {
-      const R k1 = eA / lEB, k2 = eC / hEB;
-      const R nA = -lEA * k1, nB = eB - lEC * k1 - hEA * k2, nC = -hEC * k2, nD = eD - lED * k1 - hED * k2;
-      eA = nA; eB = nB; eC = nC; eD = nD;
-    }
-    {
-      const R k1 = oA / lOB, k2 = oC / hOB;
-      const R nA = -lOA * k1, nB = oB - lOC * k1 - hOA * k2, nC = -hOC * k2, nD = oD - lOD * k1 - hOD * k2;
-      oA = nA; oB = nB; oC = nC; oD = nD;
-    }
-  }
-  const R x0 = eD / eB;
-  const R xl = oD / oB;
-  // back-substitution
-  d[0] = x0;
-  for (int k = 1; k < m - 1; ++k) d[k] = d[k] - a[k] * x0 - c[k] * xl;
-  d[m - 1] = xl;
-}
-
+// chunks (pitch mp), plus the reduced system (two sets of the 2G normalised
+// rows a, c, d).
+__host__ __device__ constexpr size_t line_smem_elems(int G, int mp) { return (size_t)4 * G * mp + (size_t)12 * G; }
 
 // Barrier of the G threads that solve one line when a CTA holds TL lines of
 // whole warps (a named barrier per line, so lines do not wait for each
@@ -812,17 +715,15 @@ struct Chunk {
 // per line (thread t: line t / G, chunk k = t % G, rows k*m .. k*m+m-1 at
 // offset k*mp of the line's row arrays).  Every thread eliminates its chunk
 // (m >= 3 rows) down to two rows coupled only to the neighbouring chunks'
-// end rows (a forward and a backward "modified Thomas" sweep); the 2G
-// reduced rows of each line are then solved either by parallel cyclic
-// reduction over all G threads in shared memory (RS_PCR, log2(2G) steps) or
-// by one warp per line with the warp Thomas-PCR hybrid (RS_WARP); finally
-// every thread back-substitutes its chunk.  This is the Thomas-PCR hybrid of
-// Laszlo, Giles and Appleyard (ACM TOMS 42(4), 2016) applied twice.
-// Reciprocals use fast_rcp (two Newton steps).  The solution replaces the
-// right-hand side.  Called by all TL*G threads;
+// end rows (a forward and a backward "modified Thomas" sweep), in registers
+// when the chunk is compile-time (M > 0); the 2G reduced rows of each line
+// are then solved by reduced_pcr, and every thread back-substitutes its
+// chunk.  This is the Thomas-PCR hybrid of Laszlo, Giles and Appleyard (ACM
+// TOMS 42(4), 2016).  Reciprocals use fast_rcp (two Newton steps).  The
+// solution replaces the right-hand side.  Called by all TL*G threads;
 // threads of lines with `active` false only take part in the barriers.
 template <class R, int G, int TL = 1, int M = 0>
-__device__ __forceinline__ void chunk_solve(R* line, int m, int mp, bool active, int rs) {
+__device__ __forceinline__ void chunk_solve(R* line, int m, int mp, bool active) {
   const int k = threadIdx.x % G;
   constexpr bool HALF = sizeof(R) == 8;
   R* a = line + k * mp;
@@ -830,8 +731,8 @@ __device__ __forceinline__ void chunk_solve(R* line, int m, int mp, bool active,
   R* c = b + (size_t)G * mp;
   R* d = c + (size_t)G * mp;
   R* red = line + (size_t)4 * G * mp;
+  R x0, xl;
   if constexpr (M > 0) {
-    // the chunk in registers; shared memory only for the reduced system
     Chunk<R, M> ch;
 #pragma unroll
     for (int i = 0; i < M; ++i) {
@@ -839,7 +740,6 @@ __device__ __forceinline__ void chunk_solve(R* line, int m, int mp, bool active,
       if (active) { ch.a[i] = a[i]; ch.b[i] = b[i]; ch.c[i] = c[i]; ch.d[i] = d[i]; }
     }
     ch.eliminate();
-    R x0, xl;
     reduced_pcr<R, HALF>(red, G, 1, G, k, k, active, ch.eA, ch.eC, ch.eD, ch.oA, ch.oC, ch.oD, x0, xl,
                          [] { line_sync<G, TL>(); });
     if (active) {
@@ -847,67 +747,42 @@ __device__ __forceinline__ void chunk_solve(R* line, int m, int mp, bool active,
 #pragma unroll
       for (int i = 0; i < M; ++i) d[i] = ch.d[i];
     }
-    return;
-  }
-  constexpr int M2 = warp_chunk(G);
-  constexpr int M2P = M2 | 1;
-  R eA = R(0), eC = R(0), eD = R(0), oA = R(0), oC = R(0), oD = R(0);
-  if (active) {
-    // forward: rows 1..m-1 -> x_k + a'_k x_0 + c'_k x_{k+1} = d'_k
-    const R a0 = a[0], b0 = b[0], c0 = c[0], d0 = d[0];
-    R inv = fast_rcp(b[1]);
-    R ap = a[1] * inv, cp = c[1] * inv, dp = d[1] * inv;
-    a[1] = ap; c[1] = cp; d[1] = dp;
-    for (int i = 2; i < m; ++i) {
-      const R ai = a[i];
-      const R r = fast_rcp(fmaT(-ai, cp, b[i]));
-      ap = -ai * ap * r;
-      dp = fmaT(-ai, dp, d[i]) * r;
-      cp = c[i] * r;
-      a[i] = ap; c[i] = cp; d[i] = dp;
-    }
-    // backward: rows m-3..1 -> x_i + a''_i x_0 + c''_i x_{m-1} = d''_i
-    R an = a[m - 2], cn = c[m - 2], dn = d[m - 2];
-    for (int i = m - 3; i >= 1; --i) {
-      const R ci = c[i];
-      dn = fmaT(-ci, dn, d[i]);
-      an = fmaT(-ci, an, a[i]);
-      cn = -ci * cn;
-      a[i] = an; c[i] = cn; d[i] = dn;
-    }
-    // reduced rows 2k (chunk's first row) and 2k+1 (its last row), unit diagonal
-    const R r0 = fast_rcp(fmaT(-c0, an, b0));
-    eA = a0 * r0; eC = -c0 * cn * r0; eD = fmaT(-c0, dn, d0) * r0;
-    oA = ap; oC = cp; oD = dp;
-  }
-  R x0, xl;
-  if (rs == RS_PCR) {
-    reduced_pcr<R, HALF>(red, G, 1, G, k, k, active, eA, eC, eD, oA, oC, oD, x0, xl, [] { line_sync<G, TL>(); });
   } else {
-    // reduced system in the warp solver's [32][M2P] chunk layout
-    constexpr int ARR2 = 32 * M2P;
-    auto off = [](int q) { return (q / M2) * M2P + q % M2; };
+    R eA = R(0), eC = R(0), eD = R(0), oA = R(0), oC = R(0), oD = R(0);
     if (active) {
-      int o = off(2 * k);
-      red[o] = eA; red[o + ARR2] = R(1); red[o + 2 * ARR2] = eC; red[o + 3 * ARR2] = eD;
-      o = off(2 * k + 1);
-      red[o] = oA; red[o + ARR2] = R(1); red[o + 2 * ARR2] = oC; red[o + 3 * ARR2] = oD;
+      // forward: rows 1..m-1 -> x_k + a'_k x_0 + c'_k x_{k+1} = d'_k
+      const R a0 = a[0], b0 = b[0], c0 = c[0], d0 = d[0];
+      const R inv = fast_rcp(b[1]);
+      R ap = a[1] * inv, cp = c[1] * inv, dp = d[1] * inv;
+      a[1] = ap; c[1] = cp; d[1] = dp;
+      for (int i = 2; i < m; ++i) {
+        const R ai = a[i];
+        const R r = fast_rcp(fmaT(-ai, cp, b[i]));
+        ap = -ai * ap * r;
+        dp = fmaT(-ai, dp, d[i]) * r;
+        cp = c[i] * r;
+        a[i] = ap; c[i] = cp; d[i] = dp;
+      }
+      // backward: rows m-3..1 -> x_i + a''_i x_0 + c''_i x_{m-1} = d''_i
+      R an = a[m - 2], cn = c[m - 2], dn = d[m - 2];
+      for (int i = m - 3; i >= 1; --i) {
+        const R ci = c[i];
+        dn = fmaT(-ci, dn, d[i]);
+        an = fmaT(-ci, an, a[i]);
+        cn = -ci * cn;
+        a[i] = an; c[i] = cn; d[i] = dn;
+      }
+      // reduced rows 2k (chunk's first row) and 2k+1 (its last row), unit diagonal
+      const R r0 = fast_rcp(fmaT(-c0, an, b0));
+      eA = a0 * r0; eC = -c0 * cn * r0; eD = fmaT(-c0, dn, d0) * r0;
+      oA = ap; oC = cp; oD = dp;
     }
-    // identity rows pad the reduced system to 32*M2 rows
-    for (int q = 2 * G + k; q < 32 * M2; q += G) {
-      const int o = off(q);
-      red[o] = R(0); red[o + ARR2] = R(1); red[o + 2 * ARR2] = R(0); red[o + 3 * ARR2] = R(0);
+    reduced_pcr<R, HALF>(red, G, 1, G, k, k, active, eA, eC, eD, oA, oC, oD, x0, xl, [] { line_sync<G, TL>(); });
+    if (active) {
+      d[0] = x0;
+      for (int i = 1; i < m - 1; ++i) d[i] = fmaT(-c[i], xl, fmaT(-a[i], x0, d[i]));
+      d[m - 1] = xl;
     }
-    __syncthreads();
-    if (k < 32 && active) thomas_pcr_warp(red, red + ARR2, red + 2 * ARR2, red + 3 * ARR2, M2, M2P);
-    __syncthreads();
-    x0 = red[3 * ARR2 + off(2 * k)];
-    xl = red[3 * ARR2 + off(2 * k + 1)];
-  }
-  if (active) {
-    d[0] = x0;
-    for (int i = 1; i < m - 1; ++i) d[i] = fmaT(-c[i], xl, fmaT(-a[i], x0, d[i]));
-    d[m - 1] = xl;
   }
 }
 

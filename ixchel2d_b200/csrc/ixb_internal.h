@@ -104,7 +104,6 @@ struct SweepShape {
   int g;          // threads per line
   int nt;         // threads per CTA (tl * g)
   int m, mp;      // chunk rows per thread, padded pitch
-  int rs;         // reduced-system solver (RS_PCR / RS_WARP)
   size_t smem;    // dynamic shared memory bytes
   int grid;       // CTAs
 };

@@ -297,7 +297,6 @@ SweepShape sweep_shape(int eq, int mi, int nj, int real_bytes, int tl, int g) {
   s.nt = tl * g;
   s.m = std::max(3, (s.n + g - 1) / g);
   s.mp = s.m | 1;
-  s.rs = RS_PCR;
   s.smem = line_smem_elems(g, s.mp) * real_bytes * tl;
   s.grid = (s.nfull + tl - 1) / tl;
   return s;

@@ -1,21 +1,21 @@
 // ixb_tridiag.cu -- batched tridiagonal solves over device arrays, the
 // batched form of tridiagonal (source/mod_solucionador.f90:25-47).
 //
-// layout 0 (each system contiguous, like the reference's x-lines): a CTA
-// stages TL systems into shared memory with coalesced loads, G = 256/TL
-// threads per system solve it (the chunked Thomas-PCR hybrid, or the exact
-// sequential Thomas on one thread), and the solution is written back
-// coalesced.
-//
-// layout 1 (systems interleaved, row i of system s at i*nsys+s, like the
-// y-lines of a column-major field): the hybrid solver runs the cluster
-// kernel below (tri_strided_kernel: groups of 128-byte row segments in 2-D
-// tensor tiles, n <= 4096).  The exact solver, and sizes or alignments that
-// kernel does not take, use one thread per system walking the rows;
-// consecutive threads touch consecutive addresses.  Its forward sweep keeps
-// the modified diagonal (exact) or normalised super-diagonal (hybrid) in a
-// scratch array of n*nsys elements taken from the stream-ordered allocator,
-// and the modified right-hand side in x.
+// Hybrid solver, by layout and size:
+//  layout 0 (each system contiguous, like the reference's x-lines)
+//    n <= 4864: tri_stream_kernel, one system per CTA at a time, the next one
+//               arriving by bulk copies (any alignment);
+//    longer:    tri_contig_kernel, one system staged per CTA.
+//  layout 1 (systems interleaved, row i of system s at i*nsys+s, like the
+//  y-lines of a column-major field)
+//    short:     tri_cols_kernel, whole systems in the registers of a CTA;
+//    n <= 4096 in whole 16-byte granules: tri_strided_kernel, a group of
+//               systems in a thread-block cluster;
+//    others:    tri_block_kernel, blocks of 128 rows, each read twice (the
+//               second time from L2) around the solve of the block ends.
+// The exact solver stages contiguous systems (tri_contig_kernel) and walks
+// interleaved ones with one thread each (tri_inter_kernel), in the
+// reference's operation order.
 #include <cooperative_groups.h>
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(TL * G) tri_contig_kernel(const R* __restrict_
     if (SOLVER == IXB_SOLVER_EXACT) {
       if (active && threadIdx.x % G == 0) thomas_exact(line, line + arr, line + 2 * arr, line + 3 * arr, n, m, mp);
     } else {
-      chunk_solve<R, G>(line, m, mp, active, RS_WARP);
+      chunk_solve<R, G>(line, m, mp, active);
     }
   }
   __syncthreads();
@@ -74,74 +74,62 @@ __global__ void __launch_bounds__(TL * G) tri_contig_kernel(const R* __restrict_
   }
 }
 
-// One thread per interleaved system.  EXACT keeps the reference's operation
-// order (modified diagonal in `work`); HYBRID uses the normalised Thomas form
-// (c' in `work`).
-template <class R, int SOLVER>
+// One thread per interleaved system, the reference's operation order
+// (modified diagonal in `work`, modified right-hand side in x).
+template <class R>
 __global__ void __launch_bounds__(128) tri_inter_kernel(const R* __restrict__ a, const R* __restrict__ b,
-                                                        const R* __restrict__ c, const R* __restrict__ d, R* x,
+                                                        const R* __restrict__ c, const R* d, R* x,
                                                         R* __restrict__ work, int n, int nsys) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nsys) return;
   const size_t S = (size_t)nsys;
-  if (SOLVER == IXB_SOLVER_EXACT) {
-    R bp = b[s], dp = d[s];
-    work[s] = bp;
-    x[s] = dp;
-    for (int i = 1; i < n; ++i) {
-      const size_t g = (size_t)i * S + s;
-      const R q = a[g] / bp;
-      dp = d[g] - q * dp;
-      bp = b[g] - q * c[g - S];
-      x[g] = dp;
-      work[g] = bp;
-    }
-    R xn = dp / bp;
-    x[(size_t)(n - 1) * S + s] = xn;
-    for (int i = n - 2; i >= 0; --i) {
-      const size_t g = (size_t)i * S + s;
-      xn = (x[g] - c[g] * xn) / work[g];
-      x[g] = xn;
-    }
-  } else {
-    R r = R(1) / b[s];
-    R cp = (n > 1 ? c[s] : R(0)) * r;
-    R dp = d[s] * r;
-    work[s] = cp;
-    x[s] = dp;
-    for (int i = 1; i < n; ++i) {
-      const size_t g = (size_t)i * S + s;
-      const R ai = a[g];
-      r = R(1) / (b[g] - ai * cp);
-      dp = (d[g] - ai * dp) * r;
-      cp = (i < n - 1 ? c[g] : R(0)) * r;
-      x[g] = dp;
-      work[g] = cp;
-    }
-    R xn = dp;
-    for (int i = n - 2; i >= 0; --i) {
-      const size_t g = (size_t)i * S + s;
-      xn = x[g] - work[g] * xn;
-      x[g] = xn;
-    }
+  R bp = b[s], dp = d[s];
+  work[s] = bp;
+  x[s] = dp;
+  for (int i = 1; i < n; ++i) {
+    const size_t g = (size_t)i * S + s;
+    const R q = a[g] / bp;
+    dp = d[g] - q * dp;
+    bp = b[g] - q * c[g - S];
+    x[g] = dp;
+    work[g] = bp;
+  }
+  R xn = dp / bp;
+  x[(size_t)(n - 1) * S + s] = xn;
+  for (int i = n - 2; i >= 0; --i) {
+    const size_t g = (size_t)i * S + s;
+    xn = (x[g] - c[g] * xn) / work[g];
+    x[g] = xn;
   }
 }
 
 // ---------------------------------------------------------------------------
-// Streamed contiguous solve (hybrid solver): a persistent CTA of 256 threads
-// per SM slot walks its systems; while it solves system s from registers,
-// the bulk-copy engine is already loading system s+grid into shared memory,
-// and the solution leaves through a bulk shared->global copy.  Thread t owns
-// rows t*M .. t*M+M-1 (M odd, so the 32 threads of a warp reading their own
-// row j hit 32 different banks); it eliminates them in registers down to two
-// rows (modified Thomas), the 512 reduced rows are solved by PCR in shared
-// memory, and each thread back-substitutes its rows.  Every wait on the copy
-// engine is bounded: on a timeout the CTA records it in g_tri_timeout, waits
-// (bounded) for its copies still in flight and leaves without writing.
+// Streamed contiguous solve (hybrid solver): CTAs of T threads walk their
+// systems; while one is solved from registers, the bulk-copy engine is
+// already loading the CTA's next one into shared memory, and the solution
+// leaves through a bulk shared->global copy.  Thread t owns rows t*M ..
+// t*M+M-1 (M odd, so the threads of a warp reading their own row j hit
+// different banks); it eliminates them in registers (Chunk), the reduced rows
+// go through reduced_pcr, and each thread back-substitutes its rows.
+// Long lines are bound by HBM (4096 x 4096 binary64: 6.17 TB/s, 94 % of the
+// measured copy rate; 135.2 us before the reduced system's shared-memory
+// traffic was cut, 108.8 us since), short ones by the latency of one system.
+//
+// Bulk copies move whole 16-byte granules.  A system that starts or ends
+// inside one (odd n, or an array that is not 16-byte aligned) keeps its
+// alignment in shared memory (a shift of up to 16 bytes), the bulk copy takes
+// the whole granules, and the up to 16 / sizeof(R) - 1 elements on each side
+// go by ordinary loads and stores, so nothing outside the system is touched.
+// (701-row systems, 302 of them, binary64: 22.5 us by the staged kernel
+// before, 9.8 us here.)  RAG picks that form; where every system fills whole
+// granules the fixed addresses save 5 % at 4096 x 4096 (113.0 against 107.3 us).
+//
+// Every wait on the copy engine is bounded: on a timeout the CTA records it
+// in g_tri_timeout, waits (bounded) for its copies still in flight and
+// leaves without writing.
 // ---------------------------------------------------------------------------
 namespace {
 
-constexpr int kStreamT = 256;       // threads per CTA (one system at a time)
 constexpr int kSpinLimit = 1 << 22;  // bounded mbarrier polls (a hang guard)
 __device__ int g_tri_timeout = 0;
 // Poll limit of the streamed kernel's first wait of every CTA (its other
@@ -202,42 +190,94 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, unsigned parity
   return false;
 }
 
-// Shared memory of the streamed kernel: 4 row arrays of NP = 256*M
-// elements (the copy target), the solution buffer (NP), the PCR buffers
-// (12*256) and the mbarrier.
-template <class R, int M>
+// elements per 16-byte granule
+template <class R>
+constexpr int kGran = 16 / (int)sizeof(R);
+
+// a system's rows at p: elements before the first whole granule (`head`),
+// in whole granules (`body`), and the shift that keeps p's alignment
+template <class R, bool RAG>
+struct Granules {
+  int shift, head, body;
+  __device__ __forceinline__ Granules(const R* p, int n) {
+    constexpr int E = kGran<R>;
+    if constexpr (!RAG) {  // every system starts and ends on a granule
+      shift = head = 0;
+      body = n;
+      return;
+    }
+    shift = (int)((reinterpret_cast<uintptr_t>(p) / sizeof(R)) & (E - 1));
+    head = min((E - shift) & (E - 1), n);
+    body = (n - head) & ~(E - 1);
+  }
+  // element of edge slot i (0 .. 2*kGran-1: head, then tail), -1: none
+  __device__ __forceinline__ int edge(int i, int n) const {
+    constexpr int E = kGran<R>;
+    if (i < E) return i < head ? i : -1;
+    const int r = head + body + i - E;
+    return r < n ? r : -1;
+  }
+};
+
+// Shared memory of the streamed kernel: 4 row arrays (the copy target) and
+// the solution, each T*M elements and room for the shift, the reduced
+// system (9*T) and the mbarrier.
+template <class R, int T, int M>
 __host__ __device__ constexpr size_t stream_smem_bytes() {
-  return ((size_t)5 * kStreamT * M + 12 * kStreamT) * sizeof(R) + 16;
+  return ((size_t)5 * (T * M + kGran<R>) + 9 * T) * sizeof(R) + 16;
 }
 
-template <class R, int M>
-__global__ void __launch_bounds__(kStreamT, 1) tri_stream_kernel(const R* __restrict__ a, const R* __restrict__ b,
-                                                                 const R* __restrict__ c, const R* __restrict__ d,
-                                                                 R* __restrict__ x, int n, int nsys) {
-  constexpr int NP = kStreamT * M;
+template <class R, int T, int M, bool RAG>
+__global__ void __launch_bounds__(T) tri_stream_kernel(const R* a, const R* b, const R* c, const R* d, R* x, int n,
+                                                       int nsys) {
+  constexpr int E = kGran<R>, NS = T * M + E;
+  static_assert(8 * E <= T, "one thread per edge element of the four arrays");
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  R* buf = reinterpret_cast<R*>(smem_raw);  // a | b | c | d, NP each
-  R* xbuf = buf + 4 * NP;
-  R* red = xbuf + NP;
-  uint64_t* bar = reinterpret_cast<uint64_t*>(red + 12 * kStreamT);
+  R* buf = reinterpret_cast<R*>(smem_raw);  // a | b | c | d, NS each
+  R* xbuf = buf + 4 * NS;
+  R* red = xbuf + NS;
+  uint64_t* bar = reinterpret_cast<uint64_t*>(red + 9 * T);
   const int tid = threadIdx.x;
-  const unsigned bytes = (unsigned)n * sizeof(R);
-  // identity rows pad every system to NP rows; the copies never touch them
-  for (int r = n + tid; r < NP; r += kStreamT) {
-    buf[r] = R(0); buf[NP + r] = R(1); buf[2 * NP + r] = R(0); buf[3 * NP + r] = R(0);
+  auto row_of = [&](int q) { return q == 0 ? a : q == 1 ? b : q == 2 ? c : d; };
+  if constexpr (!RAG) {  // identity rows pad every system to T*M rows; the copies never touch them
+    for (int r = n + tid; r < T * M; r += T) {
+      buf[r] = R(0); buf[NS + r] = R(1); buf[2 * NS + r] = R(0); buf[3 * NS + r] = R(0);
+    }
   }
   if (tid == 0) mbar_init(bar);
   __syncthreads();
   auto issue = [&](int s) {
     const size_t off = (size_t)s * n;
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // earlier reads of buf precede the copies
-    mbar_expect_tx(bar, 4 * bytes);
-    bulk_load(buf, a + off, bytes, bar);
-    bulk_load(buf + NP, b + off, bytes, bar);
-    bulk_load(buf + 2 * NP, c + off, bytes, bar);
-    bulk_load(buf + 3 * NP, d + off, bytes, bar);
+    unsigned bytes = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) bytes += (unsigned)(Granules<R, RAG>(row_of(q) + off, n).body * sizeof(R));
+    mbar_expect_tx(bar, bytes);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const R* p = row_of(q) + off;
+      const Granules<R, RAG> gr(p, n);
+      if (gr.body)
+        bulk_load(buf + q * NS + gr.shift + gr.head, p + gr.head, (unsigned)(gr.body * sizeof(R)), bar);
+    }
   };
-  if (tid == 0 && blockIdx.x < nsys) issue(blockIdx.x);
+  // this thread's edge element of system s: its slot in buf (or -1) and value
+  auto edge_load = [&](int s, R& v) -> int {
+    if (!RAG || tid >= 8 * E) return -1;
+    const int q = tid / (2 * E);
+    const R* p = row_of(q) + (size_t)s * n;
+    const Granules<R, RAG> gr(p, n);
+    const int r = gr.edge(tid % (2 * E), n);
+    if (r < 0) return -1;
+    v = p[r];
+    return q * NS + gr.shift + r;
+  };
+  if (blockIdx.x < nsys) {
+    if (tid == 0) issue(blockIdx.x);
+    R v;
+    const int slot = edge_load(blockIdx.x, v);
+    if (slot >= 0) buf[slot] = v;
+  }
   const int first_limit = *(volatile int*)&g_tri_first_wait_polls;
   unsigned parity = 0;
   bool failed = false;
@@ -245,56 +285,59 @@ __global__ void __launch_bounds__(kStreamT, 1) tri_stream_kernel(const R* __rest
     const bool ok = mbar_wait_bounded(bar, parity, s == (int)blockIdx.x ? first_limit : kSpinLimit);
     if (__syncthreads_or(!ok)) { failed = true; break; }
     parity ^= 1;
-    // own rows into registers (row 0 has no a, row n-1 no c)
-    R ra[M], rb[M], rc[M], rd[M];
+    // own rows into registers (row 0 has no a, row n-1 no c; identity rows past n)
+    Chunk<R, M> ch;
+    {
+      const size_t off = (size_t)s * n;
+      const R* ba = buf + Granules<R, RAG>(a + off, n).shift;
+      const R* bb = buf + NS + Granules<R, RAG>(b + off, n).shift;
+      const R* bc = buf + 2 * NS + Granules<R, RAG>(c + off, n).shift;
+      const R* bd = buf + 3 * NS + Granules<R, RAG>(d + off, n).shift;
 #pragma unroll
-    for (int j = 0; j < M; ++j) {
-      const int r = tid * M + j;
-      ra[j] = r == 0 ? R(0) : buf[r];
-      rb[j] = buf[NP + r];
-      rc[j] = r == n - 1 ? R(0) : buf[2 * NP + r];
-      rd[j] = buf[3 * NP + r];
+      for (int j = 0; j < M; ++j) {
+        const int r = tid * M + j;
+        if constexpr (RAG) {
+          const bool in = r < n;
+          ch.a[j] = in && r > 0 ? ba[r] : R(0);
+          ch.b[j] = in ? bb[r] : R(1);
+          ch.c[j] = r < n - 1 ? bc[r] : R(0);
+          ch.d[j] = in ? bd[r] : R(0);
+        } else {
+          ch.a[j] = r == 0 ? R(0) : ba[r];
+          ch.b[j] = bb[r];
+          ch.c[j] = r == n - 1 ? R(0) : bc[r];
+          ch.d[j] = bd[r];
+        }
+      }
     }
     __syncthreads();  // the row buffers are free: start loading the next system
-    if (tid == 0 && s + (int)gridDim.x < nsys) issue(s + gridDim.x);
-    // modified Thomas on the own rows: x_j + a'_j x_0 + c'_j x_{j+1} = d'_j ...
-    R inv = fast_rcp(rb[1]);
-    R ap = ra[1] * inv, cp = rc[1] * inv, dp = rd[1] * inv;
-    ra[1] = ap; rc[1] = cp; rd[1] = dp;
-#pragma unroll
-    for (int j = 2; j < M; ++j) {
-      const R aj = ra[j];
-      const R r = fast_rcp(fmaT(-aj, cp, rb[j]));
-      ap = -aj * ap * r;
-      dp = fmaT(-aj, dp, rd[j]) * r;
-      cp = rc[j] * r;
-      ra[j] = ap; rc[j] = cp; rd[j] = dp;
+    const int next = s + (int)gridDim.x;
+    R ev = R(0);
+    int eslot = -1;
+    if (next < nsys) {
+      if (tid == 0) issue(next);
+      eslot = edge_load(next, ev);
     }
-    // ... then x_j + a''_j x_0 + c''_j x_{M-1} = d''_j for j = 1..M-2
-    R an = ra[M - 2], cn = rc[M - 2], dn = rd[M - 2];
-#pragma unroll
-    for (int j = M - 3; j >= 1; --j) {
-      const R cj = rc[j];
-      dn = fmaT(-cj, dn, rd[j]);
-      an = fmaT(-cj, an, ra[j]);
-      cn = -cj * cn;
-      ra[j] = an; rc[j] = cn; rd[j] = dn;
-    }
-    const R r0 = fast_rcp(fmaT(-rc[0], an, rb[0]));
-    const R eA = ra[0] * r0, eC = -rc[0] * cn * r0, eD = fmaT(-rc[0], dn, rd[0]) * r0;
+    ch.eliminate();
     R x0, xl;
-    reduced_pcr<R, true>(red, kStreamT, 1, kStreamT, tid, tid, true, eA, eC, eD, ap, cp, dp, x0, xl,
+    reduced_pcr<R, true>(red, T, 1, T, tid, tid, true, ch.eA, ch.eC, ch.eD, ch.oA, ch.oC, ch.oD, x0, xl,
                          [] { __syncthreads(); });
+    ch.substitute(x0, xl);
     // the previous solution must have left xbuf before it is overwritten
     if (tid == 0) bulk_store_wait_read();
     __syncthreads();
-    xbuf[tid * M] = x0;
+    R* xs = x + (size_t)s * n;
+    const Granules<R, RAG> gx(xs, n);
 #pragma unroll
-    for (int j = 1; j < M - 1; ++j) xbuf[tid * M + j] = fmaT(-rc[j], xl, fmaT(-ra[j], x0, rd[j]));
-    xbuf[tid * M + M - 1] = xl;
+    for (int j = 0; j < M; ++j) xbuf[gx.shift + tid * M + j] = ch.d[j];
+    if (eslot >= 0) buf[eslot] = ev;
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic writes -> copy engine
     __syncthreads();
-    if (tid == 0) bulk_store(x + (size_t)s * n, xbuf, bytes);
+    if (tid == 0 && gx.body) bulk_store(xs + gx.head, xbuf + gx.shift + gx.head, (unsigned)(gx.body * sizeof(R)));
+    if (RAG && tid < 2 * E) {
+      const int r = gx.edge(tid, n);
+      if (r >= 0) xs[r] = xbuf[gx.shift + r];
+    }
   }
   if (failed) {
     if (tid == 0) {
@@ -305,55 +348,451 @@ __global__ void __launch_bounds__(kStreamT, 1) tri_stream_kernel(const R* __rest
   if (tid == 0) bulk_store_wait_all();
 }
 
-template <class R, int M>
-cudaError_t stream_launch(const R* a, const R* b, const R* c, const R* d, R* x, int n, int nsys, cudaStream_t st) {
-  auto k = tri_stream_kernel<R, M>;
-  const size_t smem = stream_smem_bytes<R, M>();
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  int dev = 0, nsm = 0, per_sm = 0;
-  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-  if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kStreamT, smem)) != cudaSuccess) return e;
-  if (per_sm < 1) return cudaErrorInvalidValue;
-  const int grid = std::min(nsys, nsm * per_sm);
-  k<<<grid, kStreamT, smem, st>>>(a, b, c, d, x, n, nsys);
+template <class R, int T, int M>
+cudaError_t stream_launch(const R* a, const R* b, const R* c, const R* d, R* x, int n, int nsys, int nsm,
+                          cudaStream_t st) {
+  const uintptr_t all = (uintptr_t)a | (uintptr_t)b | (uintptr_t)c | (uintptr_t)d | (uintptr_t)x;
+  const bool ragged = (all & 15) != 0 || ((size_t)n * sizeof(R)) % 16 != 0;
+  auto k = ragged ? tri_stream_kernel<R, T, M, true> : tri_stream_kernel<R, T, M, false>;
+  constexpr size_t smem = stream_smem_bytes<R, T, M>();
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  // about one wave: by shared memory (227 KB per SM, 1 KB reserved per CTA)
+  // and threads; the CTAs do not depend on one another
+  const int per_sm = std::max(1, std::min((int)(227 * 1024 / (smem + 1024)), 1024 / T));
+  k<<<std::min(nsys, nsm * per_sm), T, smem, st>>>(a, b, c, d, x, n, nsys);
   return cudaGetLastError();
 }
 
-// The streamed kernel applies when the copies are legal (16-byte aligned
-// system starts and sizes) and the rows fit one CTA: n <= 256*M for an odd
-// M <= 19 whose buffers fit the shared memory.
-template <class R>
-bool stream_fits(const R* a, const R* b, const R* c, const R* d, const R* x, int n) {
-  const uintptr_t all = (uintptr_t)a | (uintptr_t)b | (uintptr_t)c | (uintptr_t)d | (uintptr_t)x;
-  if ((all & 15) != 0 || ((size_t)n * sizeof(R)) % 16 != 0) return false;
-  return n >= 3 * kStreamT / 2 && n <= kStreamT * 19;
-}
+// Lines of up to 32, 64, 128 and 256 threads' worth of three to seven rows:
+// short chunks keep a lone system's latency down, and below 256 threads
+// more systems share an SM.  From 256 threads on, longer chunks.
+constexpr int kStreamMaxN = 256 * 19;
 
 template <class R>
 cudaError_t stream_solve(const R* a, const R* b, const R* c, const R* d, R* x, int n, int nsys, cudaStream_t st) {
-  int m = (n + kStreamT - 1) / kStreamT;
-  m |= 1;
-  if (m < 3) m = 3;
-  switch (m) {
-    case 3: return stream_launch<R, 3>(a, b, c, d, x, n, nsys, st);
-    case 5: return stream_launch<R, 5>(a, b, c, d, x, n, nsys, st);
-    case 7: return stream_launch<R, 7>(a, b, c, d, x, n, nsys, st);
-    case 9: return stream_launch<R, 9>(a, b, c, d, x, n, nsys, st);
-    case 11: return stream_launch<R, 11>(a, b, c, d, x, n, nsys, st);
-    case 13: return stream_launch<R, 13>(a, b, c, d, x, n, nsys, st);
-    case 15: return stream_launch<R, 15>(a, b, c, d, x, n, nsys, st);
-    case 17: return stream_launch<R, 17>(a, b, c, d, x, n, nsys, st);
-    case 19: return stream_launch<R, 19>(a, b, c, d, x, n, nsys, st);
-    default: return cudaErrorInvalidValue;
-  }
+  int dev = 0, nsm = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+#define IXB_STREAM_(T_, M_) \
+  if (n <= T_ * M_) return stream_launch<R, T_, M_>(a, b, c, d, x, n, nsys, nsm, st);
+  IXB_STREAM_(32, 3) IXB_STREAM_(32, 5)
+  IXB_STREAM_(64, 3) IXB_STREAM_(64, 5)
+  IXB_STREAM_(128, 3) IXB_STREAM_(128, 5)
+  IXB_STREAM_(256, 3) IXB_STREAM_(256, 5) IXB_STREAM_(256, 7) IXB_STREAM_(256, 9) IXB_STREAM_(256, 11)
+  IXB_STREAM_(256, 13) IXB_STREAM_(256, 15) IXB_STREAM_(256, 17) IXB_STREAM_(256, 19)
+#undef IXB_STREAM_
+  return cudaErrorInvalidValue;
 }
 
 }  // namespace
 
 // ---------------------------------------------------------------------------
 // Interleaved systems (row i of system s at i*nsys + s), hybrid solver.
+// A CTA holds W adjacent systems: thread t the M consecutive rows of chunk
+// t / W of system t % W, loaded straight into registers, so that every load
+// of a warp covers W adjacent elements of 32 / W rows and no alignment is
+// asked of the arrays or of nsys.
+// ---------------------------------------------------------------------------
+namespace {
+
+// rows k*M .. k*M+M-1 past row0 of system s; identity rows outside
+template <class R, int M, class Ld>
+__device__ __forceinline__ void load_chunk(Chunk<R, M>& ch, const R* a, const R* b, const R* c, const R* d,
+                                           size_t row0, int n, size_t s, int nsys, Ld ld) {
+#pragma unroll
+  for (int j = 0; j < M; ++j) {
+    const size_t r = row0 + j;
+    const bool in = s < (size_t)nsys && r < (size_t)n;
+    const size_t g = in ? r * nsys + s : 0;
+    ch.a[j] = in && r > 0 ? ld(a + g) : R(0);
+    ch.b[j] = in ? ld(b + g) : R(1);
+    ch.c[j] = in && r < (size_t)n - 1 ? ld(c + g) : R(0);
+    ch.d[j] = in ? ld(d + g) : R(0);
+  }
+}
+
+// Whole systems: n <= M * G rows on the G chunks of a CTA.
+template <class R, int W, int M>
+__global__ void __launch_bounds__(512) tri_cols_kernel(const R* a, const R* b, const R* c, const R* d, R* x, int n,
+                                                       int nsys, int G) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  R* red = reinterpret_cast<R*>(smem_raw);
+  const int w = threadIdx.x % W, k = threadIdx.x / W;
+  const size_t s = (size_t)blockIdx.x * W + w;
+  const bool active = s < (size_t)nsys;
+  Chunk<R, M> ch;
+  load_chunk(ch, a, b, c, d, (size_t)k * M, n, s, nsys, [](const R* p) { return *p; });
+  ch.eliminate();
+  R x0, xl;
+  reduced_pcr<R, true>(red, W * G, W, G, threadIdx.x, k, active, ch.eA, ch.eC, ch.eD, ch.oA, ch.oC, ch.oD, x0, xl,
+                       [] { __syncthreads(); });
+  ch.substitute(x0, xl);
+#pragma unroll
+  for (int j = 0; j < M; ++j) {
+    const int r = k * M + j;
+    if (active && r < n) x[(size_t)r * nsys + s] = ch.d[j];
+  }
+}
+
+// Blocks of 128 rows of 128 bytes' worth of systems, for lines that fit
+// neither one CTA nor the cluster kernel's copies (odd nsys, n > 4096).  Two items per block, handed out in order by a ticket:
+//   A: eliminate the block to its first and last rows as functions of the
+//      neighbouring blocks' ends; the last A of a system group then solves
+//      the group's block ends (block_ends) and raises its flag;
+//   C: the same elimination from the same inputs (mostly L2 hits: C of group
+//      g follows A of group g + lag), then, with the block's outer
+//      neighbours known, its rows.
+// DRAM sees the inputs and the solution once; nothing waits on a cluster or
+// a launch boundary.  Items wait only on items with lower tickets, which
+// running CTAs hold, and the wait is bounded (g_tri_timeout).  Bound by the
+// latency of an item (64 KB in registers, two items per SM): 4095 x 4095
+// binary64 307 us (2.19 TB/s), against 5057 us for one thread per system;
+// where the cluster kernel applies it is faster (4096 x 4096: 213 against
+// 305 us).
+template <class R>
+struct BlockCfg {
+  static constexpr int T = 256;
+  static constexpr int W = 128 / (int)sizeof(R);  // systems per group
+  static constexpr int G = T / W;                 // chunks per block
+  static constexpr int ROWS = 128;
+  static constexpr int M = ROWS / G;              // rows per chunk
+};
+
+struct BlockPlan {
+  int groups, blocks, lag;
+  long long items;
+  size_t ends, outer, ctr;  // scratch: elements of block ends and outer values, ints of counters
+};
+
+template <class R>
+BlockPlan block_plan(int n, int nsys, int resident) {
+  using B = BlockCfg<R>;
+  BlockPlan p{};
+  p.groups = (nsys + B::W - 1) / B::W;
+  p.blocks = (n + B::ROWS - 1) / B::ROWS;
+  // A runs ahead of C by the groups a full GPU has in flight, and two more
+  p.lag = std::min(p.groups, resident / p.blocks + 2);
+  p.items = 2LL * p.groups * p.blocks;
+  p.ends = (size_t)p.groups * p.blocks * 6 * B::W;
+  p.outer = (size_t)p.groups * p.blocks * 2 * B::W;
+  p.ctr = 2 + 2 * (size_t)p.groups;
+  return p;
+}
+
+template <class R>
+size_t block_scratch_bytes(const BlockPlan& p) {
+  return (p.ends + p.outer) * sizeof(R) + p.ctr * sizeof(unsigned);
+}
+
+// item t: group, block and whether it is a C item
+__device__ __forceinline__ void block_item(long long t, int groups, int blocks, int lag, int& g, int& blk, bool& c) {
+  const long long head = (long long)lag * blocks, mid = 2LL * (groups - lag) * blocks;
+  if (t < head) {
+    g = (int)(t / blocks); blk = (int)(t % blocks); c = false;
+  } else if (t < head + mid) {
+    const long long u = t - head, pos = u / (2 * blocks), v = u % (2 * blocks);
+    c = v >= blocks;
+    g = (int)pos + (c ? 0 : lag);
+    blk = (int)(v % blocks);
+  } else {
+    const long long u = t - head - mid;
+    g = groups - lag + (int)(u / blocks); blk = (int)(u % blocks); c = true;
+  }
+}
+
+// Odd rows of a block's chunks as functions of the outer unknowns:
+//   xl_k + A XL + C XF = D, XL the last unknown before the block, XF the first
+// after it.  reduced_pcr with open ends: a row without a neighbour keeps its
+// coupling to the outer unknown (the neighbour "row" is -x_outer).
+template <class R>
+__device__ __forceinline__ void block_pcr(R* red, int W, int G, int k, const R eA, const R eC, const R eD, R& oA,
+                                          R& oC, R& oD) {
+  const int N = W * G, pos = threadIdx.x;
+  red[pos] = eA; red[N + pos] = eC; red[2 * N + pos] = eD;
+  __syncthreads();
+  R hA = R(0), hC = R(-1), hD = R(0);
+  if (k + 1 < G) { hA = red[pos + W]; hC = red[N + pos + W]; hD = red[2 * N + pos + W]; }
+  pcr_row(oA, oC, oD, eA, eC, eD, hA, hC, hD);
+  R* cur = red + 3 * N;
+  R* nxt = red + 6 * N;
+#pragma unroll 1
+  for (int h = 1; h < G; h <<= 1) {
+    cur[pos] = oA; cur[N + pos] = oC; cur[2 * N + pos] = oD;
+    __syncthreads();
+    R lA = R(-1), lC = R(0), lD = R(0);
+    hA = R(0); hC = R(-1); hD = R(0);
+    if (k >= h) { const int q = pos - h * W; lA = cur[q]; lC = cur[N + q]; lD = cur[2 * N + q]; }
+    if (k + h < G) { const int q = pos + h * W; hA = cur[q]; hC = cur[N + q]; hD = cur[2 * N + q]; }
+    pcr_row(oA, oC, oD, lA, lC, lD, hA, hC, hD);
+    R* t = cur; cur = nxt; nxt = t;
+  }
+  __syncthreads();  // red is free again
+}
+
+// Block ends of one system (thread w of a group): per block, first row
+// f + al XL + be XF = de and last row l + A XL + C XF = D, with XL the previous
+// block's l and XF the next block's f.  Forward: l_b = P_b - Q_b f_{b+1} and
+// f_b = F0_b - F1_b f_{b+1}, one reciprocal per block; backward: the values,
+// and each block's XL, XF.  `ends` is overwritten by (F0, F1, P, Q).
+template <class R>
+__device__ void block_ends(R* ends, R* outer, int W, int blocks) {
+  R P = R(0), Q = R(0);
+  constexpr int U = 4;  // blocks whose ends are loaded together
+  for (int b0 = 0; b0 < blocks; b0 += U) {
+    R v[U][6];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int q = 0; q < 6; ++q) v[u][q] = b0 + u < blocks ? __ldcg(ends + ((size_t)(b0 + u) * 6 + q) * W) : R(0);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (b0 + u >= blocks) break;
+      const R al = v[u][0], be = v[u][1], de = v[u][2], A = v[u][3], Cc = v[u][4], D = v[u][5];
+      const R r = fast_rcp(fmaT(-al, Q, R(1)));
+      const R F0 = fmaT(-al, P, de) * r, F1 = be * r;
+      const R AQ = A * Q;
+      const R Pn = fmaT(AQ, F0, fmaT(-A, P, D)), Qn = fmaT(AQ, F1, Cc);
+      R* e = ends + (size_t)(b0 + u) * 6 * W;
+      __stcg(e, F0); __stcg(e + W, F1); __stcg(e + 2 * W, Pn); __stcg(e + 3 * W, Qn);
+      P = Pn; Q = Qn;
+    }
+  }
+  R fn = R(0);
+  for (int b1 = blocks - 1; b1 >= 0; b1 -= U) {
+    R v[U][4];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int b = b1 - u;
+      v[u][0] = b >= 0 ? __ldcg(ends + (size_t)b * 6 * W) : R(0);
+      v[u][1] = b >= 0 ? __ldcg(ends + ((size_t)b * 6 + 1) * W) : R(0);
+      v[u][2] = b > 0 ? __ldcg(ends + ((size_t)(b - 1) * 6 + 2) * W) : R(0);
+      v[u][3] = b > 0 ? __ldcg(ends + ((size_t)(b - 1) * 6 + 3) * W) : R(0);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int b = b1 - u;
+      if (b < 0) break;
+      const R f = fmaT(-v[u][1], fn, v[u][0]);
+      __stcg(outer + (size_t)b * 2 * W, fmaT(-v[u][3], f, v[u][2]));
+      __stcg(outer + ((size_t)b * 2 + 1) * W, fn);
+      fn = f;
+    }
+  }
+}
+
+// Bounded wait for a flag another CTA of this launch raises.
+__device__ __forceinline__ bool flag_wait_bounded(const unsigned* flag) {
+  unsigned long long t0;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+  for (int i = 0; i < kSpinLimit; ++i) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");
+    if (v) return true;
+    if ((i & 63) == 63) {
+      unsigned long long t;
+      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+      if (t - t0 > 2000000000ull) return false;
+    }
+  }
+  return false;
+}
+
+template <class R>
+__global__ void __launch_bounds__(BlockCfg<R>::T, 2)
+    tri_block_kernel(const R* a, const R* b, const R* c, const R* d, R* x, int n, int nsys, int groups, int blocks,
+                     int lag, R* ends, R* outer, unsigned* ctr) {
+  using B = BlockCfg<R>;
+  constexpr int W = B::W, G = B::G, M = B::M;
+  __shared__ R red[9 * B::T];
+  __shared__ long long s_item;
+  __shared__ int s_last;
+  const int tid = threadIdx.x, w = tid % W, k = tid / W;
+  unsigned long long* ticket = reinterpret_cast<unsigned long long*>(ctr);
+  unsigned* done = ctr + 2;
+  unsigned* flag = done + groups;
+  const long long items = 2LL * groups * blocks;
+  if (tid == 0) s_item = (long long)atomicAdd(ticket, 1ull);
+  __syncthreads();
+  long long t = s_item;
+  while (t < items) {
+    long long nt = 0;
+    if (tid == 0) nt = (long long)atomicAdd(ticket, 1ull);  // the next ticket, while this item runs
+    int g, blk;
+    bool second;
+    block_item(t, groups, blocks, lag, g, blk, second);
+    const size_t s = (size_t)g * W + w;
+    const size_t row0 = (size_t)blk * B::ROWS + k * M;
+    Chunk<R, M> ch;
+    if (second) load_chunk(ch, a, b, c, d, row0, n, s, nsys, [](const R* p) { return __ldcs(p); });
+    else load_chunk(ch, a, b, c, d, row0, n, s, nsys, [](const R* p) { return __ldcg(p); });
+    ch.eliminate();
+    const R eA = ch.eA, eC = ch.eC, eD = ch.eD;
+    R oA = ch.oA, oC = ch.oC, oD = ch.oD;
+    block_pcr(red, W, G, k, eA, eC, eD, oA, oC, oD);
+    R* my_ends = ends + ((size_t)g * blocks + blk) * 6 * W + w;
+    R* my_outer = outer + ((size_t)g * blocks + blk) * 2 * W + w;
+    if (!second) {
+      if (k == 0) {
+        __stcg(my_ends, fmaT(-eC, oA, eA));
+        __stcg(my_ends + W, -eC * oC);
+        __stcg(my_ends + 2 * W, fmaT(-eC, oD, eD));
+      }
+      if (k == G - 1) { __stcg(my_ends + 3 * W, oA); __stcg(my_ends + 4 * W, oC); __stcg(my_ends + 5 * W, oD); }
+      __threadfence();
+      __syncthreads();
+      if (tid == 0) s_last = atomicAdd(done + g, 1u) == (unsigned)blocks - 1;
+      __syncthreads();
+      if (s_last) {
+        __threadfence();
+        if (tid < W)
+          block_ends(ends + (size_t)g * blocks * 6 * W + tid, outer + (size_t)g * blocks * 2 * W + tid, W, blocks);
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(flag + g), "r"(1u) : "memory");
+      }
+    } else {
+      bool ok = true;
+      if (tid == 0) ok = flag_wait_bounded(flag + g);
+      if (__syncthreads_or(!ok)) {
+        if (tid == 0) atomicExch(&g_tri_timeout, 1);
+        return;
+      }
+      const R XL = __ldcg(my_outer), XF = __ldcg(my_outer + W);
+      const R xl = fmaT(-oC, XF, fmaT(-oA, XL, oD));
+      red[tid] = xl;
+      __syncthreads();
+      const R xm = k > 0 ? red[tid - W] : XL;
+      const R x0 = fmaT(-eC, xl, fmaT(-eA, xm, eD));
+      ch.substitute(x0, xl);
+      if (s < (size_t)nsys) {
+#pragma unroll
+        for (int j = 0; j < M; ++j)
+          if (row0 + j < (size_t)n) __stcs(x + (row0 + j) * nsys + s, ch.d[j]);
+      }
+    }
+    if (tid == 0) s_item = nt;
+    __syncthreads();
+    t = s_item;
+    __syncthreads();
+  }
+}
+
+template <class R, int W, int M>
+cudaError_t cols_launch(const R* a, const R* b, const R* c, const R* d, R* x, int n, int nsys, cudaStream_t st) {
+  constexpr int Q = W < 32 ? 32 / W : 1;  // chunks that fill a warp
+  const int G = ((n + M - 1) / M + Q - 1) / Q * Q;
+  const size_t smem = (size_t)9 * W * G * sizeof(R);
+  tri_cols_kernel<R, W, M><<<(nsys + W - 1) / W, W * G, smem, st>>>(a, b, c, d, x, n, nsys, G);
+  return cudaGetLastError();
+}
+
+// Whole systems in one CTA's registers (up to 512 threads).  64-byte row
+// pieces stream from HBM, 32-byte ones at under half its rate, but they put
+// twice as many CTAs on a GPU that 64-byte ones leave idle: used below two
+// CTAs per SM, and up to 1024 rows.
+template <class R>
+bool cols_fit(int n, int nsys, int nsm) {
+  const int W = 64 / (int)sizeof(R);
+  return n <= 512 || (n <= 1024 && (nsys + W - 1) / W < 4 * nsm);
+}
+
+template <class R>
+cudaError_t cols_solve(const R* a, const R* b, const R* c, const R* d, R* x, int n, int nsys, int nsm,
+                       cudaStream_t st) {
+  constexpr int W1 = 64 / (int)sizeof(R), W2 = W1 / 2;  // systems per 64- and 32-byte piece
+  if (n <= 512 && (nsys + W1 - 1) / W1 >= 2 * nsm) {
+    if constexpr (sizeof(R) == 8) {
+      return n <= 256 ? cols_launch<R, W1, 4>(a, b, c, d, x, n, nsys, st)
+                      : cols_launch<R, W1, 8>(a, b, c, d, x, n, nsys, st);
+    } else {
+      return n <= 256 ? cols_launch<R, W1, 8>(a, b, c, d, x, n, nsys, st)
+                      : cols_launch<R, W1, 16>(a, b, c, d, x, n, nsys, st);
+    }
+  }
+  if (n <= 2048 / W2) return cols_launch<R, W2, 4>(a, b, c, d, x, n, nsys, st);
+  if (sizeof(R) == 8 || n <= 4096 / W2) return cols_launch<R, W2, 8>(a, b, c, d, x, n, nsys, st);
+  if constexpr (sizeof(R) == 4) return cols_launch<R, W2, 16>(a, b, c, d, x, n, nsys, st);
+  return cudaErrorInvalidValue;
+}
+
+// Resident CTAs of tri_block_kernel at two per SM (its launch bound).
+template <class R>
+cudaError_t block_solve(const R* a, const R* b, const R* c, const R* d, R* x, int n, int nsys, int nsm,
+                        const BlockPlan& p, void* scratch, cudaStream_t st) {
+  R* ends = static_cast<R*>(scratch);
+  R* outer = ends + p.ends;
+  unsigned* ctr = reinterpret_cast<unsigned*>(outer + p.outer);  // W is even: 8-byte aligned
+  cudaError_t e = cudaMemsetAsync(ctr, 0, p.ctr * sizeof(unsigned), st);
+  if (e != cudaSuccess) return e;
+  const int grid = (int)std::min<long long>(p.items, 2LL * nsm);
+  tri_block_kernel<R><<<grid, BlockCfg<R>::T, 0, st>>>(a, b, c, d, x, n, nsys, p.groups, p.blocks, p.lag, ends, outer,
+                                                       ctr);
+  return cudaGetLastError();
+}
+
+// Stream-ordered scratch from a pool of the library's own (one per device
+// context), so that memory freed after a call is still mapped at the next
+// one: with the device's default pool every synchronisation unmapped it, and
+// a 0.2 ms solve that the host waits for took 4.2 ms.  The pool keeps at most
+// kPoolKeep bytes mapped across synchronisations.  While `st` is captured,
+// or if the pool cannot be had, the default allocator serves.
+constexpr unsigned long long kPoolKeep = 64ull << 20;
+constexpr int kPoolDevices = 64;
+
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t st) {
+  static std::mutex mu;
+  static cudaMemPool_t pool[kPoolDevices] = {};
+  static unsigned long long owner[kPoolDevices] = {};  // context the pool belongs to (0: none)
+  using CtxIdFn = CUresult (*)(CUcontext, unsigned long long*);
+  static CtxIdFn ctx_id = nullptr;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if ((e = cudaStreamIsCapturing(st, &cap)) != cudaSuccess) return e;
+  if (cap != cudaStreamCaptureStatusNone || dev < 0 || dev >= kPoolDevices) return cudaMallocAsync(p, bytes, st);
+  cudaMemPool_t use = nullptr;
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    if (!ctx_id) {
+      void* f = nullptr;
+      cudaDriverEntryPointQueryResult q;
+      if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) == cudaSuccess &&
+          q == cudaDriverEntryPointSuccess)
+        ctx_id = reinterpret_cast<CtxIdFn>(f);
+    }
+    unsigned long long id = 0;
+    if (ctx_id && ctx_id(nullptr, &id) == CUDA_SUCCESS) {
+      if (owner[dev] != id + 1) {  // first use, or the context was re-created (cudaDeviceReset)
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t made = nullptr;
+        unsigned long long keep = kPoolKeep;
+        if (cudaMemPoolCreate(&made, &props) == cudaSuccess &&
+            cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess) {
+          pool[dev] = made;
+          owner[dev] = id + 1;
+        } else {
+          cudaGetLastError();
+        }
+      }
+      if (owner[dev] == id + 1) use = pool[dev];
+    }
+  }
+  return use ? cudaMallocFromPoolAsync(p, bytes, use, st) : cudaMallocAsync(p, bytes, st);
+}
+
+}  // namespace
+
+// ---------------------------------------------------------------------------
+// Interleaved systems in a thread-block cluster (hybrid solver; rows of whole
+// 16-byte granules, up to 4096 of them).
 // A group of W adjacent systems occupies SEG = W*sizeof(R) contiguous bytes
 // of every row: 128-byte segments stream from HBM at full rate, 64-byte ones
 // a little below it and 32-byte ones (4 binary64 systems) at under 40 % of
@@ -446,10 +885,15 @@ __device__ __forceinline__ void bulk_send(unsigned dst, const void* src, unsigne
                : "memory");
 }
 
+template <class R>
+__device__ __forceinline__ R shfl_up_r(R x, int d) { return __shfl_up_sync(0xffffffffu, x, d); }
+template <class R>
+__device__ __forceinline__ R shfl_dn_r(R x, int d) { return __shfl_down_sync(0xffffffffu, x, d); }
+
 // One warp solves a system of 32*m rows (m >= 2) with unit diagonals:
 // x_i + a_i x_{i-1} + c_i x_{i+1} = d_i, lane l's rows at l*pitch ..
 // l*pitch+m-1 of the arrays a, c, d.  Each lane eliminates its rows to the
-// first and last (modified Thomas, as in thomas_pcr_warp, its intermediate
+// first and last (modified Thomas, its intermediate
 // rows in the scratch arrays sa, sc, sd so that the inputs are only read),
 // the 64 rows are solved by PCR over register shuffles, and each lane
 // back-substitutes.  The solution replaces d.
@@ -846,41 +1290,69 @@ static cudaError_t contig_tl(const R* a, const R* b, const R* c, const R* d, R* 
 }
 
 template <class R, int SOLVER>
-static cudaError_t tridiag_impl(const R* a, const R* b, const R* c, const R* d, R* x, int n, int nsys, int layout,
-                                cudaStream_t st) {
-  if (layout == 0) {
-    if (SOLVER == IXB_SOLVER_HYBRID && stream_fits(a, b, c, d, x, n)) {
-      const cudaError_t e = stream_solve(a, b, c, d, x, n, nsys, st);
-      if (e != cudaErrorInvalidValue) return e;  // otherwise: does not fit this GPU, use the staged kernel
-    }
-    int g = 32;
-    while (g < 256 && 3 * g < n) g <<= 1;
-    const int tl = 256 / g;
-    const int m = std::max(3, (n + g - 1) / g);
-    const int mp = m | 1;
-    const size_t smem = line_smem_elems(g, mp) * sizeof(R) * tl;
-    int dev = 0, optin = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    if (smem > (size_t)optin) return cudaErrorInvalidValue;  // line too long for one CTA
+static cudaError_t tridiag_contig(const R* a, const R* b, const R* c, const R* d, R* x, int n, int nsys,
+                                  cudaStream_t st) {
+  if (SOLVER == IXB_SOLVER_HYBRID && n <= kStreamMaxN) return stream_solve(a, b, c, d, x, n, nsys, st);
+  int g = 32;
+  while (g < 256 && 3 * g < n) g <<= 1;
+  const int tl = 256 / g;
+  const int m = std::max(3, (n + g - 1) / g);
+  const int mp = m | 1;
+  const size_t smem = line_smem_elems(g, mp) * sizeof(R) * tl;
+  int dev = 0, optin = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (smem > (size_t)optin) return cudaErrorInvalidValue;  // line too long for one CTA
+  if constexpr (SOLVER == IXB_SOLVER_EXACT) {
     switch (tl) {
-      case 1: return contig_tl<R, SOLVER, 1>(a, b, c, d, x, n, nsys, m, mp, smem, st);
       case 2: return contig_tl<R, SOLVER, 2>(a, b, c, d, x, n, nsys, m, mp, smem, st);
       case 4: return contig_tl<R, SOLVER, 4>(a, b, c, d, x, n, nsys, m, mp, smem, st);
-      default: return contig_tl<R, SOLVER, 8>(a, b, c, d, x, n, nsys, m, mp, smem, st);
+      case 8: return contig_tl<R, SOLVER, 8>(a, b, c, d, x, n, nsys, m, mp, smem, st);
+      default: break;
     }
   }
-  if (SOLVER == IXB_SOLVER_HYBRID) {
-    const cudaError_t es = strided_solve(a, b, c, d, x, n, nsys, st);
-    if (es != cudaErrorInvalidValue) return es;  // otherwise: size outside the cluster kernel's range
-  }
-  R* work = nullptr;
-  cudaError_t e = cudaMallocAsync((void**)&work, (size_t)n * nsys * sizeof(R), st);
+  return contig_tl<R, SOLVER, 1>(a, b, c, d, x, n, nsys, m, mp, smem, st);
+}
+
+// Interleaved systems.  fixed: scratch of at least fixed_bytes the caller
+// owns (the allocation-free entry point), or null to allocate what is needed.
+template <class R, int SOLVER>
+static cudaError_t tridiag_inter(const R* a, const R* b, const R* c, const R* d, R* x, int n, int nsys,
+                                 cudaStream_t st, void* fixed = nullptr, size_t fixed_bytes = 0) {
+  int dev = 0, nsm = 0;
+  cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  tri_inter_kernel<R, SOLVER><<<(nsys + 127) / 128, 128, 0, st>>>(a, b, c, d, x, work, n, nsys);
-  e = cudaGetLastError();
-  cudaError_t e2 = cudaFreeAsync(work, st);
+  if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+  BlockPlan plan{};
+  size_t bytes = (size_t)n * nsys * sizeof(R);
+  if (SOLVER == IXB_SOLVER_HYBRID) {
+    if (cols_fit<R>(n, nsys, nsm)) return cols_solve(a, b, c, d, x, n, nsys, nsm, st);
+    const cudaError_t es = strided_solve(a, b, c, d, x, n, nsys, st);
+    if (es != cudaErrorInvalidValue) return es;  // otherwise: outside the cluster kernel's range
+    plan = block_plan<R>(n, nsys, 2 * nsm);
+    bytes = block_scratch_bytes<R>(plan);
+  }
+  void* work = fixed;
+  // a few very long systems: the block ends, padded to whole groups, can
+  // exceed the fixed array, which always holds the sequential solve's scratch
+  const bool sequential = SOLVER == IXB_SOLVER_EXACT || (fixed && bytes > fixed_bytes);
+  if (!fixed && (e = scratch_alloc(&work, bytes, st)) != cudaSuccess) return e;
+  if (!sequential) {
+    e = block_solve(a, b, c, d, x, n, nsys, nsm, plan, work, st);
+  } else {
+    tri_inter_kernel<R><<<(nsys + 127) / 128, 128, 0, st>>>(a, b, c, d, x, static_cast<R*>(work), n, nsys);
+    e = cudaGetLastError();
+  }
+  if (fixed) return e;
+  const cudaError_t e2 = cudaFreeAsync(work, st);
   return e != cudaSuccess ? e : e2;
+}
+
+template <class R, int SOLVER>
+static cudaError_t tridiag_impl(const R* a, const R* b, const R* c, const R* d, R* x, int n, int nsys, int layout,
+                                cudaStream_t st) {
+  return layout == 0 ? tridiag_contig<R, SOLVER>(a, b, c, d, x, n, nsys, st)
+                     : tridiag_inter<R, SOLVER>(a, b, c, d, x, n, nsys, st);
 }
 
 // Reads and clears the timeout flag the streamed and interleaved kernels set
@@ -985,12 +1457,11 @@ extern "C" int ixb_tridiag_f64_noalloc(const double* a, const double* b, const d
     double* work = nullptr;
     e = noalloc_scratch(st, &work);
     if (e == cudaSuccess) {
-      // every work[] element is written before it is read: nothing to clear
-      if (solver == IXB_SOLVER_EXACT)
-        tri_inter_kernel<double, IXB_SOLVER_EXACT><<<(nsys + 127) / 128, 128, 0, st>>>(a, b, c, d, x, work, n, nsys);
-      else
-        tri_inter_kernel<double, IXB_SOLVER_HYBRID><<<(nsys + 127) / 128, 128, 0, st>>>(a, b, c, d, x, work, n, nsys);
-      e = cudaGetLastError();
+      // every element is written (or cleared) before it is read
+      const size_t bytes = (size_t)IXB_NOALLOC_MAX_ELEMS * sizeof(double);
+      e = solver == IXB_SOLVER_EXACT
+              ? tridiag_inter<double, IXB_SOLVER_EXACT>(a, b, c, d, x, n, nsys, st, work, bytes)
+              : tridiag_inter<double, IXB_SOLVER_HYBRID>(a, b, c, d, x, n, nsys, st, work, bytes);
     }
   }
   if (e == cudaErrorInvalidValue) return IXB_EINVAL;

@@ -38,3 +38,49 @@ def test_partition_edges(has_gpu, mi, nj, prec):
         elif k != "p":
             d = np.linalg.norm(gs[k] - os_[k]) / max(np.linalg.norm(os_[k]), 1e-300)
             assert d < 1e-4, (k, d)
+
+
+# batched line solves (device pointers): unaligned starts and ends (odd n, arrays that begin inside a
+# 16-byte granule), the edges of the chunk sizes and of the 128-row blocks, ragged system groups, one
+# system; x must be written everywhere and nothing beside it
+LINES = [(1, 3), (2, 1), (31, 7), (96, 5), (97, 300), (160, 2), (161, 33), (320, 3), (321, 17), (641, 9), (701, 302),
+         (1281, 5), (4863, 2), (4865, 3), (512, 37), (513, 37), (256, 4800), (257, 2411), (512, 2500), (1024, 15),
+         (1025, 15), (1025, 1), (1150, 2500), (1152, 33), (2049, 31), (4096, 17), (4097, 70), (9000, 3)]
+
+
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+@pytest.mark.parametrize("layout", [0, 1])
+@pytest.mark.parametrize("n,nsys", LINES)
+def test_batched_lines_any_alignment(has_gpu, n, nsys, layout, dtype):
+    if not has_gpu:
+        pytest.skip("no CUDA device")
+    import torch
+    tdt = torch.float64 if dtype == "f64" else torch.float32
+    fn = F.lib.ixb_tridiag_f64 if dtype == "f64" else F.lib.ixb_tridiag_f32
+    rng = np.random.default_rng(n + 31 * nsys + layout)
+    a = rng.uniform(-1, 0, (nsys, n)); c = rng.uniform(-1, 0, (nsys, n))
+    b = np.abs(a) + np.abs(c) + rng.uniform(0.1, 1, (nsys, n)); d = rng.uniform(-1, 1, (nsys, n))
+    ref = O.tridiagonal_batch(a, b, c, d)
+    stream = torch.cuda.current_stream().cuda_stream
+    for shift in ((0, 0, 0, 0, 0), (1, 0, 2, 3, 1)):  # elements each array starts past an aligned address
+        dev = []
+        for v, s in zip((a, b, c, d, np.full_like(d, np.nan)), shift):
+            flat = torch.full((n * nsys + 8,), -7.0, dtype=tdt, device="cuda")
+            flat[s:s + n * nsys] = torch.tensor(np.ascontiguousarray(v if layout == 0 else v.T).ravel(), dtype=tdt)
+            dev.append(flat)
+        ptr = [t.data_ptr() + s * t.element_size() for t, s in zip(dev, shift)]
+        if shift[0]:
+            ptr[4] = ptr[3]  # in place: x may alias d
+        st = fn(*ptr, n, nsys, layout, F.SOLVER_HYBRID, stream)
+        if n == 9000 and layout == 0 and dtype == "f64":  # a contiguous line must fit one CTA's shared memory
+            assert st == F.EINVAL
+            return
+        assert st == F.OK
+        out, s = (dev[3], shift[3]) if shift[0] else (dev[4], shift[4])
+        torch.cuda.synchronize()
+        assert F.lib.ixb_tridiag_status() == F.OK
+        got = out.cpu().numpy().astype(np.float64)
+        assert np.all(got[:s] == -7.0) and np.all(got[s + n * nsys:] == -7.0)
+        x = got[s:s + n * nsys].reshape((nsys, n) if layout == 0 else (n, nsys))
+        x = x if layout == 0 else x.T
+        assert relerr(x, ref) < (1e-12 if dtype == "f64" else 2e-5), relerr(x, ref)
