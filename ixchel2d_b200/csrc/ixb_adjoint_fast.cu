@@ -39,8 +39,9 @@ __global__ void adj_coef_kernel(const Geo<double> G, const SweepIO<double> io, d
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= ni * (G.nj - 1)) return;
   const int ii = 2 + idx % ni, jj = 2 + idx / ni;
-  const Row<double> rx = assemble_tx<true>(G, io, ii, jj);  // a = AI, c = AD, b = diagonal
-  const Row<double> ry = assemble_ty<true>(G, io, ii, jj);  // a = BS, c = BN
+  const CellView<double, double> cell{G, io, ii, jj};
+  const Row<double> rx = assemble_tx<true>(G, cell);  // a = AI, c = AD, b = diagonal
+  const Row<double> ry = assemble_ty<true>(G, cell);  // a = BS, c = BN
   const int c0 = G.at(ii, jj);
   coef[C_AI * fsz + c0] = rx.a;
   coef[C_AD * fsz + c0] = rx.c;

@@ -23,6 +23,7 @@
 
 #include "ixb_ctl.cuh"
 #include "ixb_handle.h"
+#include "ixb_loop.h"
 
 using namespace ixb;
 
@@ -227,19 +228,79 @@ int read_norms(ixb_handle* h) {
     if (s_ != IXB_OK) return s_; \
   } while (0)
 
+// Bring every ping-pong field to buffer 0 (the parity the graph expects).
+int normalize_parity(ixb_handle* h) {
+  const size_t bytes = h->fsz * sizeof(double);
+  if (h->cu) { CK(cudaMemcpyAsync(h->u[0], h->u[1], bytes, cudaMemcpyDeviceToDevice, h->stream)); h->cu = 0; }
+  if (h->cv) { CK(cudaMemcpyAsync(h->v[0], h->v[1], bytes, cudaMemcpyDeviceToDevice, h->stream)); h->cv = 0; }
+  if (h->cT) { CK(cudaMemcpyAsync(h->T[0], h->T[1], bytes, cudaMemcpyDeviceToDevice, h->stream)); h->cT = 0; }
+  if (h->cpc) { CK(cudaMemcpyAsync(h->pc[0], h->pc[1], bytes, cudaMemcpyDeviceToDevice, h->stream)); h->cpc = 0; }
+  return IXB_OK;
+}
+
+// ---------------------------------------------------------------------------
+// the resident loop kernel (ixb_loop.cuh)
+// ---------------------------------------------------------------------------
+bool do_while_loops();
+// Whether it serves this handle: its grids, the hybrid and mixed line solves,
+// and no launch shape set by the caller (those name the kernels of single
+// sweeps).
+bool loop_usable(const ixb_handle* h) {
+  if (!h->coop || h->prm.solver != IXB_SOLVER_HYBRID) return false;
+  for (bool s : h->shape_set)
+    if (s) return false;
+  LoopShape shape;
+  return fused_enabled() && do_while_loops() && loop_shape(h->mi, h->nj, h->nsm, &shape);
+}
+bool use_loop(const ixb_handle* h) { return h->use_graph && loop_usable(h); }
+
+// Outer passes of one launch (0.05 to 0.2 s).
+constexpr int kLoopPasses = 2048;
+
+LoopArgs loop_args(const ixb_handle* h, int part) {
+  LoopArgs a{};
+  loop_shape(h->mi, h->nj, h->nsm, &a.s);
+  a.G = make_geo(h);
+  for (int k = 0; k < 2; ++k) { a.u[k] = h->u[k]; a.v[k] = h->v[k]; a.T[k] = h->T[k]; a.pc[k] = h->pc[k]; }
+  a.p = h->p; a.au = h->au; a.av = h->av; a.b_o = h->b_o; a.resu = h->resu;
+  a.u_ant = h->u_ant; a.v_ant = h->v_ant; a.T_ant = h->T_ant;
+  for (int k = 0; k < 3; ++k) { a.fcon[k] = h->fcon[k]; a.flin[k] = h->flin[k]; }
+  a.bc = h->bc; a.bcstride = h->bcstride;
+  a.ctl = h->ctl_d; a.partials = h->partials; a.bar = &h->ctl_d->bar; a.norms = h->norms;
+  a.max_outer = kLoopPasses;
+  a.part = part;
+  return a;
+}
+
+// One part of an outer pass (host-driven loop); its norms arrive in h_norms.
+int loop_part(ixb_handle* h, int part) {
+  CK(cudaMemsetAsync(h->ctl_d, 0, sizeof(Ctl), h->stream));
+  CK(loop_launch(solver_form(h), loop_args(h, part), h->stream));
+  CK(cudaMemcpyAsync(h->h_norms, h->norms, N_COUNT * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaMemcpyAsync(&h->ctl_h->abort_flag, &h->ctl_d->abort_flag, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaStreamSynchronize(h->stream));
+  return h->ctl_h->abort_flag ? IXB_ETIMEOUT : IXB_OK;
+}
+
 // ---------------------------------------------------------------------------
 // host-driven body (one sync per inner pass), main.f90:404-1215
 // ---------------------------------------------------------------------------
 int body_host(ixb_handle* h, bool outer_test, ixb_report* rep, int* exit_code) {
   const ixb_params& P = h->prm;
+  const bool resident = loop_usable(h);  // the parts of the loop kernel, else single sweeps
+  if (resident) TRY(normalize_parity(h));
   // ecuacion_momento
   for (;;) {
-    TRY(sweep(h, EQ_UY, nullptr, false));
-    TRY(sweep(h, EQ_UX, nullptr, false));
-    const double* v_start = h->v[h->cv];
-    TRY(sweep(h, EQ_VY, nullptr, false));
-    TRY(sweep(h, EQ_VX, v_start, true));
-    TRY(read_norms(h));
+    if (resident) {
+      TRY(loop_part(h, LOOP_MOMENTUM));
+    } else {
+      TRY(sweep(h, EQ_UY, nullptr, false));
+      TRY(sweep(h, EQ_UX, nullptr, false));
+      const double* v_start = h->v[h->cv];
+      TRY(sweep(h, EQ_VY, nullptr, false));
+      TRY(sweep(h, EQ_VX, v_start, true));
+      TRY(read_norms(h));
+    }
     const double err = h->h_norms[N_DV];
     rep->err_u = err;
     rep->n_momen++;
@@ -249,12 +310,16 @@ int body_host(ixb_handle* h, bool outer_test, ixb_report* rep, int* exit_code) {
     else h->iter_ecuaci++;
   }
   // correccion_presion
-  CK(cudaMemsetAsync(h->pc[h->cpc], 0, h->fsz * sizeof(double), h->stream));
-  for (;;) {
-    const double* pc_start = h->pc[h->cpc];
-    TRY(sweep(h, EQ_PY, nullptr, false));
-    TRY(sweep(h, EQ_PX, pc_start, true));
-    TRY(read_norms(h));
+  if (!resident) CK(cudaMemsetAsync(h->pc[h->cpc], 0, h->fsz * sizeof(double), h->stream));
+  for (bool first = true;; first = false) {
+    if (resident) {
+      TRY(loop_part(h, first ? LOOP_PRESSURE_FIRST : LOOP_PRESSURE));
+    } else {
+      const double* pc_start = h->pc[h->cpc];
+      TRY(sweep(h, EQ_PY, nullptr, false));
+      TRY(sweep(h, EQ_PX, pc_start, true));
+      TRY(read_norms(h));
+    }
     const double err = h->h_norms[N_DP];
     rep->err_p = err;
     rep->maxbo = h->h_norms[N_BO];
@@ -264,13 +329,18 @@ int body_host(ixb_handle* h, bool outer_test, ixb_report* rep, int* exit_code) {
     else if (h->iter_ecuaci > P.iter_ecuaci_max) { h->iter_ecuaci = 0; break; }
     else h->iter_ecuaci++;
   }
-  TRY(correct(h));
+  if (resident) TRY(loop_part(h, LOOP_CORRECT));
+  else TRY(correct(h));
   // solucion_energia
   for (;;) {
-    const double* t_start = h->T[h->cT];
-    TRY(sweep(h, EQ_TY, nullptr, false));
-    TRY(sweep(h, EQ_TX, t_start, true));
-    TRY(read_norms(h));
+    if (resident) {
+      TRY(loop_part(h, LOOP_ENERGY));
+    } else {
+      const double* t_start = h->T[h->cT];
+      TRY(sweep(h, EQ_TY, nullptr, false));
+      TRY(sweep(h, EQ_TX, t_start, true));
+      TRY(read_norms(h));
+    }
     const double err = h->h_norms[N_DT];
     rep->err_t = err;
     rep->n_ener++;
@@ -279,8 +349,12 @@ int body_host(ixb_handle* h, bool outer_test, ixb_report* rep, int* exit_code) {
     else if (h->iter_ecuaci > P.iter_ecuaci_max) { h->iter_ecuaci = 0; break; }
     else h->iter_ecuaci++;
   }
-  TRY(residual(h));
-  TRY(read_norms(h));
+  if (resident) {
+    TRY(loop_part(h, LOOP_RESIDUAL));
+  } else {
+    TRY(residual(h));
+    TRY(read_norms(h));
+  }
   rep->residuo = h->h_norms[N_RES];
   rep->n_simple++;
   if (!std::isfinite(rep->residuo)) return IXB_ENONFINITE;
@@ -500,7 +574,7 @@ int build_graph(ixb_handle* h, int kind, cudaGraph_t* graph, cudaGraphExec_t* ex
     TRY(add_outer_loop(h, mbody, &n_bb, c_outer, unroll, &n_outer));
     const Geo<double> G = make_geo(h);
     TRY(capture_into(h, mbody, &n_outer, [&]() {
-      return launch_nusselt_f64(G, h->T[h->cT], h->xp_d, h->yp_d, 0, 1, 1, h->nu_d, h->stream, h->ctl_d, c_top) ==
+      return launch_nusselt_f64(G, h->T[h->cT], h->xp_d, h->yp_d, 0, 1, 1, h->nu_d, h->stream, h->ctl_d, 1, c_top) ==
                      cudaSuccess ? IXB_OK : IXB_ECUDA;
     }, &n_nu));
   }
@@ -525,22 +599,8 @@ int ensure_graph(ixb_handle* h, int kind, cudaGraphExec_t* exec) {
   return IXB_OK;
 }
 
-// Bring every ping-pong field to buffer 0 (the parity the graph expects).
-int normalize_parity(ixb_handle* h) {
-  const size_t bytes = h->fsz * sizeof(double);
-  if (h->cu) { CK(cudaMemcpyAsync(h->u[0], h->u[1], bytes, cudaMemcpyDeviceToDevice, h->stream)); h->cu = 0; }
-  if (h->cv) { CK(cudaMemcpyAsync(h->v[0], h->v[1], bytes, cudaMemcpyDeviceToDevice, h->stream)); h->cv = 0; }
-  if (h->cT) { CK(cudaMemcpyAsync(h->T[0], h->T[1], bytes, cudaMemcpyDeviceToDevice, h->stream)); h->cT = 0; }
-  if (h->cpc) { CK(cudaMemcpyAsync(h->pc[0], h->pc[1], bytes, cudaMemcpyDeviceToDevice, h->stream)); h->cpc = 0; }
-  return IXB_OK;
-}
-
-// Launch the graph of `kind` with the loop inputs of the handle; `mon`
-// (monitor graphs only) sets the Nusselt monitor's inputs.
-int run_graph_once(ixb_handle* h, int kind, int fixed_count, ixb_report* rep, const ixb_nu_monitor* mon = nullptr) {
-  cudaGraphExec_t exec = nullptr;
-  TRY(ensure_graph(h, kind, &exec));
-  TRY(normalize_parity(h));
+// The control block of a run: its inputs and the handle's counters in ...
+void fill_ctl(ixb_handle* h, int fixed_count, const ixb_nu_monitor* mon) {
   Ctl* c = h->ctl_h;
   std::memset(c, 0, sizeof(Ctl));
   if (mon) {
@@ -558,10 +618,11 @@ int run_graph_once(ixb_handle* h, int kind, int fixed_count, ixb_report* rep, co
   c->fixed_count = fixed_count;
   c->iter_ecuaci = h->iter_ecuaci;
   c->iter_simple = h->iter_simple;
-  CK(cudaMemcpyAsync(h->ctl_d, c, sizeof(Ctl), cudaMemcpyHostToDevice, h->stream));
-  CK(cudaGraphLaunch(exec, h->stream));
-  CK(cudaMemcpyAsync(c, h->ctl_d, sizeof(Ctl), cudaMemcpyDeviceToHost, h->stream));
-  CK(cudaStreamSynchronize(h->stream));
+}
+
+// ... and its report and counters out.
+int read_ctl(ixb_handle* h, ixb_report* rep) {
+  const Ctl* c = h->ctl_h;
   rep->maxbo = c->maxbo; rep->residuo = c->residuo;
   rep->err_u = c->err_u; rep->err_p = c->err_p; rep->err_t = c->err_t;
   rep->n_simple = c->n_simple; rep->n_momen = c->n_momen; rep->n_pres = c->n_pres; rep->n_ener = c->n_ener;
@@ -571,12 +632,64 @@ int run_graph_once(ixb_handle* h, int kind, int fixed_count, ixb_report* rep, co
   return c->status;
 }
 
+// Launch the graph of `kind` with the loop inputs of the handle; `mon`
+// (monitor graphs only) sets the Nusselt monitor's inputs.
+int run_graph_once(ixb_handle* h, int kind, int fixed_count, ixb_report* rep, const ixb_nu_monitor* mon = nullptr) {
+  cudaGraphExec_t exec = nullptr;
+  TRY(ensure_graph(h, kind, &exec));
+  TRY(normalize_parity(h));
+  Ctl* c = h->ctl_h;
+  fill_ctl(h, fixed_count, mon);
+  CK(cudaMemcpyAsync(h->ctl_d, c, sizeof(Ctl), cudaMemcpyHostToDevice, h->stream));
+  CK(cudaGraphLaunch(exec, h->stream));
+  CK(cudaMemcpyAsync(c, h->ctl_d, sizeof(Ctl), cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaStreamSynchronize(h->stream));
+  return read_ctl(h, rep);
+}
+
+// Launches of the resident kernel queued between two looks at the control
+// block.
+constexpr int kLoopAhead = 8;
+
+// The SIMPLE loop through the resident kernel: a fixed count, the loop to its
+// exit test (fixed_count 0), or blocks of fixed_count passes with the Nusselt
+// monitor between them (`mon`).
+int run_loop(ixb_handle* h, int fixed_count, ixb_report* rep, const ixb_nu_monitor* mon = nullptr) {
+  TRY(normalize_parity(h));
+  fill_ctl(h, fixed_count, mon);
+  LoopArgs a = loop_args(h, LOOP_ALL);
+  const int form = solver_form(h);
+  CK(cudaMemcpyAsync(h->ctl_d, h->ctl_h, sizeof(Ctl), cudaMemcpyHostToDevice, h->stream));
+  bool fresh = true;  // the upload cleared the barrier
+  // launches of one block of passes (unknown without a fixed count: one at a time)
+  const int per_block = fixed_count > 0 ? (fixed_count + kLoopPasses - 1) / kLoopPasses : 1;
+  long long launched = 0;  // of the current block
+  for (;;) {
+    for (int q = 0; q < (fixed_count > 0 ? kLoopAhead : 1); ++q) {
+      if (!fresh) CK(cudaMemsetAsync(&h->ctl_d->bar, 0, sizeof(unsigned), h->stream));
+      fresh = false;
+      CK(loop_launch(form, a, h->stream));
+      if (++launched == per_block) {
+        if (!mon) { if (fixed_count > 0) break; launched = 0; continue; }
+        launched = 0;
+        CK(launch_nusselt_f64(a.G, h->T[0], h->xp_d, h->yp_d, 0, 1, 1, h->nu_d, h->stream, h->ctl_d));
+      }
+    }
+    CK(cudaMemcpyAsync(h->ctl_h, h->ctl_d, sizeof(Ctl), cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaStreamSynchronize(h->stream));
+    if (h->ctl_h->abort_flag) { h->ctl_h->status = IXB_ETIMEOUT; break; }
+    if (mon ? h->ctl_h->mon_over : h->ctl_h->stop) break;
+  }
+  return read_ctl(h, rep);
+}
+
 // The SIMPLE loop on the device: a fixed count that is a positive multiple
 // of kOuterUnroll runs through the unrolled graph (one WHILE body launch per
 // kOuterUnroll passes), anything else through the plain one.  (Splitting
 // other counts into the two graphs costs a second launch and host sync per
 // call, more than the unrolling saves on small grids.)
 int run_graph(ixb_handle* h, int fixed_count, ixb_report* rep) {
+  if (use_loop(h)) return run_loop(h, fixed_count, rep);
   const bool unrolled = fixed_count > 0 && fixed_count % kOuterUnroll == 0;
   return run_graph_once(h, unrolled ? GRAPH_UNROLLED : GRAPH_PLAIN, fixed_count, rep);
 }
@@ -808,6 +921,8 @@ int ixb_create(int mi, int nj, int prec_mode, ixb_handle** out) {
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
       return fail(IXB_ECUDA);
+    int coop = 0;
+    h->coop = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && coop;
   }
   const char* env = std::getenv("IXB_NO_GRAPH");
   if (env && env[0] == '1') h->use_graph = 0;
@@ -1099,7 +1214,7 @@ int ixb_simple_converge(ixb_handle* h, const ixb_nu_monitor* mon, ixb_report* re
   int st;
   if (h->use_graph) {
     const int kind = mon->every % kOuterUnroll == 0 ? GRAPH_MON_UNROLLED : GRAPH_MON_PLAIN;
-    st = run_graph_once(h, kind, mon->every, r, mon);
+    st = use_loop(h) ? run_loop(h, mon->every, r, mon) : run_graph_once(h, kind, mon->every, r, mon);
     const Ctl* c = h->ctl_h;
     nu2[0] = c->mon_nu[0];
     nu2[1] = c->mon_nu[1];
@@ -1218,6 +1333,10 @@ int ixb_time_phases(ixb_handle* h, int reps, size_t flush_bytes, double* ms) {
 
 int ixb_iteration_launches(ixb_handle* h, int* launches) {
   if (!h || !launches) return IXB_EINVAL;
+  if (use_loop(h)) {  // the resident kernel: launched once per call, not per iteration
+    *launches = 0;
+    return IXB_OK;
+  }
   // p/u/v correction, u residual, and the p' reset kernel unless the graph
   // runs the inner loops in do-while form (whose first pressure pass reads zeros)
   int k = (h->use_graph && do_while_loops()) ? 2 : 3;
@@ -1234,6 +1353,7 @@ int ixb_set_sweep_shape(ixb_handle* h, int sweep, int lines_per_cta, int threads
   if (!h || sweep < 0 || sweep >= EQ_COUNT) return IXB_EINVAL;
   if (lines_per_cta == 0) {  // back to the default choice
     h->shape_tl[sweep] = h->shape_g[sweep] = 0;
+    h->shape_set[sweep] = false;
     h->graph_dirty = h->egraph_dirty = h->agraph_dirty = true;
     return IXB_OK;
   }
@@ -1245,6 +1365,7 @@ int ixb_set_sweep_shape(ixb_handle* h, int sweep, int lines_per_cta, int threads
   if (sweep_occupancy(sweep, solver_form(h), s) <= 0) return IXB_EINVAL;
   h->shape_tl[sweep] = lines_per_cta;
   h->shape_g[sweep] = threads_per_line;
+  h->shape_set[sweep] = true;
   h->graph_dirty = h->egraph_dirty = h->agraph_dirty = true;
   return IXB_OK;
 }
@@ -1262,6 +1383,8 @@ int ixb_autotune(ixb_handle* h, int reps, size_t flush_bytes, int* chosen, doubl
   void* flush = nullptr;
   if (flush_bytes > 0 && cudaMalloc(&flush, flush_bytes) != cudaSuccess) { cudaFree(save); return IXB_ENOMEM; }
   const int cu = h->cu, cv = h->cv, cT = h->cT, cpc = h->cpc;
+  std::array<bool, EQ_COUNT> set_by_caller;
+  std::copy(std::begin(h->shape_set), std::end(h->shape_set), set_by_caller.begin());
   int st = IXB_OK;
   for (int k = 0; k < nsave && st == IXB_OK; ++k)
     if (cudaMemcpyAsync(save + k * h->fsz, bufs[k], fb, cudaMemcpyDeviceToDevice, h->stream) != cudaSuccess)
@@ -1301,6 +1424,7 @@ int ixb_autotune(ixb_handle* h, int reps, size_t flush_bytes, int* chosen, doubl
   for (int k = 0; k < nsave; ++k)
     cudaMemcpyAsync(bufs[k], save + k * h->fsz, fb, cudaMemcpyDeviceToDevice, h->stream);
   h->cu = cu; h->cv = cv; h->cT = cT; h->cpc = cpc;
+  std::copy(set_by_caller.begin(), set_by_caller.end(), std::begin(h->shape_set));  // trials are not the caller's choice
   if (cudaStreamSynchronize(h->stream) != cudaSuccess && st == IXB_OK) st = IXB_ECUDA;
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);

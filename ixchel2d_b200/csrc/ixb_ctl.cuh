@@ -83,7 +83,9 @@ static __device__ void ctl_outer_step(Ctl* c, const double* norms, cudaGraphCond
 // monitored wall, then stop the monitor loop (exit_code 3) when that change
 // is below mon_tol_dnu, (4) when maxbo is below mon_tol_maxbo, (5) once
 // mon_max_iters outer passes are done, or on an error status of the passes.
-static __device__ void ctl_monitor_step(Ctl* c, const double* nu2, cudaGraphConditionalHandle mon) {
+// In a graph the loop is the conditional node `mon`; the resident loop's
+// launches read `stop` instead.
+static __device__ void ctl_monitor_step(Ctl* c, const double* nu2, bool in_graph, cudaGraphConditionalHandle mon) {
   c->mon_nu[0] = nu2[0];
   c->mon_nu[1] = nu2[1];
   const double nu = nu2[c->mon_wall];
@@ -104,7 +106,13 @@ static __device__ void ctl_monitor_step(Ctl* c, const double* nu2, cudaGraphCond
   } else {
     stop = false;
   }
-  cudaGraphSetConditional(mon, stop ? 0u : 1u);
+  if (in_graph) {
+    cudaGraphSetConditional(mon, stop ? 0u : 1u);
+  } else {
+    c->mon_over = stop;
+    c->stop = stop;
+    c->outer_done = 0;  // the next block counts from zero
+  }
 }
 
 }  // namespace ixb

@@ -33,10 +33,14 @@ namespace ixb {
 // forms the diffusive conductances gamma*delta/d of the 2-D tables below
 // from 1-D factors (a uniform gamma makes them separable): M_GRDXP =
 // gamma_momen/dxp, M_GRDYV = gamma_momen/dyv, M_GRDXU = gamma_momen/dxu,
-// M_GRDYP = gamma_momen/dyp, M_HRDXU = M_HXU/dxu, M_HRDYV = M_HYV/dyv.
+// M_GRDYP = gamma_momen/dyp, M_HRDXU = M_HXU/dxu, M_HRDYV = M_HYV/dyv.  M_PE*
+// are the factors of |velocity| in 0.1|Peclet| (0.1 * spacing / diffusivity):
+// of gamma_momen with dxp, dyv, dxu and dyp, and of the energy faces (M_PHXU,
+// M_PHYV).
 enum Metric {
   M_DXP = 0, M_DYP, M_DXU, M_DYU, M_DXV, M_DYV, M_FEXP, M_FEYP, M_FEXU, M_FEYV,
-  M_HXU, M_HYV, M_RHXU, M_RHYV, M_GRDXP, M_GRDYV, M_GRDXU, M_GRDYP, M_HRDXU, M_HRDYV, M_COUNT
+  M_HXU, M_HYV, M_RHXU, M_RHYV, M_GRDXP, M_GRDYV, M_GRDXU, M_GRDYP, M_HRDXU, M_HRDYV,
+  M_PEXP, M_PEYV, M_PEXU, M_PEYP, M_PHXU, M_PHYV, M_COUNT
 };
 
 // Mesh-constant 2-D tables (field layout).  With the uniform diffusion
@@ -87,6 +91,12 @@ __device__ __forceinline__ R ldg(const R* p, int i) { return __ldg(p + i); }
 // the field and the arithmetic are both binary64)
 template <class R, class F>
 __device__ __forceinline__ R ld(const F* p, int i) { return R(__ldg(p + i)); }
+// A binary64 field that other CTAs of the same launch write between grid
+// barriers (the loop kernel): ordinary loads, which see those writes, in
+// place of the read-only path.
+struct Live { double v; };
+template <class R>
+__device__ __forceinline__ R ld(const Live* p, int i) { return p[i].v; }
 template <class R>
 struct Geo {
   int mi, nj, LD, mstride;
@@ -100,36 +110,58 @@ struct Geo {
   __device__ __forceinline__ R t(int which, int ii, int jj) const { return __ldg(tab + which * tstride + at(ii, jj)); }
 };
 
-// Diffusive conductances of the assembly.  Exact form: the 2-D table entry
-// (the reference's operands in its order).  Fast form: the product of the
-// cell's 1-D mesh factor, which the caller holds already (`f`), and a 1-D
-// reciprocal factor, an L1-resident load in place of a 2-D table read; it
-// differs from the table by rounding (the face diffusivities of a uniform
-// gamma are gamma itself up to rounding, as in the Peclet numbers).
-//   u: T_CU1(ii,jj) = dyu(jj) * GRDXP(ii);   T_CU2(ii,jj) = dxu(ii) * GRDYV(jj)
-//   v: T_CV1(ii,jj) = dyv(jj) * GRDXU(ii-1); T_CV2(ii,jj) = dxv(ii) * GRDYP(jj)
-//   T: T_CT1(ii,jj) = dyp(jj) * HRDXU(ii-1); T_CT2(ii,jj) = dxp(ii) * HRDYV(jj)
-template <bool FAST, class R>
-__device__ __forceinline__ R cond_t(const Geo<R>& G, int table, int ii, int jj, R f, int metric, int k) {
-  if constexpr (FAST) return f * G.met(metric, k);
-  else return G.t(table, ii, jj);
-}
-
 template <class R>
 struct SweepIO {
   const R *u, *v, *T, *p, *pc;        // current fields
-  const R *u_ant, *v_ant, *T_ant;
+  const double *u_ant, *v_ant, *T_ant;
   const R *au, *av;
-  const R *fcon, *flin;               // sources of this equation (null when none)
+  const double *fcon, *flin;          // sources of this equation (null when none)
   const R* in;                        // swept field, current values
-  R* out;                             // swept field, new values
-  const R* prev;                      // field at the start of the inner pass (null: zero)
-  R* aux;                             // au (u-x), av (v-x), b_o (p'-x)
+  double* out;                        // swept field, new values
+  const double* prev;                 // field at the start of the inner pass (null: zero)
+  double* aux;                        // au (u-x), av (v-x), b_o (p'-x)
   const BCEntry* bc_first;            // indexed by line
   const BCEntry* bc_last;
   NormSlot nrm0;                      // ||out - prev|| over interior rows of solved lines
   NormSlot nrm1;                      // ||b_o|| (p'-x)
 };
+
+// What an assembly reads at and around cell (ii,jj): the swept field `in`,
+// the other fields, the previous time level and the sources at the cell, the
+// 1-D metrics and the mesh tables, all by offset.  CellView loads each value
+// where it is asked for; the resident loop's column view holds three cells'
+// values in registers (ixb_loop.cuh).
+template <class R, class F>
+struct CellView {
+  const Geo<R>& G;
+  const SweepIO<F>& io;
+  int ii, jj;
+  __device__ __forceinline__ int at(int di, int dj) const { return G.at(ii + di, jj + dj); }
+  __device__ __forceinline__ R in(int di, int dj) const { return ld<R>(io.in, at(di, dj)); }
+  __device__ __forceinline__ R u(int di, int dj) const { return ld<R>(io.u, at(di, dj)); }
+  __device__ __forceinline__ R v(int di, int dj) const { return ld<R>(io.v, at(di, dj)); }
+  __device__ __forceinline__ R T(int di, int dj) const { return ld<R>(io.T, at(di, dj)); }
+  __device__ __forceinline__ R p(int di, int dj) const { return ld<R>(io.p, at(di, dj)); }
+  __device__ __forceinline__ R au(int di, int dj) const { return ld<R>(io.au, at(di, dj)); }
+  __device__ __forceinline__ R av(int di, int dj) const { return ld<R>(io.av, at(di, dj)); }
+  __device__ __forceinline__ R u_ant() const { return ld<R>(io.u_ant, at(0, 0)); }
+  __device__ __forceinline__ R v_ant() const { return ld<R>(io.v_ant, at(0, 0)); }
+  __device__ __forceinline__ R T_ant() const { return ld<R>(io.T_ant, at(0, 0)); }
+  // no sources: no loads (the values would be +0)
+  __device__ __forceinline__ R fcon() const { return io.fcon ? ld<R>(io.fcon, at(0, 0)) : R(0); }
+  __device__ __forceinline__ R flin() const { return io.flin ? ld<R>(io.flin, at(0, 0)) : R(0); }
+  __device__ __forceinline__ R mx(int which, int di) const { return G.met(which, ii + di); }  // metrics along x
+  __device__ __forceinline__ R my(int which, int dj) const { return G.met(which, jj + dj); }  // and along y
+  __device__ __forceinline__ R tab(int which, int di, int dj) const { return G.t(which, ii + di, jj + dj); }
+};
+
+// Diffusive conductances.  The exact form reads the 2-D table entry (the
+// reference's operands in its order); the fast form multiplies the cell's 1-D
+// mesh factor by a 1-D reciprocal factor, an L1-resident load in place of a
+// 2-D table read, which differs from the table by rounding:
+//   u: T_CU1(ii,jj) = dyu(jj) * GRDXP(ii);   T_CU2(ii,jj) = dxu(ii) * GRDYV(jj)
+//   v: T_CV1(ii,jj) = dyv(jj) * GRDXU(ii-1); T_CV2(ii,jj) = dxv(ii) * GRDYP(jj)
+//   T: T_CT1(ii,jj) = dyp(jj) * HRDXU(ii-1); T_CT2(ii,jj) = dxp(ii) * HRDYV(jj)
 
 template <class R>
 struct Row { R a, b, c, d; };
@@ -152,6 +184,21 @@ __device__ __forceinline__ R plaw(R pe) {
 }
 template <class R>
 __device__ __forceinline__ R dmax0(R x) { return fmaxT(R(0), x); }
+// max(0, x) by the sign bit (three integer operations; the binary64 maximum
+// takes the binary64 pipe, which the fast rows keep busy).  NaN stays NaN.
+__device__ __forceinline__ double pos(double x) {
+  const int hi = __double2hiint(x), keep = ~(hi >> 31);
+  return __hiloint2double(hi & keep, __double2loint(x) & keep);
+}
+// Fast form of a neighbour coefficient (with its sign): conductance
+// max(0, 1 - 0.1|Pe|)^5 plus the upwind part of the flux, 0.1|Pe| = |vel| m.
+__device__ __forceinline__ double plaw_fast(double vel, double m) {
+  const double t = pos(fma(-fabs(vel), m, 1.0)), t2 = t * t;
+  return t * (t2 * t2);
+}
+__device__ __forceinline__ double link_fast(double cond, double law, double flux) {
+  return -fma(cond, law, pos(flux));
+}
 
 // harmonic face interpolation g1*g2/(g1*(1-f)+g2*f) of the reference
 // (e.g. source/mod_ec_momento.f90:462-465) with its operand order
@@ -189,154 +236,137 @@ __device__ __forceinline__ R qdiv(R a, R b) { if constexpr (FAST) return a * fas
 // The four neighbour coefficients of the u row (:512-526), face velocities
 // interpolated as in :447-455, diffusivities and conductances from the
 // tables (gammai = gammad = gamma_momen).
-template <bool FAST, class R, class F>
-__device__ __forceinline__ void u_parts(const Geo<R>& G, const SweepIO<F>& io, const F* u, int ii, int jj,
-                                        R& AI, R& AD, R& BS, R& BN, R& deltax, R& deltay, R& temp_int) {
-  const F* v = io.v;
-  const R fexu_i = G.met(M_FEXU, ii), fexu_m = G.met(M_FEXU, ii - 1);
-  const R fexp_i = G.met(M_FEXP, ii);
-  R ud = fexu_i * ld<R>(u, G.at(ii + 1, jj)) + (R(1) - fexu_i) * ld<R>(u, G.at(ii, jj));
-  R ui = fexu_m * ld<R>(u, G.at(ii, jj)) + (R(1) - fexu_m) * ld<R>(u, G.at(ii - 1, jj));
-  R vn = fexp_i * ld<R>(v, G.at(ii + 1, jj)) + (R(1) - fexp_i) * ld<R>(v, G.at(ii, jj));
-  R vs = fexp_i * ld<R>(v, G.at(ii + 1, jj - 1)) + (R(1) - fexp_i) * ld<R>(v, G.at(ii, jj - 1));
-  const R g = G.gm;
-  R gamman, gammas, rgn = R(0), rgs = R(0);
+// Without buoyancy (coefficient 0) the fast form leaves T unread.
+template <bool FAST, class R, class V>
+__device__ __forceinline__ void u_parts(const Geo<R>& G, const V& c, R& AI, R& AD, R& BS, R& BN, R& deltax, R& deltay,
+                                        R& temp_int) {
+  const R fexu_i = c.mx(M_FEXU, 0), fexu_m = c.mx(M_FEXU, -1);
+  const R fexp_i = c.mx(M_FEXP, 0);
+  R ud = fexu_i * c.in(1, 0) + (R(1) - fexu_i) * c.in(0, 0);
+  R ui = fexu_m * c.in(0, 0) + (R(1) - fexu_m) * c.in(-1, 0);
+  R vn = fexp_i * c.v(1, 0) + (R(1) - fexp_i) * c.v(0, 0);
+  R vs = fexp_i * c.v(1, -1) + (R(1) - fexp_i) * c.v(0, -1);
+  deltax = c.mx(M_DXU, 0);
+  deltay = c.my(M_DYU, 0);
   if constexpr (FAST) {
-    // the face diffusivity is the harmonic mean of a uniform gamma_momen
-    // (ixb_params holds one value), i.e. gamma_momen up to rounding: its
-    // reciprocal is the scalar 1/gamma_momen, no table load
-    rgn = rgs = G.inv_gm;
-    gamman = gammas = R(0);
+    // the face diffusivities are harmonic means of a uniform gamma_momen
+    // (ixb_params holds one value), i.e. gamma_momen up to rounding
+    temp_int = R(0);
+    if (G.Ri != R(0)) temp_int = fexp_i * c.T(1, 0) + (R(1) - fexp_i) * c.T(0, 0);
+    AI = link_fast(deltay * c.mx(M_GRDXP, 0), plaw_fast(ui, c.mx(M_PEXP, 0)), ui * deltay);
+    AD = link_fast(deltay * c.mx(M_GRDXP, 1), plaw_fast(ud, c.mx(M_PEXP, 1)), -ud * deltay);
+    BS = link_fast(deltax * c.my(M_GRDYV, -1), plaw_fast(vs, c.my(M_PEYV, -1)), vs * deltax);
+    BN = link_fast(deltax * c.my(M_GRDYV, 0), plaw_fast(vn, c.my(M_PEYV, 0)), -vn * deltax);
   } else {
-    gamman = G.t(T_GU, ii, jj);
-    gammas = G.t(T_GU, ii, jj - 1);
+    const R g = G.gm;
+    const R gamman = c.tab(T_GU, 0, 0), gammas = c.tab(T_GU, 0, -1);
+    R di = c.mx(M_DXP, 0), dd = c.mx(M_DXP, 1), ds = c.my(M_DYV, -1), dn = c.my(M_DYV, 0);
+    temp_int = fexp_i * c.T(1, 0) + (R(1) - fexp_i) * c.T(0, 0);
+    AI = -(c.tab(T_CU1, 0, 0) * plaw(ui * di / g) + dmax0(ui * deltay));
+    AD = -(c.tab(T_CU1, 1, 0) * plaw(ud * dd / g) + dmax0(-ud * deltay));
+    BS = -(c.tab(T_CU2, 0, -1) * plaw(vs * ds / gammas) + dmax0(vs * deltax));
+    BN = -(c.tab(T_CU2, 0, 0) * plaw(vn * dn / gamman) + dmax0(-vn * deltax));
   }
-  R di = G.met(M_DXP, ii), dd = G.met(M_DXP, ii + 1), ds = G.met(M_DYV, jj - 1), dn = G.met(M_DYV, jj);
-  deltax = G.met(M_DXU, ii);
-  deltay = G.met(M_DYU, jj);
-  temp_int = fexp_i * ld<R>(io.T, G.at(ii + 1, jj)) + (R(1) - fexp_i) * ld<R>(io.T, G.at(ii, jj));
-  AI = -(cond_t<FAST>(G, T_CU1, ii, jj, deltay, M_GRDXP, ii) * plaw(qdiv<FAST>(ui * di, g, G.inv_gm)) + dmax0(ui * deltay));
-  AD = -(cond_t<FAST>(G, T_CU1, ii + 1, jj, deltay, M_GRDXP, ii + 1) * plaw(qdiv<FAST>(ud * dd, g, G.inv_gm)) +
-         dmax0(-ud * deltay));
-  BS = -(cond_t<FAST>(G, T_CU2, ii, jj - 1, deltax, M_GRDYV, jj - 1) * plaw(qdiv<FAST>(vs * ds, gammas, rgs)) +
-         dmax0(vs * deltax));
-  BN = -(cond_t<FAST>(G, T_CU2, ii, jj, deltax, M_GRDYV, jj) * plaw(qdiv<FAST>(vn * dn, gamman, rgn)) +
-         dmax0(-vn * deltax));
 }
 
 // X form (ensambla_velu_x): a=AI c=AD b=AC d=Rx, aux = au = AC*rel
-template <bool FAST, class R, class F>
-__device__ __forceinline__ Row<R> assemble_ux(const Geo<R>& G, const SweepIO<F>& io, int ii, int jj, R& au) {
-  const F* u = io.in;
+template <bool FAST, class R, class V>
+__device__ __forceinline__ Row<R> assemble_ux(const Geo<R>& G, const V& c, R& au) {
   R AI, AD, BS, BN, dx, dy, tint;
-  u_parts<FAST>(G, io, u, ii, jj, AI, AD, BS, BN, dx, dy, tint);
-  const int c0 = G.at(ii, jj);
-  const R flin = io.flin ? ld<R>(io.flin, c0) : R(0);  // no sources: no loads (the values would be +0)
-  const R fcon = io.fcon ? ld<R>(io.fcon, c0) : R(0);
+  u_parts<FAST>(G, c, AI, AD, BS, BN, dx, dy, tint);
+  const R flin = c.flin(), fcon = c.fcon();
   Row<R> r;
   r.a = AI;
   r.c = AD;
   r.b = qdiv<FAST>(-AI - AD - BS - BN - dx * dy * flin + qdiv<FAST>(dx * dy, G.dt, G.inv_dt), G.rel_vel,
                    G.inv_rel_vel);
-  r.d = -BS * ld<R>(u, G.at(ii, jj - 1)) - BN * ld<R>(u, G.at(ii, jj + 1)) - dx * dy * G.Ri * tint + dx * dy * fcon +
-        qdiv<FAST>(dx * dy * ld<R>(io.u_ant, c0), G.dt, G.inv_dt) + (ld<R>(io.p, c0) - ld<R>(io.p, G.at(ii + 1, jj))) * dy +
-        r.b * (R(1) - G.rel_vel) * ld<R>(u, c0);
+  r.d = -BS * c.in(0, -1) - BN * c.in(0, 1) - dx * dy * G.Ri * tint + dx * dy * fcon +
+        qdiv<FAST>(dx * dy * c.u_ant(), G.dt, G.inv_dt) + (c.p(0, 0) - c.p(1, 0)) * dy +
+        r.b * (R(1) - G.rel_vel) * c.in(0, 0);
   au = r.b * G.rel_vel;
   return r;
 }
 
 // Y form (ensambla_velu_y): a=BS c=BN b=BC d=Ry
-template <bool FAST, class R, class F>
-__device__ __forceinline__ Row<R> assemble_uy(const Geo<R>& G, const SweepIO<F>& io, int ii, int jj) {
-  const F* u = io.in;
+template <bool FAST, class R, class V>
+__device__ __forceinline__ Row<R> assemble_uy(const Geo<R>& G, const V& c) {
   R AI, AD, BS, BN, dx, dy, tint;
-  u_parts<FAST>(G, io, u, ii, jj, AI, AD, BS, BN, dx, dy, tint);
-  const int c0 = G.at(ii, jj);
-  const R flin = io.flin ? ld<R>(io.flin, c0) : R(0);  // no sources: no loads (the values would be +0)
-  const R fcon = io.fcon ? ld<R>(io.fcon, c0) : R(0);
+  u_parts<FAST>(G, c, AI, AD, BS, BN, dx, dy, tint);
+  const R flin = c.flin(), fcon = c.fcon();
   Row<R> r;
   r.a = BS;
   r.c = BN;
   r.b = qdiv<FAST>(-AI - AD - BS - BN - dx * dy * flin + qdiv<FAST>(dx * dy, G.dt, G.inv_dt), G.rel_vel,
                    G.inv_rel_vel);
-  r.d = -AI * ld<R>(u, G.at(ii - 1, jj)) - AD * ld<R>(u, G.at(ii + 1, jj)) - dx * dy * G.Ri * tint + dx * dy * fcon +
-        qdiv<FAST>(dx * dy * ld<R>(io.u_ant, c0), G.dt, G.inv_dt) + (ld<R>(io.p, c0) - ld<R>(io.p, G.at(ii + 1, jj))) * dy +
-        r.b * (R(1) - G.rel_vel) * ld<R>(u, c0);
+  r.d = -AI * c.in(-1, 0) - AD * c.in(1, 0) - dx * dy * G.Ri * tint + dx * dy * fcon +
+        qdiv<FAST>(dx * dy * c.u_ant(), G.dt, G.inv_dt) + (c.p(0, 0) - c.p(1, 0)) * dy +
+        r.b * (R(1) - G.rel_vel) * c.in(0, 0);
   return r;
 }
 
 // ---------------------------------------------------------------------------
 // v momentum (ensambla_velv_x/_y, source/mod_ec_momento.f90:736-1098)
 // ---------------------------------------------------------------------------
-template <bool FAST, class R, class F>
-__device__ __forceinline__ void v_parts(const Geo<R>& G, const SweepIO<F>& io, const F* v, int ii, int jj,
-                                        R& AI, R& AD, R& BS, R& BN, R& temp_int) {
-  const F* u = io.u;
-  const R feyp_j = G.met(M_FEYP, jj);
-  const R feyv_j = G.met(M_FEYV, jj), feyv_m = G.met(M_FEYV, jj - 1);
-  R ud = feyp_j * ld<R>(u, G.at(ii, jj + 1)) + (R(1) - feyp_j) * ld<R>(u, G.at(ii, jj));
-  R ui = feyp_j * ld<R>(u, G.at(ii - 1, jj + 1)) + (R(1) - feyp_j) * ld<R>(u, G.at(ii - 1, jj));
-  R vn = feyv_j * ld<R>(v, G.at(ii, jj + 1)) + (R(1) - feyv_j) * ld<R>(v, G.at(ii, jj));
-  R vs = feyv_m * ld<R>(v, G.at(ii, jj)) + (R(1) - feyv_m) * ld<R>(v, G.at(ii, jj - 1));
-  const R g = G.gm;  // gamman = gammas = gamma_momen (:854-858)
-  R gammad, gammai, rgd = R(0), rgi = R(0);
+template <bool FAST, class R, class V>
+__device__ __forceinline__ void v_parts(const Geo<R>& G, const V& c, R& AI, R& AD, R& BS, R& BN, R& temp_int) {
+  const R feyp_j = c.my(M_FEYP, 0);
+  const R feyv_j = c.my(M_FEYV, 0), feyv_m = c.my(M_FEYV, -1);
+  R ud = feyp_j * c.u(0, 1) + (R(1) - feyp_j) * c.u(0, 0);
+  R ui = feyp_j * c.u(-1, 1) + (R(1) - feyp_j) * c.u(-1, 0);
+  R vn = feyv_j * c.in(0, 1) + (R(1) - feyv_j) * c.in(0, 0);
+  R vs = feyv_m * c.in(0, 0) + (R(1) - feyv_m) * c.in(0, -1);
+  const R dyv = c.my(M_DYV, 0), dxv = c.mx(M_DXV, 0);
   if constexpr (FAST) {
-    rgd = rgi = G.inv_gm;  // uniform gamma_momen, as in u_parts
-    gammad = gammai = R(0);
+    temp_int = R(0);
+    if (G.Riy != R(0)) temp_int = feyp_j * c.T(0, 1) + (R(1) - feyp_j) * c.T(0, 0);
+    AI = link_fast(dyv * c.mx(M_GRDXU, -1), plaw_fast(ui, c.mx(M_PEXU, -1)), ui * dyv);
+    AD = link_fast(dyv * c.mx(M_GRDXU, 0), plaw_fast(ud, c.mx(M_PEXU, 0)), -ud * dyv);
+    BS = link_fast(dxv * c.my(M_GRDYP, 0), plaw_fast(vs, c.my(M_PEYP, 0)), vs * dxv);
+    BN = link_fast(dxv * c.my(M_GRDYP, 1), plaw_fast(vn, c.my(M_PEYP, 1)), -vn * dxv);
   } else {
-    gammad = G.t(T_GV, ii, jj);
-    gammai = G.t(T_GV, ii - 1, jj);
+    const R g = G.gm;  // gamman = gammas = gamma_momen (:854-858)
+    const R gammad = c.tab(T_GV, 0, 0), gammai = c.tab(T_GV, -1, 0);
+    R di = c.mx(M_DXU, -1), dd = c.mx(M_DXU, 0), ds = c.my(M_DYP, 0), dn = c.my(M_DYP, 1);
+    temp_int = feyp_j * c.T(0, 1) + (R(1) - feyp_j) * c.T(0, 0);
+    AI = -(c.tab(T_CV1, 0, 0) * plaw(ui * di / gammai) + dmax0(ui * dyv));
+    AD = -(c.tab(T_CV1, 1, 0) * plaw(ud * dd / gammad) + dmax0(-ud * dyv));
+    BS = -(c.tab(T_CV2, 0, 0) * plaw(vs * ds / g) + dmax0(vs * dxv));
+    BN = -(c.tab(T_CV2, 0, 1) * plaw(vn * dn / g) + dmax0(-vn * dxv));
   }
-  R di = G.met(M_DXU, ii - 1), dd = G.met(M_DXU, ii), ds = G.met(M_DYP, jj), dn = G.met(M_DYP, jj + 1);
-  const R dyv = G.met(M_DYV, jj), dxv = G.met(M_DXV, ii);
-  temp_int = feyp_j * ld<R>(io.T, G.at(ii, jj + 1)) + (R(1) - feyp_j) * ld<R>(io.T, G.at(ii, jj));
-  AI = -(cond_t<FAST>(G, T_CV1, ii, jj, dyv, M_GRDXU, ii - 1) * plaw(qdiv<FAST>(ui * di, gammai, rgi)) +
-         dmax0(ui * dyv));
-  AD = -(cond_t<FAST>(G, T_CV1, ii + 1, jj, dyv, M_GRDXU, ii) * plaw(qdiv<FAST>(ud * dd, gammad, rgd)) +
-         dmax0(-ud * dyv));
-  BS = -(cond_t<FAST>(G, T_CV2, ii, jj, dxv, M_GRDYP, jj) * plaw(qdiv<FAST>(vs * ds, g, G.inv_gm)) + dmax0(vs * dxv));
-  BN = -(cond_t<FAST>(G, T_CV2, ii, jj + 1, dxv, M_GRDYP, jj + 1) * plaw(qdiv<FAST>(vn * dn, g, G.inv_gm)) +
-         dmax0(-vn * dxv));
 }
 
-template <bool FAST, class R, class F>
-__device__ __forceinline__ Row<R> assemble_vx(const Geo<R>& G, const SweepIO<F>& io, int ii, int jj, R& av) {
-  const F* v = io.in;
+template <bool FAST, class R, class V>
+__device__ __forceinline__ Row<R> assemble_vx(const Geo<R>& G, const V& c, R& av) {
   R AI, AD, BS, BN, tint;
-  v_parts<FAST>(G, io, v, ii, jj, AI, AD, BS, BN, tint);
-  const int c0 = G.at(ii, jj);
-  const R dxv = G.met(M_DXV, ii), dyv = G.met(M_DYV, jj);
+  v_parts<FAST>(G, c, AI, AD, BS, BN, tint);
+  const R dxv = c.mx(M_DXV, 0), dyv = c.my(M_DYV, 0);
   const R dxdy = dxv * dyv;
-  const R flin = io.flin ? ld<R>(io.flin, c0) : R(0);  // no sources: no loads (the values would be +0)
-  const R fcon = io.fcon ? ld<R>(io.fcon, c0) : R(0);
+  const R flin = c.flin(), fcon = c.fcon();
   Row<R> r;
   r.a = AI;
   r.c = AD;
   r.b = qdiv<FAST>(-AI - AD - BS - BN - dxdy * flin + qdiv<FAST>(dxdy, G.dt, G.inv_dt), G.rel_vel, G.inv_rel_vel);
-  r.d = -BS * ld<R>(v, G.at(ii, jj - 1)) - BN * ld<R>(v, G.at(ii, jj + 1)) - dxdy * G.Riy * tint + dxdy * fcon +
-        qdiv<FAST>(dxdy * ld<R>(io.v_ant, c0), G.dt, G.inv_dt) + (ld<R>(io.p, c0) - ld<R>(io.p, G.at(ii, jj + 1))) * dxv +
-        r.b * (R(1) - G.rel_vel) * ld<R>(v, c0);
+  r.d = -BS * c.in(0, -1) - BN * c.in(0, 1) - dxdy * G.Riy * tint + dxdy * fcon +
+        qdiv<FAST>(dxdy * c.v_ant(), G.dt, G.inv_dt) + (c.p(0, 0) - c.p(0, 1)) * dxv +
+        r.b * (R(1) - G.rel_vel) * c.in(0, 0);
   av = r.b * G.rel_vel;
   return r;
 }
 
-template <bool FAST, class R, class F>
-__device__ __forceinline__ Row<R> assemble_vy(const Geo<R>& G, const SweepIO<F>& io, int ii, int jj) {
-  const F* v = io.in;
+template <bool FAST, class R, class V>
+__device__ __forceinline__ Row<R> assemble_vy(const Geo<R>& G, const V& c) {
   R AI, AD, BS, BN, tint;
-  v_parts<FAST>(G, io, v, ii, jj, AI, AD, BS, BN, tint);
-  const int c0 = G.at(ii, jj);
-  const R dxv = G.met(M_DXV, ii), dyv = G.met(M_DYV, jj);
+  v_parts<FAST>(G, c, AI, AD, BS, BN, tint);
+  const R dxv = c.mx(M_DXV, 0), dyv = c.my(M_DYV, 0);
   const R dxdy = dxv * dyv;
-  const R flin = io.flin ? ld<R>(io.flin, c0) : R(0);  // no sources: no loads (the values would be +0)
-  const R fcon = io.fcon ? ld<R>(io.fcon, c0) : R(0);
+  const R flin = c.flin(), fcon = c.fcon();
   Row<R> r;
   r.a = BS;
   r.c = BN;
   r.b = qdiv<FAST>(-AI - AD - BS - BN - dxdy * flin + qdiv<FAST>(dxdy, G.dt, G.inv_dt), G.rel_vel, G.inv_rel_vel);
-  r.d = -AI * ld<R>(v, G.at(ii - 1, jj)) - AD * ld<R>(v, G.at(ii + 1, jj)) - dxdy * G.Riy * tint + dxdy * fcon +
-        qdiv<FAST>(dxdy * ld<R>(io.v_ant, c0), G.dt, G.inv_dt) + (ld<R>(io.p, c0) - ld<R>(io.p, G.at(ii, jj + 1))) * dxv +
-        r.b * (R(1) - G.rel_vel) * ld<R>(v, c0);
+  r.d = -AI * c.in(-1, 0) - AD * c.in(1, 0) - dxdy * G.Riy * tint + dxdy * fcon +
+        qdiv<FAST>(dxdy * c.v_ant(), G.dt, G.inv_dt) + (c.p(0, 0) - c.p(0, 1)) * dxv +
+        r.b * (R(1) - G.rel_vel) * c.in(0, 0);
   return r;
 }
 
@@ -344,171 +374,134 @@ __device__ __forceinline__ Row<R> assemble_vy(const Geo<R>& G, const SweepIO<F>&
 // energy (ensambla_energia_x/_y, source/mod_ec_energia.f90:119-443).  The
 // calls in main.f90:989 and :1060 bind fexu/feyv to the dummies fexpo/feypo.
 // ---------------------------------------------------------------------------
-template <bool FAST, class R, class F>
-__device__ __forceinline__ void t_parts(const Geo<R>& G, const SweepIO<F>& io, int ii, int jj, R& AI, R& AD,
-                                        R& BS, R& BN) {
-  const R ud = ld<R>(io.u, G.at(ii, jj)), ui = ld<R>(io.u, G.at(ii - 1, jj));
-  const R vn = ld<R>(io.v, G.at(ii, jj)), vs = ld<R>(io.v, G.at(ii, jj - 1));
-  const R di = G.met(M_DXU, ii - 1), dd = G.met(M_DXU, ii), ds = G.met(M_DYV, jj - 1), dn = G.met(M_DYV, jj);
-  const R dyp = G.met(M_DYP, jj), dxp = G.met(M_DXP, ii);
+template <bool FAST, class R, class V>
+__device__ __forceinline__ void t_parts(const Geo<R>& G, const V& c, R& AI, R& AD, R& BS, R& BN) {
+  const R ud = c.u(0, 0), ui = c.u(-1, 0);
+  const R vn = c.v(0, 0), vs = c.v(0, -1);
+  const R dyp = c.my(M_DYP, 0), dxp = c.mx(M_DXP, 0);
   if constexpr (FAST) {
-    AI = -(cond_t<true>(G, T_CT1, ii, jj, dyp, M_HRDXU, ii - 1) * plaw(ui * di * G.met(M_RHXU, ii - 1)) +
-           dmax0(ui * dyp));
-    AD = -(cond_t<true>(G, T_CT1, ii + 1, jj, dyp, M_HRDXU, ii) * plaw(ud * dd * G.met(M_RHXU, ii)) + dmax0(-ud * dyp));
-    BS = -(cond_t<true>(G, T_CT2, ii, jj - 1, dxp, M_HRDYV, jj - 1) * plaw(vs * ds * G.met(M_RHYV, jj - 1)) +
-           dmax0(vs * dxp));
-    BN = -(cond_t<true>(G, T_CT2, ii, jj, dxp, M_HRDYV, jj) * plaw(vn * dn * G.met(M_RHYV, jj)) + dmax0(-vn * dxp));
+    AI = link_fast(dyp * c.mx(M_HRDXU, -1), plaw_fast(ui, c.mx(M_PHXU, -1)), ui * dyp);
+    AD = link_fast(dyp * c.mx(M_HRDXU, 0), plaw_fast(ud, c.mx(M_PHXU, 0)), -ud * dyp);
+    BS = link_fast(dxp * c.my(M_HRDYV, -1), plaw_fast(vs, c.my(M_PHYV, -1)), vs * dxp);
+    BN = link_fast(dxp * c.my(M_HRDYV, 0), plaw_fast(vn, c.my(M_PHYV, 0)), -vn * dxp);
   } else {
-    const R gammad = G.met(M_HXU, ii);
-    const R gammai = G.met(M_HXU, ii - 1);
-    const R gamman = G.met(M_HYV, jj);
-    const R gammas = G.met(M_HYV, jj - 1);
-    AI = -(G.t(T_CT1, ii, jj) * plaw(ui * di / gammai) + dmax0(ui * dyp));
-    AD = -(G.t(T_CT1, ii + 1, jj) * plaw(ud * dd / gammad) + dmax0(-ud * dyp));
-    BS = -(G.t(T_CT2, ii, jj - 1) * plaw(vs * ds / gammas) + dmax0(vs * dxp));
-    BN = -(G.t(T_CT2, ii, jj) * plaw(vn * dn / gamman) + dmax0(-vn * dxp));
+    const R di = c.mx(M_DXU, -1), dd = c.mx(M_DXU, 0), ds = c.my(M_DYV, -1), dn = c.my(M_DYV, 0);
+    const R gammad = c.mx(M_HXU, 0);
+    const R gammai = c.mx(M_HXU, -1);
+    const R gamman = c.my(M_HYV, 0);
+    const R gammas = c.my(M_HYV, -1);
+    AI = -(c.tab(T_CT1, 0, 0) * plaw(ui * di / gammai) + dmax0(ui * dyp));
+    AD = -(c.tab(T_CT1, 1, 0) * plaw(ud * dd / gammad) + dmax0(-ud * dyp));
+    BS = -(c.tab(T_CT2, 0, -1) * plaw(vs * ds / gammas) + dmax0(vs * dxp));
+    BN = -(c.tab(T_CT2, 0, 0) * plaw(vn * dn / gamman) + dmax0(-vn * dxp));
   }
 }
 
-template <bool FAST, class R, class F>
-__device__ __forceinline__ Row<R> assemble_tx(const Geo<R>& G, const SweepIO<F>& io, int ii, int jj) {
-  const F* T = io.in;
+template <bool FAST, class R, class V>
+__device__ __forceinline__ Row<R> assemble_tx(const Geo<R>& G, const V& c) {
   R AI, AD, BS, BN;
-  t_parts<FAST>(G, io, ii, jj, AI, AD, BS, BN);
-  const int c0 = G.at(ii, jj);
-  const R dxdy = G.met(M_DXP, ii) * G.met(M_DYP, jj);
-  const R flin = io.flin ? ld<R>(io.flin, c0) : R(0);  // no sources: no loads (the values would be +0)
-  const R fcon = io.fcon ? ld<R>(io.fcon, c0) : R(0);
+  t_parts<FAST>(G, c, AI, AD, BS, BN);
+  const R dxdy = c.mx(M_DXP, 0) * c.my(M_DYP, 0);
+  const R flin = c.flin(), fcon = c.fcon();
   Row<R> r;
   r.a = AI;
   r.c = AD;
   r.b = qdiv<FAST>(-AI - AD - BS - BN - dxdy * flin + qdiv<FAST>(dxdy, G.dt, G.inv_dt), G.rel_ener, G.inv_rel_ener);
-  r.d = -BS * ld<R>(T, G.at(ii, jj - 1)) - BN * ld<R>(T, G.at(ii, jj + 1)) + dxdy * fcon +
-        qdiv<FAST>(dxdy * ld<R>(io.T_ant, c0), G.dt, G.inv_dt) + r.b * (R(1) - G.rel_ener) * ld<R>(T, c0);
+  r.d = -BS * c.in(0, -1) - BN * c.in(0, 1) + dxdy * fcon + qdiv<FAST>(dxdy * c.T_ant(), G.dt, G.inv_dt) +
+        r.b * (R(1) - G.rel_ener) * c.in(0, 0);
   return r;
 }
 
-template <bool FAST, class R, class F>
-__device__ __forceinline__ Row<R> assemble_ty(const Geo<R>& G, const SweepIO<F>& io, int ii, int jj) {
-  const F* T = io.in;
+template <bool FAST, class R, class V>
+__device__ __forceinline__ Row<R> assemble_ty(const Geo<R>& G, const V& c) {
   R AI, AD, BS, BN;
-  t_parts<FAST>(G, io, ii, jj, AI, AD, BS, BN);
-  const int c0 = G.at(ii, jj);
-  const R dxdy = G.met(M_DXP, ii) * G.met(M_DYP, jj);
-  const R flin = io.flin ? ld<R>(io.flin, c0) : R(0);  // no sources: no loads (the values would be +0)
-  const R fcon = io.fcon ? ld<R>(io.fcon, c0) : R(0);
+  t_parts<FAST>(G, c, AI, AD, BS, BN);
+  const R dxdy = c.mx(M_DXP, 0) * c.my(M_DYP, 0);
+  const R flin = c.flin(), fcon = c.fcon();
   Row<R> r;
   r.a = BS;
   r.c = BN;
   r.b = qdiv<FAST>(-AI - AD - BS - BN - dxdy * flin + qdiv<FAST>(dxdy, G.dt, G.inv_dt), G.rel_ener, G.inv_rel_ener);
-  r.d = -AI * ld<R>(T, G.at(ii - 1, jj)) - AD * ld<R>(T, G.at(ii + 1, jj)) + dxdy * fcon +
-        qdiv<FAST>(dxdy * ld<R>(io.T_ant, c0), G.dt, G.inv_dt) + r.b * (R(1) - G.rel_ener) * ld<R>(T, c0);
+  r.d = -AI * c.in(-1, 0) - AD * c.in(1, 0) + dxdy * fcon + qdiv<FAST>(dxdy * c.T_ant(), G.dt, G.inv_dt) +
+        r.b * (R(1) - G.rel_ener) * c.in(0, 0);
   return r;
 }
 
 // ---------------------------------------------------------------------------
 // pressure correction (ensambla_corr_pres_x/_y, source/mod_ec_momento.f90:145-355)
 // ---------------------------------------------------------------------------
-template <class R, class F>
-__device__ __forceinline__ R pc_at(const SweepIO<F>& io, const Geo<R>& G, int ii, int jj) {
-  return ld<R>(io.in, G.at(ii, jj));
-}
-
 // Mass source b_o = (u_w - u_e) dy + (v_s - v_n) dx of the p' rows, always
 // in the fields' precision (binary64) with binary64 metrics, whatever the
 // precision of the coefficients.
-template <class R, class F>
-__device__ __forceinline__ F mass_residual(const Geo<R>& G, const SweepIO<F>& io, int ii, int jj) {
-  const int c0 = G.at(ii, jj);
-  const F ud = ldg(io.u, c0), ui = ldg(io.u, G.at(ii - 1, jj)), vn = ldg(io.v, c0), vs = ldg(io.v, G.at(ii, jj - 1));
-  return (ui - ud) * F(G.met(M_DYP, jj)) + (vs - vn) * F(G.met(M_DXP, ii));
+template <class R, class V>
+__device__ __forceinline__ double mass_residual(const Geo<R>& G, const V& c) {
+  const double ud = c.u(0, 0), ui = c.u(-1, 0), vn = c.v(0, 0), vs = c.v(0, -1);
+  return (ui - ud) * double(c.my(M_DYP, 0)) + (vs - vn) * double(c.mx(M_DXP, 0));
 }
 
-template <bool FAST, class R, class F>
-__device__ __forceinline__ Row<R> assemble_px(const Geo<R>& G, const SweepIO<F>& io, int ii, int jj, F& bo) {
-  const int c0 = G.at(ii, jj);
-  const R ai = ld<R>(io.au, G.at(ii - 1, jj)), ad = ld<R>(io.au, c0), as = ld<R>(io.av, G.at(ii, jj - 1)),
-          an = ld<R>(io.av, c0);
-  const R dyp = G.met(M_DYP, jj), dxp = G.met(M_DXP, ii);
+template <bool FAST, class R, class V>
+__device__ __forceinline__ Row<R> assemble_px(const Geo<R>& G, const V& c, double& bo) {
+  const R ai = c.au(-1, 0), ad = c.au(0, 0), as = c.av(0, -1), an = c.av(0, 0);
+  const R dyp = c.my(M_DYP, 0), dxp = c.mx(M_DXP, 0);
   Row<R> r;
   r.a = -qdiv<FAST>(dyp * dyp, ai);
   r.c = -qdiv<FAST>(dyp * dyp, ad);
   const R BS = -qdiv<FAST>(dxp * dxp, as);
   const R BN = -qdiv<FAST>(dxp * dxp, an);
   r.b = qdiv<FAST>(-r.a - r.c - BS - BN, G.rel_pres, G.inv_rel_pres);
-  bo = mass_residual(G, io, ii, jj);
-  r.d = -BS * pc_at<R>(io, G, ii, jj - 1) - BN * pc_at<R>(io, G, ii, jj + 1) + R(bo) +
-        (R(1) - G.rel_pres) * r.b * pc_at<R>(io, G, ii, jj);
+  bo = mass_residual(G, c);
+  r.d = -BS * c.in(0, -1) - BN * c.in(0, 1) + R(bo) + (R(1) - G.rel_pres) * r.b * c.in(0, 0);
   return r;
 }
 
-template <bool FAST, class R, class F>
-__device__ __forceinline__ Row<R> assemble_py(const Geo<R>& G, const SweepIO<F>& io, int ii, int jj) {
-  const int c0 = G.at(ii, jj);
-  const R ai = ld<R>(io.au, G.at(ii - 1, jj)), ad = ld<R>(io.au, c0), as = ld<R>(io.av, G.at(ii, jj - 1)),
-          an = ld<R>(io.av, c0);
-  const R dyp = G.met(M_DYP, jj), dxp = G.met(M_DXP, ii);
+template <bool FAST, class R, class V>
+__device__ __forceinline__ Row<R> assemble_py(const Geo<R>& G, const V& c) {
+  const R ai = c.au(-1, 0), ad = c.au(0, 0), as = c.av(0, -1), an = c.av(0, 0);
+  const R dyp = c.my(M_DYP, 0), dxp = c.mx(M_DXP, 0);
   const R AI = -qdiv<FAST>(dyp * dyp, ai);
   const R AD = -qdiv<FAST>(dyp * dyp, ad);
   Row<R> r;
   r.a = -qdiv<FAST>(dxp * dxp, as);
   r.c = -qdiv<FAST>(dxp * dxp, an);
   r.b = qdiv<FAST>(-AI - AD - r.a - r.c, G.rel_pres, G.inv_rel_pres);
-  const R bo = R(mass_residual(G, io, ii, jj));
-  r.d = -AI * pc_at<R>(io, G, ii - 1, jj) - AD * pc_at<R>(io, G, ii + 1, jj) + bo +
-        (R(1) - G.rel_pres) * r.b * pc_at<R>(io, G, ii, jj);
+  const R bo = R(mass_residual(G, c));
+  r.d = -AI * c.in(-1, 0) - AD * c.in(1, 0) + bo + (R(1) - G.rel_pres) * r.b * c.in(0, 0);
   return r;
 }
 
 // ---------------------------------------------------------------------------
-// u residual (residuo_u, source/mod_ec_momento.f90:1107-1266).  With a
-// uniform gamma the reference's different south numerator (:1208) has the
-// same value as in ensambla_velu_x, so it shares the u tables.
+// u residual (residuo_u, source/mod_ec_momento.f90:1107-1266) of the cell's
+// u (`in` of the view).  With a uniform gamma the reference's different south
+// numerator (:1208) has the same value as in ensambla_velu_x, so it shares
+// the u coefficients.
 // ---------------------------------------------------------------------------
-// T_WRITTEN: T was written earlier in the calling kernel (a fused T-x sweep
-// evaluating the residual of the rows it solved), so it is read with
-// ordinary coherent loads instead of the read-only path.
+template <bool FAST, class R, class V>
+__device__ __forceinline__ R residual_u(const Geo<R>& G, const V& c) {
+  R AI, AD, BS, BN, dxu, dyu, temp_int;
+  u_parts<FAST>(G, c, AI, AD, BS, BN, dxu, dyu, temp_int);
+  AI = -AI; AD = -AD; BS = -BS; BN = -BN;
+  const R fl = c.flin(), fc = c.fcon();
+  R AC = AI + AD + BS + BN - dxu * dyu * fl + qdiv<FAST>(dxu * dyu, G.dt, G.inv_dt);
+  return AI * c.in(-1, 0) - AC * c.in(0, 0) + AD * c.in(1, 0) + BS * c.in(0, -1) + BN * c.in(0, 1) -
+         dxu * dyu * G.Ri * temp_int + dxu * dyu * fc + qdiv<FAST>(dxu * dyu * c.u_ant(), G.dt, G.inv_dt) +
+         (c.p(0, 0) - c.p(1, 0)) * dyu;
+}
+// the same from field pointers; T_WRITTEN: T was written earlier in the
+// calling kernel (a fused T-x sweep evaluating the residual of the rows it
+// solved), so it is read with ordinary coherent loads
+template <class R, bool T_WRITTEN>
+struct ResidView : CellView<R, R> {
+  __device__ __forceinline__ R T(int di, int dj) const {
+    const int k = this->at(di, dj);
+    return T_WRITTEN ? this->io.T[k] : ldg(this->io.T, k);
+  }
+};
 template <bool FAST, class R, bool T_WRITTEN = false>
 __device__ __forceinline__ R residual_u(const Geo<R>& G, const R* u, const R* v, const R* T, const R* p,
                                         const R* u_ant, const R* fcon, const R* flin, int ii, int jj) {
-  const R fexu_i = G.met(M_FEXU, ii), fexu_m = G.met(M_FEXU, ii - 1);
-  const R fexp_i = G.met(M_FEXP, ii);
-  R ud = fexu_i * ldg(u, G.at(ii + 1, jj)) + (R(1) - fexu_i) * ldg(u, G.at(ii, jj));
-  R ui = fexu_m * ldg(u, G.at(ii, jj)) + (R(1) - fexu_m) * ldg(u, G.at(ii - 1, jj));
-  R vn = fexp_i * ldg(v, G.at(ii + 1, jj)) + (R(1) - fexp_i) * ldg(v, G.at(ii, jj));
-  R vs = fexp_i * ldg(v, G.at(ii + 1, jj - 1)) + (R(1) - fexp_i) * ldg(v, G.at(ii, jj - 1));
-  const R g = G.gm;
-  R gamman, gammas, rgn = R(0), rgs = R(0);
-  if constexpr (FAST) {
-    // the face diffusivity is the harmonic mean of a uniform gamma_momen
-    // (ixb_params holds one value), i.e. gamma_momen up to rounding: its
-    // reciprocal is the scalar 1/gamma_momen, no table load
-    rgn = rgs = G.inv_gm;
-    gamman = gammas = R(0);
-  } else {
-    gamman = G.t(T_GU, ii, jj);
-    gammas = G.t(T_GU, ii, jj - 1);
-  }
-  R di = G.met(M_DXP, ii), dd = G.met(M_DXP, ii + 1), ds = G.met(M_DYV, jj - 1), dn = G.met(M_DYV, jj);
-  const R dxu = G.met(M_DXU, ii), dyu = G.met(M_DYU, jj);
-  const int c0 = G.at(ii, jj);
-  const R t_e = T_WRITTEN ? T[G.at(ii + 1, jj)] : ldg(T, G.at(ii + 1, jj));
-  const R t_c = T_WRITTEN ? T[c0] : ldg(T, c0);
-  R temp_int = fexp_i * t_e + (R(1) - fexp_i) * t_c;
-  R AI = (cond_t<FAST>(G, T_CU1, ii, jj, dyu, M_GRDXP, ii) * plaw(qdiv<FAST>(ui * di, g, G.inv_gm)) + dmax0(ui * dyu));
-  R AD = (cond_t<FAST>(G, T_CU1, ii + 1, jj, dyu, M_GRDXP, ii + 1) * plaw(qdiv<FAST>(ud * dd, g, G.inv_gm)) +
-          dmax0(-ud * dyu));
-  R BS = (cond_t<FAST>(G, T_CU2, ii, jj - 1, dxu, M_GRDYV, jj - 1) * plaw(qdiv<FAST>(vs * ds, gammas, rgs)) +
-          dmax0(vs * dxu));
-  R BN = (cond_t<FAST>(G, T_CU2, ii, jj, dxu, M_GRDYV, jj) * plaw(qdiv<FAST>(vn * dn, gamman, rgn)) +
-          dmax0(-vn * dxu));
-  const R fl = flin ? ldg(flin, c0) : R(0);
-  const R fc = fcon ? ldg(fcon, c0) : R(0);
-  R AC = AI + AD + BS + BN - dxu * dyu * fl + qdiv<FAST>(dxu * dyu, G.dt, G.inv_dt);
-  return AI * ldg(u, G.at(ii - 1, jj)) - AC * ldg(u, c0) + AD * ldg(u, G.at(ii + 1, jj)) +
-         BS * ldg(u, G.at(ii, jj - 1)) + BN * ldg(u, G.at(ii, jj + 1)) - dxu * dyu * G.Ri * temp_int +
-         dxu * dyu * fc + qdiv<FAST>(dxu * dyu * ldg(u_ant, c0), G.dt, G.inv_dt) +
-         (ldg(p, c0) - ldg(p, G.at(ii + 1, jj))) * dyu;
+  SweepIO<R> io{};
+  io.in = u; io.v = v; io.T = T; io.p = p; io.u_ant = u_ant; io.fcon = fcon; io.flin = flin;
+  return residual_u<FAST>(G, ResidView<R, T_WRITTEN>{{G, io, ii, jj}});
 }
 
 // ---------------------------------------------------------------------------
@@ -547,16 +540,25 @@ __device__ void thomas_exact(R* sa, R* sb, R* sc, R* sd, int n, int m, int mp) {
 // rows a, c, d).
 __host__ __device__ constexpr size_t line_smem_elems(int G, int mp) { return (size_t)4 * G * mp + (size_t)12 * G; }
 
+// Barrier `id` (1..15) of n threads (whole warps); returns whether q holds in
+// any of them.
+__device__ __forceinline__ bool barrier_or(int id, int n, bool q) {
+  int r;
+  asm volatile(
+      "{ .reg .pred p, a; setp.ne.s32 a, %3, 0; barrier.cta.red.or.pred p, %1, %2, a; selp.s32 %0, 1, 0, p; }"
+      : "=r"(r)
+      : "r"(id), "r"(n), "r"((int)q)
+      : "memory");
+  return r != 0;
+}
+
 // Barrier of the G threads that solve one line when a CTA holds TL lines of
 // whole warps (a named barrier per line, so lines do not wait for each
 // other), else of the whole CTA.
 template <int G, int TL>
-__device__ __forceinline__ void line_sync() {
-  if constexpr (TL > 1 && TL <= 8 && G % 32 == 0) {
-    asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)threadIdx.x / G), "r"(G) : "memory");
-  } else {
-    __syncthreads();
-  }
+__device__ __forceinline__ bool line_sync(bool q) {
+  if constexpr (TL > 1 && TL <= 8 && G % 32 == 0) return barrier_or(1 + (int)threadIdx.x / G, G, q);
+  else return __syncthreads_or(q);
 }
 
 // One parallel-cyclic-reduction step of a row with unit diagonal,
@@ -586,10 +588,20 @@ __device__ __forceinline__ void pcr_row(R& A, R& C, R& D, R lA, R lC, R lD, R hA
 //    so the form whose rounding they had is kept).
 // The textbook form (rows re-read every step) moved 24 words.
 //
+// Each step squares the couplings (they are below one in diagonally dominant
+// rows), and once every coupling of the line is below pcr_tiny the remaining
+// steps could only add products too small to be seen next to the unit
+// diagonal: the barrier that publishes the rows also tells whether any is
+// larger, and the loop ends when none is.  (Relaxed transport lines end after
+// four to six of eight steps; lines that do not decay take them all.)
+//
 // N elements per array in `red` (9N used with HALF, else 12N); the rows of
 // neighbouring chunks are TS elements apart.  All threads of the line(s)
-// call `sync`, which orders shared memory between them; `active` false:
-// barriers only.
+// call `sync(q)`, which orders shared memory between them and returns
+// whether q holds in any of them; `active` false: barriers only.
+template <class R>
+__device__ __forceinline__ R pcr_tiny() { return sizeof(R) == 8 ? R(3.5e-18) : R(5.7e-14); }  // 2^-58, 2^-44
+
 template <class R, bool HALF, class Sync>
 __device__ __forceinline__ void reduced_pcr(R* red, const int N, const int TS, const int G, const int pos,
                                             const int k, const bool active, R eA, R eC, R eD, R oA, R oC, R oD,
@@ -597,7 +609,7 @@ __device__ __forceinline__ void reduced_pcr(R* red, const int N, const int TS, c
   const bool lo1 = active && k > 0, hi1 = active && k + 1 < G;
   if constexpr (HALF) {
     if (active) { red[pos] = eA; red[N + pos] = eC; red[2 * N + pos] = eD; }
-    sync();
+    sync(false);
     R hA = R(0), hC = R(0), hD = R(0);
     if (hi1) { hA = red[pos + TS]; hC = red[N + pos + TS]; hD = red[2 * N + pos + TS]; }
     pcr_row(oA, oC, oD, eA, eC, eD, hA, hC, hD);
@@ -606,7 +618,7 @@ __device__ __forceinline__ void reduced_pcr(R* red, const int N, const int TS, c
 #pragma unroll 1
     for (int h = 1; h < G; h <<= 1) {
       if (active) { cur[pos] = oA; cur[N + pos] = oC; cur[2 * N + pos] = oD; }
-      sync();
+      if (!sync(active && fmaxT(fabsT(oA), fabsT(oC)) > pcr_tiny<R>())) break;
       R lA = R(0), lC = R(0), lD = R(0);
       hA = hC = hD = R(0);
       if (active && k >= h) {
@@ -621,8 +633,8 @@ __device__ __forceinline__ void reduced_pcr(R* red, const int N, const int TS, c
       R* t = cur; cur = nxt; nxt = t;
     }
     xl = oD;
-    if (active) cur[pos] = xl;
-    sync();
+    if (active) cur[pos] = xl;  // a buffer nobody reads any more: no step follows the one it was published for
+    sync(false);
     const R xm = lo1 ? cur[pos - TS] : R(0);
     x0 = fmaT(-eC, xl, fmaT(-eA, xm, eD));
   } else {
@@ -632,7 +644,7 @@ __device__ __forceinline__ void reduced_pcr(R* red, const int N, const int TS, c
       cur[pos] = eA; cur[N + pos] = eC; cur[2 * N + pos] = eD;
       cur[3 * N + pos] = oA; cur[4 * N + pos] = oC; cur[5 * N + pos] = oD;
     }
-    sync();
+    sync(false);
     {
       R lA = R(0), lC = R(0), lD = R(0), hA = R(0), hC = R(0), hD = R(0);
       if (lo1) { lA = cur[3 * N + pos - TS]; lC = cur[4 * N + pos - TS]; lD = cur[5 * N + pos - TS]; }
@@ -648,7 +660,8 @@ __device__ __forceinline__ void reduced_pcr(R* red, const int N, const int TS, c
         cur[pos] = eA; cur[N + pos] = eC; cur[2 * N + pos] = eD;
         cur[3 * N + pos] = oA; cur[4 * N + pos] = oC; cur[5 * N + pos] = oD;
       }
-      sync();
+      const R big = fmaxT(fmaxT(fabsT(eA), fabsT(eC)), fmaxT(fabsT(oA), fabsT(oC)));
+      if (!sync(active && big > pcr_tiny<R>())) break;
       R lA = R(0), lC = R(0), lD = R(0), hA = R(0), hC = R(0), hD = R(0);
       R mA = R(0), mC = R(0), mD = R(0), gA = R(0), gC = R(0), gD = R(0);
       if (active && k >= h) {
@@ -741,7 +754,7 @@ __device__ __forceinline__ void chunk_solve(R* line, int m, int mp, bool active)
     }
     ch.eliminate();
     reduced_pcr<R, HALF>(red, G, 1, G, k, k, active, ch.eA, ch.eC, ch.eD, ch.oA, ch.oC, ch.oD, x0, xl,
-                         [] { line_sync<G, TL>(); });
+                         [](bool q) { return line_sync<G, TL>(q); });
     if (active) {
       ch.substitute(x0, xl);
 #pragma unroll
@@ -777,7 +790,7 @@ __device__ __forceinline__ void chunk_solve(R* line, int m, int mp, bool active)
       eA = a0 * r0; eC = -c0 * cn * r0; eD = fmaT(-c0, dn, d0) * r0;
       oA = ap; oC = cp; oD = dp;
     }
-    reduced_pcr<R, HALF>(red, G, 1, G, k, k, active, eA, eC, eD, oA, oC, oD, x0, xl, [] { line_sync<G, TL>(); });
+    reduced_pcr<R, HALF>(red, G, 1, G, k, k, active, eA, eC, eD, oA, oC, oD, x0, xl, [](bool q) { return line_sync<G, TL>(q); });
     if (active) {
       d[0] = x0;
       for (int i = 1; i < m - 1; ++i) d[i] = fmaT(-c[i], xl, fmaT(-a[i], x0, d[i]));

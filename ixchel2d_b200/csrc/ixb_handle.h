@@ -24,6 +24,8 @@ struct Ctl {
   int exit_code, status;
   long long n_simple, n_momen, n_pres, n_ener;
   double err_u, err_p, err_t, maxbo, residuo;
+  // resident loop (ixb_loop.cuh): the run is over; a bounded grid wait ran out
+  int stop, abort_flag, mon_over;
   // Nusselt monitor (ixb_simple_converge): inputs
   int mon_vertical, mon_k0, mon_k1, mon_wall;
   long long mon_max_iters;
@@ -31,6 +33,8 @@ struct Ctl {
   // Nusselt monitor: state
   long long mon_evals;
   double mon_nu[2], mon_nu_prev, mon_dnu;
+  // arrivals of the resident loop's grid barrier, on a line of its own
+  alignas(128) unsigned bar;
 };
 
 // the SIMPLE loop graphs of a handle
@@ -98,6 +102,8 @@ struct ixb_handle {
   int use_graph = 1;
   int shape_tl[ixb::EQ_COUNT] = {};  // launch shape per sweep (0 = not chosen yet)
   int shape_g[ixb::EQ_COUNT] = {};
+  bool shape_set[ixb::EQ_COUNT] = {};  // set by the caller (ixb_set_sweep_shape): the loop keeps to the per-sweep kernels
+  bool coop = false;                   // the device takes cooperative launches
   int nsm = 148;
   // adjoint workspace (ixb_adjoint_energy), allocated on first use
   double* xfer = nullptr;  // seven host-shaped (column-major, unpadded) state arrays: the state transfers' staging, allocated on the first transfer

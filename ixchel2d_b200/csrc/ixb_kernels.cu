@@ -31,18 +31,24 @@ __global__ void table1d_kernel(Geo<R> G, R* met) {
     met[M_HXU * G.mstride + k] = h;
     met[M_RHXU * G.mstride + k] = R(1) / h;
     met[M_HRDXU * G.mstride + k] = ratio(h, G.met(M_DXU, k));
+    met[M_PHXU * G.mstride + k] = R(0.1) * G.met(M_DXU, k) / h;
   }
   if (k >= 1 && k <= G.nj) {
     const R h = hmean(ge, ge, G.met(M_FEYV, k));
     met[M_HYV * G.mstride + k] = h;
     met[M_RHYV * G.mstride + k] = R(1) / h;
     met[M_HRDYV * G.mstride + k] = ratio(h, G.met(M_DYV, k));
+    met[M_PHYV * G.mstride + k] = R(0.1) * G.met(M_DYV, k) / h;
   }
   if (k >= 1 && k < G.mstride) {
     met[M_GRDXP * G.mstride + k] = ratio(g, G.met(M_DXP, k));
     met[M_GRDYV * G.mstride + k] = ratio(g, G.met(M_DYV, k));
     met[M_GRDXU * G.mstride + k] = ratio(g, G.met(M_DXU, k));
     met[M_GRDYP * G.mstride + k] = ratio(g, G.met(M_DYP, k));
+    met[M_PEXP * G.mstride + k] = R(0.1) * G.met(M_DXP, k) / g;
+    met[M_PEYV * G.mstride + k] = R(0.1) * G.met(M_DYV, k) / g;
+    met[M_PEXU * G.mstride + k] = R(0.1) * G.met(M_DXU, k) / g;
+    met[M_PEYP * G.mstride + k] = R(0.1) * G.met(M_DYP, k) / g;
   }
 }
 
@@ -236,9 +242,10 @@ constexpr int kNuThreads = 256;
 __global__ void __launch_bounds__(kNuThreads)
     nusselt_kernel(const Geo<double> G, const double* __restrict__ T, const double* __restrict__ xp,
                    const double* __restrict__ yp, int vertical, int k0, int k1, double* __restrict__ out2, Ctl* mon,
-                   cudaGraphConditionalHandle cond) {
+                   int in_graph, cudaGraphConditionalHandle cond) {
   __shared__ double terms[2][3][kNuThreads];
   if (mon) {
+    if (!in_graph && mon->mon_over) return;  // launched ahead of the block that ended the run
     vertical = mon->mon_vertical;
     k0 = mon->mon_k0;
     k1 = mon->mon_k1;
@@ -272,7 +279,7 @@ __global__ void __launch_bounds__(kNuThreads)
   }
   if (tid == 0 || tid == 32) out2[my_wall] = -acc;
   __syncthreads();
-  if (mon && tid == 0) ctl_monitor_step(mon, out2, cond);
+  if (mon && tid == 0) ctl_monitor_step(mon, out2, in_graph != 0, cond);
 }
 
 // ---------------------------------------------------------------------------
@@ -441,9 +448,9 @@ cudaError_t launch_residual_f64(const Geo<double>& G, const double* u, const dou
 }
 
 cudaError_t launch_nusselt_f64(const Geo<double>& G, const double* T, const double* xp, const double* yp,
-                               int vertical, int k0, int k1, double* out2, cudaStream_t st, Ctl* mon,
+                               int vertical, int k0, int k1, double* out2, cudaStream_t st, Ctl* mon, int in_graph,
                                cudaGraphConditionalHandle cond) {
-  nusselt_kernel<<<1, kNuThreads, 0, st>>>(G, T, xp, yp, vertical, k0, k1, out2, mon, cond);
+  nusselt_kernel<<<1, kNuThreads, 0, st>>>(G, T, xp, yp, vertical, k0, k1, out2, mon, in_graph, cond);
   return cudaGetLastError();
 }
 

@@ -29,41 +29,22 @@ namespace ixb {
 // per-equation assembly dispatch
 // ---------------------------------------------------------------------------
 
-// Row of cell (ii,jj); the side outputs (au, av, b_o and the b_o norm) are
-// written only when `keep` is set.
-template <class R, int EQ, bool FAST, class F>
-__device__ __forceinline__ Row<R> assemble_cell(const Geo<R>& G, const SweepIO<F>& io, int ii, int jj,
-                                                double& acc_bo, bool keep) {
-  if constexpr (EQ == EQ_UY) {
-    return assemble_uy<FAST>(G, io, ii, jj);
-  } else if constexpr (EQ == EQ_UX) {
-    R au;
-    Row<R> r = assemble_ux<FAST>(G, io, ii, jj, au);
-    if (keep) io.aux[G.at(ii, jj)] = F(au);
-    return r;
-  } else if constexpr (EQ == EQ_VY) {
-    return assemble_vy<FAST>(G, io, ii, jj);
-  } else if constexpr (EQ == EQ_VX) {
-    R av;
-    Row<R> r = assemble_vx<FAST>(G, io, ii, jj, av);
-    if (keep) io.aux[G.at(ii, jj)] = F(av);
-    return r;
-  } else if constexpr (EQ == EQ_PY) {
-    return assemble_py<FAST>(G, io, ii, jj);
-  } else if constexpr (EQ == EQ_PX) {
-    F bo;
-    Row<R> r = assemble_px<FAST>(G, io, ii, jj, bo);
-    if (keep) {
-      io.aux[G.at(ii, jj)] = bo;
-      acc_bo += (double)bo * (double)bo;
-    }
-    return r;
-  } else if constexpr (EQ == EQ_TY) {
-    return assemble_ty<FAST>(G, io, ii, jj);
-  } else {
-    return assemble_tx<FAST>(G, io, ii, jj);
-  }
+// Row of the view's cell; aux: the value of its side output (au, av, b_o).
+template <int EQ, bool FAST, class R, class V>
+__device__ __forceinline__ Row<R> assemble_cell(const Geo<R>& G, const V& c, double& aux) {
+  if constexpr (EQ == EQ_UY) return assemble_uy<FAST>(G, c);
+  else if constexpr (EQ == EQ_UX) return assemble_ux<FAST>(G, c, aux);
+  else if constexpr (EQ == EQ_VY) return assemble_vy<FAST>(G, c);
+  else if constexpr (EQ == EQ_VX) return assemble_vx<FAST>(G, c, aux);
+  else if constexpr (EQ == EQ_PY) return assemble_py<FAST>(G, c);
+  else if constexpr (EQ == EQ_PX) return assemble_px<FAST>(G, c, aux);
+  else if constexpr (EQ == EQ_TY) return assemble_ty<FAST>(G, c);
+  else return assemble_tx<FAST>(G, c);
 }
+
+// sweeps with a side output: au (u-x), av (v-x), b_o and its norm (p'-x)
+template <int EQ>
+struct EqHasAux { static constexpr bool value = EQ == EQ_UX || EQ == EQ_VX || EQ == EQ_PX; };
 
 // Boundary rows of impone_cond_frontera (source/mod_cond_frontera.f90:280-416):
 // first row of a line: diri (0,1,0|val), neum (0,-1,1|val);
@@ -87,22 +68,38 @@ __device__ __forceinline__ Row<R> bc_last_row(const BCEntry* t, int L) {
 // ---------------------------------------------------------------------------
 // assembly kernel
 // ---------------------------------------------------------------------------
-// Row of line L, position r (0-based along the line) of sweep EQ, or an
-// identity row outside the line.  Rows outside the interior are assembled
-// at the nearest interior cell and then replaced, so every load is in bounds
-// and no branch separates a thread's loads.
-template <int EQ, int SOLVER>
-__device__ __forceinline__ Row<double> staged_row(
-    const Geo<double>& Gm, const SweepIO<double>& io, int L, int r, int n, int line_lo,
-    int line_hi, bool valid, double& acc_bo) {
+// the row's right-hand side -> its binary64 residual at xm, x0, xp
+__device__ __forceinline__ void row_defect(Row<double>& row, double xm, double x0, double xp) {
+  double res = fma(-row.b, x0, row.d);
+  res = fma(-row.a, xm, res);
+  res = fma(-row.c, xp, res);
+  row.d = res;
+}
+// unit diagonal before the binary32 staging; the solution is unchanged (a
+// Newton-refined reciprocal: the scaled row is rounded to binary32)
+__device__ __forceinline__ void row_scale(Row<double>& row) {
+  const double sc = fast_rcp(row.b);
+  row.a *= sc;
+  row.c *= sc;
+  row.d *= sc;
+  row.b = 1.0;
+}
+
+// Row of line L, position r (0-based along the line) of sweep EQ.  Rows
+// outside the interior are assembled at the nearest interior cell and then
+// replaced, so every load is in bounds and no branch separates a thread's
+// loads.  Returns the row; aux: its side output, to be stored where
+// `interior` (1 <= r <= n-2 of a solved line).
+template <int EQ, int SOLVER, class F>
+__device__ __forceinline__ Row<double> sweep_row(const Geo<double>& Gm, const SweepIO<F>& io, int L, int r, int n,
+                                                 int line_lo, int line_hi, double& aux) {
   using ST = SweepTypes<SOLVER, EQ>;
   using A = double;
   constexpr bool X = EqIsX<EQ>::value;
   const int Lc = min(max(L, line_lo), line_hi);
   const int rc = min(max(r, 1), n - 2);
-  const bool interior = valid && r >= 1 && r <= n - 2;
-  Row<A> row = assemble_cell<A, EQ, SOLVER != IXB_SOLVER_EXACT>(Gm, io, X ? rc + 1 : Lc, X ? Lc : rc + 1, acc_bo,
-                                                                interior);
+  const CellView<A, F> cell{Gm, io, X ? rc + 1 : Lc, X ? Lc : rc + 1};
+  Row<A> row = assemble_cell<EQ, SOLVER != IXB_SOLVER_EXACT>(Gm, cell, aux);
   const Row<A> first = bc_first_row<A>(io.bc_first, Lc);
   const Row<A> last = bc_last_row<A>(io.bc_last, Lc);
   if (r == 0) row = first;
@@ -112,22 +109,26 @@ __device__ __forceinline__ Row<double> staged_row(
     const int rr = min(max(r, 0), n - 1);
     const int g = Gm.at(X ? rr + 1 : Lc, X ? Lc : rr + 1);
     const int step = X ? 1 : Gm.LD;
-    const double xm = __ldg(io.in + (rr > 0 ? g - step : g));
-    const double x0 = __ldg(io.in + g);
-    const double xp = __ldg(io.in + (rr < n - 1 ? g + step : g));
-    double res = fma(-row.b, x0, row.d);
-    res = fma(-row.a, xm, res);
-    res = fma(-row.c, xp, res);
-    row.d = res;
+    const double xm = ld<double>(io.in, rr > 0 ? g - step : g);
+    const double x0 = ld<double>(io.in, g);
+    const double xp = ld<double>(io.in, rr < n - 1 ? g + step : g);
+    row_defect(row, xm, x0, xp);
   }
-  if constexpr (ST::MIX) {
-    // unit diagonal before the binary32 staging; the solution is unchanged
-    // (a Newton-refined reciprocal: the scaled row is rounded to binary32)
-    const double sc = fast_rcp(row.b);
-    row.a *= sc;
-    row.c *= sc;
-    row.d *= sc;
-    row.b = 1.0;
+  if constexpr (ST::MIX) row_scale(row);
+  return row;
+}
+
+// sweep_row, its side output stored and added to the b_o norm.
+template <int EQ, int SOLVER>
+__device__ __forceinline__ Row<double> staged_row(const Geo<double>& Gm, const SweepIO<double>& io, int L, int r,
+                                                  int n, int line_lo, int line_hi, bool valid, double& acc_bo) {
+  double aux = 0.0;
+  const Row<double> row = sweep_row<EQ, SOLVER>(Gm, io, L, r, n, line_lo, line_hi, aux);
+  if constexpr (EqHasAux<EQ>::value) {
+    if (valid && r >= 1 && r <= n - 2) {
+      io.aux[EqIsX<EQ>::value ? Gm.at(r + 1, L) : Gm.at(L, r + 1)] = aux;
+      if (EQ == EQ_PX) acc_bo += aux * aux;
+    }
   }
   return row;
 }
@@ -321,7 +322,7 @@ __device__ __forceinline__ double fused_y_lines(typename SweepTypes<SOLVER, EQ>:
   ch.eliminate();
   S x0, xl;
   reduced_pcr<S, sizeof(S) == 8>(red, TL * G, TL, G, threadIdx.x, k, active, ch.eA, ch.eC, ch.eD, ch.oA, ch.oC,
-                                 ch.oD, x0, xl, [] { __syncthreads(); });
+                                 ch.oD, x0, xl, [](bool q) { return (bool)__syncthreads_or(q); });
   ch.substitute(x0, xl);
   double acc = 0.0;
 #pragma unroll

@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(T) tri_stream_kernel(const R* a, const R* b, c
     ch.eliminate();
     R x0, xl;
     reduced_pcr<R, true>(red, T, 1, T, tid, tid, true, ch.eA, ch.eC, ch.eD, ch.oA, ch.oC, ch.oD, x0, xl,
-                         [] { __syncthreads(); });
+                         [](bool q) { return (bool)__syncthreads_or(q); });
     ch.substitute(x0, xl);
     // the previous solution must have left xbuf before it is overwritten
     if (tid == 0) bulk_store_wait_read();
@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(512) tri_cols_kernel(const R* a, const R* b, c
   ch.eliminate();
   R x0, xl;
   reduced_pcr<R, true>(red, W * G, W, G, threadIdx.x, k, active, ch.eA, ch.eC, ch.eD, ch.oA, ch.oC, ch.oD, x0, xl,
-                       [] { __syncthreads(); });
+                       [](bool q) { return (bool)__syncthreads_or(q); });
   ch.substitute(x0, xl);
 #pragma unroll
   for (int j = 0; j < M; ++j) {
