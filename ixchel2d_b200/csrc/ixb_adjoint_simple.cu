@@ -15,23 +15,30 @@
 //   s_bar += sum over rows r of  mu_r d(d_r)/ds - mu_r (x_{r-1} d(a_r)/ds
 //            + x_r d(b_r)/ds + x_{r+1} d(c_r)/ds)
 //   x_in_bar += lambda                       (on the unsolved lines)
-// The row's derivatives with respect to the ~10 stencil values it reads come
-// from evaluating the row once more in forward-mode dual numbers, one
-// derivative slot per stencil input, and the products with the weights
-// (-mu x, mu) are scattered to the stencil positions with atomic adds.  The
-// rows are restated here from ixb_device.cuh (the reference's formulas,
-// mod_ec_momento.f90:365-1098, :145-355, mod_ec_energia.f90:119-443) in a
-// form generic over the scalar type; the forward kernels are untouched.
-// The velocity/pressure update (main.f90:931-962) has a hand-written adjoint.
+// The row's derivatives are taken in reverse: for the weights (-mu x, mu) of
+// (a, b, c, d) the adjoints of the row's coefficients, face velocities and
+// stencil values follow by hand (about twice the row's own arithmetic, where
+// one dual number per stencil value took thirteen times it), and are added to
+// the stencil positions with atomic adds.  The rows are those of
+// ixb_device.cuh in the fast form (the reference's formulas,
+// mod_ec_momento.f90:365-1098, :145-355, mod_ec_energia.f90:119-443).  The
+// velocity/pressure update (main.f90:931-962) has a hand-written adjoint.
 //
-// Forward: K outer iterations phase by phase (ixb_phase: the same kernels as
-// the graph; the pressure loop starts from p' = 0), the state saved every C
-// iterations.  Reverse, segment by segment from the last: restore the
-// segment's checkpoint, recompute its iterations storing the state after
-// every phase, then reverse the phases of each iteration from the last.
+// A reversed sweep is one kernel: a CTA evaluates its lines' rows, places
+// them transposed in shared memory, solves, and scatters.  As row, transpose,
+// line-solve and scatter kernels it was 44 launches per reversed iteration
+// instead of 9, and bound by them up to 256x256 (128x128, 30 iterations, a
+// checkpoint every 10: 20.3 ms per gradient then).
+//
+// Forward: K outer iterations (the library's loop, one pass of each equation),
+// the state saved every C iterations.  Reverse, segment by segment from the
+// last: restore the segment's checkpoint, recompute its iterations sweep by
+// sweep, each writing its field of the store directly, then reverse the
+// phases of each iteration from the last.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <utility>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -43,239 +50,15 @@ namespace ixb {
 namespace {
 
 // ---------------------------------------------------------------------------
-// forward-mode dual numbers with N derivative slots
-// ---------------------------------------------------------------------------
-template <int N>
-struct Dual {
-  double v;
-  double d[N];
-};
-
-template <int N>
-__device__ __forceinline__ Dual<N> cst(double x) {
-  Dual<N> r;
-  r.v = x;
-#pragma unroll
-  for (int k = 0; k < N; ++k) r.d[k] = 0.0;
-  return r;
-}
-template <int N>
-__device__ __forceinline__ Dual<N> seed(double x, int slot) {
-  Dual<N> r = cst<N>(x);
-  r.d[slot] = 1.0;
-  return r;
-}
-template <int N>
-__device__ __forceinline__ Dual<N> operator+(const Dual<N>& a, const Dual<N>& b) {
-  Dual<N> r;
-  r.v = a.v + b.v;
-#pragma unroll
-  for (int k = 0; k < N; ++k) r.d[k] = a.d[k] + b.d[k];
-  return r;
-}
-template <int N>
-__device__ __forceinline__ Dual<N> operator-(const Dual<N>& a, const Dual<N>& b) {
-  Dual<N> r;
-  r.v = a.v - b.v;
-#pragma unroll
-  for (int k = 0; k < N; ++k) r.d[k] = a.d[k] - b.d[k];
-  return r;
-}
-template <int N>
-__device__ __forceinline__ Dual<N> operator-(const Dual<N>& a) {
-  Dual<N> r;
-  r.v = -a.v;
-#pragma unroll
-  for (int k = 0; k < N; ++k) r.d[k] = -a.d[k];
-  return r;
-}
-template <int N>
-__device__ __forceinline__ Dual<N> operator*(const Dual<N>& a, const Dual<N>& b) {
-  Dual<N> r;
-  r.v = a.v * b.v;
-#pragma unroll
-  for (int k = 0; k < N; ++k) r.d[k] = a.d[k] * b.v + a.v * b.d[k];
-  return r;
-}
-template <int N>
-__device__ __forceinline__ Dual<N> operator*(const Dual<N>& a, double s) {
-  Dual<N> r;
-  r.v = a.v * s;
-#pragma unroll
-  for (int k = 0; k < N; ++k) r.d[k] = a.d[k] * s;
-  return r;
-}
-template <int N>
-__device__ __forceinline__ Dual<N> operator*(double s, const Dual<N>& a) { return a * s; }
-template <int N>
-__device__ __forceinline__ Dual<N> operator+(const Dual<N>& a, double s) {
-  Dual<N> r = a;
-  r.v += s;
-  return r;
-}
-template <int N>
-__device__ __forceinline__ Dual<N> operator/(const Dual<N>& a, const Dual<N>& b) {
-  Dual<N> r;
-  const double ib = 1.0 / b.v;
-  r.v = a.v * ib;
-#pragma unroll
-  for (int k = 0; k < N; ++k) r.d[k] = (a.d[k] - r.v * b.d[k]) * ib;
-  return r;
-}
-template <int N>
-__device__ __forceinline__ Dual<N> operator/(const Dual<N>& a, double s) { return a * (1.0 / s); }
-template <int N>
-__device__ __forceinline__ Dual<N> operator/(double s, const Dual<N>& b) { return cst<N>(s) / b; }
-
-// |x| and DMAX1(0, x) on plain doubles and on dual numbers
-__device__ __forceinline__ double gabs(double x) { return fabs(x); }
-template <int N>
-__device__ __forceinline__ Dual<N> gabs(const Dual<N>& x) { return x.v < 0.0 ? -x : x; }
-__device__ __forceinline__ double gpos(double x) { return x > 0.0 ? x : 0.0; }
-template <int N>
-__device__ __forceinline__ Dual<N> gpos(const Dual<N>& x) { return x.v > 0.0 ? x : cst<N>(0.0); }
-
-// DMAX1(0, (1 - 0.1|P|)**5) and DMAX1(0, x)
-template <class S>
-__device__ __forceinline__ S aplaw(const S& pe) {
-  const S t = 1.0 - 0.1 * gabs(pe);
-  const S t2 = t * t;
-  return gpos(t * (t2 * t2));
-}
-template <int N>
-__device__ __forceinline__ Dual<N> operator-(double s, const Dual<N>& a) {
-  Dual<N> r = -a;
-  r.v += s;
-  return r;
-}
-template <int N>
-__device__ __forceinline__ Dual<N> operator-(const Dual<N>& a, double s) {
-  Dual<N> r = a;
-  r.v -= s;
-  return r;
-}
-template <int N>
-__device__ __forceinline__ Dual<N> operator+(double s, const Dual<N>& a) { return a + s; }
-
-// ---------------------------------------------------------------------------
-// the rows of the four equations, generic over the scalar type, from the
-// stencil values x[0..12] (layouts in kStencil below).  Constants (metrics,
-// mesh tables, u_ant / v_ant / T_ant, sources) are plain doubles.  The
-// exact (IEEE-division) forms of ixb_device.cuh.
-// ---------------------------------------------------------------------------
-constexpr int NS = 13;  // stencil inputs of a row (the energy rows use 9)
-
-template <class S>
-struct GRow {
-  S a, b, c, d;
-};
-
-// u momentum (ensambla_velu_x/_y, mod_ec_momento.f90:365-724) at (ii, jj)
-template <class S>
-__device__ GRow<S> row_u(const Geo<double>& G, const S* x, double u_ant, double fcon, double flin, int ii, int jj,
-                         bool xform, S* aux) {
-  const double fexu_i = G.met(M_FEXU, ii), fexu_m = G.met(M_FEXU, ii - 1), fexp_i = G.met(M_FEXP, ii);
-  const S ud = fexu_i * x[1] + (1.0 - fexu_i) * x[0];
-  const S ui = fexu_m * x[0] + (1.0 - fexu_m) * x[2];
-  const S vn = fexp_i * x[6] + (1.0 - fexp_i) * x[5];
-  const S vs = fexp_i * x[8] + (1.0 - fexp_i) * x[7];
-  const S tint = fexp_i * x[10] + (1.0 - fexp_i) * x[9];
-  const double g = G.gm, gamman = G.t(T_GU, ii, jj), gammas = G.t(T_GU, ii, jj - 1);
-  const double di = G.met(M_DXP, ii), dd = G.met(M_DXP, ii + 1), ds = G.met(M_DYV, jj - 1), dn = G.met(M_DYV, jj);
-  const double dx = G.met(M_DXU, ii), dy = G.met(M_DYU, jj);
-  const S AI = -(G.t(T_CU1, ii, jj) * aplaw(ui * di / g) + gpos(ui * dy));
-  const S AD = -(G.t(T_CU1, ii + 1, jj) * aplaw(ud * dd / g) + gpos(-ud * dy));
-  const S BS = -(G.t(T_CU2, ii, jj - 1) * aplaw(vs * ds / gammas) + gpos(vs * dx));
-  const S BN = -(G.t(T_CU2, ii, jj) * aplaw(vn * dn / gamman) + gpos(-vn * dx));
-  const double dxdy = dx * dy;
-  const S b = (-AI - AD - BS - BN - dxdy * flin + dxdy / G.dt) / G.rel_vel;
-  const S rest = -dxdy * G.Ri * tint + dxdy * fcon + dxdy * u_ant / G.dt + (x[11] - x[12]) * dy +
-                 b * (1.0 - G.rel_vel) * x[0];
-  GRow<S> r;
-  r.b = b;
-  if (xform) { r.a = AI; r.c = AD; r.d = -BS * x[3] - BN * x[4] + rest; }
-  else { r.a = BS; r.c = BN; r.d = -AI * x[2] - AD * x[1] + rest; }
-  if (aux) *aux = b * G.rel_vel;
-  return r;
-}
-
-// v momentum (ensambla_velv_x/_y, mod_ec_momento.f90:736-1098) at (ii, jj)
-template <class S>
-__device__ GRow<S> row_v(const Geo<double>& G, const S* x, double v_ant, double fcon, double flin, int ii, int jj,
-                         bool xform, S* aux) {
-  const double feyp_j = G.met(M_FEYP, jj), feyv_j = G.met(M_FEYV, jj), feyv_m = G.met(M_FEYV, jj - 1);
-  const S ud = feyp_j * x[6] + (1.0 - feyp_j) * x[5];
-  const S ui = feyp_j * x[8] + (1.0 - feyp_j) * x[7];
-  const S vn = feyv_j * x[1] + (1.0 - feyv_j) * x[0];
-  const S vs = feyv_m * x[0] + (1.0 - feyv_m) * x[2];
-  const S tint = feyp_j * x[10] + (1.0 - feyp_j) * x[9];
-  const double g = G.gm, gammad = G.t(T_GV, ii, jj), gammai = G.t(T_GV, ii - 1, jj);
-  const double di = G.met(M_DXU, ii - 1), dd = G.met(M_DXU, ii), ds = G.met(M_DYP, jj), dn = G.met(M_DYP, jj + 1);
-  const double dyv = G.met(M_DYV, jj), dxv = G.met(M_DXV, ii);
-  const S AI = -(G.t(T_CV1, ii, jj) * aplaw(ui * di / gammai) + gpos(ui * dyv));
-  const S AD = -(G.t(T_CV1, ii + 1, jj) * aplaw(ud * dd / gammad) + gpos(-ud * dyv));
-  const S BS = -(G.t(T_CV2, ii, jj) * aplaw(vs * ds / g) + gpos(vs * dxv));
-  const S BN = -(G.t(T_CV2, ii, jj + 1) * aplaw(vn * dn / g) + gpos(-vn * dxv));
-  const double dxdy = dxv * dyv;
-  const S b = (-AI - AD - BS - BN - dxdy * flin + dxdy / G.dt) / G.rel_vel;
-  const S rest = -dxdy * G.Riy * tint + dxdy * fcon + dxdy * v_ant / G.dt + (x[11] - x[12]) * dxv +
-                 b * (1.0 - G.rel_vel) * x[0];
-  GRow<S> r;
-  r.b = b;
-  if (xform) { r.a = AI; r.c = AD; r.d = -BS * x[2] - BN * x[1] + rest; }
-  else { r.a = BS; r.c = BN; r.d = -AI * x[3] - AD * x[4] + rest; }
-  if (aux) *aux = b * G.rel_vel;
-  return r;
-}
-
-// pressure correction (ensambla_corr_pres_x/_y, mod_ec_momento.f90:145-355) at (ii, jj)
-template <class S>
-__device__ GRow<S> row_p(const Geo<double>& G, const S* x, int ii, int jj, bool xform) {
-  const double dyp = G.met(M_DYP, jj), dxp = G.met(M_DXP, ii);
-  const S AI = -(dyp * dyp) / x[5], AD = -(dyp * dyp) / x[6];
-  const S BS = -(dxp * dxp) / x[7], BN = -(dxp * dxp) / x[8];
-  const S b = (-AI - AD - BS - BN) / G.rel_pres;
-  const S bo = (x[10] - x[9]) * dyp + (x[12] - x[11]) * dxp;
-  const S rest = bo + (1.0 - G.rel_pres) * b * x[0];
-  GRow<S> r;
-  r.b = b;
-  if (xform) { r.a = AI; r.c = AD; r.d = -BS * x[3] - BN * x[4] + rest; }
-  else { r.a = BS; r.c = BN; r.d = -AI * x[2] - AD * x[1] + rest; }
-  return r;
-}
-
-// energy (ensambla_energia_x/_y, mod_ec_energia.f90:119-443) at (ii, jj)
-template <class S>
-__device__ GRow<S> row_t(const Geo<double>& G, const S* x, double T_ant, double fcon, double flin, int ii, int jj,
-                         bool xform) {
-  const S ud = x[5], ui = x[6], vn = x[7], vs = x[8];
-  const double di = G.met(M_DXU, ii - 1), dd = G.met(M_DXU, ii), ds = G.met(M_DYV, jj - 1), dn = G.met(M_DYV, jj);
-  const double dyp = G.met(M_DYP, jj), dxp = G.met(M_DXP, ii);
-  const double gammad = G.met(M_HXU, ii), gammai = G.met(M_HXU, ii - 1);
-  const double gamman = G.met(M_HYV, jj), gammas = G.met(M_HYV, jj - 1);
-  const S AI = -(G.t(T_CT1, ii, jj) * aplaw(ui * di / gammai) + gpos(ui * dyp));
-  const S AD = -(G.t(T_CT1, ii + 1, jj) * aplaw(ud * dd / gammad) + gpos(-ud * dyp));
-  const S BS = -(G.t(T_CT2, ii, jj - 1) * aplaw(vs * ds / gammas) + gpos(vs * dxp));
-  const S BN = -(G.t(T_CT2, ii, jj) * aplaw(vn * dn / gamman) + gpos(-vn * dxp));
-  const double dxdy = dxp * dyp;
-  const S b = (-AI - AD - BS - BN - dxdy * flin + dxdy / G.dt) / G.rel_ener;
-  const S rest = dxdy * fcon + dxdy * T_ant / G.dt + b * (1.0 - G.rel_ener) * x[0];
-  GRow<S> r;
-  r.b = b;
-  if (xform) { r.a = AI; r.c = AD; r.d = -BS * x[3] - BN * x[4] + rest; }
-  else { r.a = BS; r.c = BN; r.d = -AI * x[2] - AD * x[1] + rest; }
-  return r;
-}
-
-// ---------------------------------------------------------------------------
 // stencils: the field and offset of every row input
 // ---------------------------------------------------------------------------
 enum Fld { F_U = 0, F_V, F_T, F_P, F_PC, F_AU, F_AV, F_COUNT, F_NONE = -1 };
 struct Tap {
   int f, di, dj;
 };
+constexpr int NS = 13;  // stencil inputs of a row (the energy rows use 9)
 // groups: 0 u rows, 1 v rows, 2 p' rows, 3 T rows
-__constant__ Tap kStencil[4][NS] = {
+constexpr Tap kStencil[4][NS] = {
     {{F_U, 0, 0}, {F_U, 1, 0}, {F_U, -1, 0}, {F_U, 0, -1}, {F_U, 0, 1}, {F_V, 0, 0}, {F_V, 1, 0}, {F_V, 0, -1},
      {F_V, 1, -1}, {F_T, 0, 0}, {F_T, 1, 0}, {F_P, 0, 0}, {F_P, 1, 0}},
     {{F_V, 0, 0}, {F_V, 0, 1}, {F_V, 0, -1}, {F_V, -1, 0}, {F_V, 1, 0}, {F_U, 0, 0}, {F_U, 0, 1}, {F_U, -1, 0},
@@ -284,8 +67,9 @@ __constant__ Tap kStencil[4][NS] = {
      {F_AV, 0, -1}, {F_AV, 0, 0}, {F_U, 0, 0}, {F_U, -1, 0}, {F_V, 0, 0}, {F_V, 0, -1}},
     {{F_T, 0, 0}, {F_T, 1, 0}, {F_T, -1, 0}, {F_T, 0, -1}, {F_T, 0, 1}, {F_U, 0, 0}, {F_U, -1, 0}, {F_V, 0, 0},
      {F_V, 0, -1}, {F_NONE, 0, 0}, {F_NONE, 0, 0}, {F_NONE, 0, 0}, {F_NONE, 0, 0}}};
-
-__host__ __device__ constexpr int eq_group(int eq) { return eq / 2 == 0 ? 0 : eq / 2 == 1 ? 1 : eq / 2 == 2 ? 2 : 3; }
+constexpr int eq_group(int eq) { return eq / 2; }
+// the swept field of a group
+constexpr int group_field(int g) { return g == 0 ? F_U : g == 1 ? F_V : g == 2 ? F_PC : F_T; }
 
 // The pre-sweep state a sweep's rows read, its constants and boundary rows.
 struct SweepState {
@@ -296,135 +80,284 @@ struct SweepState {
   const double* flin;
   const BCEntry* first;       // boundary rows (null: p', Dirichlet 0)
   const BCEntry* last;
-  int eq, n, line_lo, line_hi;
+  int eq, n, line_lo, line_hi, nfull;
 };
-
-template <class S>
-__device__ __forceinline__ GRow<S> eval_row(const Geo<double>& G, const SweepState& s, const S* x, int ii, int jj,
-                                            S* aux) {
-  const bool X = (s.eq & 1) != 0;
-  const int c0 = G.at(ii, jj);
-  const double fc = s.fcon ? s.fcon[c0] : 0.0, fl = s.flin ? s.flin[c0] : 0.0;
-  switch (eq_group(s.eq)) {
-    case 0: return row_u(G, x, s.ant[c0], fc, fl, ii, jj, X, aux);
-    case 1: return row_v(G, x, s.ant[c0], fc, fl, ii, jj, X, aux);
-    case 2: return row_p(G, x, ii, jj, X);
-    default: return row_t(G, x, s.ant[c0], fc, fl, ii, jj, X);
-  }
-}
-
-__device__ __forceinline__ void cell_of(const SweepState& s, int L, int r, int& ii, int& jj) {
-  if (s.eq & 1) { ii = r + 1; jj = L; }
-  else { ii = L; jj = r + 1; }
-}
-
-// Forward rows (a, b, c) of every solved line at the pre-sweep state,
-// contiguous per line: line L at (L - line_lo) * n.  Boundary rows follow
-// impone_cond_frontera (p' rows: Dirichlet 0).
-__global__ void adj_rows_kernel(const Geo<double> G, const SweepState s, double* __restrict__ fa,
-                                double* __restrict__ fb, double* __restrict__ fc) {
-  const int nl = s.line_hi - s.line_lo + 1;
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= nl * s.n) return;
-  const int li = idx / s.n, r = idx - li * s.n, L = s.line_lo + li;
-  double a, b, c;
-  if (r == 0 || r == s.n - 1) {
-    const BCEntry* t = r == 0 ? s.first : s.last;
-    const int type = t ? t[L].type : 1;
-    a = 0.0; b = 1.0; c = 0.0;
-    if (type == 2) {
-      if (r == 0) { b = -1.0; c = 1.0; }
-      else { a = -1.0; }
-    }
-  } else {
-    int ii, jj;
-    cell_of(s, L, r, ii, jj);
-    const int grp = eq_group(s.eq);
-    double x[NS];
-#pragma unroll
-    for (int k = 0; k < NS; ++k) {
-      const Tap tp = kStencil[grp][k];
-      x[k] = tp.f == F_NONE ? 0.0 : s.f[tp.f][G.at(ii + tp.di, jj + tp.dj)];
-    }
-    const GRow<double> row = eval_row<double>(G, s, x, ii, jj, nullptr);
-    a = row.a; b = row.b; c = row.c;
-  }
-  fa[idx] = a; fb[idx] = b; fc[idx] = c;
-}
-
-// Transposed rows (a'_r = c_{r-1}, b'_r = b_r, c'_r = a_{r+1}) with right-hand
-// side lambda (the adjoint of the swept field after the sweep); the adjoint
-// of the solved lines is then cleared (their x_in reaches x_out only through
-// the rows, whose contributions adj_jac_kernel adds).
-__global__ void adj_transpose_kernel(const Geo<double> G, const SweepState s, const double* __restrict__ fa,
-                                     const double* __restrict__ fb, const double* __restrict__ fc,
-                                     double* __restrict__ lam, double* __restrict__ ta, double* __restrict__ tb,
-                                     double* __restrict__ tc, double* __restrict__ td) {
-  const int nl = s.line_hi - s.line_lo + 1;
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= nl * s.n) return;
-  const int li = idx / s.n, r = idx - li * s.n, L = s.line_lo + li;
-  ta[idx] = r > 0 ? fc[idx - 1] : 0.0;
-  tb[idx] = fb[idx];
-  tc[idx] = r < s.n - 1 ? fa[idx + 1] : 0.0;
-  int ii, jj;
-  cell_of(s, L, r, ii, jj);
-  const int c0 = G.at(ii, jj);
-  td[idx] = lam[c0];
-  lam[c0] = 0.0;
-}
 
 struct AdjFields {
   double* f[F_COUNT];  // adjoints of u, v, T, p, p', au, av (field layout)
 };
 
-// Contributions of every interior row of the solved lines to the adjoints of
-// the stencil values it read: with mu_r from the transposed solve and x the
-// swept field after the sweep, the weights of (a, b, c, d) are
-// (-mu_r x_{r-1}, -mu_r x_r, -mu_r x_{r+1}, mu_r); aux_bar (u-x, v-x) adds
-// au_bar * rel_vel to b's weight (au = b rel_vel).
-__global__ void __launch_bounds__(128) adj_jac_kernel(const Geo<double> G, const SweepState s,
-                                                      const double* __restrict__ mu, const double* aux_bar,
-                                                      AdjFields adj) {
-  const int nl = s.line_hi - s.line_lo + 1, rows = s.n - 2;
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= nl * rows) return;
-  const int li = idx / rows, r = 1 + idx % rows, L = s.line_lo + li;
-  int ii, jj, im, jm, ip, jp;
-  cell_of(s, L, r, ii, jj);
-  cell_of(s, L, r - 1, im, jm);
-  cell_of(s, L, r + 1, ip, jp);
-  const double m0 = mu[(size_t)li * s.n + r];
-  const double wa = -m0 * s.x_out[G.at(im, jm)];
-  double wb = -m0 * s.x_out[G.at(ii, jj)];
-  const double wc = -m0 * s.x_out[G.at(ip, jp)];
-  const double wd = m0;
-  if (aux_bar) wb += aux_bar[G.at(ii, jj)] * G.rel_vel;
-  if (wa == 0.0 && wb == 0.0 && wc == 0.0 && wd == 0.0) return;
-  const int grp = eq_group(s.eq);
-  Dual<NS> x[NS];
-#pragma unroll
-  for (int k = 0; k < NS; ++k) {
-    const Tap tp = kStencil[grp][k];
-    x[k] = tp.f == F_NONE ? cst<NS>(0.0) : seed<NS>(s.f[tp.f][G.at(ii + tp.di, jj + tp.dj)], k);
+// The coefficients of a row (AI, AD, BS, BN negative, b the relaxed diagonal)
+// and, with the face velocities (ui, ud, vs, vn) or au, av (p'), the
+// derivative of each coefficient by its own face value.
+struct Links {
+  double AI, AD, BS, BN, b;
+  double dI, dD, dS, dN;
+  double dx, dy;  // the cell's widths
+};
+
+// Coefficient -(cond max(0, 1 - |vel| m)^5 + max(0, vel w)) and its derivative
+// by vel; at the kinks of |.| and max the branch taken counts.
+__device__ __forceinline__ void link_d(double cond, double m, double vel, double w, double& val, double& der) {
+  const double t = fmax(0.0, fma(-fabs(vel), m, 1.0)), t2 = t * t, t4 = t2 * t2;
+  const bool up = vel * w > 0.0;
+  val = -fma(cond, t * t4, up ? vel * w : 0.0);
+  const double dl = 5.0 * cond * t4 * m;
+  der = (vel < 0.0 ? -dl : dl) - (up ? w : 0.0);
+}
+
+template <int GRP>
+__device__ __forceinline__ Links links(const Geo<double>& G, const double (&x)[NS], double flin, int ii, int jj) {
+  Links k;
+  if constexpr (GRP == 0) {
+    const double fi = G.met(M_FEXU, ii), fm = G.met(M_FEXU, ii - 1), fp = G.met(M_FEXP, ii);
+    k.dx = G.met(M_DXU, ii);
+    k.dy = G.met(M_DYU, jj);
+    const double ud = fi * x[1] + (1.0 - fi) * x[0], ui = fm * x[0] + (1.0 - fm) * x[2];
+    const double vn = fp * x[6] + (1.0 - fp) * x[5], vs = fp * x[8] + (1.0 - fp) * x[7];
+    link_d(k.dy * G.met(M_GRDXP, ii), G.met(M_PEXP, ii), ui, k.dy, k.AI, k.dI);
+    link_d(k.dy * G.met(M_GRDXP, ii + 1), G.met(M_PEXP, ii + 1), ud, -k.dy, k.AD, k.dD);
+    link_d(k.dx * G.met(M_GRDYV, jj - 1), G.met(M_PEYV, jj - 1), vs, k.dx, k.BS, k.dS);
+    link_d(k.dx * G.met(M_GRDYV, jj), G.met(M_PEYV, jj), vn, -k.dx, k.BN, k.dN);
+  } else if constexpr (GRP == 1) {
+    const double fp = G.met(M_FEYP, jj), fj = G.met(M_FEYV, jj), fm = G.met(M_FEYV, jj - 1);
+    k.dx = G.met(M_DXV, ii);
+    k.dy = G.met(M_DYV, jj);
+    const double ud = fp * x[6] + (1.0 - fp) * x[5], ui = fp * x[8] + (1.0 - fp) * x[7];
+    const double vn = fj * x[1] + (1.0 - fj) * x[0], vs = fm * x[0] + (1.0 - fm) * x[2];
+    link_d(k.dy * G.met(M_GRDXU, ii - 1), G.met(M_PEXU, ii - 1), ui, k.dy, k.AI, k.dI);
+    link_d(k.dy * G.met(M_GRDXU, ii), G.met(M_PEXU, ii), ud, -k.dy, k.AD, k.dD);
+    link_d(k.dx * G.met(M_GRDYP, jj), G.met(M_PEYP, jj), vs, k.dx, k.BS, k.dS);
+    link_d(k.dx * G.met(M_GRDYP, jj + 1), G.met(M_PEYP, jj + 1), vn, -k.dx, k.BN, k.dN);
+  } else if constexpr (GRP == 2) {
+    k.dx = G.met(M_DXP, ii);
+    k.dy = G.met(M_DYP, jj);
+    const double ri = fast_rcp(x[5]), rd = fast_rcp(x[6]), rs = fast_rcp(x[7]), rn = fast_rcp(x[8]);
+    k.AI = -(k.dy * k.dy) * ri; k.AD = -(k.dy * k.dy) * rd;
+    k.BS = -(k.dx * k.dx) * rs; k.BN = -(k.dx * k.dx) * rn;
+    k.dI = -k.AI * ri; k.dD = -k.AD * rd; k.dS = -k.BS * rs; k.dN = -k.BN * rn;
+    k.b = (-k.AI - k.AD - k.BS - k.BN) * G.inv_rel_pres;
+    return k;
+  } else {
+    k.dx = G.met(M_DXP, ii);
+    k.dy = G.met(M_DYP, jj);
+    link_d(k.dy * G.met(M_HRDXU, ii - 1), G.met(M_PHXU, ii - 1), x[6], k.dy, k.AI, k.dI);
+    link_d(k.dy * G.met(M_HRDXU, ii), G.met(M_PHXU, ii), x[5], -k.dy, k.AD, k.dD);
+    link_d(k.dx * G.met(M_HRDYV, jj - 1), G.met(M_PHYV, jj - 1), x[8], k.dx, k.BS, k.dS);
+    link_d(k.dx * G.met(M_HRDYV, jj), G.met(M_PHYV, jj), x[7], -k.dx, k.BN, k.dN);
   }
-  const GRow<Dual<NS>> row = eval_row<Dual<NS>>(G, s, x, ii, jj, nullptr);
+  const double S = k.dx * k.dy;
+  k.b = (-k.AI - k.AD - k.BS - k.BN - S * flin + S * G.inv_dt) * (GRP == 3 ? G.inv_rel_ener : G.inv_rel_vel);
+  return k;
+}
+
+// Adjoints g of the stencil values of a row for the weights wa, wb, wc, wd of
+// (a, b, c, d); X: the row along x (a = AI, c = AD), else along y.
+template <int GRP, bool X>
+__device__ __forceinline__ void row_back(const Geo<double>& G, const Links& k, const double (&x)[NS], int ii, int jj,
+                                         double wa, double wb, double wc, double wd, double (&g)[NS]) {
+  const double rel = GRP == 2 ? G.rel_pres : GRP == 3 ? G.rel_ener : G.rel_vel;
+  const double irel = GRP == 2 ? G.inv_rel_pres : GRP == 3 ? G.inv_rel_ener : G.inv_rel_vel;
 #pragma unroll
-  for (int k = 0; k < NS; ++k) {
-    const Tap tp = kStencil[grp][k];
-    if (tp.f == F_NONE) continue;
-    const double g = wa * row.a.d[k] + wb * row.b.d[k] + wc * row.c.d[k] + wd * row.d.d[k];
-    if (g != 0.0) atomicAdd(adj.f[tp.f] + G.at(ii + tp.di, jj + tp.dj), g);
+  for (int q = 0; q < NS; ++q) g[q] = 0.0;
+  // stencil indices of the west, east, south and north swept values
+  constexpr int W = GRP == 1 ? 3 : 2, E = GRP == 1 ? 4 : 1, S = GRP == 1 ? 2 : 3, N = GRP == 1 ? 1 : 4;
+  const double bb = (wb + wd * (1.0 - rel) * x[0]) * irel;  // what -AI, -AD, -BS, -BN of the diagonal receive
+  const double AIb = (X ? wa : -wd * x[W]) - bb, ADb = (X ? wc : -wd * x[E]) - bb;
+  const double BSb = (X ? -wd * x[S] : wa) - bb, BNb = (X ? -wd * x[N] : wc) - bb;
+  g[0] += wd * k.b * (1.0 - rel);
+  if (X) { g[S] += -wd * k.BS; g[N] += -wd * k.BN; }
+  else { g[W] += -wd * k.AI; g[E] += -wd * k.AD; }
+  const double ui = AIb * k.dI, ud = ADb * k.dD, vs = BSb * k.dS, vn = BNb * k.dN;
+  if constexpr (GRP == 0) {
+    const double fi = G.met(M_FEXU, ii), fm = G.met(M_FEXU, ii - 1), fp = G.met(M_FEXP, ii);
+    g[1] += fi * ud; g[0] += (1.0 - fi) * ud;
+    g[0] += fm * ui; g[2] += (1.0 - fm) * ui;
+    g[6] += fp * vn; g[5] += (1.0 - fp) * vn;
+    g[8] += fp * vs; g[7] += (1.0 - fp) * vs;
+    const double tb = -wd * k.dx * k.dy * G.Ri;
+    g[10] += fp * tb; g[9] += (1.0 - fp) * tb;
+    g[11] += wd * k.dy; g[12] += -wd * k.dy;
+  } else if constexpr (GRP == 1) {
+    const double fp = G.met(M_FEYP, jj), fj = G.met(M_FEYV, jj), fm = G.met(M_FEYV, jj - 1);
+    g[6] += fp * ud; g[5] += (1.0 - fp) * ud;
+    g[8] += fp * ui; g[7] += (1.0 - fp) * ui;
+    g[1] += fj * vn; g[0] += (1.0 - fj) * vn;
+    g[0] += fm * vs; g[2] += (1.0 - fm) * vs;
+    const double tb = -wd * k.dx * k.dy * G.Riy;
+    g[10] += fp * tb; g[9] += (1.0 - fp) * tb;
+    g[11] += wd * k.dx; g[12] += -wd * k.dx;
+  } else if constexpr (GRP == 2) {
+    g[5] += ui; g[6] += ud; g[7] += vs; g[8] += vn;
+    g[10] += wd * k.dy; g[9] += -wd * k.dy;
+    g[12] += wd * k.dx; g[11] += -wd * k.dx;
+  } else {
+    g[5] += ud; g[6] += ui; g[7] += vn; g[8] += vs;
   }
 }
 
-// Side-a boundary rows of the T x-sweep: row 0 of line jj is (0, 1, 0 | value)
-// (or the Neumann row with the value as flux), so d x_out / d value = A^-1 e_0
-// and the value's gradient is mu at row 0.
-__global__ void adj_bcgrad_kernel(const SweepState s, const double* __restrict__ mu, double* __restrict__ grad) {
-  const int li = blockIdx.x * blockDim.x + threadIdx.x;
-  if (li > s.line_hi - s.line_lo) return;
-  grad[s.line_lo + li] += mu[(size_t)li * s.n];
+// f(q, tap) for every tap of a group, both compile-time constants
+template <int GRP, class F, int... Q>
+__device__ __forceinline__ void each_tap_(F&& f, std::integer_sequence<int, Q...>) {
+  auto one = [&](auto q) {
+    constexpr Tap t = kStencil[GRP][decltype(q)::value];
+    if constexpr (t.f != F_NONE) f(q, std::integral_constant<int, t.f>{}, t.di, t.dj);
+  };
+  (one(std::integral_constant<int, Q>{}), ...);
+}
+template <int GRP, class F>
+__device__ __forceinline__ void each_tap(F&& f) {
+  each_tap_<GRP>(f, std::make_integer_sequence<int, NS>{});
+}
+
+template <int GRP>
+__device__ __forceinline__ void load_stencil(const Geo<double>& G, const SweepState& s, int ii, int jj,
+                                             double (&x)[NS]) {
+  each_tap<GRP>([&](auto q, auto f, int di, int dj) { x[q] = __ldg(s.f[f] + G.at(ii + di, jj + dj)); });
+}
+
+// One sweep reversed.  A CTA takes TL adjacent lines, G threads per line, m
+// rows per thread (n <= G*m).  lam: the swept field's adjoint after the sweep,
+// read and cleared here; every contribution to it before the sweep goes to
+// adj.f[swept field], another buffer, zero on entry (null: dropped, p' before
+// its first sweep).  aux_bar (u-x, v-x): the adjoint of au or av, read and
+// cleared.  grad (T-x): d / d value of the side-a boundary rows, += mu of row
+// 0 (the row is (0, 1, 0 | value), or the Neumann row with the value as flux).
+template <int EQ, int TL, int GT, int M>
+__global__ void __launch_bounds__(TL * GT)
+    adj_sweep_kernel(const Geo<double> G, const SweepState s, double* __restrict__ lam, double* aux_bar, AdjFields adj,
+                     double* grad, int m_, int mp_) {
+  constexpr int GRP = eq_group(EQ);
+  constexpr bool X = (EQ & 1) != 0;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double* sm = reinterpret_cast<double*>(smem_raw);
+  const int m = M > 0 ? M : m_, mp = M > 0 ? (M | 1) : mp_;
+  const int n = s.n, npad = GT * m, arr = GT * mp, LS = (int)line_smem_elems(GT, mp);
+  const int L0 = 1 + blockIdx.x * TL;
+  auto slot = [&](int l, int r) { return l * LS + (r / m) * mp + r % m; };
+  auto cell = [&](int L, int r) { return X ? G.at(r + 1, L) : G.at(L, r + 1); };
+  // rows, transposed: a'_r = c_{r-1}, b'_r = b_r, c'_r = a_{r+1}; identity rows pad the line
+  for (int idx = threadIdx.x; idx < TL * npad; idx += TL * GT) {
+    const int l = X ? idx / npad : idx % TL, r = X ? idx - l * npad : idx / TL, L = L0 + l;
+    if (L > s.nfull) continue;
+    const bool solved = L >= s.line_lo && L <= s.line_hi;
+    double a = 0.0, b = 1.0, c = 0.0, d = 0.0;
+    if (r < n) {
+      const int g = cell(L, r);
+      d = lam[g];
+      lam[g] = 0.0;
+      if (!solved) {  // the sweep copies this line
+        if (d != 0.0 && adj.f[group_field(GRP)]) atomicAdd(adj.f[group_field(GRP)] + g, d);
+        continue;
+      }
+      if (r == 0 || r == n - 1) {
+        const BCEntry* t = r == 0 ? s.first : s.last;
+        if (t && t[L].type == 2) {
+          if (r == 0) { b = -1.0; c = 1.0; }
+          else { a = -1.0; }
+        }
+      } else {
+        const int ii = X ? r + 1 : L, jj = X ? L : r + 1;
+        double x[NS];
+        load_stencil<GRP>(G, s, ii, jj, x);
+        const Links k = links<GRP>(G, x, s.flin ? s.flin[g] : 0.0, ii, jj);
+        a = X ? k.AI : k.BS; b = k.b; c = X ? k.AD : k.BN;
+      }
+    }
+    if (!solved) continue;
+    sm[slot(l, r) + arr] = b;
+    sm[slot(l, r) + 3 * arr] = d;
+    if (r == 0 || r >= n) sm[slot(l, r)] = 0.0;
+    if (r >= n - 1) sm[slot(l, r) + 2 * arr] = 0.0;
+    if (r + 1 < n) sm[slot(l, r + 1)] = c;
+    if (r >= 1 && r < n) sm[slot(l, r - 1) + 2 * arr] = a;
+  }
+  __syncthreads();
+  {
+    const int l = threadIdx.x / GT, L = L0 + l;
+    chunk_solve<double, GT, TL, M>(sm + l * LS, m, mp, L >= s.line_lo && L <= s.line_hi);
+  }
+  __syncthreads();
+  // scatter of the interior rows
+  for (int idx = threadIdx.x; idx < TL * n; idx += TL * GT) {
+    const int l = X ? idx / n : idx % TL, r = X ? idx - l * n : idx / TL, L = L0 + l;
+    if (L < s.line_lo || L > s.line_hi) continue;
+    const double mu = sm[slot(l, r) + 3 * arr];
+    if (r == 0 && grad) grad[L] += mu;
+    if (r == 0 || r == n - 1) continue;
+    const int g = cell(L, r), st = X ? 1 : G.LD;
+    const int ii = X ? r + 1 : L, jj = X ? L : r + 1;
+    const double wa = -mu * __ldg(s.x_out + g - st), wc = -mu * __ldg(s.x_out + g + st);
+    double wb = -mu * __ldg(s.x_out + g);
+    if (aux_bar) {
+      wb += aux_bar[g] * G.rel_vel;
+      aux_bar[g] = 0.0;
+    }
+    if (wa == 0.0 && wb == 0.0 && wc == 0.0 && mu == 0.0) continue;
+    double x[NS], out[NS];
+    load_stencil<GRP>(G, s, ii, jj, x);
+    const Links k = links<GRP>(G, x, s.flin ? s.flin[g] : 0.0, ii, jj);
+    row_back<GRP, X>(G, k, x, ii, jj, wa, wb, wc, mu, out);
+    each_tap<GRP>([&](auto q, auto f, int di, int dj) {
+      double* to = adj.f[f];
+      if (out[q] != 0.0 && (f != F_PC || to)) atomicAdd(to + G.at(ii + di, jj + dj), out[q]);
+    });
+  }
+}
+
+// x-lines one per CTA; y-lines four adjacent ones (32-byte pieces of a row).
+// Three rows per thread up to 768 rows, longer chunks beyond.
+template <int EQ>
+cudaError_t adj_sweep_launch(const Geo<double>& G, const SweepState& s, double* lam, double* aux_bar,
+                             const AdjFields& adj, double* grad, cudaStream_t st) {
+  constexpr bool X = (EQ & 1) != 0;
+  auto go = [&](auto k, int tl, int g, int m) -> cudaError_t {
+    const size_t smem = line_smem_elems(g, m | 1) * sizeof(double) * tl;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k<<<(s.nfull + tl - 1) / tl, tl * g, smem, st>>>(G, s, lam, aux_bar, adj, grad, m, m | 1);
+    return cudaGetLastError();
+  };
+  constexpr int TL = X ? 1 : 4;
+  if (s.n <= 192) return go(adj_sweep_kernel<EQ, TL, 64, 3>, TL, 64, 3);
+  if (s.n <= 384) return go(adj_sweep_kernel<EQ, TL, 128, 3>, TL, 128, 3);
+  if (X && s.n <= 768) return go(adj_sweep_kernel<EQ, 1, 256, 3>, 1, 256, 3);
+  if (!X && s.n <= 1024) return go(adj_sweep_kernel<EQ, TL, 128, 0>, TL, 128, (s.n + 127) / 128);
+  return go(adj_sweep_kernel<EQ, 1, 256, 0>, 1, 256, std::max(3, (s.n + 255) / 256));
+}
+
+cudaError_t adj_sweep(const Geo<double>& G, const SweepState& s, double* lam, double* aux_bar, const AdjFields& adj,
+                      double* grad, cudaStream_t st) {
+  switch (s.eq) {
+    case EQ_UY: return adj_sweep_launch<EQ_UY>(G, s, lam, aux_bar, adj, grad, st);
+    case EQ_UX: return adj_sweep_launch<EQ_UX>(G, s, lam, aux_bar, adj, grad, st);
+    case EQ_VY: return adj_sweep_launch<EQ_VY>(G, s, lam, aux_bar, adj, grad, st);
+    case EQ_VX: return adj_sweep_launch<EQ_VX>(G, s, lam, aux_bar, adj, grad, st);
+    case EQ_PY: return adj_sweep_launch<EQ_PY>(G, s, lam, aux_bar, adj, grad, st);
+    case EQ_PX: return adj_sweep_launch<EQ_PX>(G, s, lam, aux_bar, adj, grad, st);
+    case EQ_TY: return adj_sweep_launch<EQ_TY>(G, s, lam, aux_bar, adj, grad, st);
+    default: return adj_sweep_launch<EQ_TX>(G, s, lam, aux_bar, adj, grad, st);
+  }
+}
+
+// pressure and velocity correction (main.f90:931-962) out of place: u3, v3, p1
+// from u2, v2, p0; entries the update leaves alone are copied
+__global__ void correct_to_kernel(const Geo<double> G, const double* __restrict__ u2, const double* __restrict__ v2,
+                                  const double* __restrict__ p0, const double* __restrict__ pc,
+                                  const double* __restrict__ au, const double* __restrict__ av, double* __restrict__ u3,
+                                  double* __restrict__ v3, double* __restrict__ p1) {
+  const int ii = 1 + blockIdx.x * blockDim.x + threadIdx.x, jj = 1 + blockIdx.y;
+  if (ii > G.mi + 1) return;
+  const int c0 = G.at(ii, jj);
+  const bool in = ii >= 2 && ii <= G.mi && jj >= 2 && jj <= G.nj;
+  const double q = in ? pc[c0] : 0.0;
+  p1[c0] = in ? p0[c0] + G.p_update * q : p0[c0];
+  u3[c0] = in && ii <= G.mi - 1 ? u2[c0] + G.met(M_DYU, jj) * (q - pc[c0 + 1]) * fast_rcp(au[c0]) : u2[c0];
+  v3[c0] = in && jj <= G.nj - 1 ? v2[c0] + G.met(M_DXV, ii) * (q - pc[c0 + G.LD]) * fast_rcp(av[c0]) : v2[c0];
+}
+
+__global__ void fill_kernel(double* f, size_t n, double v) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) f[i] = v;
 }
 
 // Adjoint of the velocity and pressure update (main.f90:931-962, correct_cell):
@@ -484,49 +417,57 @@ using namespace ixb;
 
 namespace {
 
-// the fields stored after every phase of one outer iteration
-enum Snap { S_U0 = 0, S_V0, S_P0, S_T0, S_U1, S_U2, S_AU, S_V1, S_V2, S_AV, S_PC1, S_PC2, S_U3, S_V3, S_T1, S_T2,
-            S_COUNT };
+// The fields of one outer iteration, each written by the phase that produces
+// it (S_U0 .. S_T0: the state before it; the state after it is the next
+// iteration's S_U0 .. S_T0).
+enum Snap { S_U0 = 0, S_V0, S_P0, S_T0, S_U1, S_U2, S_AU, S_V1, S_V2, S_AV, S_PC1, S_PC2, S_T1, S_COUNT };
 
 struct SimpleAdjoint {
   ixb_handle* h;
   size_t fsz = 0;
   Geo<double> G{};
-  std::vector<void*> allocs;
-  double* store = nullptr;  // C iterations x S_COUNT fields
-  double* ckpt = nullptr;   // (segments + 1) x (u, v, p, T)
+  double* pool = nullptr;   // everything below
+  double* store = nullptr;  // C + 1 iterations x S_COUNT fields
+  double* ckpt = nullptr;   // segments x (u, v, p, T)
   AdjFields adj{};
-  double *fa = nullptr, *fb = nullptr, *fc = nullptr, *ta = nullptr, *tb = nullptr, *tc = nullptr, *td = nullptr,
-         *mu = nullptr, *gd = nullptr;
+  double* other[F_COUNT] = {};  // second buffers of the swept fields' adjoints
+  double* gd = nullptr;
 
   ~SimpleAdjoint() {
+    if (pool) cudaFreeAsync(pool, h->stream);
     if (h && h->stream) cudaStreamSynchronize(h->stream);
-    for (void* p : allocs) cudaFree(p);
-  }
-  int alloc(double** p, size_t n) {
-    if (cudaMalloc((void**)p, n * sizeof(double)) != cudaSuccess) {
-      cudaGetLastError();
-      return IXB_ENOMEM;
-    }
-    allocs.push_back(*p);
-    return IXB_OK;
   }
 
   int init(int C, int segments) {
     fsz = h->fsz;
     G = handle_geo(h);
-    STRY(alloc(&store, (size_t)C * S_COUNT * fsz));
-    STRY(alloc(&ckpt, (size_t)(segments + 1) * 4 * fsz));
-    for (int k = 0; k < F_COUNT; ++k) {
-      STRY(alloc(&adj.f[k], fsz));
-      SCK(cudaMemsetAsync(adj.f[k], 0, fsz * sizeof(double), h->stream));
+    const size_t nadj = F_COUNT + 4, ngd = (size_t)h->nj + 2;
+    const size_t total = ((size_t)(C + 1) * S_COUNT + (size_t)segments * 4 + nadj) * fsz + ngd;
+    const cudaError_t e = scratch_alloc(reinterpret_cast<void**>(&pool), total * sizeof(double), h->stream);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      pool = nullptr;
+      return e == cudaErrorMemoryAllocation ? IXB_ENOMEM : IXB_ECUDA;
     }
-    const size_t nst = (size_t)std::max(h->mi + 1, h->nj + 1) * (size_t)std::max(h->mi + 1, h->nj + 1);
-    for (double** p : {&fa, &fb, &fc, &ta, &tb, &tc, &td, &mu}) STRY(alloc(p, nst));
-    STRY(alloc(&gd, (size_t)h->nj + 2));
-    SCK(cudaMemsetAsync(gd, 0, ((size_t)h->nj + 2) * sizeof(double), h->stream));
+    h->scratch_used = true;
+    store = pool;
+    ckpt = store + (size_t)(C + 1) * S_COUNT * fsz;
+    double* a = ckpt + (size_t)segments * 4 * fsz;
+    // adjoints and gradient start from zero; fields of the store from zero
+    // too, but for au and av, whose unswept entries are 1e40 (main.f90:309-310)
+    SCK(cudaMemsetAsync(a, 0, (nadj * fsz + ngd) * sizeof(double), h->stream));
+    for (int k = 0; k < F_COUNT; ++k, a += fsz) adj.f[k] = a;
+    for (int f : {F_U, F_V, F_T, F_PC}) { other[f] = a; a += fsz; }
+    gd = a;
+    SCK(cudaMemsetAsync(store, 0, (size_t)(C + 1) * S_COUNT * fsz * sizeof(double), h->stream));
+    for (int it = 0; it < C; ++it)
+      for (int f : {S_AU, S_AV}) {
+        fill_kernel<<<148, 256, 0, h->stream>>>(slot(it, f), fsz, 1.e40);
+        SCK(cudaGetLastError());
+      }
     return IXB_OK;
   }
+  double* slot(int it, int k) const { return store + ((size_t)it * S_COUNT + k) * fsz; }
 
   int copy(double* dst, const double* src) {
     SCK(cudaMemcpyAsync(dst, src, fsz * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
@@ -538,43 +479,51 @@ struct SimpleAdjoint {
     STRY(copy(dst + 2 * fsz, h->p));
     return copy(dst + 3 * fsz, h->T[h->cT]);
   }
-  int restore(const double* src) {
-    STRY(copy(h->u[h->cu], src));
-    STRY(copy(h->v[h->cv], src + fsz));
-    STRY(copy(h->p, src + 2 * fsz));
-    return copy(h->T[h->cT], src + 3 * fsz);
+  // the state of checkpoint k into the store
+  int load(int k) {
+    for (int q = 0; q < 4; ++q) STRY(copy(slot(0, S_U0 + q), ckpt + ((size_t)k * 4 + q) * fsz));
+    return IXB_OK;
+  }
+  // count iterations from checkpoint k by the library's loop; it stops at
+  // values that are not finite, the sweeps of the store carry them along
+  int forward(int k, int count) {
+    STRY(save(ckpt + (size_t)k * 4 * fsz));
+    const int st = handle_single_passes(h, count);
+    if (st != IXB_ENONFINITE) return st;
+    STRY(load(k));
+    for (int it = 0; it < count; ++it) STRY(iterate(it));
+    STRY(copy(h->u[h->cu], slot(count, S_U0)));
+    STRY(copy(h->v[h->cv], slot(count, S_V0)));
+    STRY(copy(h->p, slot(count, S_P0)));
+    return copy(h->T[h->cT], slot(count, S_T0));
   }
 
-  // One outer iteration, one pass of each equation, phase by phase; with
-  // `st`, the state after every phase is stored there.
-  int iterate(double* st) {
-    auto snap = [&](int k, const double* src) { return st ? copy(st + (size_t)k * fsz, src) : IXB_OK; };
-    STRY(snap(S_U0, h->u[h->cu]));
-    STRY(snap(S_V0, h->v[h->cv]));
-    STRY(snap(S_P0, h->p));
-    STRY(snap(S_T0, h->T[h->cT]));
-    STRY(ixb_phase(h, 0));
-    STRY(snap(S_U1, h->u[h->cu]));
-    STRY(ixb_phase(h, 1));
-    STRY(snap(S_U2, h->u[h->cu]));
-    STRY(snap(S_AU, h->au));
-    STRY(ixb_phase(h, 2));
-    STRY(snap(S_V1, h->v[h->cv]));
-    STRY(ixb_phase(h, 3));
-    STRY(snap(S_V2, h->v[h->cv]));
-    STRY(snap(S_AV, h->av));
-    SCK(cudaMemsetAsync(h->pc[h->cpc], 0, fsz * sizeof(double), h->stream));  // p' starts from zero
-    STRY(ixb_phase(h, 4));
-    STRY(snap(S_PC1, h->pc[h->cpc]));
-    STRY(ixb_phase(h, 5));
-    STRY(snap(S_PC2, h->pc[h->cpc]));
-    STRY(ixb_phase(h, 6));
-    STRY(snap(S_U3, h->u[h->cu]));
-    STRY(snap(S_V3, h->v[h->cv]));
-    STRY(ixb_phase(h, 7));
-    STRY(snap(S_T1, h->T[h->cT]));
-    STRY(ixb_phase(h, 8));
-    return snap(S_T2, h->T[h->cT]);
+  // Iteration `it` of the store, sweep by sweep, one pass of each equation:
+  // reads the state in its slots S_U0 .. S_T0, fills its other slots and the
+  // next iteration's S_U0 .. S_T0.
+  int iterate(int it) {
+    auto S = [&](int k) { return slot(it, k); };
+    auto sw = [&](int eq, const double* in, double* out, const double* u, const double* v, double* aux) -> int {
+      SweepIO<double> io = handle_fixed_io(h, eq);
+      io.in = in; io.out = out; io.aux = aux;
+      io.u = u; io.v = v; io.T = S(S_T0); io.p = S(S_P0); io.pc = in;
+      io.au = S(S_AU); io.av = S(S_AV);
+      return handle_sweep_to(h, eq, io);
+    };
+    const double *u0 = S(S_U0), *v0 = S(S_V0);
+    STRY(sw(EQ_UY, u0, S(S_U1), u0, v0, nullptr));
+    STRY(sw(EQ_UX, S(S_U1), S(S_U2), S(S_U1), v0, S(S_AU)));
+    STRY(sw(EQ_VY, v0, S(S_V1), S(S_U2), v0, nullptr));
+    STRY(sw(EQ_VX, S(S_V1), S(S_V2), S(S_U2), S(S_V1), S(S_AV)));
+    STRY(sw(EQ_PY, h->zero, S(S_PC1), S(S_U2), S(S_V2), nullptr));
+    STRY(sw(EQ_PX, S(S_PC1), S(S_PC2), S(S_U2), S(S_V2), h->b_o));
+    double *u3 = slot(it + 1, S_U0), *v3 = slot(it + 1, S_V0);
+    const dim3 grid((h->mi + 1 + 127) / 128, h->nj + 1);
+    correct_to_kernel<<<grid, 128, 0, h->stream>>>(G, S(S_U2), S(S_V2), S(S_P0), S(S_PC2), S(S_AU), S(S_AV), u3, v3,
+                                                   slot(it + 1, S_P0));
+    SCK(cudaGetLastError());
+    STRY(sw(EQ_TY, S(S_T0), S(S_T1), u3, v3, nullptr));
+    return sw(EQ_TX, S(S_T1), slot(it + 1, S_T0), u3, v3, nullptr);
   }
 
   // the boundary tables of variable var (0 u, 1 v, 2 T) for x- or y-lines
@@ -584,23 +533,24 @@ struct SimpleAdjoint {
     s.first = base + (size_t)(x ? 0 : 1) * h->bcstride;
     s.last = base + (size_t)(x ? 2 : 3) * h->bcstride;
   }
-  SweepState state(int eq, const double* st) {
+  SweepState state(int eq, int it) {
     SweepState s{};
     s.eq = eq;
     const SweepShape sh = sweep_shape(eq, h->mi, h->nj, 8, 1, 128);
     s.n = sh.n;
     s.line_lo = sh.line_lo;
     s.line_hi = sh.line_hi;
-    auto S = [&](int k) { return st + (size_t)k * fsz; };
+    s.nfull = sh.nfull;
+    auto S = [&](int k) { return slot(it, k); };
     switch (eq) {
       case EQ_UY: case EQ_UX:
         s.f[F_U] = S(eq == EQ_UY ? S_U0 : S_U1); s.f[F_V] = S(S_V0); s.f[F_T] = S(S_T0); s.f[F_P] = S(S_P0);
-        s.x_out = S(eq == EQ_UY ? S_U1 : S_U2); s.ant = h->u_ant; s.fcon = h->fcon[0]; s.flin = h->flin[0];
+        s.x_out = S(eq == EQ_UY ? S_U1 : S_U2); s.flin = h->flin[0];
         tables(s, 0);
         break;
       case EQ_VY: case EQ_VX:
         s.f[F_V] = S(eq == EQ_VY ? S_V0 : S_V1); s.f[F_U] = S(S_U2); s.f[F_T] = S(S_T0); s.f[F_P] = S(S_P0);
-        s.x_out = S(eq == EQ_VY ? S_V1 : S_V2); s.ant = h->v_ant; s.fcon = h->fcon[1]; s.flin = h->flin[1];
+        s.x_out = S(eq == EQ_VY ? S_V1 : S_V2); s.flin = h->flin[1];
         tables(s, 1);
         break;
       case EQ_PY: case EQ_PX:
@@ -609,52 +559,41 @@ struct SimpleAdjoint {
         s.x_out = S(eq == EQ_PY ? S_PC1 : S_PC2);
         break;
       default:
-        s.f[F_T] = S(eq == EQ_TY ? S_T0 : S_T1); s.f[F_U] = S(S_U3); s.f[F_V] = S(S_V3);
-        s.x_out = S(eq == EQ_TY ? S_T1 : S_T2); s.ant = h->T_ant; s.fcon = h->fcon[2]; s.flin = h->flin[2];
+        s.f[F_T] = S(eq == EQ_TY ? S_T0 : S_T1); s.f[F_U] = slot(it + 1, S_U0); s.f[F_V] = slot(it + 1, S_V0);
+        s.x_out = eq == EQ_TY ? S(S_T1) : slot(it + 1, S_T0); s.flin = h->flin[2];
         tables(s, 2);
         break;
     }
     return s;
   }
 
-  // One sweep reversed: lam (the swept field's adjoint) holds the adjoint of
-  // x_out on entry and of x_in on exit; the other fields' adjoints collect.
-  int sweep_back(const SweepState& s, double* lam, const double* aux_bar, bool bc_grad) {
-    const int nl = s.line_hi - s.line_lo + 1, rows = nl * s.n;
-    adj_rows_kernel<<<(rows + 255) / 256, 256, 0, h->stream>>>(G, s, fa, fb, fc);
-    SCK(cudaGetLastError());
-    adj_transpose_kernel<<<(rows + 255) / 256, 256, 0, h->stream>>>(G, s, fa, fb, fc, lam, ta, tb, tc, td);
-    SCK(cudaGetLastError());
-    SCK(tridiag_f64(ta, tb, tc, td, mu, s.n, nl, 0, IXB_SOLVER_HYBRID, h->stream));
-    if (bc_grad) {
-      adj_bcgrad_kernel<<<(nl + 127) / 128, 128, 0, h->stream>>>(s, mu, gd);
-      SCK(cudaGetLastError());
-    }
-    const int cells = nl * (s.n - 2);
-    adj_jac_kernel<<<(cells + 127) / 128, 128, 0, h->stream>>>(G, s, mu, aux_bar, adj);
-    SCK(cudaGetLastError());
+  // One sweep reversed: the adjoint of the swept field moves to its other
+  // buffer (keep false: it is dropped); the other fields' adjoints collect.
+  int sweep_back(int eq, int it, double* aux_bar, double* grad, bool keep = true) {
+    const int f = eq == EQ_UY || eq == EQ_UX ? F_U : eq == EQ_VY || eq == EQ_VX ? F_V : eq == EQ_PY || eq == EQ_PX ? F_PC : F_T;
+    double* lam = adj.f[f];
+    std::swap(adj.f[f], other[f]);
+    AdjFields a = adj;
+    if (!keep) a.f[f] = nullptr;
+    SCK(adj_sweep(G, state(eq, it), lam, aux_bar, a, grad, h->stream));
     return IXB_OK;
   }
 
   // One outer iteration reversed, from its stored phases.
-  int iteration_back(const double* st) {
-    auto S = [&](int k) { return st + (size_t)k * fsz; };
-    STRY(sweep_back(state(EQ_TX, st), adj.f[F_T], nullptr, true));
-    STRY(sweep_back(state(EQ_TY, st), adj.f[F_T], nullptr, false));
+  int iteration_back(int it) {
+    STRY(sweep_back(EQ_TX, it, nullptr, gd));
+    STRY(sweep_back(EQ_TY, it, nullptr, nullptr));
     const int ncell = (h->mi - 1) * (h->nj - 1);
-    adj_correct_kernel<<<(ncell + 255) / 256, 256, 0, h->stream>>>(G, S(S_PC2), S(S_AU), S(S_AV), adj.f[F_U],
-                                                                 adj.f[F_V], adj.f[F_P], adj.f[F_PC], adj.f[F_AU],
-                                                                 adj.f[F_AV]);
+    adj_correct_kernel<<<(ncell + 255) / 256, 256, 0, h->stream>>>(G, slot(it, S_PC2), slot(it, S_AU), slot(it, S_AV),
+                                                                 adj.f[F_U], adj.f[F_V], adj.f[F_P], adj.f[F_PC],
+                                                                 adj.f[F_AU], adj.f[F_AV]);
     SCK(cudaGetLastError());
-    STRY(sweep_back(state(EQ_PX, st), adj.f[F_PC], nullptr, false));
-    STRY(sweep_back(state(EQ_PY, st), adj.f[F_PC], nullptr, false));
-    SCK(cudaMemsetAsync(adj.f[F_PC], 0, fsz * sizeof(double), h->stream));  // p' starts from the zero field
-    STRY(sweep_back(state(EQ_VX, st), adj.f[F_V], adj.f[F_AV], false));
-    SCK(cudaMemsetAsync(adj.f[F_AV], 0, fsz * sizeof(double), h->stream));  // av is written by the v-x sweep
-    STRY(sweep_back(state(EQ_VY, st), adj.f[F_V], nullptr, false));
-    STRY(sweep_back(state(EQ_UX, st), adj.f[F_U], adj.f[F_AU], false));
-    SCK(cudaMemsetAsync(adj.f[F_AU], 0, fsz * sizeof(double), h->stream));  // au is written by the u-x sweep
-    return sweep_back(state(EQ_UY, st), adj.f[F_U], nullptr, false);
+    STRY(sweep_back(EQ_PX, it, nullptr, nullptr));
+    STRY(sweep_back(EQ_PY, it, nullptr, nullptr, false));  // p' starts from the zero field
+    STRY(sweep_back(EQ_VX, it, adj.f[F_AV], nullptr));     // av is written by the v-x sweep
+    STRY(sweep_back(EQ_VY, it, nullptr, nullptr));
+    STRY(sweep_back(EQ_UX, it, adj.f[F_AU], nullptr));     // au is written by the u-x sweep
+    return sweep_back(EQ_UY, it, nullptr, nullptr);
   }
 
   // lambda_T = d Nu / d T: the Nusselt number is linear in T; its weights
@@ -688,31 +627,22 @@ extern "C" int ixb_adjoint_simple(ixb_handle* h, int K, int C, int j0, int j1, d
   const int segments = (K + C - 1) / C;
   SimpleAdjoint A{h};
   STRY(A.init(std::min(C, K), segments));
-  // forward, with a checkpoint at the start of every segment and at the end
-  for (int sgm = 0; sgm < segments; ++sgm) {
-    STRY(A.save(A.ckpt + (size_t)sgm * 4 * A.fsz));
-    const int count = std::min(C, K - sgm * C);
-    for (int it = 0; it < count; ++it) STRY(A.iterate(nullptr));
-  }
-  STRY(A.save(A.ckpt + (size_t)segments * 4 * A.fsz));
+  // forward, with a checkpoint at the start of every segment
+  for (int sgm = 0; sgm < segments; ++sgm) STRY(A.forward(sgm, std::min(C, K - sgm * C)));
   double nu = 0.0;
   STRY(ixb_nusselt_x(h, j0, j1, &nu, nullptr));
   if (nu0) *nu0 = nu;
   if (!grad) return IXB_OK;
   STRY(A.objective(j0, j1));
   for (int sgm = segments - 1; sgm >= 0; --sgm) {
-    STRY(A.restore(A.ckpt + (size_t)sgm * 4 * A.fsz));
+    STRY(A.load(sgm));
     const int count = std::min(C, K - sgm * C);
-    for (int it = 0; it < count; ++it) STRY(A.iterate(A.store + (size_t)it * S_COUNT * A.fsz));
-    for (int it = count - 1; it >= 0; --it) STRY(A.iteration_back(A.store + (size_t)it * S_COUNT * A.fsz));
+    for (int it = 0; it < count; ++it) STRY(A.iterate(it));
+    for (int it = count - 1; it >= 0; --it) STRY(A.iteration_back(it));
   }
-  STRY(A.restore(A.ckpt + (size_t)segments * 4 * A.fsz));  // the state of the forward run
   std::vector<double> g((size_t)h->nj + 2);
   SCK(cudaMemcpyAsync(g.data(), A.gd, g.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
   SCK(cudaStreamSynchronize(h->stream));
-  int timed_out = 0;
-  SCK(tridiag_take_timeout(&timed_out));
-  if (timed_out) return IXB_ETIMEOUT;
   for (int jj = 1; jj <= h->nj + 1; ++jj) grad[jj - 1] = g[jj];
   return IXB_OK;
 }

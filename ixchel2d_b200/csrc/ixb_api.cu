@@ -935,8 +935,10 @@ int ixb_create(int mi, int nj, int prec_mode, ixb_handle** out) {
 int ixb_destroy(ixb_handle* h) {
   if (!h) return IXB_EINVAL;
   if (h->stream) cudaStreamSynchronize(h->stream);
+  const bool trim = h->scratch_used;
   free_all(h);
   delete h;
+  if (trim) scratch_trim();
   return IXB_OK;
 }
 
@@ -1545,4 +1547,31 @@ int handle_solver_form(const ixb_handle* h) { return solver_form(h); }
 int handle_ready(ixb_handle* h) { return ready(h); }
 SweepIO<double> handle_sweep_io(ixb_handle* h, int eq, const double* prev) { return sweep_io(h, eq, prev, false); }
 int handle_real_bytes(const ixb_handle* h) { return real_bytes(h); }
+SweepIO<double> handle_fixed_io(ixb_handle* h, int eq) {
+  const int cu = h->cu, cv = h->cv, cT = h->cT, cpc = h->cpc;
+  const SweepIO<double> io = sweep_io(h, eq, nullptr, false);
+  h->cu = cu; h->cv = cv; h->cT = cT; h->cpc = cpc;
+  return io;
+}
+int handle_sweep_to(ixb_handle* h, int eq, const SweepIO<double>& io) {
+  if (h->shape_tl[eq] == 0) pick_shape(h, eq);
+  const SweepShape s = sweep_shape(eq, h->mi, h->nj, real_bytes(h), h->shape_tl[eq], h->shape_g[eq]);
+  CK(launch_sweep_f64(eq, solver_form(h), s, make_geo(h), io, StageBuf{h->stage, h->stage_stride, h->stage_P},
+                      h->stream));
+  return IXB_OK;
+}
+int handle_single_passes(ixb_handle* h, int n) {
+  // every inner test met after its first pass
+  const ixb_params prm = h->prm;
+  const int ie = h->iter_ecuaci, is = h->iter_simple;
+  h->prm.conv_u = h->prm.conv_p = h->prm.conv_t = INFINITY;
+  h->prm.iter_ecuaci_max = 0;
+  h->iter_ecuaci = 0;
+  ixb_report rep;
+  const int st = ixb_simple_iterations(h, n, &rep);
+  h->prm = prm;
+  h->iter_ecuaci = ie;
+  h->iter_simple = is;
+  return st;
+}
 }  // namespace ixb

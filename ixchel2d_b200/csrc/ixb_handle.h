@@ -103,6 +103,7 @@ struct ixb_handle {
   int shape_tl[ixb::EQ_COUNT] = {};  // launch shape per sweep (0 = not chosen yet)
   int shape_g[ixb::EQ_COUNT] = {};
   bool shape_set[ixb::EQ_COUNT] = {};  // set by the caller (ixb_set_sweep_shape): the loop keeps to the per-sweep kernels
+  bool scratch_used = false;           // a gradient has grown the scratch pool
   bool coop = false;                   // the device takes cooperative launches
   int nsm = 148;
   // adjoint workspace (ixb_adjoint_energy), allocated on first use
@@ -134,5 +135,13 @@ int handle_build_loop_graph(ixb_handle* h, const std::function<int()>& pass, int
                             cudaGraphExec_t* exec);
 int handle_run_loop_graph(ixb_handle* h, cudaGraphExec_t exec, int iterations);
 SweepIO<double> handle_sweep_io(ixb_handle* h, int eq, const double* prev);
+// sweep `eq` between fields of the caller's choice, in the handle's launch
+// shape: handle_fixed_io gives the inputs that are the handle's own (previous
+// time level, sources, boundary tables), the caller fills in the rest
+SweepIO<double> handle_fixed_io(ixb_handle* h, int eq);
+int handle_sweep_to(ixb_handle* h, int eq, const SweepIO<double>& io);
+// n outer iterations of one pass of each equation, whatever the parameters'
+// tests say; the loop counters are left alone
+int handle_single_passes(ixb_handle* h, int n);
 int handle_real_bytes(const ixb_handle* h);  // element size of the staged rows
 }  // namespace ixb

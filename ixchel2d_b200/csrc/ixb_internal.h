@@ -280,6 +280,11 @@ cudaError_t tridiag_f64(const double* a, const double* b, const double* c, const
                         int nsys, int layout, int solver, cudaStream_t st);
 cudaError_t tridiag_f32(const float* a, const float* b, const float* c, const float* d, float* x, int n,
                         int nsys, int layout, int solver, cudaStream_t st);
+// stream-ordered device memory from a bounded pool of the library's own
+// (free with cudaFreeAsync)
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t st);
+// gives the pool's idle memory on the current device back
+void scratch_trim();
 // reads and clears the flag set when a line-solve kernel's bounded wait on
 // its copies expired (synchronous)
 cudaError_t tridiag_take_timeout(int* flag);

@@ -738,57 +738,68 @@ cudaError_t block_solve(const R* a, const R* b, const R* c, const R* d, R* x, in
 // context), so that memory freed after a call is still mapped at the next
 // one: with the device's default pool every synchronisation unmapped it, and
 // a 0.2 ms solve that the host waits for took 4.2 ms.  The pool keeps at most
-// kPoolKeep bytes mapped across synchronisations.  While `st` is captured,
-// or if the pool cannot be had, the default allocator serves.
-constexpr unsigned long long kPoolKeep = 64ull << 20;
+// kPoolKeep bytes mapped across synchronisations (a 128x128 gradient of the
+// coupled iteration with a checkpoint every 10 holds 21 MB: as thirty
+// cudaMalloc / cudaFree pairs its workspace cost 2 to 10 ms per call); a
+// handle that has used it for a gradient gives the idle memory back when it
+// is destroyed.  While `st` is captured, or if the pool cannot be had, the
+// default allocator serves.
+constexpr unsigned long long kPoolKeep = 256ull << 20;
 constexpr int kPoolDevices = 64;
 
-cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t st) {
+// the pool of the current device's context; made on first use with `make`,
+// else null if there is none
+cudaMemPool_t scratch_pool(int dev, bool make) {
   static std::mutex mu;
   static cudaMemPool_t pool[kPoolDevices] = {};
   static unsigned long long owner[kPoolDevices] = {};  // context the pool belongs to (0: none)
   using CtxIdFn = CUresult (*)(CUcontext, unsigned long long*);
   static CtxIdFn ctx_id = nullptr;
+  if (dev < 0 || dev >= kPoolDevices) return nullptr;
+  std::lock_guard<std::mutex> lock(mu);
+  if (!ctx_id) {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      ctx_id = reinterpret_cast<CtxIdFn>(f);
+  }
+  unsigned long long id = 0;
+  if (!ctx_id || ctx_id(nullptr, &id) != CUDA_SUCCESS) return nullptr;
+  if (owner[dev] != id + 1 && make) {  // first use, or the context was re-created (cudaDeviceReset)
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t made = nullptr;
+    unsigned long long keep = kPoolKeep;
+    if (cudaMemPoolCreate(&made, &props) == cudaSuccess &&
+        cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess) {
+      pool[dev] = made;
+      owner[dev] = id + 1;
+    } else {
+      cudaGetLastError();
+    }
+  }
+  return owner[dev] == id + 1 ? pool[dev] : nullptr;
+}
+}  // namespace
+
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t st) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if ((e = cudaStreamIsCapturing(st, &cap)) != cudaSuccess) return e;
-  if (cap != cudaStreamCaptureStatusNone || dev < 0 || dev >= kPoolDevices) return cudaMallocAsync(p, bytes, st);
-  cudaMemPool_t use = nullptr;
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    if (!ctx_id) {
-      void* f = nullptr;
-      cudaDriverEntryPointQueryResult q;
-      if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) == cudaSuccess &&
-          q == cudaDriverEntryPointSuccess)
-        ctx_id = reinterpret_cast<CtxIdFn>(f);
-    }
-    unsigned long long id = 0;
-    if (ctx_id && ctx_id(nullptr, &id) == CUDA_SUCCESS) {
-      if (owner[dev] != id + 1) {  // first use, or the context was re-created (cudaDeviceReset)
-        cudaMemPoolProps props{};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = dev;
-        cudaMemPool_t made = nullptr;
-        unsigned long long keep = kPoolKeep;
-        if (cudaMemPoolCreate(&made, &props) == cudaSuccess &&
-            cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess) {
-          pool[dev] = made;
-          owner[dev] = id + 1;
-        } else {
-          cudaGetLastError();
-        }
-      }
-      if (owner[dev] == id + 1) use = pool[dev];
-    }
-  }
+  cudaMemPool_t use = cap == cudaStreamCaptureStatusNone ? scratch_pool(dev, true) : nullptr;
   return use ? cudaMallocFromPoolAsync(p, bytes, use, st) : cudaMallocAsync(p, bytes, st);
 }
 
-}  // namespace
+void scratch_trim() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return;
+  if (cudaMemPool_t pool = scratch_pool(dev, false)) cudaMemPoolTrimTo(pool, 0);
+}
 
 // ---------------------------------------------------------------------------
 // Interleaved systems in a thread-block cluster (hybrid solver; rows of whole
