@@ -20,6 +20,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <new>
+#include <numeric>
 #include <type_traits>
 #include <vector>
 
@@ -130,13 +131,23 @@ cudaError_t upload(T** dst, const std::vector<T>& v) {
 
 int form_of(const ixb_batch* b) { return b->prec == IXB_PREC_FP32_REFINED ? SOLVER_MIXED : IXB_SOLVER_HYBRID; }
 
+// The instances from the largest to the smallest: the order of their work
+// items, so that a launch's last wave is made of its smallest items.
+std::vector<int> by_size(const ixb_batch* b) {
+  std::vector<int> o(b->count);
+  std::iota(o.begin(), o.end(), 0);
+  auto cells = [&](int i) { return (long long)b->h[i]->mi * b->h[i]->nj; };
+  std::stable_sort(o.begin(), o.end(), [&](int p, int q) { return cells(p) > cells(q); });
+  return o;
+}
+
 // assembly descriptors of sweep EQ for every instance, typed for the form
 template <int EQ, int SOLVER>
 cudaError_t build_asm(ixb_batch* b, const std::vector<SweepIO<double>>& io, std::vector<int2>& items) {
   using ST = SweepTypes<SOLVER, EQ>;
   using S = typename ST::S;
   std::vector<AsmInst<S>> v(b->count);
-  for (int i = 0; i < b->count; ++i) {
+  for (const int i : by_size(b)) {
     ixb_handle* h = b->h[i];
     const SweepShape s = sweep_shape(EQ, h->mi, h->nj, (int)sizeof(S), 1, 128);
     AsmInst<S>& d = v[i];
@@ -211,7 +222,7 @@ cudaError_t launch_fused_eq(ixb_batch* b, int eq, const BatchNorm& an, const Bat
 // the b_o norm (p'-x), sn: the pass norm.
 cudaError_t sweep_batch(ixb_batch* b, int eq, const BatchNorm& an, const BatchNorm& sn) {
   const int form = form_of(b);
-  if (fused_enabled() && fused_shape(eq, b->tl[eq], b->g[eq])) {
+  if (fused_enabled() && fused_shape(eq, b->tl[eq], b->g[eq], true)) {
     const cudaError_t e = form == SOLVER_MIXED ? launch_fused_eq<SOLVER_MIXED>(b, eq, an, sn)
                                                : launch_fused_eq<IXB_SOLVER_HYBRID>(b, eq, an, sn);
     if (e != cudaErrorNotSupported) return e;
@@ -227,17 +238,33 @@ BatchNorm norm_of(ixb_batch* b, int k) {
   return BatchNorm{b->partials[k], b->counters + (size_t)k * b->count, b->results + (size_t)k * b->count};
 }
 
+// Default launch shape of a sweep: fused, four lines of 64 threads per CTA.
+// Per outer iteration, against assembly and solve launches of 2 x 64: 12
+// instances of 64 to 384 cells a side 291 against 388 us refined; 12 of 100
+// to 300 245 against 297 us binary64; 12 of 24 to 60 72 against 85; 2 of 24
+// and 40 68 against 80.  In binary64 the four lines' rows fill an SM's
+// shared memory from about 320 rows on: x-lines then run one per CTA with
+// 128 threads (64 to 384: 323 against 348 us), and beyond 512 rows all lines
+// get twice the threads (4 of 513 to 700: 587 against 628 us).  The refined
+// form keeps 64 threads: its binary32 solves depend on the partition.
+void pick_shape(ixb_batch* b, int eq) {
+  int rows = 0;
+  for (const ixb_handle* h : b->h) rows = std::max(rows, (eq & 1) ? h->mi + 1 : h->nj + 1);
+  const bool x = (eq & 1) != 0, wide = b->prec == IXB_PREC_FP64;
+  b->tl[eq] = 4;
+  b->g[eq] = 64;
+  if (wide && rows > 512) b->g[eq] = x ? 256 : 128;
+  else if (wide && rows > 320 && x) b->g[eq] = 128;
+  if (x && b->g[eq] != 64) b->tl[eq] = 1;
+}
+
 // Descriptors and work items of one outer iteration for every instance
 // (buffer parity 0 at the start of the iteration, back at 0 at its end).
 int build_tables(ixb_batch* b) {
   free_tables(b);
   const int form = form_of(b);
-  for (int eq = 0; eq < EQ_COUNT; ++eq) {
-    if (b->tl[eq] == 0) {  // default line-solve shape: 2 lines x 64 threads
-      b->tl[eq] = 2;
-      b->g[eq] = 64;
-    }
-  }
+  for (int eq = 0; eq < EQ_COUNT; ++eq)
+    if (b->tl[eq] == 0) pick_shape(b, eq);
   for (int i = 0; i < b->count; ++i) {
     ixb_handle* h = b->h[i];
     BTRY(handle_ready(h));
@@ -274,7 +301,8 @@ int build_tables(ixb_batch* b) {
     std::vector<SolveInst> sv(b->count);
     std::vector<int2> sitems;
     size_t smem = 0;
-    for (int i = 0; i < b->count; ++i) {
+    const bool fused = fused_enabled() && fused_shape(eq, b->tl[eq], b->g[eq], true);
+    for (const int i : by_size(b)) {
       ixb_handle* h = b->h[i];
       const SweepShape s = sweep_shape(eq, h->mi, h->nj, handle_real_bytes(h), b->tl[eq], b->g[eq]);
       SolveInst& d = sv[i];
@@ -285,7 +313,7 @@ int build_tables(ixb_batch* b) {
       d.first = (int)sitems.size();
       d.count = s.grid;
       for (int t = 0; t < s.grid; ++t) sitems.push_back(make_int2(i, t));
-      smem = std::max(smem, s.smem);
+      smem = std::max(smem, fused ? fused_batch_smem(eq, s, handle_real_bytes(h)) : s.smem);
     }
     BCK(upload(&b->sol_inst[eq], sv));
     std::vector<FusedInst> fv(b->count);
@@ -299,7 +327,7 @@ int build_tables(ixb_batch* b) {
   // correction and residual
   std::vector<CellInst> cv(b->count);
   std::vector<int2> citems, ritems;
-  for (int i = 0; i < b->count; ++i) {
+  for (const int i : by_size(b)) {
     ixb_handle* h = b->h[i];
     CellInst& d = cv[i];
     d.G = handle_geo(h);

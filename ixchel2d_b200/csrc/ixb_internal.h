@@ -194,10 +194,13 @@ constexpr int kShapeList[kNumShapes][2] = {{1, 128}, {1, 256}, {1, 512}, {2, 64}
 #define IXB_FUSED_Y_SHAPES(X_) \
   X_(4, 32) X_(4, 64) X_(4, 128) X_(5, 64) X_(5, 128) X_(6, 64) X_(6, 128) X_(8, 32) X_(8, 64) X_(8, 128) \
   X_(16, 16) X_(16, 32)
-inline bool fused_shape(int eq, int tl, int g) {
+// batched x-sweeps run fused with 64 threads per line too
+#define IXB_FUSED_BATCH_X_SHAPES(X_) IXB_FUSED_X_SHAPES(X_) X_(2, 64) X_(4, 64)
+inline bool fused_shape(int eq, int tl, int g, bool batch = false) {
   bool hit = false;
 #define IXB_HIT_(TL_, G_) hit = hit || (tl == TL_ && g == G_);
-  if (eq & 1) { IXB_FUSED_X_SHAPES(IXB_HIT_) }  // x-sweeps are the odd ones (EqIsX)
+  if ((eq & 1) && batch) { IXB_FUSED_BATCH_X_SHAPES(IXB_HIT_) }
+  else if (eq & 1) { IXB_FUSED_X_SHAPES(IXB_HIT_) }  // x-sweeps are the odd ones (EqIsX)
   else { IXB_FUSED_Y_SHAPES(IXB_HIT_) }
 #undef IXB_HIT_
   return hit;
@@ -207,6 +210,15 @@ inline bool fused_shape(int eq, int tl, int g) {
 template <int EQ, int SOLVER>
 cudaError_t fused_launch(const SweepShape& s, const Geo<double>& G, const SweepIO<double>& io, const SolveIO& so,
                            cudaStream_t st);
+// Batched y-sweeps of 4 x 64 threads hold chunks of up to kBatchRegM rows in
+// registers (fused_y_lines): shared memory then only carries the reduced
+// systems, 18 KB (binary64) instead of 82 KB per CTA at 384 rows.
+constexpr int kBatchRegM = 8;
+constexpr __host__ __device__ bool batch_y_regs(int eq, int tl, int g) { return (eq & 1) == 0 && tl == 4 && g == 64; }
+inline size_t fused_batch_smem(int eq, const SweepShape& s, int real_bytes) {
+  return batch_y_regs(eq, s.tl, s.g) && s.m <= kBatchRegM ? (size_t)(real_bytes == 8 ? 9 : 12) * s.tl * s.g * real_bytes
+                                                          : s.smem;
+}
 // one instance of a batched line solve
 struct SolveInst {
   SolveIO io;

@@ -435,7 +435,9 @@ __global__ void __launch_bounds__(TL * G, TL > 1 ? 1 : (G >= 512 ? 2 : 3))
 // CTA walks the items grid-stride, skipping instances that no longer
 // iterate; the b_o norm (p'-x) and the pass norm are reduced per instance.
 template <int EQ, int SOLVER, int TL, int G>
-__global__ void __launch_bounds__(TL * G)
+__global__ void __launch_bounds__(TL * G, TL * G > 256                                                  ? 1
+                                          : batch_y_regs(EQ, TL, G) && SOLVER == IXB_SOLVER_HYBRID ? 2
+                                                                                                   : 768 / (TL * G))
     fused_batch_kernel(const FusedInst* __restrict__ inst, const int2* __restrict__ items, const int nitems,
                        const int* __restrict__ active, const BatchNorm bn_asm, const BatchNorm bn_sol) {
   IXB_PDL_ENTRY();
@@ -448,12 +450,29 @@ __global__ void __launch_bounds__(TL * G)
     if (!active[wi.x]) continue;  // uniform across the CTA
     const FusedInst& d = inst[wi.x];
     const int L0 = 1 + wi.y * TL;
-    double acc_bo = 0.0;
-    fused_assemble<EQ, SOLVER, TL, G, 0>(sm, d.G, d.io, d.s.io.m, d.s.io.mp, d.s.n, d.s.line_lo, d.s.line_hi, L0,
-                                         acc_bo);
-    __syncthreads();
-    const double acc = solve_lines<S, EqIsX<EQ>::value, ST::DC, false, TL, G, 0>(sm, d.s.io, d.s.n, d.s.line_lo,
-                                                                                d.s.line_hi, d.s.nfull, L0);
+    double acc_bo = 0.0, acc = 0.0;
+    if (batch_y_regs(EQ, TL, G) && d.s.io.m <= kBatchRegM) {
+      if constexpr (batch_y_regs(EQ, TL, G)) {
+        auto lines = [&](auto mc) {
+          return fused_y_lines<EQ, SOLVER, TL, G, decltype(mc)::value>(sm, d.G, d.io, d.s.io, d.s.n, d.s.line_lo,
+                                                                       d.s.line_hi, d.s.nfull, L0);
+        };
+        switch (d.s.io.m) {
+          case 3: acc = lines(std::integral_constant<int, 3>{}); break;
+          case 4: acc = lines(std::integral_constant<int, 4>{}); break;
+          case 5: acc = lines(std::integral_constant<int, 5>{}); break;
+          case 6: acc = lines(std::integral_constant<int, 6>{}); break;
+          case 7: acc = lines(std::integral_constant<int, 7>{}); break;
+          default: acc = lines(std::integral_constant<int, 8>{}); break;
+        }
+      }
+    } else {
+      fused_assemble<EQ, SOLVER, TL, G, 0>(sm, d.G, d.io, d.s.io.m, d.s.io.mp, d.s.n, d.s.line_lo, d.s.line_hi, L0,
+                                           acc_bo);
+      __syncthreads();
+      acc = solve_lines<S, EqIsX<EQ>::value, ST::DC, false, TL, G, 0>(sm, d.s.io, d.s.n, d.s.line_lo, d.s.line_hi,
+                                                                      d.s.nfull, L0);
+    }
     if (bn_asm.partials) finish_item_norm(bn_asm, wi.x, d.s.first, d.s.count, it, block_sum(acc_bo));
     if (bn_sol.partials) finish_item_norm(bn_sol, wi.x, d.s.first, d.s.count, it, block_sum(acc));
     __syncthreads();  // the next item reuses the shared memory
@@ -545,7 +564,7 @@ cudaError_t fused_batch_launch(int tl, int g, size_t smem, const FusedInst* inst
 #define IXB_FBATCH_(TL_, G_) \
   if (tl == TL_ && g == G_) return go(fused_batch_kernel<EQ, SOLVER, TL_, G_>, TL_ * G_);
   if constexpr (EqIsX<EQ>::value) {
-    IXB_FUSED_X_SHAPES(IXB_FBATCH_)
+    IXB_FUSED_BATCH_X_SHAPES(IXB_FBATCH_)
   } else {
     IXB_FUSED_Y_SHAPES(IXB_FBATCH_)
   }
