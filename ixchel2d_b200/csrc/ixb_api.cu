@@ -86,32 +86,48 @@ int ensure_tables(ixb_handle* h) {
 
 
 // Default launch shape of a sweep, from per-shape timings of every sweep on
-// 64x64, 256x256 and 701x301 grids in both precision forms: x-lines one per
-// CTA with 256 threads for lines of more than 384 rows, else 128; y-lines in
-// the fused form with the fewest of 4, 5, 6 or 8 adjacent lines per CTA that
-// keeps one CTA per SM (8 beyond that), and 128 threads per line for lines
-// of 160 rows or more, else 64 (at 701x301: 5 x 128, one CTA on each of 141
-// SMs, where 8 x 128 leaves 60 SMs idle; the u-y sweep measured 17.5 against
-// 19.3 us, the other y-sweeps within 1 %).
-// Those shapes were within about 5 % of the best (at worst 15 %, binary64
-// y-sweeps at 701x301), where the rule below was 20-50 % behind.  When the
-// shape cannot be resident: the fewest waves of CTAs, then the shortest
-// chunks, then the most SMs busy (CTAs up to the SM count), then the larger CTA.
+// 64x64 to 2000x600 grids in both precision forms: x-lines one per CTA with
+// 256 threads for lines of more than 384 rows, else 128 (512 threads at
+// 1501x1001: u-x 36.9 against 33.3 us, and 51.2 against 43.6 at 2000x600);
+// y-lines in the fused form with 128 threads per line for lines of 160 rows
+// or more, else 64, and 4, 5, 6 or 8 adjacent lines per CTA: a CTA fills its
+// SM, and a wave of them measured nearly (lines + 4) times a constant of the
+// grid (refined 1501x1001 u-y, per wave: 17.7, 19.6, 23.0, 28.1 us for 4, 5,
+// 6, 8 lines; 2000x600: 9.5, 11.2, 12.6, 14.8), so the least waves x
+// (lines + 4) is taken among those that can be resident (binary64 900x700
+// u-y 25.2 us with 4 x 128 against 33.4 for the rule below).
+// When none can: the fewest waves of CTAs, then the shortest chunks, then
+// the most SMs busy (CTAs up to the SM count), then the larger CTA; the
+// refined form goes there from the widest shape already, because its
+// binary32 solves depend on the threads per line.
 void pick_shape(ixb_handle* h, int eq) {
   {
     const bool x = (eq & 1) != 0;
     SweepShape probe = sweep_shape(eq, h->mi, h->nj, real_bytes(h), 1, 128);
     const int lines = probe.nfull, n = probe.n;
-    int tl = 1;
-    if (!x) {
-      tl = 8;
-      for (const int t : {4, 5, 6})
-        if ((lines + t - 1) / t <= h->nsm) { tl = t; break; }
-    }
     const int g = x ? (n > 384 ? 256 : 128) : (n >= 160 ? 128 : 64);
-    const SweepShape s = sweep_shape(eq, h->mi, h->nj, real_bytes(h), tl, g);
-    if (sweep_occupancy(eq, solver_form(h), s) > 0) {
-      h->shape_tl[eq] = tl;
+    const bool mixed = solver_form(h) == SOLVER_MIXED;
+    auto resident = [&](int tl) {
+      return sweep_occupancy(eq, solver_form(h), sweep_shape(eq, h->mi, h->nj, real_bytes(h), tl, g)) > 0;
+    };
+    int best_tl = 0;
+    if (x) {
+      if (resident(1)) best_tl = 1;
+    } else {
+      int first = 8;
+      for (const int t : {6, 5, 4})
+        if ((lines + t - 1) / t <= h->nsm) first = t;
+      long long best_cost = 0;
+      for (const int t : {4, 5, 6, 8}) {
+        const long long waves = ((lines + t - 1) / t + h->nsm - 1) / h->nsm, cost = waves * (t + 4);
+        if ((best_tl && cost >= best_cost) || !resident(t)) continue;
+        best_tl = t;
+        best_cost = cost;
+      }
+      if (mixed && !resident(first)) best_tl = 0;
+    }
+    if (best_tl) {
+      h->shape_tl[eq] = best_tl;
       h->shape_g[eq] = g;
       return;
     }

@@ -735,7 +735,13 @@ struct Chunk {
 // TOMS 42(4), 2016).  Reciprocals use fast_rcp (two Newton steps).  The
 // solution replaces the right-hand side.  Called by all TL*G threads;
 // threads of lines with `active` false only take part in the barriers.
-template <class R, int G, int TL = 1, int M = 0>
+// ALIAS (compile-time chunk): the reduced system takes the place of the
+// coefficients, which are in registers by then; it ends before the
+// right-hand sides (binary64 keeps 9G of it, binary32 12G, the first three
+// row arrays hold 3*G*mp).
+template <class R, int M>
+__host__ __device__ constexpr bool chunk_alias() { return M > 0 && (sizeof(R) == 8 ? 3 : 4) <= (M | 1); }
+template <class R, int G, int TL = 1, int M = 0, bool ALIAS = false>
 __device__ __forceinline__ void chunk_solve(R* line, int m, int mp, bool active) {
   const int k = threadIdx.x % G;
   constexpr bool HALF = sizeof(R) == 8;
@@ -743,7 +749,8 @@ __device__ __forceinline__ void chunk_solve(R* line, int m, int mp, bool active)
   R* b = a + (size_t)G * mp;
   R* c = b + (size_t)G * mp;
   R* d = c + (size_t)G * mp;
-  R* red = line + (size_t)4 * G * mp;
+  static_assert(!ALIAS || chunk_alias<R, M>(), "the reduced system would reach the right-hand sides");
+  R* red = line + (ALIAS ? (size_t)0 : (size_t)4 * G * mp);
   R x0, xl;
   if constexpr (M > 0) {
     Chunk<R, M> ch;
@@ -753,6 +760,7 @@ __device__ __forceinline__ void chunk_solve(R* line, int m, int mp, bool active)
       if (active) { ch.a[i] = a[i]; ch.b[i] = b[i]; ch.c[i] = c[i]; ch.d[i] = d[i]; }
     }
     ch.eliminate();
+    if constexpr (ALIAS) line_sync<G, TL>(false);  // every chunk is in registers
     reduced_pcr<R, HALF>(red, G, 1, G, k, k, active, ch.eA, ch.eC, ch.eD, ch.oA, ch.oC, ch.oD, x0, xl,
                          [](bool q) { return line_sync<G, TL>(q); });
     if (active) {

@@ -16,7 +16,7 @@ namespace ixb {
 // ||new - prev||^2 over the interior rows of the solved lines.  y-lines are
 // written TL adjacent ii at a time.  Called by all threads of the CTA (it
 // holds barriers).
-template <class S, bool X, bool DC, bool EXACT, int TL, int G, int M>
+template <class S, bool X, bool DC, bool EXACT, int TL, int G, int M, bool ALIAS = false>
 __device__ __forceinline__ double solve_lines(S* sm, const SolveIO& io, const int n, const int line_lo,
                                               const int line_hi, const int nfull, const int L0) {
   constexpr int NT = TL * G;
@@ -32,7 +32,7 @@ __device__ __forceinline__ double solve_lines(S* sm, const SolveIO& io, const in
     if constexpr (EXACT) {
       if (active && threadIdx.x % G == 0) thomas_exact(line, line + arr, line + 2 * arr, line + 3 * arr, n, m, mp);
     } else {
-      chunk_solve<S, G, TL, M>(line, m, mp, active);
+      chunk_solve<S, G, TL, M, ALIAS>(line, m, mp, active);
     }
   }
   __syncthreads();

@@ -397,8 +397,8 @@ __global__ void __launch_bounds__(TL * G, TL > 1 ? 1 : (G >= 512 ? 2 : 3))
   } else {
     fused_assemble<EQ, SOLVER, TL, G, M>(sm, G_, io, m, mp, n, line_lo, line_hi, L0, acc_bo);
     __syncthreads();
-    acc = solve_lines<S, EqIsX<EQ>::value, ST::DC, SOLVER == IXB_SOLVER_EXACT, TL, G, M>(sm, so, n, line_lo, line_hi,
-                                                                                        nfull, L0);
+    acc = solve_lines<S, EqIsX<EQ>::value, ST::DC, SOLVER == IXB_SOLVER_EXACT, TL, G, M, chunk_alias<S, M>()>(
+        sm, so, n, line_lo, line_hi, nfull, L0);
   }
   if constexpr (EQ == EQ_TX) {
     if (so.res.resu) {
@@ -516,6 +516,14 @@ cudaError_t fused_go(const SweepShape& s, const Geo<double>& G, const SweepIO<do
   return launch_k(K, s.grid, s.tl * s.g, s.smem, st, G, io, so, s.n, s.line_lo, s.line_hi, s.nfull);
 }
 
+// Compile-time chunks (M) of up to 6 rows for x-lines of 256 threads and up to
+// 8 for y-lines of 4 x 128: the chunk is in registers while the reduced
+// system is solved, so an x-line's shared memory is its staged rows alone
+// (1501 rows binary64: 57 instead of 82 KB, three CTAs per SM instead of
+// two) and a y-line's the reduced system alone (36 instead of 196 KB).
+// Measured against the run-time chunk at 1501x1001 binary64: u-x 49.6 ->
+// 33.3, v-x 73.2 -> 47.1, p'-x 65.0 -> 42.5, T-x 57.7 -> 38.3, u-y 53.4 ->
+// 45.4, p'-y 49.0 -> 38.5 us.
 // Launches the fused form of sweep EQ for the shapes of IXB_FUSED_X_SHAPES /
 // IXB_FUSED_Y_SHAPES; any other shape: cudaErrorNotSupported (the caller
 // runs the two-kernel sweep).
@@ -528,10 +536,23 @@ cudaError_t fused_launch(const SweepShape& s, const Geo<double>& G, const SweepI
   if (s.tl == TL_ && s.g == G_) {                                                               \
     if constexpr (!EXACT) {                                                                     \
       SweepShape r = s;                                                                         \
-      if constexpr (!EqIsX<EQ>::value) r.smem = fused_y_smem<S, TL_, G_>();                     \
+      if (!EqIsX<EQ>::value) r.smem = fused_y_smem<S, TL_, G_>();                               \
+      else if (s.m > 3 || chunk_alias<S, 3>()) r.smem = sizeof(S) * 4 * G_ * s.mp;              \
       if (s.m == 3) return fused_go<fused_sweep_kernel<EQ, SOLVER, TL_, G_, 3>>(r, G, io, so, st); \
       if constexpr (!EqIsX<EQ>::value)                                                          \
         if (s.m == 5) return fused_go<fused_sweep_kernel<EQ, SOLVER, TL_, G_, 5>>(r, G, io, so, st); \
+      if constexpr (EqIsX<EQ>::value && G_ == 256) {                                            \
+        if (s.m == 4) return fused_go<fused_sweep_kernel<EQ, SOLVER, TL_, G_, 4>>(r, G, io, so, st); \
+        if (s.m == 5) return fused_go<fused_sweep_kernel<EQ, SOLVER, TL_, G_, 5>>(r, G, io, so, st); \
+        if (s.m == 6) return fused_go<fused_sweep_kernel<EQ, SOLVER, TL_, G_, 6>>(r, G, io, so, st); \
+      }                                                                                         \
+      if constexpr (!EqIsX<EQ>::value && TL_ <= 6 && G_ == 128)                                 \
+        if (s.m == 4) return fused_go<fused_sweep_kernel<EQ, SOLVER, TL_, G_, 4>>(r, G, io, so, st); \
+      if constexpr (!EqIsX<EQ>::value && TL_ == 4 && G_ == 128) {                                \
+        if (s.m == 6) return fused_go<fused_sweep_kernel<EQ, SOLVER, TL_, G_, 6>>(r, G, io, so, st); \
+        if (s.m == 7) return fused_go<fused_sweep_kernel<EQ, SOLVER, TL_, G_, 7>>(r, G, io, so, st); \
+        if (s.m == 8) return fused_go<fused_sweep_kernel<EQ, SOLVER, TL_, G_, 8>>(r, G, io, so, st); \
+      }                                                                                         \
     }                                                                                           \
     return fused_go<fused_sweep_kernel<EQ, SOLVER, TL_, G_, 0>>(s, G, io, so, st);                \
   }

@@ -40,6 +40,17 @@ def test_partition_edges(has_gpu, mi, nj, prec):
             assert d < 1e-4, (k, d)
 
 
+# lines beyond the resident loop's: chunks of 4 to 9 rows, and grids whose y-lines come 4, 5, 6 or 8 per CTA
+LONG = [(1023, 6), (1025, 5), (1280, 7), (1281, 6), (1536, 5), (1537, 6), (1700, 4), (6, 512), (7, 513), (6, 641),
+        (5, 768), (6, 896), (7, 1024), (6, 1025), (700, 400), (820, 500), (900, 390), (1250, 400)]
+
+
+@pytest.mark.parametrize("mi,nj", LONG)
+@pytest.mark.parametrize("prec", [F.PREC_FP64, F.PREC_FP32_REFINED])
+def test_longer_lines(has_gpu, mi, nj, prec):
+    test_partition_edges(has_gpu, mi, nj, prec)
+
+
 # batched line solves (device pointers): unaligned starts and ends (odd n, arrays that begin inside a
 # 16-byte granule), the edges of the chunk sizes and of the 128-row blocks, ragged system groups, one
 # system; x must be written everywhere and nothing beside it
