@@ -315,8 +315,7 @@ int ixb_tridiag_f64_noalloc(const double* a, const double* b, const double* c, c
  * grad[jj-1] = d nu0 / d value(jj), jj = 1..nj+1 (zero where the line is not
  * solved).  The map is affine in T with u, v fixed, so the gradient is exact
  * (transposed line solves, no stored forward states); the state is left
- * unchanged; IXB_ETIMEOUT if a transposed line solve's copies did not arrive
- * within their bounded wait.  ixb_set_bc_values sets the per-line values of one side of a
+ * unchanged.  ixb_set_bc_values sets the per-line values of one side of a
  * boundary table (a per-node profile, beyond the reference's 15 segments),
  * keeping each line's type. */
 /* ---- discrete adjoint of the full coupled SIMPLE iteration ----

@@ -12,6 +12,12 @@
 // mu = A^-T lambda (a transposed batched line solve) followed by
 // lambda_in = R^T mu plus the lines the sweep copies, and the side-a
 // boundary rows of the x-sweeps collect d Nu / d value += mu[row 0].
+// A reversed sweep is one kernel that reads the sweep reversed before it as
+// its mu and forms that one's R^T mu while it loads its right-hand sides, so
+// that neither lambda nor the transposed rows pass through memory: 2
+// launches and 6 loads per row and pass where staging, solving and
+// scattering took 6 launches (256 x 256, 200 passes with the forward run:
+// 7.8 ms then).
 // Built with FMA contraction, like the fast forward assembly, whose
 // coefficients it re-evaluates.  ixb_adjoint_energy_coupled extends this to
 // K outer SIMPLE iterations of a flow that evolves but does not depend on
@@ -58,79 +64,118 @@ struct Sweep {
   const BCEntry* last;
 };
 
-// Forward row r of solved line L: (a, b, c) of impone_cond_frontera's boundary
-// rows or of the energy assembly.
-__device__ __forceinline__ void fwd_row(const Geo<double>& G, const Sweep& s, const double* coef, size_t fsz, int L,
-                                        int r, double& a, double& b, double& c) {
-  if (r == 0) {
-    const BCEntry e = s.first[L];
-    a = 0.0; b = e.type == 2 ? -1.0 : 1.0; c = e.type == 2 ? 1.0 : 0.0;
-  } else if (r == s.n - 1) {
-    const BCEntry e = s.last[L];
-    a = e.type == 2 ? -1.0 : 0.0; b = 1.0; c = 0.0;
-  } else {
-    const int c0 = s.x ? G.at(r + 1, L) : G.at(L, r + 1);
-    a = coef[(s.x ? C_AI : C_BS) * fsz + c0];
-    c = coef[(s.x ? C_AD : C_BN) * fsz + c0];
-    b = coef[C_DG * fsz + c0];
-  }
-}
-
-// Transposed rows (a'_r = c_{r-1}, b'_r = b_r, c'_r = a_{r+1}) and right-hand
-// side lambda of every solved line, contiguous per line.
-__global__ void adj_stage_kernel(const Geo<double> G, const Sweep s, const double* __restrict__ coef, size_t fsz,
-                                 const double* __restrict__ lam, double* __restrict__ ta, double* __restrict__ tb,
-                                 double* __restrict__ tc, double* __restrict__ td) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= s.nl * s.n) return;
-  const int li = idx / s.n, r = idx - li * s.n, L = li + 2;
-  double a, b, c, t;
-  fwd_row(G, s, coef, fsz, L, r, a, b, c);
-  ta[idx] = 0.0;
-  tc[idx] = 0.0;
-  if (r > 0) { fwd_row(G, s, coef, fsz, L, r - 1, t, t, c); ta[idx] = c; }
-  if (r < s.n - 1) { fwd_row(G, s, coef, fsz, L, r + 1, a, t, t); tc[idx] = a; }
-  fwd_row(G, s, coef, fsz, L, r, a, b, c);
-  tb[idx] = b;
-  td[idx] = lam[s.x ? G.at(r + 1, L) : G.at(L, r + 1)];
-}
-
-// lambda_in = R^T mu + copies of the unsolved lines; x-sweeps also add the
-// side-a boundary rows' sensitivities to grad (indexed by line).
-__global__ void adj_scatter_kernel(const Geo<double> G, const Sweep s, const double* __restrict__ coef, size_t fsz,
-                                   double rel, const double* __restrict__ mu, const double* __restrict__ lam_out,
-                                   double* __restrict__ lam_in, double* __restrict__ grad) {
-  const int nx = G.mi + 1, ny = G.nj + 1;
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= nx * ny) return;
-  const int ii = 1 + idx % nx, jj = 1 + idx / nx;
-  const int L = s.x ? jj : ii;  // line of this cell
-  const int r = s.x ? ii - 1 : jj - 1;
-  const int nfull = s.nl + 2;
+// lambda at a cell after sweep `s` was reversed: R^T mu + the lines it copies.
+// `f` holds mu on the solved lines and lambda on the copied ones.
+__device__ __forceinline__ double lambda_at(const Geo<double>& G, const Sweep& s, const double* coef, size_t fsz,
+                                            double keep, const double* f, int ii, int jj) {
+  const int L = s.x ? jj : ii, r = s.x ? ii - 1 : jj - 1, st = s.x ? G.LD : 1;
+  const int c0 = G.at(ii, jj);
   auto solved = [&](int l) { return l >= 2 && l <= s.nl + 1; };
-  auto mu_at = [&](int l, int rr) { return mu[(size_t)(l - 2) * s.n + rr]; };
   const bool interior = r >= 1 && r <= s.n - 2;
   double v = 0.0;
-  if (L >= 1 && L <= nfull) {
-    if (solved(L)) {
-      if (interior) v += coef[C_DG * fsz + G.at(ii, jj)] * (1.0 - rel) * mu_at(L, r);
-      if (s.x && r == 0) grad[L] += mu_at(L, 0);
-    } else {
-      v += lam_out[G.at(ii, jj)];
-    }
-    // rows of the neighbouring lines that read this cell through d
-    if (interior) {
-      if (solved(L + 1)) {
-        const int cn = s.x ? G.at(ii, jj + 1) : G.at(ii + 1, jj);
-        v -= coef[(s.x ? C_BS : C_AI) * fsz + cn] * mu_at(L + 1, r);
+  if (!solved(L)) v = __ldg(f + c0);
+  else if (interior) v = coef[C_DG * fsz + c0] * keep * __ldg(f + c0);
+  // rows of the neighbouring lines that read this cell through d
+  if (interior && solved(L + 1)) v -= coef[(s.x ? C_BS : C_AI) * fsz + c0 + st] * __ldg(f + c0 + st);
+  if (interior && solved(L - 1)) v -= coef[(s.x ? C_BN : C_AD) * fsz + c0 - st] * __ldg(f + c0 - st);
+  return v;
+}
+
+__global__ void adj_lambda_kernel(const Geo<double> G, const Sweep s, const double* __restrict__ coef, size_t fsz,
+                                  double keep, const double* __restrict__ f, double* __restrict__ lam) {
+  const int ii = 1 + blockIdx.x * blockDim.x + threadIdx.x, jj = 1 + blockIdx.y;
+  if (ii <= G.mi + 1) lam[G.at(ii, jj)] = lambda_at(G, s, coef, fsz, keep, f, ii, jj);
+}
+
+// One sweep reversed: CTA = TL adjacent lines, thread t: chunk t / TL (M rows)
+// of line L0 + t % TL, in registers from the loads to mu.  The right-hand
+// sides are lambda after the sweep `prev` (FIRST: `f` is lambda itself); the
+// matrix is the transposed one (a'_r = c_{r-1}, b'_r = b_r, c'_r = a_{r+1}).
+// Bound by latency: one wave of CTAs, a chunk's loads, the reduced system.
+template <bool X, bool FIRST, int TL, int GT, int M>
+__global__ void __launch_bounds__(TL * GT)
+    adj_sweep_kernel(const Geo<double> G, const Sweep s, const Sweep prev, const double* __restrict__ coef, size_t fsz,
+                     double keep, const double* __restrict__ f, double* __restrict__ mu, double* __restrict__ grad) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double* red = reinterpret_cast<double*>(smem_raw);
+  const int t = threadIdx.x, l = t % TL, k = t / TL, L = 1 + blockIdx.x * TL + l;
+  const bool active = L >= 2 && L <= s.nl + 1, there = L <= s.nl + 2;
+  const double *ca = coef + (X ? C_AI : C_BS) * fsz, *cc = coef + (X ? C_AD : C_BN) * fsz, *cd = coef + C_DG * fsz;
+  const int c00 = X ? G.at(1, L) : G.at(L, 1), st = X ? 1 : G.LD;
+  int t0 = 1, t1 = 1;  // boundary row types
+  if (active) { t0 = s.first[L].type; t1 = s.last[L].type; }
+  Chunk<double, M> ch;
+#pragma unroll
+  for (int it = 0; it < M; ++it) {
+    const int r = k * M + it, c0 = c00 + r * st;
+    double a = 0.0, b = 1.0, c = 0.0, d = 0.0;
+    if (there && r < s.n) {
+      const int ii = X ? r + 1 : L, jj = X ? L : r + 1;
+      d = FIRST ? __ldg(f + c0) : lambda_at(G, prev, coef, fsz, keep, f, ii, jj);
+      if (!active) {
+        mu[c0] = d;
+        d = 0.0;
+      } else {
+        if (r == 0) b = t0 == 2 ? -1.0 : 1.0;
+        else if (r < s.n - 1) b = __ldg(cd + c0);
+        if (r == 1) a = t0 == 2 ? 1.0 : 0.0;
+        else if (r > 1) a = __ldg(cc + c0 - st);
+        if (r == s.n - 2) c = t1 == 2 ? -1.0 : 0.0;
+        else if (r < s.n - 2) c = __ldg(ca + c0 + st);
       }
-      if (solved(L - 1)) {
-        const int cp = s.x ? G.at(ii, jj - 1) : G.at(ii - 1, jj);
-        v -= coef[(s.x ? C_BN : C_AD) * fsz + cp] * mu_at(L - 1, r);
-      }
     }
+    ch.a[it] = a; ch.b[it] = b; ch.c[it] = c; ch.d[it] = d;
   }
-  lam_in[G.at(ii, jj)] = v;
+  ch.eliminate();
+  double x0, xl;
+  reduced_pcr<double, true>(red, TL * GT, TL, GT, t, k, active, ch.eA, ch.eC, ch.eD, ch.oA, ch.oC, ch.oD, x0, xl,
+                            [](bool q) { return (bool)__syncthreads_or(q); });
+  ch.substitute(x0, xl);
+  if (!active) return;
+#pragma unroll
+  for (int it = 0; it < M; ++it) {
+    const int r = k * M + it;
+    if (r < s.n) mu[c00 + r * st] = ch.d[it];
+    if (X && r == 0) grad[L] += ch.d[it];
+  }
+}
+
+struct SweepArgs {
+  Geo<double> G;
+  Sweep s, prev;
+  const double* coef;
+  size_t fsz;
+  double keep;
+  const double* f;
+  double* mu;
+  double* grad;
+};
+
+template <bool X, bool FIRST, int TL, int GT, int M>
+cudaError_t adj_sweep_go(const SweepArgs& q, cudaStream_t st) {
+  auto k = adj_sweep_kernel<X, FIRST, TL, GT, M>;
+  const size_t smem = (size_t)9 * TL * GT * sizeof(double);
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  k<<<(q.s.nl + 2 + TL - 1) / TL, TL * GT, smem, st>>>(q.G, q.s, q.prev, q.coef, q.fsz, q.keep, q.f, q.mu, q.grad);
+  return cudaGetLastError();
+}
+
+// The fewest threads that leave 3 rows each, up to 256 per x-line and 128 per
+// y-line (four of them make 32-byte pieces of a row), then longer chunks;
+// lines beyond those by 1024 threads.  A line has at most 6001 rows.
+template <bool X, bool FIRST>
+cudaError_t adj_sweep(const SweepArgs& q, cudaStream_t st) {
+  constexpr int TL = X ? 1 : 4, GM = X ? 256 : 128;
+  const int n = q.s.n;
+  if (n <= 192) return adj_sweep_go<X, FIRST, TL, 64, 3>(q, st);
+  if (n <= 384) return adj_sweep_go<X, FIRST, TL, 128, 3>(q, st);
+  if (X && n <= 768) return adj_sweep_go<X, FIRST, TL, GM, 3>(q, st);
+  if (n <= 4 * GM) return adj_sweep_go<X, FIRST, TL, GM, 4>(q, st);
+  if (n <= 6 * GM) return adj_sweep_go<X, FIRST, TL, GM, 6>(q, st);
+  if (n <= 8 * GM) return adj_sweep_go<X, FIRST, TL, GM, 8>(q, st);
+  if (n <= 3072) return adj_sweep_go<X, FIRST, 1, 1024, 3>(q, st);
+  return adj_sweep_go<X, FIRST, 1, 1024, 6>(q, st);
 }
 
 }  // namespace
@@ -159,18 +204,16 @@ namespace {
 struct AdjCtx {
   ixb_handle* h;
   size_t fsz = 0;
-  double *coef = nullptr, *lam = nullptr, *lam2 = nullptr, *ta = nullptr, *tb = nullptr, *tc = nullptr,
-         *td = nullptr, *mu = nullptr, *gd = nullptr;
+  double *coef = nullptr, *lam = nullptr, *mx = nullptr, *my = nullptr, *gd = nullptr;
   Geo<double> G{};
   Sweep sx{}, sy{};
-  double rel = 0.0;
-  int cells = 0;
+  double keep = 0.0;     // 1 - relaxation
+  bool started = false;  // the T-y sweep reversed last left its mu in my; else lam holds lambda
 
   int init(int j0, int j1) {
     const int mi = h->mi, nj = h->nj;
     fsz = h->fsz;
-    const size_t nst = (size_t)std::max((nj - 1) * (mi + 1), (mi - 1) * (nj + 1));
-    const size_t need = (C_COUNT + 2) * fsz + 5 * nst + (size_t)(nj + 2);
+    const size_t need = (C_COUNT + 3) * fsz + (size_t)(nj + 2);
     if (h->adj_size < need) {
       if (h->adj_pool) cudaFree(h->adj_pool);
       h->adj_pool = nullptr;
@@ -180,19 +223,15 @@ struct AdjCtx {
     }
     coef = h->adj_pool;
     lam = coef + C_COUNT * fsz;
-    lam2 = lam + fsz;
-    ta = lam2 + fsz;
-    tb = ta + nst;
-    tc = tb + nst;
-    td = tc + nst;
-    mu = td + nst;
-    gd = mu + nst;
+    mx = lam + fsz;
+    my = mx + fsz;
+    gd = my + fsz;
+    started = false;
     G = handle_geo(h);
     const BCEntry* base = h->bc + (size_t)2 * 4 * h->bcstride;  // T tables, sides a b c d
     sx = Sweep{true, mi + 1, nj - 1, base + 0 * (size_t)h->bcstride, base + 2 * (size_t)h->bcstride};
     sy = Sweep{false, nj + 1, mi - 1, base + 1 * (size_t)h->bcstride, base + 3 * (size_t)h->bcstride};
-    rel = h->prm.rel_ener;
-    cells = (mi + 1) * (nj + 1);
+    keep = 1.0 - h->prm.rel_ener;
     // the objective's weights: Nu is linear in T (the wall-normal 3-point
     // derivative integrated panel by panel), evaluated here on unit fields
     std::vector<double> along(nj + 2, 0.0), across(mi + 2, 0.0);
@@ -200,18 +239,22 @@ struct AdjCtx {
     for (int i = 1; i <= mi + 1; ++i) across[i] = h->xp[i - 1];
     std::vector<double> w((size_t)fsz, 0.0);
     for (int k = j0; k <= j1 + 2; ++k)
-      for (int l = 1; l <= 3; ++l) {
-        auto f = [&](int kk, int ll) { return (kk == k && ll == l) ? 1.0 : 0.0; };
-        w[(size_t)(k - 1) * h->LD + (l - 1)] = nusselt_wall(f, along.data(), across.data(), mi + 1, 0, 0, j0, j1);
-      }
+      for (int l = 1; l <= 3; ++l)
+        w[(size_t)(k - 1) * h->LD + (l - 1)] = nusselt_weight(along.data(), across.data(), mi + 1, j0, j1, k, l);
     ACK(cudaMemcpyAsync(lam, w.data(), fsz * sizeof(double), cudaMemcpyHostToDevice, h->stream));
     ACK(cudaMemsetAsync(gd, 0, (nj + 2) * sizeof(double), h->stream));
     ACK(cudaStreamSynchronize(h->stream));  // w leaves scope
     return IXB_OK;
   }
 
-  // coefficients of the energy rows at the handle's current velocities
+  // coefficients of the energy rows at the handle's current velocities; the
+  // last reversed sweep's lambda is formed with the ones it ran with first
   int coefficients() {
+    if (started) {
+      adj_lambda_kernel<<<dim3((h->mi + 1 + 127) / 128, h->nj + 1), 128, 0, h->stream>>>(G, sy, coef, fsz, keep, my, lam);
+      ACK(cudaGetLastError());
+      started = false;
+    }
     const int cT = h->cT;
     SweepIO<double> io = handle_sweep_io(h, EQ_TX, nullptr);
     h->cT = cT;
@@ -222,20 +265,14 @@ struct AdjCtx {
     return IXB_OK;
   }
 
-  int reverse(const Sweep& s, const double* lam_out, double* lam_in) {
-    const int rows = s.nl * s.n;
-    adj_stage_kernel<<<(rows + 255) / 256, 256, 0, h->stream>>>(G, s, coef, fsz, lam_out, ta, tb, tc, td);
-    ACK(cudaGetLastError());
-    ACK(tridiag_f64(ta, tb, tc, td, mu, s.n, s.nl, 0, IXB_SOLVER_HYBRID, h->stream));
-    adj_scatter_kernel<<<(cells + 255) / 256, 256, 0, h->stream>>>(G, s, coef, fsz, rel, mu, lam_out, lam_in, gd);
-    ACK(cudaGetLastError());
-    return IXB_OK;
-  }
-
   // one (T-y, T-x) pass, reversed: T-x first
   int pass() {
-    const int r1 = reverse(sx, lam, lam2);
-    return r1 != IXB_OK ? r1 : reverse(sy, lam2, lam);
+    const SweepArgs x{G, sx, sy, coef, fsz, keep, started ? my : lam, mx, gd};
+    const SweepArgs y{G, sy, sx, coef, fsz, keep, mx, my, gd};
+    ACK((started ? adj_sweep<true, false>(x, h->stream) : adj_sweep<true, true>(x, h->stream)));
+    ACK((adj_sweep<false, false>(y, h->stream)));
+    started = true;
+    return IXB_OK;
   }
 
   int finish(double* grad) {
@@ -243,9 +280,6 @@ struct AdjCtx {
     std::vector<double> g(nj + 2);
     ACK(cudaMemcpyAsync(g.data(), gd, (nj + 2) * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     ACK(cudaStreamSynchronize(h->stream));
-    int timed_out = 0;
-    ACK(tridiag_take_timeout(&timed_out));  // a line solve whose copies did not arrive in time
-    if (timed_out) return IXB_ETIMEOUT;
     for (int jj = 1; jj <= nj + 1; ++jj) grad[jj - 1] = g[jj];
     return IXB_OK;
   }
@@ -268,21 +302,23 @@ extern "C" int ixb_adjoint_energy(ixb_handle* h, int K, int j0, int j1, double* 
   AdjCtx A{h};
   TRY(A.init(j0, j1));
   TRY(A.coefficients());  // the frozen velocities
-  // K passes of (T-y, T-x), reversed.  A WHILE graph runs them kLoopUnroll
-  // at a time (rebuilt when the handle or its workspace changes); the
-  // remaining K mod kLoopUnroll are plain launches
+  // K passes of (T-y, T-x), reversed: the first reads the objective's weights,
+  // a WHILE graph runs the others kLoopUnroll at a time (rebuilt when the
+  // handle or its workspace changes), the remaining ones are plain launches
+  if (K > 0) TRY(A.pass());
+  const int left = std::max(K - 1, 0);
   const std::function<int()> pass = [&A]() -> int { return A.pass(); };
-  if (K >= kLoopUnroll) {
+  if (left >= kLoopUnroll) {
     if (h->agraph_dirty || !h->agraph_exec || h->agraph_pool != h->adj_pool) {
       const int r = handle_build_loop_graph(h, pass, kLoopUnroll, &h->agraph, &h->agraph_exec);
       if (r != IXB_OK) return r;
       h->agraph_dirty = false;
       h->agraph_pool = h->adj_pool;
     }
-    const int r = handle_run_loop_graph(h, h->agraph_exec, K / kLoopUnroll);
+    const int r = handle_run_loop_graph(h, h->agraph_exec, left / kLoopUnroll);
     if (r != IXB_OK) return r;
   }
-  for (int k = 0; k < K % kLoopUnroll; ++k) TRY(pass());
+  for (int k = 0; k < left % kLoopUnroll; ++k) TRY(pass());
   return A.finish(grad);
 }
 

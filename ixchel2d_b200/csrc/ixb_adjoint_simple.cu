@@ -605,10 +605,8 @@ struct SimpleAdjoint {
     for (int i = 1; i <= mi + 1; ++i) across[i] = h->xp[i - 1];
     std::vector<double> w(fsz, 0.0);
     for (int k = j0; k <= j1 + 2; ++k)
-      for (int l = 1; l <= 3; ++l) {
-        auto f = [&](int kk, int ll) { return (kk == k && ll == l) ? 1.0 : 0.0; };
-        w[(size_t)(k - 1) * h->LD + (l - 1)] = nusselt_wall(f, along.data(), across.data(), mi + 1, 0, 0, j0, j1);
-      }
+      for (int l = 1; l <= 3; ++l)
+        w[(size_t)(k - 1) * h->LD + (l - 1)] = nusselt_weight(along.data(), across.data(), mi + 1, j0, j1, k, l);
     SCK(cudaMemcpyAsync(adj.f[F_T], w.data(), fsz * sizeof(double), cudaMemcpyHostToDevice, h->stream));
     SCK(cudaStreamSynchronize(h->stream));
     return IXB_OK;

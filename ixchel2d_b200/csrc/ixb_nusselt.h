@@ -54,4 +54,20 @@ __host__ __device__ double nusselt_wall(F f, const double* along, const double* 
   return -nu;
 }
 
+// d nusselt_wall(f, ..., wall 0, no quirk, k0, k1) / d f(k, l): its value on
+// the unit field of (k, l), of which only the panels that reach position k
+// are not zero (summing all panels for every k was most of the host time of
+// a gradient: 1.2 ms at 257 positions).
+inline double nusselt_weight(const double* along, const double* across, int n_across, int k0, int k1, int k, int l) {
+  const auto f = [&](int kk, int ll) { return kk == k && ll == l ? 1.0 : 0.0; };
+  double nu = 0.0;
+  for (int ii = k - 2; ii <= k; ++ii) {
+    if (ii < k0 || ii > k1 || (ii - k0) % 2 != 0) continue;
+    double t[3];
+    nusselt_panel(f, along, across, n_across, 0, 0, k1, ii, t);
+    nu = nu + t[0] + t[1] + t[2];
+  }
+  return -nu;
+}
+
 }  // namespace ixb
