@@ -813,17 +813,23 @@ void scratch_trim() {
 // arrives as four tiles (a, b, c, d; boxes of W x 256 rows, copied by the
 // tensor engine without multicast) in shared memory while the CTA is still
 // solving the previous group from registers.  Every thread eliminates its
-// 16 rows (modified Thomas) to two rows coupled to the neighbouring chunks.
-// The reduced rows of system w are solved in cluster rank w % Q (its owner)
-// by one warp (Thomas-PCR on 32 lanes): every CTA stages its reduced rows in
-// the owners' layout and sends each owner its runs by bulk shared-to-shared
-// copies that complete on the owner's mbarrier.  After a cluster barrier
-// every thread reads its two solutions back and back-substitutes into a
-// solution tile that the tensor engine stores.  The reduced rows are
-// double-buffered across groups.  Every wait on a copy is bounded
+// rows (modified Thomas) to two rows coupled to the neighbouring chunks; the
+// CTA sends the reduced rows of each system to its owner, cluster rank w % Q,
+// by one bulk shared-to-shared copy that completes on the owner's mbarrier.
+// All threads of every CTA solve the systems it owns (reduced_pcr: as many
+// chunks as threads) and each CTA of the cluster gets the solutions of its
+// chunks the same way; every thread back-substitutes into a solution tile
+// that the tensor engine stores.  No cluster barrier: rows of the next group
+// are sent only after the solutions of this one have come, so every buffer
+// has been read before it is written again (each wait follows from the one
+// before it).  Bound by this chain of some 7,000 cycles per group, one group
+// per SM at a time, with the tile copies under it.  Every wait on a copy is bounded
 // (g_tri_timeout, as above).  (SEG, ROWS) = (128, 256) for lines of up to
-// 2048 rows; (64, 512) above, which halves W and so the cluster size that
-// holds a 4096-row group (8 instead of 16 CTAs: more clusters fit the GPU).
+// 1024 rows; (64, 512) above, which halves W and so the cluster size that
+// holds a group (4096 rows: 8 instead of 16 CTAs; more clusters fit the GPU).
+// 4096 x 4096 binary64: 153 us, 4.4 TB/s on the 120 SMs that clusters of 8
+// fill; with each owned system on one warp and the solutions read across the
+// cluster between two barriers 213 us (2048 x 2048: 43.8 against 55.8).
 // ---------------------------------------------------------------------------
 namespace {
 
@@ -843,25 +849,20 @@ struct StridedCfg {
   static constexpr int T = W * C;                 // threads per CTA
   static constexpr int TILE = W * ROWS;           // elements per tile
   static constexpr int BOXES = ROWS / kStrBox;    // tile boxes per array
-  // The 2*C*Q reduced rows of a system are 32 lane chunks of m = C*Q/16
-  // rows, at pitch m + 2 (even, so that a chunk's two reduced rows are one
-  // aligned pair).  The owner of a system solves m rows per lane, so m is
-  // 4, 8 or 16 (warp_unit_solve): Q <= QMAX.
-  static constexpr int QMAX = (256 / C < W ? 256 / C : W) < 16 ? (256 / C < W ? 256 / C : W) : 16;
-  // one set of gathered reduced rows: a | c | d of the W / Q owned systems,
-  // W * (2C + 64 / Q) elements per array, at most W * (2C + 16) (Q = 4)
-  static constexpr int SETA = W * (2 * C + 16);
-  // a CTA's rows for one owned system of one owner are one run of (32 / Q)
-  // lane chunks: 2C + 64 / Q elements, at most 2C + 16 (Q = 4); W runs per array
-  static constexpr int RUN = 2 * C + 16;
+  static constexpr int QMAX = W < 16 ? W : 16;  // every CTA of a cluster owns W / Q systems
+  // an owner's reduced rows (W / Q systems of 2*C*Q rows, a | c | d per
+  // sender), and in their place the working arrays of reduced_pcr once read
+  static constexpr int RED = (sizeof(R) == 8 ? 9 : 12) * T;
+  static constexpr int RUN = 6 * C;  // what a CTA sends of one system: a | c | d of its C chunks
 };
 
-// shared memory (bytes): 4 input tiles, the solution tile, 2 sets of
-// gathered reduced rows, the outgoing runs, 3 mbarriers (tiles, 2 sets)
+// shared memory (bytes): 4 input tiles, the solution tile, the reduced
+// systems, outgoing rows (later outgoing solutions), incoming solutions,
+// 3 mbarriers (tiles, reduced rows, solutions)
 template <class R, int SEG, int ROWS>
 __host__ __device__ constexpr size_t strided_smem_bytes() {
   using SC = StridedCfg<R, SEG, ROWS>;
-  return ((size_t)5 * SC::TILE + 2 * 3 * (size_t)SC::SETA + 3 * (size_t)SC::W * SC::RUN) * sizeof(R) + 32;
+  return ((size_t)5 * SC::TILE + SC::RED + (6 + 2 + 2) * (size_t)SC::T) * sizeof(R) + 32;
 }
 
 __device__ __forceinline__ void tile_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
@@ -896,95 +897,6 @@ __device__ __forceinline__ void bulk_send(unsigned dst, const void* src, unsigne
                : "memory");
 }
 
-template <class R>
-__device__ __forceinline__ R shfl_up_r(R x, int d) { return __shfl_up_sync(0xffffffffu, x, d); }
-template <class R>
-__device__ __forceinline__ R shfl_dn_r(R x, int d) { return __shfl_down_sync(0xffffffffu, x, d); }
-
-// One warp solves a system of 32*m rows (m >= 2) with unit diagonals:
-// x_i + a_i x_{i-1} + c_i x_{i+1} = d_i, lane l's rows at l*pitch ..
-// l*pitch+m-1 of the arrays a, c, d.  Each lane eliminates its rows to the
-// first and last (modified Thomas, its intermediate
-// rows in the scratch arrays sa, sc, sd so that the inputs are only read),
-// the 64 rows are solved by PCR over register shuffles, and each lane
-// back-substitutes.  The solution replaces d.
-template <class R, int m>
-__device__ __forceinline__ void warp_unit_solve(const R* __restrict__ a, const R* __restrict__ c, R* __restrict__ d,
-                                                R* __restrict__ sa, R* __restrict__ sc, R* __restrict__ sd,
-                                                int pitch) {
-  const int lane = threadIdx.x & 31;
-  const R* la = a + lane * pitch;
-  const R* lc = c + lane * pitch;
-  R* ld = d + lane * pitch;
-  R* xa = sa + lane * pitch;
-  R* xc = sc + lane * pitch;
-  R* xd = sd + lane * pitch;
-  R eA, eC, eD, oA, oC, oD;
-  if constexpr (m == 2) {
-    eA = la[0]; eC = lc[0]; eD = ld[0];
-    oA = la[1]; oC = lc[1]; oD = ld[1];
-  } else {
-    // forward: rows 1..m-1 -> x_k + a'_k x_0 + c'_k x_{k+1} = d'_k
-    R ap = la[1], cp = lc[1], dp = ld[1];
-    xa[1] = ap; xc[1] = cp; xd[1] = dp;
-#pragma unroll
-    for (int k = 2; k < m; ++k) {
-      const R ak = la[k];
-      const R r = fast_rcp(fmaT(-ak, cp, R(1)));
-      ap = -ak * ap * r;
-      dp = fmaT(-ak, dp, ld[k]) * r;
-      cp = lc[k] * r;
-      xa[k] = ap; xc[k] = cp; xd[k] = dp;
-    }
-    oA = ap; oC = cp; oD = dp;
-    // backward: rows m-3..1 -> x_k + a''_k x_0 + c''_k x_{m-1} = d''_k
-    R an = xa[m - 2], cn = xc[m - 2], dn = xd[m - 2];
-#pragma unroll
-    for (int k = m - 3; k >= 1; --k) {
-      const R ck = xc[k];
-      dn = fmaT(-ck, dn, xd[k]);
-      an = fmaT(-ck, an, xa[k]);
-      cn = -ck * cn;
-      xa[k] = an; xc[k] = cn; xd[k] = dn;
-    }
-    const R c0 = lc[0];
-    const R r0 = fast_rcp(fmaT(-c0, an, R(1)));
-    eA = la[0] * r0; eC = -c0 * cn * r0; eD = fmaT(-c0, dn, ld[0]) * r0;
-  }
-  // PCR on the 64 interleaved rows (even: first rows, odd: last rows), unit
-  // diagonals kept by normalising every step
-  auto step = [](R& A, R& C, R& D, R lA, R lC, R lD, R hA, R hC, R hD) {
-    const R r = fast_rcp(fmaT(-C, hA, fmaT(-A, lC, R(1))));
-    const R nA = -A * lA * r, nC = -C * hC * r, nD = fmaT(-C, hD, fmaT(-A, lD, D)) * r;
-    A = nA; C = nC; D = nD;
-  };
-  {  // row stride 1: even rows see the odd row of lane-1 and their own; odd rows their own even and lane+1's
-    R lA = shfl_up_r(oA, 1), lC = shfl_up_r(oC, 1), lD = shfl_up_r(oD, 1);
-    R hA = shfl_dn_r(eA, 1), hC = shfl_dn_r(eC, 1), hD = shfl_dn_r(eD, 1);
-    if (lane == 0) { lA = R(0); lC = R(0); lD = R(0); }
-    if (lane == 31) { hA = R(0); hC = R(0); hD = R(0); }
-    const R e0A = eA, e0C = eC, e0D = eD;
-    step(eA, eC, eD, lA, lC, lD, oA, oC, oD);
-    step(oA, oC, oD, e0A, e0C, e0D, hA, hC, hD);
-  }
-#pragma unroll
-  for (int dl = 1; dl < 32; dl <<= 1) {  // row stride 2*dl: same-parity rows of lanes +-dl
-    R lEA = shfl_up_r(eA, dl), lEC = shfl_up_r(eC, dl), lED = shfl_up_r(eD, dl);
-    R hEA = shfl_dn_r(eA, dl), hEC = shfl_dn_r(eC, dl), hED = shfl_dn_r(eD, dl);
-    R lOA = shfl_up_r(oA, dl), lOC = shfl_up_r(oC, dl), lOD = shfl_up_r(oD, dl);
-    R hOA = shfl_dn_r(oA, dl), hOC = shfl_dn_r(oC, dl), hOD = shfl_dn_r(oD, dl);
-    if (lane < dl) { lEA = R(0); lEC = R(0); lED = R(0); lOA = R(0); lOC = R(0); lOD = R(0); }
-    if (lane + dl > 31) { hEA = R(0); hEC = R(0); hED = R(0); hOA = R(0); hOC = R(0); hOD = R(0); }
-    step(eA, eC, eD, lEA, lEC, lED, hEA, hEC, hED);
-    step(oA, oC, oD, lOA, lOC, lOD, hOA, hOC, hOD);
-  }
-  const R x0 = eD, xl = oD;
-  ld[0] = x0;
-#pragma unroll
-  for (int k = 1; k < m - 1; ++k) ld[k] = fmaT(-xc[k], xl, fmaT(-xa[k], x0, xd[k]));
-  ld[m - 1] = xl;
-}
-
 // pairs of adjacent elements (16 bytes in binary64, 8 in binary32)
 template <class R>
 struct Pair2;
@@ -1004,34 +916,28 @@ __global__ void __launch_bounds__(StridedCfg<R, SEG, ROWS>::T, 1)
   extern __shared__ __align__(128) unsigned char smem_raw[];
   R* tile = reinterpret_cast<R*>(smem_raw);  // a | b | c | d, [row][system] each
   R* xt = tile + 4 * SC::TILE;               // solution tile
-  R* sets = xt + SC::TILE;                   // 2 x (a | c | d), SETA each
-  R* outr = sets + 2 * 3 * SC::SETA;         // outgoing runs: [array][w][RUN]
-  uint64_t* bar = reinterpret_cast<uint64_t*>(outr + 3 * W * SC::RUN);  // tiles
-  uint64_t* rbar = bar + 1;                                            // reduced rows of set 0, 1
+  R* red = xt + SC::TILE;                    // owned systems: a | c | d, 2*T each; then reduced_pcr's
+  R* outr = red + SC::RED;                   // outgoing reduced rows: [system][a | c | d][chunk]
+  R* outx = outr + 6 * T;                    // outgoing solutions: [owned system][chunk]
+  R* xs = outx + 2 * T;                      // incoming solutions: [system][own chunk]
+  uint64_t* bar = reinterpret_cast<uint64_t*>(xs + 2 * T);  // tiles
+  uint64_t* rbar = bar + 1;                                 // reduced rows
+  uint64_t* xbar = bar + 2;                                 // solutions
   cg::cluster_group cluster = cg::this_cluster();
   const int Q = (int)cluster.num_blocks();  // 4 .. SC::QMAX, a power of two
   const int rank = (int)cluster.block_rank();
-  const int S = W / Q;                       // systems each CTA owns
-  const int m = CH * Q / 16;                 // reduced rows per lane chunk: 4, 8 or 16
-  const int pitch = m + 2;                   // lane chunks of m reduced rows, padded
-  const int sysP = 32 * pitch;               // one owned system in a set array
-  const int run = (32 / Q) * pitch;          // this CTA's part of one owned system
   const int tid = threadIdx.x;
   const int w = tid % W, k = tid / W;
-  const int owner = w % Q, slot = w / Q;  // system w's reduced rows: rank `owner`, slot `slot`
   const int row0 = rank * ROWS + k * M;
   const int nclusters = gridDim.x / Q;
   const int cl = blockIdx.x / Q;
   const int ngroups = (nsys + W - 1) / W;
   const bool stores = rank * ROWS < n;  // CTAs wholly past the last row store nothing
-  // this chunk's reduced rows 2i, 2i+1 (i = rank*C + k): their pair in the
-  // run for system w and in the owner's set (m and 2i are even: one lane
-  // chunk, even position)
-  const int i2 = 2 * (rank * CH + k);
-  const int q_run = ((2 * k) / m) * pitch + (2 * k) % m;
-  const int p_e = slot * sysP + (i2 / m) * pitch + i2 % m;
-  // bytes an owner receives per group: Q senders x S systems x 3 arrays x run
-  const unsigned recv_bytes = (unsigned)(3 * W * run * sizeof(R));
+  const int G = CH * Q;  // chunks per system; the W / Q owned systems have T
+  const int c = tid % G, slot = tid / G;  // the chunk this thread solves for
+  P2* const my_rows = reinterpret_cast<P2*>(outr + w * SC::RUN) + k;
+  const P2* const my_red = reinterpret_cast<const P2*>(red + (slot * Q + c / CH) * SC::RUN) + c % CH;
+  const unsigned rows_bytes = (unsigned)(6 * T * sizeof(R)), xs_bytes = (unsigned)(2 * T * sizeof(R));
   constexpr unsigned kTileBytes = (unsigned)(SC::TILE * sizeof(R));
   auto issue = [&](int g) {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // earlier reads of the tiles precede the copies
@@ -1048,17 +954,17 @@ __global__ void __launch_bounds__(StridedCfg<R, SEG, ROWS>::T, 1)
   if (tid == 0) {
     mbar_init(bar);
     mbar_init(rbar);
-    mbar_init(rbar + 1);
+    mbar_init(xbar);
+    mbar_expect_tx(rbar, rows_bytes);
+    mbar_expect_tx(xbar, xs_bytes);
   }
   cluster.sync();  // every CTA of the cluster runs and its mbarriers are set up
   if (tid == 0 && cl < ngroups) issue(cl);
-  unsigned parity = 0, rpar = 0;
+  unsigned parity = 0, xpar = 0;
   bool failed = false;
-  int set = 0;
-  for (int g = cl; g < ngroups; g += nclusters, set ^= 1) {
+  for (int g = cl; g < ngroups; g += nclusters, xpar ^= 1) {
     const int sys = g * W + w;
     const bool live = sys < nsys;
-    if (tid == 0) mbar_expect_tx(rbar + set, recv_bytes);  // this group's reduced rows, from every CTA
     if (!failed) {
       const bool ok = mbar_wait_bounded(bar, parity);
       failed = __syncthreads_or(!ok);
@@ -1067,13 +973,22 @@ __global__ void __launch_bounds__(StridedCfg<R, SEG, ROWS>::T, 1)
     // own rows into registers; row 0 has no a, row n-1 no c, and rows or
     // systems outside the problem (zeros in the tiles) become identity rows
     R ra[M], rb[M], rc[M], rd[M];
+    // (64-byte rows: chunks of odd k take each pair of rows in the other
+    // order, or the chunks of a warp would meet in one half of the banks; at
+    // 4096 rows binary64 the loads of a group took 2490 cycles without)
+    const bool swap = SEG == 64 && (k & 1);
+    const int o0 = (k * M + (swap ? 1 : 0)) * W + w, o1 = (k * M + (swap ? 0 : 1)) * W + w;
+    auto pair = [&](const R* t, R& first, R& second, int j) {
+      const R p = t[o0 + j * W], q = t[o1 + j * W];
+      first = swap ? q : p;
+      second = swap ? p : q;
+    };
 #pragma unroll
-    for (int j = 0; j < M; ++j) {
-      const int o = (k * M + j) * W + w;
-      ra[j] = tile[o];
-      rb[j] = tile[SC::TILE + o];
-      rc[j] = tile[2 * SC::TILE + o];
-      rd[j] = tile[3 * SC::TILE + o];
+    for (int j = 0; j < M; j += 2) {
+      pair(tile, ra[j], ra[j + 1], j);
+      pair(tile + SC::TILE, rb[j], rb[j + 1], j);
+      pair(tile + 2 * SC::TILE, rc[j], rc[j + 1], j);
+      pair(tile + 3 * SC::TILE, rd[j], rd[j + 1], j);
     }
     if (!(live && row0 >= 1 && row0 + M <= n - 1)) {
 #pragma unroll
@@ -1113,54 +1028,50 @@ __global__ void __launch_bounds__(StridedCfg<R, SEG, ROWS>::T, 1)
     }
     const R r0 = fast_rcp(fmaT(-rc[0], an, rb[0]));
     const R eA = ra[0] * r0, eC = -rc[0] * cn * r0, eD = fmaT(-rc[0], dn, rd[0]) * r0;
-    // the chunk's reduced rows -> the run for its system, then every run to
-    // its owner (the previous group's runs were read before its barrier)
-    {
-      P2* o = reinterpret_cast<P2*>(outr + w * SC::RUN + q_run);
-      o[0] = P2{eA, ap};
-      o[W * SC::RUN / 2] = P2{eC, cp};
-      o[W * SC::RUN] = P2{eD, dp};
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic writes -> copy engine
+    my_rows[0] = P2{eA, ap};
+    my_rows[CH] = P2{eC, cp};
+    my_rows[2 * CH] = P2{eD, dp};
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic accesses -> copy engine
     __syncthreads();
-    R* own = sets + (size_t)set * 3 * SC::SETA;  // this group's set: a | c | d
-    if (tid < 3 * W && !failed) {
-      const int arr = tid / W, ws = tid % W;  // run of system ws, array arr
-      const int dst = arr * SC::SETA + (ws / Q) * sysP + (32 / Q) * rank * pitch;
-      bulk_send(cluster_smem_addr(own + dst, ws % Q), outr + (arr * W + ws) * SC::RUN,
-                (unsigned)(run * sizeof(R)), cluster_smem_addr(rbar + set, ws % Q));
-    }
+    if (tid < W && !failed)
+      bulk_send(cluster_smem_addr(red + ((tid / Q) * Q + rank) * SC::RUN, tid % Q), outr + tid * SC::RUN,
+                (unsigned)(SC::RUN * sizeof(R)), cluster_smem_addr(rbar, tid % Q));
     if (!failed) {
-      const bool ok = mbar_wait_bounded(rbar + set, (rpar >> set) & 1u);
+      const bool ok = mbar_wait_bounded(rbar, xpar);
       failed = __syncthreads_or(!ok);
-      rpar ^= 1u << set;
     }
-    // one warp per owned system (S of them, 32Q rows each); the other set,
-    // idle until this group's barrier, holds the intermediate rows
     {
-      R* scr = sets + (size_t)(set ^ 1) * 3 * SC::SETA;
-      for (int s = tid >> 5; s < S; s += T / 32) {
-        const int o = s * sysP;
-        R* A = own + o;
-        R* Cc = own + SC::SETA + o;
-        R* D = own + 2 * SC::SETA + o;
-        R* sa = scr + o;
-        R* sc = scr + SC::SETA + o;
-        R* sd = scr + 2 * SC::SETA + o;
-        switch (m) {
-          case 4: warp_unit_solve<R, 4>(A, Cc, D, sa, sc, sd, pitch); break;
-          case 8: warp_unit_solve<R, 8>(A, Cc, D, sa, sc, sd, pitch); break;
-          default: warp_unit_solve<R, 16>(A, Cc, D, sa, sc, sd, pitch); break;
-        }
-      }
+      const P2 A = my_red[0], C = my_red[CH], D = my_red[2 * CH];
+      __syncthreads();
+      R x0, xl;
+      reduced_pcr<R, sizeof(R) == 8>(red, T, 1, G, tid, c, true, A.x, C.x, D.x, A.y, C.y, D.y, x0, xl,
+                                     [](bool q) { return (bool)__syncthreads_or(q); });
+      reinterpret_cast<P2*>(outx)[tid] = P2{x0, xl};
     }
-    if (tid == 0) bulk_store_wait_read();  // the previous solution tile has been read out
-    cluster.sync();
-    const P2 sol = *reinterpret_cast<const P2*>(cluster.map_shared_rank(own + 2 * SC::SETA, owner) + p_e);
+    if (tid == 0) {
+      mbar_expect_tx(rbar, rows_bytes);  // the next group's rows come only after these solutions
+      bulk_store_wait_read();            // the previous solution tile has been read out
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic accesses -> copy engine
+    __syncthreads();
+    if (tid < W && !failed)  // owned system tid / Q, the chunks of rank tid % Q
+      bulk_send(cluster_smem_addr(xs + ((tid / Q) * Q + rank) * 2 * CH, tid % Q),
+                outx + 2 * ((tid / Q) * G + (tid % Q) * CH), (unsigned)(2 * CH * sizeof(R)),
+                cluster_smem_addr(xbar, tid % Q));
+    if (!failed) {
+      const bool ok = mbar_wait_bounded(xbar, xpar);
+      failed = __syncthreads_or(!ok);
+    }
+    if (tid == 0) mbar_expect_tx(xbar, xs_bytes);  // the next ones come only after the rows sent below
+    const P2 sol = reinterpret_cast<const P2*>(xs)[w * CH + k];
     const R x0 = sol.x, xl = sol.y;
+    auto row = [&](int j) { return j == 0 ? x0 : (j == M - 1 ? xl : fmaT(-rc[j], xl, fmaT(-ra[j], x0, rd[j]))); };
 #pragma unroll
-    for (int j = 0; j < M; ++j)
-      xt[(k * M + j) * W + w] = j == 0 ? x0 : (j == M - 1 ? xl : fmaT(-rc[j], xl, fmaT(-ra[j], x0, rd[j])));
+    for (int j = 0; j < M; j += 2) {
+      const R p = row(j), q = row(j + 1);
+      xt[o0 + j * W] = swap ? q : p;
+      xt[o1 + j * W] = swap ? p : q;
+    }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic writes -> tensor engine
     __syncthreads();
     // rows past n and systems past nsys fall outside the map and are not written
@@ -1174,8 +1085,8 @@ __global__ void __launch_bounds__(StridedCfg<R, SEG, ROWS>::T, 1)
     if (failed) {
       atomicExch(&g_tri_timeout, 1);
       mbar_wait_bounded(bar, parity);  // copies still in flight land before the CTA leaves
-      mbar_wait_bounded(rbar, rpar & 1u);
-      mbar_wait_bounded(rbar + 1, (rpar >> 1) & 1u);
+      mbar_wait_bounded(rbar, xpar);
+      mbar_wait_bounded(xbar, xpar);
     }
     bulk_store_wait_all();
   }
@@ -1260,9 +1171,10 @@ cudaError_t strided_launch(const R* a, const R* b, const R* c, const R* d, R* x,
 }
 
 // IXB_STRIDED_SEG=64 or 128 forces one configuration; otherwise lines of
-// more than 2048 rows use 64-byte segments with 512-row CTAs (clusters of
-// 8 instead of 16, so more of them fit the GPU at once), shorter lines
-// 128-byte segments with 256-row CTAs (less padding).
+// more than 1024 rows use 64-byte segments with 512-row CTAs (half the CTAs
+// per cluster, so more clusters fit the GPU at once: binary64 1500 x 1500
+// 33.2 against 39.3 us, 4096 x 4096 153 against 167), shorter lines 128-byte
+// segments with 256-row CTAs (less padding).
 int strided_seg_choice() {
   static const int v = [] {
     const char* e = std::getenv("IXB_STRIDED_SEG");
@@ -1280,7 +1192,7 @@ cudaError_t strided_solve(const R* a, const R* b, const R* c, const R* d, R* x, 
   const uintptr_t all = (uintptr_t)a | (uintptr_t)b | (uintptr_t)c | (uintptr_t)d | (uintptr_t)x;
   if ((all & 15) != 0 || ((size_t)nsys * sizeof(R)) % 16 != 0) return cudaErrorInvalidValue;
   const int seg = strided_seg_choice();
-  if (seg == 64 || (seg != 128 && n > 8 * kStrBox)) {
+  if (seg == 64 || (seg != 128 && n > 4 * kStrBox)) {
     const cudaError_t e = strided_launch<R, 64, 512>(a, b, c, d, x, n, nsys, st);
     if (e != cudaErrorInvalidValue) return e;
   }

@@ -95,3 +95,12 @@ def test_batched_lines_any_alignment(has_gpu, n, nsys, layout, dtype):
         x = got[s:s + n * nsys].reshape((nsys, n) if layout == 0 else (n, nsys))
         x = x if layout == 0 else x.T
         assert relerr(x, ref) < (1e-12 if dtype == "f64" else 2e-5), relerr(x, ref)
+
+
+# interleaved systems in thread-block clusters: the row limits of the two configurations and of their cluster
+# sizes, a last group that is not full, several groups per cluster
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+@pytest.mark.parametrize("n,nsys", [(513, 36), (1024, 2052), (1025, 64), (2048, 2500), (2049, 16), (3000, 8),
+                                    (4096, 40), (4096, 1036)])
+def test_interleaved_lines_in_clusters(has_gpu, n, nsys, dtype):
+    test_batched_lines_any_alignment(has_gpu, n, nsys, 1, dtype)
