@@ -32,29 +32,10 @@
 
 #include "ixb_handle.h"
 #include "ixb_nusselt.h"
+#include "ixb_passes.h"
 
 namespace ixb {
 namespace {
-
-// coefficient arrays (field layout) of the energy rows: AI, AD, BS, BN, diag
-enum { C_AI = 0, C_AD, C_BS, C_BN, C_DG, C_COUNT };
-
-__global__ void adj_coef_kernel(const Geo<double> G, const SweepIO<double> io, double* __restrict__ coef,
-                                size_t fsz) {
-  const int ni = G.mi - 1;  // ii = 2..mi, jj = 2..nj
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= ni * (G.nj - 1)) return;
-  const int ii = 2 + idx % ni, jj = 2 + idx / ni;
-  const CellView<double, double> cell{G, io, ii, jj};
-  const Row<double> rx = assemble_tx<true>(G, cell);  // a = AI, c = AD, b = diagonal
-  const Row<double> ry = assemble_ty<true>(G, cell);  // a = BS, c = BN
-  const int c0 = G.at(ii, jj);
-  coef[C_AI * fsz + c0] = rx.a;
-  coef[C_AD * fsz + c0] = rx.c;
-  coef[C_BS * fsz + c0] = ry.a;
-  coef[C_BN * fsz + c0] = ry.c;
-  coef[C_DG * fsz + c0] = rx.b;
-}
 
 struct Sweep {
   bool x;               // x-lines (fixed jj) or y-lines (fixed ii)
@@ -213,7 +194,7 @@ struct AdjCtx {
   int init(int j0, int j1) {
     const int mi = h->mi, nj = h->nj;
     fsz = h->fsz;
-    const size_t need = (C_COUNT + 3) * fsz + (size_t)(nj + 2);
+    const size_t need = (C_COUNT + 3) * fsz + (size_t)(nj + 2) + 1;  // the last: barrier and flag of the resident passes
     if (h->adj_size < need) {
       if (h->adj_pool) cudaFree(h->adj_pool);
       h->adj_pool = nullptr;
@@ -255,13 +236,9 @@ struct AdjCtx {
       ACK(cudaGetLastError());
       started = false;
     }
-    const int cT = h->cT;
-    SweepIO<double> io = handle_sweep_io(h, EQ_TX, nullptr);
-    h->cT = cT;
-    ACK(cudaMemsetAsync(coef, 0, C_COUNT * fsz * sizeof(double), h->stream));
-    const int n = (h->mi - 1) * (h->nj - 1);
-    adj_coef_kernel<<<(n + 255) / 256, 256, 0, h->stream>>>(G, io, coef, fsz);
-    ACK(cudaGetLastError());
+    SweepIO<double> io = handle_fixed_io(h, EQ_TX);
+    io.in = h->zero;
+    ACK(energy_coef_launch(G, io, coef, fsz, h->stream));
     return IXB_OK;
   }
 
@@ -302,11 +279,19 @@ extern "C" int ixb_adjoint_energy(ixb_handle* h, int K, int j0, int j1, double* 
   AdjCtx A{h};
   TRY(A.init(j0, j1));
   TRY(A.coefficients());  // the frozen velocities
-  // K passes of (T-y, T-x), reversed: the first reads the objective's weights,
-  // a WHILE graph runs the others kLoopUnroll at a time (rebuilt when the
-  // handle or its workspace changes), the remaining ones are plain launches
+  // K passes of (T-y, T-x), reversed: the first reads the objective's weights;
+  // the others run in one resident kernel where the grid fits it, else in a
+  // WHILE graph kLoopUnroll at a time (rebuilt when the handle or its
+  // workspace changes) and what is left as plain launches
   if (K > 0) TRY(A.pass());
   const int left = std::max(K - 1, 0);
+  PassArgs P{};
+  if (left > 0 && handle_resident_passes(h, &P)) {
+    P.coef = A.coef; P.f0 = A.my; P.f1 = A.mx; P.grad = A.gd; P.passes = left;
+    unsigned* w = reinterpret_cast<unsigned*>(A.gd + h->nj + 2);
+    TRY(handle_run_passes(h, true, P, w));
+    return A.finish(grad);
+  }
   const std::function<int()> pass = [&A]() -> int { return A.pass(); };
   if (left >= kLoopUnroll) {
     if (h->agraph_dirty || !h->agraph_exec || h->agraph_pool != h->adj_pool) {

@@ -1469,6 +1469,27 @@ int ixb_energy_iterations(ixb_handle* h, int n) {
   if (!h || n < 0) return IXB_EINVAL;
   TRY(ready(h));
   if (n == 0) return IXB_OK;
+  // the resident passes factor their rows first: from a few passes on, in
+  // binary64 and without launch shapes of the caller's
+  PassArgs P{};
+  const bool own_shape = h->shape_set[EQ_TY] || h->shape_set[EQ_TX];
+  if (n >= 4 && !own_shape && solver_form(h) == IXB_SOLVER_HYBRID && handle_resident_passes(h, &P)) {
+    double* work = nullptr;
+    const cudaError_t e = scratch_alloc(reinterpret_cast<void**>(&work), (C_COUNT * h->fsz + 1) * sizeof(double), h->stream);
+    if (e == cudaSuccess) {
+      h->scratch_used = true;
+      SweepIO<double> io = handle_fixed_io(h, EQ_TX);
+      io.in = h->zero;
+      cudaError_t k = energy_coef_launch(P.G, io, work, h->fsz, h->stream);
+      P.coef = work; P.f0 = h->T[h->cT]; P.f1 = h->T[h->cT ^ 1]; P.passes = n;
+      int st = IXB_ECUDA;
+      if (k == cudaSuccess) st = handle_run_passes(h, false, P, reinterpret_cast<unsigned*>(work + C_COUNT * h->fsz));
+      else h->last_cuda = k;
+      cudaFreeAsync(work, h->stream);
+      return st;
+    }
+    cudaGetLastError();  // no room for the factors: the sweeps
+  }
   // one pass, T-y then T-x (buffer parity back to 0); kLoopUnroll of them
   // form the body of a WHILE loop, the rest run as plain launches
   const std::function<int()> pass = [h]() -> int {
@@ -1575,6 +1596,29 @@ int handle_sweep_to(ixb_handle* h, int eq, const SweepIO<double>& io) {
   CK(launch_sweep_f64(eq, solver_form(h), s, make_geo(h), io, StageBuf{h->stage, h->stage_stride, h->stage_P},
                       h->stream));
   return IXB_OK;
+}
+bool handle_resident_passes(ixb_handle* h, PassArgs* a) {
+  if (!h->coop || !h->use_graph || !fused_enabled() || !do_while_loops()) return false;
+  if (!energy_passes_fit(h->mi, h->nj, h->nsm, a)) return false;
+  a->G = make_geo(h);
+  a->fsz = h->fsz;
+  a->keep = 1.0 - h->prm.rel_ener;
+  const BCEntry* base = h->bc + (size_t)2 * 4 * h->bcstride;  // T tables, sides a b c d
+  a->first_x = base;
+  a->first_y = base + (size_t)h->bcstride;
+  a->last_x = base + 2 * (size_t)h->bcstride;
+  a->last_y = base + 3 * (size_t)h->bcstride;
+  return true;
+}
+int handle_run_passes(ixb_handle* h, bool reverse, PassArgs& a, unsigned* w) {
+  a.bar = w;
+  a.abort_flag = reinterpret_cast<int*>(w + 1);
+  CK(cudaMemsetAsync(w, 0, 2 * sizeof(unsigned), h->stream));
+  CK(energy_passes_launch(reverse, a, h->stream));
+  int gave_up = 0;
+  CK(cudaMemcpyAsync(&gave_up, a.abort_flag, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaStreamSynchronize(h->stream));
+  return gave_up ? IXB_ETIMEOUT : IXB_OK;
 }
 int handle_single_passes(ixb_handle* h, int n) {
   // every inner test met after its first pass

@@ -7,6 +7,7 @@
 
 #include <vector>
 
+#include "ixb_passes.h"
 #include "ixb_internal.h"
 
 namespace ixb {
@@ -140,6 +141,11 @@ SweepIO<double> handle_sweep_io(ixb_handle* h, int eq, const double* prev);
 // time level, sources, boundary tables), the caller fills in the rest
 SweepIO<double> handle_fixed_io(ixb_handle* h, int eq);
 int handle_sweep_to(ixb_handle* h, int eq, const SweepIO<double>& io);
+// Whether the resident energy passes (ixb_passes.h) serve the handle's grid;
+// fills the fields of `a` that follow from the handle (fixed velocities).
+bool handle_resident_passes(ixb_handle* h, ixb::PassArgs* a);
+// runs them and waits; w: two words on the device (barrier, flag)
+int handle_run_passes(ixb_handle* h, bool reverse, ixb::PassArgs& a, unsigned* w);
 // n outer iterations of one pass of each equation, whatever the parameters'
 // tests say; the loop counters are left alone
 int handle_single_passes(ixb_handle* h, int n);
