@@ -28,7 +28,9 @@
 // them transposed in shared memory, solves, and scatters.  As row, transpose,
 // line-solve and scatter kernels it was 44 launches per reversed iteration
 // instead of 9, and bound by them up to 256x256 (128x128, 30 iterations, a
-// checkpoint every 10: 20.3 ms per gradient then).
+// checkpoint every 10: 20.3 ms per gradient then).  The recomputed sweeps and
+// the reversed ones are launched with programmatic serialisation: each is a
+// few microseconds of latency, and the next one's launch overlaps it.
 //
 // Forward: K outer iterations (the library's loop, one pass of each equation),
 // the state saved every C iterations.  Reverse, segment by segment from the
@@ -216,19 +218,23 @@ __device__ __forceinline__ void load_stencil(const Geo<double>& G, const SweepSt
   each_tap<GRP>([&](auto q, auto f, int di, int dj) { x[q] = __ldg(s.f[f] + G.at(ii + di, jj + dj)); });
 }
 
-// One sweep reversed.  A CTA takes TL adjacent lines, G threads per line, m
-// rows per thread (n <= G*m).  lam: the swept field's adjoint after the sweep,
+// One sweep reversed.  A CTA takes TL adjacent lines, GT threads per line for
+// the solve, m rows per thread (n <= GT*m), and RP times as many for the rows
+// and the scatter (their stencil loads and link arithmetic, one row after
+// another, were most of a reversed sweep at one thread per chunk).  lam: the swept field's adjoint after the sweep,
 // read and cleared here; every contribution to it before the sweep goes to
 // adj.f[swept field], another buffer, zero on entry (null: dropped, p' before
 // its first sweep).  aux_bar (u-x, v-x): the adjoint of au or av, read and
 // cleared.  grad (T-x): d / d value of the side-a boundary rows, += mu of row
 // 0 (the row is (0, 1, 0 | value), or the Neumann row with the value as flux).
-template <int EQ, int TL, int GT, int M>
-__global__ void __launch_bounds__(TL * GT)
+template <int EQ, int TL, int GT, int RP, int M>
+__global__ void __launch_bounds__(TL * GT * RP)
     adj_sweep_kernel(const Geo<double> G, const SweepState s, double* __restrict__ lam, double* aux_bar, AdjFields adj,
                      double* grad, int m_, int mp_) {
   constexpr int GRP = eq_group(EQ);
   constexpr bool X = (EQ & 1) != 0;
+  constexpr int NT = TL * GT * RP;
+  IXB_PDL_ENTRY();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double* sm = reinterpret_cast<double*>(smem_raw);
   const int m = M > 0 ? M : m_, mp = M > 0 ? (M | 1) : mp_;
@@ -237,7 +243,7 @@ __global__ void __launch_bounds__(TL * GT)
   auto slot = [&](int l, int r) { return l * LS + (r / m) * mp + r % m; };
   auto cell = [&](int L, int r) { return X ? G.at(r + 1, L) : G.at(L, r + 1); };
   // rows, transposed: a'_r = c_{r-1}, b'_r = b_r, c'_r = a_{r+1}; identity rows pad the line
-  for (int idx = threadIdx.x; idx < TL * npad; idx += TL * GT) {
+  for (int idx = threadIdx.x; idx < TL * npad; idx += NT) {
     const int l = X ? idx / npad : idx % TL, r = X ? idx - l * npad : idx / TL, L = L0 + l;
     if (L > s.nfull) continue;
     const bool solved = L >= s.line_lo && L <= s.line_hi;
@@ -273,13 +279,14 @@ __global__ void __launch_bounds__(TL * GT)
     if (r >= 1 && r < n) sm[slot(l, r - 1) + 2 * arr] = a;
   }
   __syncthreads();
-  {
+  if (threadIdx.x < TL * GT) {
+    // (lines barriers of their own, TL > 1, when not all threads solve)
     const int l = threadIdx.x / GT, L = L0 + l;
-    chunk_solve<double, GT, TL, M>(sm + l * LS, m, mp, L >= s.line_lo && L <= s.line_hi);
+    chunk_solve<double, GT, (RP > 1 ? 2 : TL), M>(sm + l * LS, m, mp, L >= s.line_lo && L <= s.line_hi);
   }
   __syncthreads();
   // scatter of the interior rows
-  for (int idx = threadIdx.x; idx < TL * n; idx += TL * GT) {
+  for (int idx = threadIdx.x; idx < TL * n; idx += NT) {
     const int l = X ? idx / n : idx % TL, r = X ? idx - l * n : idx / TL, L = L0 + l;
     if (L < s.line_lo || L > s.line_hi) continue;
     const double mu = sm[slot(l, r) + 3 * arr];
@@ -305,38 +312,47 @@ __global__ void __launch_bounds__(TL * GT)
   }
 }
 
-// x-lines one per CTA; y-lines four adjacent ones (32-byte pieces of a row).
-// Three rows per thread up to 768 rows, longer chunks beyond.
+// x-lines one per CTA; y-lines two adjacent ones while that gives a CTA per SM
+// at most, else four (32-byte pieces of a row).  Three rows per thread of the
+// solve up to 768 rows, longer chunks beyond.
 template <int EQ>
 cudaError_t adj_sweep_launch(const Geo<double>& G, const SweepState& s, double* lam, double* aux_bar,
-                             const AdjFields& adj, double* grad, cudaStream_t st) {
+                             const AdjFields& adj, double* grad, int nsm, cudaStream_t st) {
   constexpr bool X = (EQ & 1) != 0;
-  auto go = [&](auto k, int tl, int g, int m) -> cudaError_t {
+  auto go = [&](auto k, int tl, int g, int rp, int m) -> cudaError_t {
     const size_t smem = line_smem_elems(g, m | 1) * sizeof(double) * tl;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    k<<<(s.nfull + tl - 1) / tl, tl * g, smem, st>>>(G, s, lam, aux_bar, adj, grad, m, m | 1);
-    return cudaGetLastError();
+    if (smem > 48 * 1024) {  // beyond the default limit
+      const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+    }
+    return launch_pdl(true, k, (s.nfull + tl - 1) / tl, tl * g * rp, smem, st, G, s, lam, aux_bar, adj, grad, m, m | 1);
   };
-  constexpr int TL = X ? 1 : 4;
-  if (s.n <= 192) return go(adj_sweep_kernel<EQ, TL, 64, 3>, TL, 64, 3);
-  if (s.n <= 384) return go(adj_sweep_kernel<EQ, TL, 128, 3>, TL, 128, 3);
-  if (X && s.n <= 768) return go(adj_sweep_kernel<EQ, 1, 256, 3>, 1, 256, 3);
-  if (!X && s.n <= 1024) return go(adj_sweep_kernel<EQ, TL, 128, 0>, TL, 128, (s.n + 127) / 128);
-  return go(adj_sweep_kernel<EQ, 1, 256, 0>, 1, 256, std::max(3, (s.n + 255) / 256));
+  if constexpr (X) {
+    if (s.n <= 192) return go(adj_sweep_kernel<EQ, 1, 64, 3, 3>, 1, 64, 3, 3);
+    if (s.n <= 384) return go(adj_sweep_kernel<EQ, 1, 128, 3, 3>, 1, 128, 3, 3);
+    if (s.n <= 768) return go(adj_sweep_kernel<EQ, 1, 256, 3, 3>, 1, 256, 3, 3);
+  } else {
+    const bool two = s.nfull <= 2 * nsm;
+    if (s.n <= 192 && two) return go(adj_sweep_kernel<EQ, 2, 64, 3, 3>, 2, 64, 3, 3);
+    if (s.n <= 192) return go(adj_sweep_kernel<EQ, 4, 64, 3, 3>, 4, 64, 3, 3);
+    if (s.n <= 384 && two) return go(adj_sweep_kernel<EQ, 2, 128, 3, 3>, 2, 128, 3, 3);
+    if (s.n <= 384) return go(adj_sweep_kernel<EQ, 4, 128, 1, 3>, 4, 128, 1, 3);
+    if (s.n <= 1024) return go(adj_sweep_kernel<EQ, 4, 128, 1, 0>, 4, 128, 1, (s.n + 127) / 128);
+  }
+  return go(adj_sweep_kernel<EQ, 1, 256, 1, 0>, 1, 256, 1, std::max(3, (s.n + 255) / 256));
 }
 
 cudaError_t adj_sweep(const Geo<double>& G, const SweepState& s, double* lam, double* aux_bar, const AdjFields& adj,
-                      double* grad, cudaStream_t st) {
+                      double* grad, int nsm, cudaStream_t st) {
   switch (s.eq) {
-    case EQ_UY: return adj_sweep_launch<EQ_UY>(G, s, lam, aux_bar, adj, grad, st);
-    case EQ_UX: return adj_sweep_launch<EQ_UX>(G, s, lam, aux_bar, adj, grad, st);
-    case EQ_VY: return adj_sweep_launch<EQ_VY>(G, s, lam, aux_bar, adj, grad, st);
-    case EQ_VX: return adj_sweep_launch<EQ_VX>(G, s, lam, aux_bar, adj, grad, st);
-    case EQ_PY: return adj_sweep_launch<EQ_PY>(G, s, lam, aux_bar, adj, grad, st);
-    case EQ_PX: return adj_sweep_launch<EQ_PX>(G, s, lam, aux_bar, adj, grad, st);
-    case EQ_TY: return adj_sweep_launch<EQ_TY>(G, s, lam, aux_bar, adj, grad, st);
-    default: return adj_sweep_launch<EQ_TX>(G, s, lam, aux_bar, adj, grad, st);
+    case EQ_UY: return adj_sweep_launch<EQ_UY>(G, s, lam, aux_bar, adj, grad, nsm, st);
+    case EQ_UX: return adj_sweep_launch<EQ_UX>(G, s, lam, aux_bar, adj, grad, nsm, st);
+    case EQ_VY: return adj_sweep_launch<EQ_VY>(G, s, lam, aux_bar, adj, grad, nsm, st);
+    case EQ_VX: return adj_sweep_launch<EQ_VX>(G, s, lam, aux_bar, adj, grad, nsm, st);
+    case EQ_PY: return adj_sweep_launch<EQ_PY>(G, s, lam, aux_bar, adj, grad, nsm, st);
+    case EQ_PX: return adj_sweep_launch<EQ_PX>(G, s, lam, aux_bar, adj, grad, nsm, st);
+    case EQ_TY: return adj_sweep_launch<EQ_TY>(G, s, lam, aux_bar, adj, grad, nsm, st);
+    default: return adj_sweep_launch<EQ_TX>(G, s, lam, aux_bar, adj, grad, nsm, st);
   }
 }
 
@@ -346,6 +362,7 @@ __global__ void correct_to_kernel(const Geo<double> G, const double* __restrict_
                                   const double* __restrict__ p0, const double* __restrict__ pc,
                                   const double* __restrict__ au, const double* __restrict__ av, double* __restrict__ u3,
                                   double* __restrict__ v3, double* __restrict__ p1) {
+  IXB_PDL_ENTRY();
   const int ii = 1 + blockIdx.x * blockDim.x + threadIdx.x, jj = 1 + blockIdx.y;
   if (ii > G.mi + 1) return;
   const int c0 = G.at(ii, jj);
@@ -368,6 +385,7 @@ __global__ void adj_correct_kernel(const Geo<double> G, const double* __restrict
                                    const double* __restrict__ av, const double* __restrict__ ub,
                                    const double* __restrict__ vb, const double* __restrict__ pb, double* pcb,
                                    double* aub, double* avb) {
+  IXB_PDL_ENTRY();
   const int ni = G.mi - 1;
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= ni * (G.nj - 1)) return;
@@ -508,7 +526,7 @@ struct SimpleAdjoint {
       io.in = in; io.out = out; io.aux = aux;
       io.u = u; io.v = v; io.T = S(S_T0); io.p = S(S_P0); io.pc = in;
       io.au = S(S_AU); io.av = S(S_AV);
-      return handle_sweep_to(h, eq, io);
+      return handle_sweep_to(h, eq, io, true);
     };
     const double *u0 = S(S_U0), *v0 = S(S_V0);
     STRY(sw(EQ_UY, u0, S(S_U1), u0, v0, nullptr));
@@ -519,9 +537,8 @@ struct SimpleAdjoint {
     STRY(sw(EQ_PX, S(S_PC1), S(S_PC2), S(S_U2), S(S_V2), h->b_o));
     double *u3 = slot(it + 1, S_U0), *v3 = slot(it + 1, S_V0);
     const dim3 grid((h->mi + 1 + 127) / 128, h->nj + 1);
-    correct_to_kernel<<<grid, 128, 0, h->stream>>>(G, S(S_U2), S(S_V2), S(S_P0), S(S_PC2), S(S_AU), S(S_AV), u3, v3,
-                                                   slot(it + 1, S_P0));
-    SCK(cudaGetLastError());
+    SCK(launch_pdl(true, correct_to_kernel, grid, 128, 0, h->stream, G, S(S_U2), S(S_V2), S(S_P0), S(S_PC2), S(S_AU),
+                   S(S_AV), u3, v3, slot(it + 1, S_P0)));
     STRY(sw(EQ_TY, S(S_T0), S(S_T1), u3, v3, nullptr));
     return sw(EQ_TX, S(S_T1), slot(it + 1, S_T0), u3, v3, nullptr);
   }
@@ -575,7 +592,7 @@ struct SimpleAdjoint {
     std::swap(adj.f[f], other[f]);
     AdjFields a = adj;
     if (!keep) a.f[f] = nullptr;
-    SCK(adj_sweep(G, state(eq, it), lam, aux_bar, a, grad, h->stream));
+    SCK(adj_sweep(G, state(eq, it), lam, aux_bar, a, grad, h->nsm, h->stream));
     return IXB_OK;
   }
 
@@ -584,10 +601,8 @@ struct SimpleAdjoint {
     STRY(sweep_back(EQ_TX, it, nullptr, gd));
     STRY(sweep_back(EQ_TY, it, nullptr, nullptr));
     const int ncell = (h->mi - 1) * (h->nj - 1);
-    adj_correct_kernel<<<(ncell + 255) / 256, 256, 0, h->stream>>>(G, slot(it, S_PC2), slot(it, S_AU), slot(it, S_AV),
-                                                                 adj.f[F_U], adj.f[F_V], adj.f[F_P], adj.f[F_PC],
-                                                                 adj.f[F_AU], adj.f[F_AV]);
-    SCK(cudaGetLastError());
+    SCK(launch_pdl(true, adj_correct_kernel, (ncell + 255) / 256, 256, 0, h->stream, G, slot(it, S_PC2), slot(it, S_AU),
+                   slot(it, S_AV), adj.f[F_U], adj.f[F_V], adj.f[F_P], adj.f[F_PC], adj.f[F_AU], adj.f[F_AV]));
     STRY(sweep_back(EQ_PX, it, nullptr, nullptr));
     STRY(sweep_back(EQ_PY, it, nullptr, nullptr, false));  // p' starts from the zero field
     STRY(sweep_back(EQ_VX, it, adj.f[F_AV], nullptr));     // av is written by the v-x sweep

@@ -1590,9 +1590,10 @@ SweepIO<double> handle_fixed_io(ixb_handle* h, int eq) {
   h->cu = cu; h->cv = cv; h->cT = cT; h->cpc = cpc;
   return io;
 }
-int handle_sweep_to(ixb_handle* h, int eq, const SweepIO<double>& io) {
+int handle_sweep_to(ixb_handle* h, int eq, const SweepIO<double>& io, bool early) {
   if (h->shape_tl[eq] == 0) pick_shape(h, eq);
-  const SweepShape s = sweep_shape(eq, h->mi, h->nj, real_bytes(h), h->shape_tl[eq], h->shape_g[eq]);
+  SweepShape s = sweep_shape(eq, h->mi, h->nj, real_bytes(h), h->shape_tl[eq], h->shape_g[eq]);
+  s.early = early;
   CK(launch_sweep_f64(eq, solver_form(h), s, make_geo(h), io, StageBuf{h->stage, h->stage_stride, h->stage_P},
                       h->stream));
   return IXB_OK;

@@ -138,9 +138,10 @@ int handle_run_loop_graph(ixb_handle* h, cudaGraphExec_t exec, int iterations);
 SweepIO<double> handle_sweep_io(ixb_handle* h, int eq, const double* prev);
 // sweep `eq` between fields of the caller's choice, in the handle's launch
 // shape: handle_fixed_io gives the inputs that are the handle's own (previous
-// time level, sources, boundary tables), the caller fills in the rest
+// time level, sources, boundary tables), the caller fills in the rest (early: see
+// SweepShape; the kernel before it is one of this library's)
 SweepIO<double> handle_fixed_io(ixb_handle* h, int eq);
-int handle_sweep_to(ixb_handle* h, int eq, const SweepIO<double>& io);
+int handle_sweep_to(ixb_handle* h, int eq, const SweepIO<double>& io, bool early);
 // Whether the resident energy passes (ixb_passes.h) serve the handle's grid;
 // fills the fields of `a` that follow from the handle (fixed velocities).
 bool handle_resident_passes(ixb_handle* h, ixb::PassArgs* a);

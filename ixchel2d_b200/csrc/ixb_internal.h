@@ -24,9 +24,10 @@ bool pdl_enabled();
 bool carveout_enabled();
 // fused sweeps (one kernel per sweep) unless IXB_SPLIT=1
 bool fused_enabled();
+// `early`: programmatic serialisation for this launch whatever the default.
 template <class... KArgs, class... Args>
-inline cudaError_t launch_k(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                            Args&&... args) {
+inline cudaError_t launch_pdl(bool early, void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                              Args&&... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -36,8 +37,13 @@ inline cudaError_t launch_k(void (*k)(KArgs...), dim3 grid, dim3 block, size_t s
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = pdl_enabled() ? 1 : 0;
+  cfg.numAttrs = early || pdl_enabled() ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, k, std::forward<Args>(args)...);
+}
+template <class... KArgs, class... Args>
+inline cudaError_t launch_k(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                            Args&&... args) {
+  return launch_pdl(false, k, grid, block, smem, st, std::forward<Args>(args)...);
 }
 
 enum NormId { N_DV = 0, N_DP, N_BO, N_DT, N_RES, N_COUNT };
@@ -104,6 +110,7 @@ struct SweepShape {
   int g;          // threads per line
   int nt;         // threads per CTA (tl * g)
   int m, mp;      // chunk rows per thread, padded pitch
+  bool early;     // fused launch with programmatic serialisation (launch_pdl)
   size_t smem;    // dynamic shared memory bytes
   int grid;       // CTAs
 };

@@ -513,7 +513,7 @@ cudaError_t fused_go(const SweepShape& s, const Geo<double>& G, const SweepIO<do
       pct_set[dev] = pct;
     }
   }
-  return launch_k(K, s.grid, s.tl * s.g, s.smem, st, G, io, so, s.n, s.line_lo, s.line_hi, s.nfull);
+  return launch_pdl(s.early, K, s.grid, s.tl * s.g, s.smem, st, G, io, so, s.n, s.line_lo, s.line_hi, s.nfull);
 }
 
 // Compile-time chunks (M) of up to 6 rows for x-lines of 256 threads and up to
