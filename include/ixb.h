@@ -221,8 +221,11 @@ int ixb_time_phases(ixb_handle* h, int reps, size_t flush_bytes, double* ms);
  * (8,32) (8,64) (8,128) (16,16) (16,32); each thread eliminates a chunk of
  * max(3, ceil(n/threads_per_line)) rows.  lines_per_cta = 0 restores the
  * default: x-lines one per CTA, 256 threads above 384 rows, else 128;
- * y-lines the fewest of 4, 5, 6 or 8 adjacent lines per CTA that keeps one
- * CTA per SM (8 beyond that), 128 threads per line from 160 rows, else 64.
+ * y-lines 4, 5, 6 or 8 adjacent lines per CTA, by the waves of CTAs that
+ * gives, 128 threads per line from 160 rows, else 64.  With every sweep at
+ * its default, grids of up to 767 x 383 (depending on the SM count) run the
+ * whole loop as one resident kernel instead of one launch per sweep; a shape
+ * set here keeps the loop to the per-sweep kernels.
  * No reference counterpart: the reference runs one sequential tridiagonal
  * per OpenACC gang. */
 int ixb_set_sweep_shape(ixb_handle* h, int sweep, int lines_per_cta, int threads_per_line);
@@ -232,12 +235,13 @@ int ixb_set_sweep_shape(ixb_handle* h, int sweep, int lines_per_cta, int threads
  * 16 lines per CTA), two per other sweep, plus the p/u/v correction and the
  * u residual, and the p' reset when the loop is host-driven
  * (IXB_NO_GRAPH=1) or IXB_DOWHILE=0.  IXB_SPLIT=1 in the environment keeps
- * every sweep at two kernels. */
+ * every sweep at two kernels.  0 where the resident loop kernel runs: the
+ * iterations of a call are one launch (one per 2048 of them). */
 int ixb_iteration_launches(ixb_handle* h, int* launches);
 /* Autotuner for the launch shapes: for every sweep, times each candidate
  * shape `reps` times on the current state (a scratch buffer of flush_bytes
  * is written before every timed launch when flush_bytes > 0) and keeps the
- * fastest.  The state is restored afterwards.  chosen[2k], chosen[2k+1]
+ * fastest for the calls that launch single sweeps.  The state is restored afterwards.  chosen[2k], chosen[2k+1]
  * receive sweep k's lines per CTA and threads per line; ms[k] its mean
  * milliseconds per launch (either may be NULL). */
 int ixb_autotune(ixb_handle* h, int reps, size_t flush_bytes, int* chosen, double* ms);
@@ -329,7 +333,7 @@ int ixb_tridiag_f64_noalloc(const double* a, const double* b, const double* c, c
  * through the momentum, pressure-correction and energy sweeps and their
  * coupling (buoyancy, convection): the adjoint for flows that depend on T.
  * The forward state is saved every C iterations; each segment is recomputed
- * storing the state after every phase (16 fields per iteration, so device
+ * storing what every phase writes (13 fields per iteration, so device
  * memory grows with C) and reversed with transposed line solves.  Leaves
  * the state of the K-iteration forward run.  Binary64 handles only
  * (IXB_EINVAL otherwise). */
@@ -367,9 +371,11 @@ int ixb_batch_create(int count, const int* mi, const int* nj, int prec_mode, ixb
 int ixb_batch_destroy(ixb_batch* b);
 int ixb_batch_instance(ixb_batch* b, int i, ixb_handle** h);
 /* Launch shape of sweep `sweep` (IXB_SWEEP_* order) for every instance, as
- * ixb_set_sweep_shape; 0, 0 restores the default. */
+ * ixb_set_sweep_shape; 0, 0 restores the default (one fused launch per sweep,
+ * four lines of 64 threads per CTA; binary64 with long lines: one x-line of
+ * 128 or 256 threads, four y-lines of 128). */
 int ixb_batch_set_sweep_shape(ixb_batch* b, int sweep, int lines_per_cta, int threads_per_line);
-/* Time the seven launch shapes of every sweep on the batch (reps batched
+/* Time the seventeen launch shapes of every sweep on the batch (reps batched
  * iterations each) and keep the fastest; chosen[2*s], chosen[2*s+1] and
  * ms[s] (may be null) receive the choice and its time per sweep.  The state
  * of every instance is saved before and restored after. */
