@@ -451,7 +451,7 @@ __global__ void __launch_bounds__(512) tri_cols_kernel(const R* a, const R* b, c
 // running CTAs hold, and the wait is bounded (g_tri_timeout).  Bound by the
 // latency of an item (64 KB in registers, two items per SM): 4095 x 4095
 // binary64 307 us (2.19 TB/s), against 5057 us for one thread per system;
-// where the cluster kernel applies it is faster (4096 x 4096: 213 against
+// where the cluster kernel applies it is faster (4096 x 4096: 154 against
 // 305 us).
 template <class R>
 struct BlockCfg {
