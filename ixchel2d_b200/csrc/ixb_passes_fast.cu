@@ -116,7 +116,8 @@ __device__ __forceinline__ void factor(Chunk3& h, const PassArgs& A, double* q, 
   q += t;
   q[(PQ - 2) * T] = eA;
   q[(PQ - 1) * T] = eC;
-  // the couplings of the steps of reduced_pcr: last rows by their own and the next chunk's first row, then among themselves
+  // the couplings of the steps of reduced_pcr: last rows by their own and the next chunk's first row, then among
+  // themselves (all steps: whether one still counts depends on the right-hand sides, which change with every pass)
   double *xa = ex, *xc = ex + T;
   xa[t] = eA;
   xc[t] = eC;
@@ -133,7 +134,7 @@ __device__ __forceinline__ void factor(Chunk3& h, const PassArgs& A, double* q, 
     double* pa = ex + ((lev & 1) ? 0 : 2) * T;  // the other pair: its readers are past a barrier
     pa[t] = oA;
     pa[T + t] = oC;
-    if (!__syncthreads_or(has && fmax(fabs(oA), fabs(oC)) > pcr_tiny<double>())) break;
+    __syncthreads();
     double lA = 0.0, lC = 0.0;
     hA = hC = 0.0;
     if (has && k >= s) { lA = pa[t - s * TS]; lC = pa[T + t - s * TS]; }
