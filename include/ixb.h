@@ -31,7 +31,8 @@ extern "C" {
 #define IXB_EINVAL 1     /* bad argument (NULL handle, size out of range, ...) */
 #define IXB_ECUDA 2      /* a CUDA runtime call failed */
 #define IXB_ENONFINITE 3 /* a convergence norm became NaN or Inf */
-#define IXB_ETIMEOUT 4   /* a bounded device wait expired */
+#define IXB_ETIMEOUT 4   /* a bounded device wait expired; the fields a call was sweeping are then
+                            partly swept (upload the state again) */
 #define IXB_EBC 5        /* a boundary table leaves a solved line without a row */
 #define IXB_ESTATE 6     /* call order: mesh/params/bc not set yet */
 #define IXB_EIO 7        /* file could not be read / parsed / written */
@@ -225,7 +226,11 @@ int ixb_time_phases(ixb_handle* h, int reps, size_t flush_bytes, double* ms);
  * gives, 128 threads per line from 160 rows, else 64.  With every sweep at
  * its default, grids of up to 767 x 383 (depending on the SM count) run the
  * whole loop as one resident kernel instead of one launch per sweep; a shape
- * set here keeps the loop to the per-sweep kernels.
+ * set here keeps the loop to the per-sweep kernels.  The resident kernel is a
+ * cooperative launch of up to one CTA per SM: where the GPU has no room for
+ * all of them at once, or not within 0.2 s, the call continues with the
+ * per-sweep kernels.  Once they run, they wait for one another between
+ * phases for at most two seconds, then the call returns IXB_ETIMEOUT.
  * No reference counterpart: the reference runs one sequential tridiagonal
  * per OpenACC gang. */
 int ixb_set_sweep_shape(ixb_handle* h, int sweep, int lines_per_cta, int threads_per_line);
@@ -238,6 +243,13 @@ int ixb_set_sweep_shape(ixb_handle* h, int sweep, int lines_per_cta, int threads
  * every sweep at two kernels.  0 where the resident loop kernel runs: the
  * iterations of a call are one launch (one per 2048 of them). */
 int ixb_iteration_launches(ixb_handle* h, int* launches);
+/* Failure-detection hook, no counterpart in the reference; for tests only.
+ * which 1: in the resident kernels' launches of this handle's calls (SIMPLE
+ * loop, energy passes), from the call's launch number `from` on, the CTAs wait
+ * for one more of them than there is and give up at once, so the call goes on
+ * with the per-sweep kernels; 2: the same at the first wait between phases, so
+ * the call returns IXB_ETIMEOUT; 0: neither. */
+int ixb_expire_grid_wait(ixb_handle* h, int which, int from);
 /* Autotuner for the launch shapes: for every sweep, times each candidate
  * shape `reps` times on the current state (a scratch buffer of flush_bytes
  * is written before every timed launch when flush_bytes > 0) and keeps the
@@ -319,7 +331,9 @@ int ixb_tridiag_f64_noalloc(const double* a, const double* b, const double* c, c
  * grad[jj-1] = d nu0 / d value(jj), jj = 1..nj+1 (zero where the line is not
  * solved).  The map is affine in T with u, v fixed, so the gradient is exact
  * (transposed line solves, no stored forward states); the state is left
- * unchanged.  ixb_set_bc_values sets the per-line values of one side of a
+ * unchanged.  Both run as one resident kernel on grids of up to about
+ * 445 x 445 and return IXB_ETIMEOUT as described at ixb_set_sweep_shape (T is
+ * then partly swept by ixb_energy_iterations).  ixb_set_bc_values sets the per-line values of one side of a
  * boundary table (a per-node profile, beyond the reference's 15 segments),
  * keeping each line's type. */
 /* ---- discrete adjoint of the full coupled SIMPLE iteration ----

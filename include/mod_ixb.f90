@@ -315,6 +315,12 @@ module ixb
        integer(c_int), intent(out) :: launches
      end function ixb_iteration_launches
 
+     integer(c_int) function ixb_expire_grid_wait(h, which, from) bind(C, name="ixb_expire_grid_wait")
+       import :: c_int, c_ptr
+       type(c_ptr), value :: h
+       integer(c_int), value :: which, from
+     end function ixb_expire_grid_wait
+
      integer(c_int) function ixb_autotune(h, reps, flush_bytes, chosen, ms) bind(C, name="ixb_autotune")
        import :: c_int, c_ptr, c_size_t, c_double
        type(c_ptr), value :: h

@@ -194,7 +194,7 @@ struct AdjCtx {
   int init(int j0, int j1) {
     const int mi = h->mi, nj = h->nj;
     fsz = h->fsz;
-    const size_t need = (C_COUNT + 3) * fsz + (size_t)(nj + 2) + 1;  // the last: barrier and flag of the resident passes
+    const size_t need = (C_COUNT + 3) * fsz + (size_t)(nj + 2) + sizeof(GridWords) / sizeof(double);
     if (h->adj_size < need) {
       if (h->adj_pool) cudaFree(h->adj_pool);
       h->adj_pool = nullptr;
@@ -284,13 +284,13 @@ extern "C" int ixb_adjoint_energy(ixb_handle* h, int K, int j0, int j1, double* 
   // WHILE graph kLoopUnroll at a time (rebuilt when the handle or its
   // workspace changes) and what is left as plain launches
   if (K > 0) TRY(A.pass());
-  const int left = std::max(K - 1, 0);
+  int left = std::max(K - 1, 0);
   PassArgs P{};
   if (left > 0 && handle_resident_passes(h, &P)) {
     P.coef = A.coef; P.f0 = A.my; P.f1 = A.mx; P.grad = A.gd; P.passes = left;
-    unsigned* w = reinterpret_cast<unsigned*>(A.gd + h->nj + 2);
-    TRY(handle_run_passes(h, true, P, w));
-    return A.finish(grad);
+    int done = 0;
+    TRY(handle_run_passes(h, true, P, reinterpret_cast<GridWords*>(A.gd + h->nj + 2), &done));
+    left -= done;
   }
   const std::function<int()> pass = [&A]() -> int { return A.pass(); };
   if (left >= kLoopUnroll) {

@@ -268,7 +268,7 @@ bool loop_usable(const ixb_handle* h) {
   LoopShape shape;
   return fused_enabled() && do_while_loops() && loop_shape(h->mi, h->nj, h->nsm, &shape);
 }
-bool use_loop(const ixb_handle* h) { return h->use_graph && loop_usable(h); }
+bool use_loop(const ixb_handle* h) { return h->use_graph && !h->loop_off && loop_usable(h); }
 
 // Outer passes of one launch (0.05 to 0.2 s).
 constexpr int kLoopPasses = 2048;
@@ -282,20 +282,33 @@ LoopArgs loop_args(const ixb_handle* h, int part) {
   a.u_ant = h->u_ant; a.v_ant = h->v_ant; a.T_ant = h->T_ant;
   for (int k = 0; k < 3; ++k) { a.fcon[k] = h->fcon[k]; a.flin[k] = h->flin[k]; }
   a.bc = h->bc; a.bcstride = h->bcstride;
-  a.ctl = h->ctl_d; a.partials = h->partials; a.bar = &h->ctl_d->bar; a.norms = h->norms;
+  a.ctl = h->ctl_d; a.partials = h->partials; a.norms = h->norms;
+  a.waits = GridWaits{&h->ctl_d->grid, h->grid_expire_from > 0 ? GRID_EXPIRE_NONE : h->grid_expire};
   a.max_outer = kLoopPasses;
   a.part = part;
   return a;
 }
 
+// A launch of the resident kernel; *placed: the device has room for its grid
+// (a partition of the GPU may have fewer SMs than the device reports).
+int loop_start(ixb_handle* h, const LoopArgs& a, bool* placed) {
+  const cudaError_t e = loop_launch(solver_form(h), a, h->stream);
+  *placed = e != cudaErrorCooperativeLaunchTooLarge;
+  if (!*placed) { cudaGetLastError(); return IXB_OK; }
+  CK(e);
+  return IXB_OK;
+}
+
 // One part of an outer pass (host-driven loop); its norms arrive in h_norms.
-int loop_part(ixb_handle* h, int part) {
+// *ran false: the CTAs did not all start, nothing was done.
+int loop_part(ixb_handle* h, int part, bool* ran) {
   CK(cudaMemsetAsync(h->ctl_d, 0, sizeof(Ctl), h->stream));
-  CK(loop_launch(solver_form(h), loop_args(h, part), h->stream));
+  TRY(loop_start(h, loop_args(h, part), ran));
   CK(cudaMemcpyAsync(h->h_norms, h->norms, N_COUNT * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  CK(cudaMemcpyAsync(&h->ctl_h->abort_flag, &h->ctl_d->abort_flag, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaMemcpyAsync(&h->ctl_h->grid, &h->ctl_d->grid, sizeof(GridWords), cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
-  return h->ctl_h->abort_flag ? IXB_ETIMEOUT : IXB_OK;
+  if (h->ctl_h->grid.gave_up == GRID_NOT_MET) *ran = false;
+  return h->ctl_h->grid.gave_up == GRID_GAVE_UP ? IXB_ETIMEOUT : IXB_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -303,20 +316,26 @@ int loop_part(ixb_handle* h, int part) {
 // ---------------------------------------------------------------------------
 int body_host(ixb_handle* h, bool outer_test, ixb_report* rep, int* exit_code) {
   const ixb_params& P = h->prm;
-  const bool resident = loop_usable(h);  // the parts of the loop kernel, else single sweeps
+  bool resident = loop_usable(h);  // the parts of the loop kernel, else single sweeps
   if (resident) TRY(normalize_parity(h));
+  // a part of the pass by the loop kernel, or by `single`; its norms in h_norms
+  const auto part = [&](int which, const auto& single) -> int {
+    if (resident) {
+      TRY(loop_part(h, which, &resident));
+      if (resident) return IXB_OK;
+    }
+    TRY(single());
+    return read_norms(h);
+  };
   // ecuacion_momento
   for (;;) {
-    if (resident) {
-      TRY(loop_part(h, LOOP_MOMENTUM));
-    } else {
+    TRY(part(LOOP_MOMENTUM, [&]() -> int {
       TRY(sweep(h, EQ_UY, nullptr, false));
       TRY(sweep(h, EQ_UX, nullptr, false));
       const double* v_start = h->v[h->cv];
       TRY(sweep(h, EQ_VY, nullptr, false));
-      TRY(sweep(h, EQ_VX, v_start, true));
-      TRY(read_norms(h));
-    }
+      return sweep(h, EQ_VX, v_start, true);
+    }));
     const double err = h->h_norms[N_DV];
     rep->err_u = err;
     rep->n_momen++;
@@ -326,16 +345,13 @@ int body_host(ixb_handle* h, bool outer_test, ixb_report* rep, int* exit_code) {
     else h->iter_ecuaci++;
   }
   // correccion_presion
-  if (!resident) CK(cudaMemsetAsync(h->pc[h->cpc], 0, h->fsz * sizeof(double), h->stream));
   for (bool first = true;; first = false) {
-    if (resident) {
-      TRY(loop_part(h, first ? LOOP_PRESSURE_FIRST : LOOP_PRESSURE));
-    } else {
+    TRY(part(first ? LOOP_PRESSURE_FIRST : LOOP_PRESSURE, [&]() -> int {
+      if (first) CK(cudaMemsetAsync(h->pc[h->cpc], 0, h->fsz * sizeof(double), h->stream));
       const double* pc_start = h->pc[h->cpc];
       TRY(sweep(h, EQ_PY, nullptr, false));
-      TRY(sweep(h, EQ_PX, pc_start, true));
-      TRY(read_norms(h));
-    }
+      return sweep(h, EQ_PX, pc_start, true);
+    }));
     const double err = h->h_norms[N_DP];
     rep->err_p = err;
     rep->maxbo = h->h_norms[N_BO];
@@ -345,18 +361,14 @@ int body_host(ixb_handle* h, bool outer_test, ixb_report* rep, int* exit_code) {
     else if (h->iter_ecuaci > P.iter_ecuaci_max) { h->iter_ecuaci = 0; break; }
     else h->iter_ecuaci++;
   }
-  if (resident) TRY(loop_part(h, LOOP_CORRECT));
-  else TRY(correct(h));
+  TRY(part(LOOP_CORRECT, [&]() { return correct(h); }));
   // solucion_energia
   for (;;) {
-    if (resident) {
-      TRY(loop_part(h, LOOP_ENERGY));
-    } else {
+    TRY(part(LOOP_ENERGY, [&]() -> int {
       const double* t_start = h->T[h->cT];
       TRY(sweep(h, EQ_TY, nullptr, false));
-      TRY(sweep(h, EQ_TX, t_start, true));
-      TRY(read_norms(h));
-    }
+      return sweep(h, EQ_TX, t_start, true);
+    }));
     const double err = h->h_norms[N_DT];
     rep->err_t = err;
     rep->n_ener++;
@@ -365,12 +377,7 @@ int body_host(ixb_handle* h, bool outer_test, ixb_report* rep, int* exit_code) {
     else if (h->iter_ecuaci > P.iter_ecuaci_max) { h->iter_ecuaci = 0; break; }
     else h->iter_ecuaci++;
   }
-  if (resident) {
-    TRY(loop_part(h, LOOP_RESIDUAL));
-  } else {
-    TRY(residual(h));
-    TRY(read_norms(h));
-  }
+  TRY(part(LOOP_RESIDUAL, [&]() { return residual(h); }));
   rep->residuo = h->h_norms[N_RES];
   rep->n_simple++;
   if (!std::isfinite(rep->residuo)) return IXB_ENONFINITE;
@@ -669,22 +676,26 @@ constexpr int kLoopAhead = 8;
 
 // The SIMPLE loop through the resident kernel: a fixed count, the loop to its
 // exit test (fixed_count 0), or blocks of fixed_count passes with the Nusselt
-// monitor between them (`mon`).
-int run_loop(ixb_handle* h, int fixed_count, ixb_report* rep, const ixb_nu_monitor* mon = nullptr) {
+// monitor between them (`mon`).  *whole false (with IXB_OK): the CTAs of a
+// launch did not all start; the passes up to it are done and in `rep`, the
+// control block (ctl_h) holds where the run stands.
+int run_loop(ixb_handle* h, int fixed_count, ixb_report* rep, const ixb_nu_monitor* mon, bool* whole) {
   TRY(normalize_parity(h));
   fill_ctl(h, fixed_count, mon);
   LoopArgs a = loop_args(h, LOOP_ALL);
-  const int form = solver_form(h);
   CK(cudaMemcpyAsync(h->ctl_d, h->ctl_h, sizeof(Ctl), cudaMemcpyHostToDevice, h->stream));
-  bool fresh = true;  // the upload cleared the barrier
   // launches of one block of passes (unknown without a fixed count: one at a time)
   const int per_block = fixed_count > 0 ? (fixed_count + kLoopPasses - 1) / kLoopPasses : 1;
-  long long launched = 0;  // of the current block
+  long long launched = 0, all = 0;  // of the current block, of the call
+  bool placed = true;
+  *whole = true;
   for (;;) {
     for (int q = 0; q < (fixed_count > 0 ? kLoopAhead : 1); ++q) {
-      if (!fresh) CK(cudaMemsetAsync(&h->ctl_d->bar, 0, sizeof(unsigned), h->stream));
-      fresh = false;
-      CK(loop_launch(form, a, h->stream));
+      if (all > 0) CK(cudaMemsetAsync(&h->ctl_d->grid, 0, 2 * sizeof(unsigned), h->stream));
+      a.waits.expire = all >= h->grid_expire_from ? h->grid_expire : GRID_EXPIRE_NONE;
+      TRY(loop_start(h, a, &placed));
+      if (!placed) break;
+      ++all;
       if (++launched == per_block) {
         if (!mon) { if (fixed_count > 0) break; launched = 0; continue; }
         launched = 0;
@@ -693,21 +704,42 @@ int run_loop(ixb_handle* h, int fixed_count, ixb_report* rep, const ixb_nu_monit
     }
     CK(cudaMemcpyAsync(h->ctl_h, h->ctl_d, sizeof(Ctl), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
-    if (h->ctl_h->abort_flag) { h->ctl_h->status = IXB_ETIMEOUT; break; }
+    const int gave_up = h->ctl_h->grid.gave_up;
+    if (gave_up == GRID_GAVE_UP) { h->ctl_h->status = IXB_ETIMEOUT; break; }
     if (mon ? h->ctl_h->mon_over : h->ctl_h->stop) break;
+    if (gave_up == GRID_NOT_MET || !placed) { *whole = false; break; }
   }
   return read_ctl(h, rep);
 }
 
-// The SIMPLE loop on the device: a fixed count that is a positive multiple
-// of kOuterUnroll runs through the unrolled graph (one WHILE body launch per
-// kOuterUnroll passes), anything else through the plain one.  (Splitting
-// other counts into the two graphs costs a second launch and host sync per
-// call, more than the unrolling saves on small grids.)
-int run_graph(ixb_handle* h, int fixed_count, ixb_report* rep) {
-  if (use_loop(h)) return run_loop(h, fixed_count, rep);
+// The SIMPLE loop through a graph of sweeps: a fixed count that is a positive
+// multiple of kOuterUnroll runs through the unrolled graph (one WHILE body
+// launch per kOuterUnroll passes), anything else through the plain one.
+// (Splitting other counts into the two graphs costs a second launch and host
+// sync per call, more than the unrolling saves on small grids.)
+int run_sweep_graph(ixb_handle* h, int fixed_count, ixb_report* rep) {
   const bool unrolled = fixed_count > 0 && fixed_count % kOuterUnroll == 0;
   return run_graph_once(h, unrolled ? GRAPH_UNROLLED : GRAPH_PLAIN, fixed_count, rep);
+}
+
+// `more` of the same run into `rep`.
+void add_report(ixb_report* rep, const ixb_report& more) {
+  const ixb_report had = *rep;
+  *rep = more;
+  rep->n_simple += had.n_simple; rep->n_momen += had.n_momen; rep->n_pres += had.n_pres; rep->n_ener += had.n_ener;
+}
+
+// The SIMPLE loop on the device: the resident kernel where it serves the
+// handle, and the graph for what that could not run.
+int run_graph(ixb_handle* h, int fixed_count, ixb_report* rep) {
+  if (!use_loop(h)) return run_sweep_graph(h, fixed_count, rep);
+  bool whole;
+  TRY(run_loop(h, fixed_count, rep, nullptr, &whole));
+  if (whole) return IXB_OK;
+  ixb_report more{};
+  const int st = run_sweep_graph(h, fixed_count > 0 ? fixed_count - h->ctl_h->outer_done : 0, &more);
+  add_report(rep, more);
+  return st;
 }
 
 void free_all(ixb_handle* h) {
@@ -1267,25 +1299,37 @@ int ixb_simple_converge(ixb_handle* h, const ixb_nu_monitor* mon, ixb_report* re
   ixb_report* r = rep ? rep : &local;
   rep_clear(r);
   double nu2[2] = {0.0, 0.0}, d = INFINITY;
-  int st;
+  int st = IXB_OK;
+  // host-driven, from the start or from where the resident kernel left off
+  bool by_host = !h->use_graph;
+  int block = mon->every;  // passes to the next evaluation
+  long long evals = 0;
+  double prev = 0.0;
   if (h->use_graph) {
     const int kind = mon->every % kOuterUnroll == 0 ? GRAPH_MON_UNROLLED : GRAPH_MON_PLAIN;
-    st = use_loop(h) ? run_loop(h, mon->every, r, mon) : run_graph_once(h, kind, mon->every, r, mon);
+    bool whole = true;
+    st = use_loop(h) ? run_loop(h, mon->every, r, mon, &whole) : run_graph_once(h, kind, mon->every, r, mon);
     const Ctl* c = h->ctl_h;
     nu2[0] = c->mon_nu[0];
     nu2[1] = c->mon_nu[1];
     d = c->mon_dnu;
-  } else {
-    // host-driven: blocks of `every` passes, the Nusselt number and the
-    // monitor's test on the host, in the order the graph applies them
-    st = IXB_OK;
-    long long evals = 0;
-    double prev = 0.0;
-    while (st == IXB_OK) {
+    if (!whole && st == IXB_OK) {
+      by_host = true;
+      h->loop_off = true;
+      block -= c->outer_done;
+      evals = c->mon_evals;
+      prev = c->mon_nu_prev;
+    }
+  }
+  if (by_host) {
+    // blocks of `every` passes, the Nusselt number and the monitor's test on
+    // the host, in the order the graph applies them
+    for (; st == IXB_OK; block = mon->every) {
       ixb_report b;
-      st = ixb_simple_iterations(h, mon->every, &b);
-      r->n_simple += b.n_simple; r->n_momen += b.n_momen; r->n_pres += b.n_pres; r->n_ener += b.n_ener;
-      r->maxbo = b.maxbo; r->residuo = b.residuo; r->err_u = b.err_u; r->err_p = b.err_p; r->err_t = b.err_t;
+      st = ixb_simple_iterations(h, block, &b);
+      const int code = r->exit_code;
+      add_report(r, b);
+      r->exit_code = code;
       if (st != IXB_OK) break;
       st = nusselt(h, mon->vertical, mon->k0, mon->k1, &nu2[0], &nu2[1]);
       if (st != IXB_OK) break;
@@ -1298,6 +1342,7 @@ int ixb_simple_converge(ixb_handle* h, const ixb_nu_monitor* mon, ixb_report* re
       if (r->maxbo < mon->tol_maxbo) { r->exit_code = 4; break; }
       if (r->n_simple >= mon->max_iters) { r->exit_code = 5; break; }
     }
+    h->loop_off = false;
   }
   if (nu) { nu[0] = nu2[0]; nu[1] = nu2[1]; }
   if (dnu) *dnu = d;
@@ -1513,20 +1558,25 @@ int ixb_energy_iterations(ixb_handle* h, int n) {
   const bool own_shape = h->shape_set[EQ_TY] || h->shape_set[EQ_TX];
   if (n >= 4 && !own_shape && solver_form(h) == IXB_SOLVER_HYBRID && handle_resident_passes(h, &P)) {
     double* work = nullptr;
-    const cudaError_t e = scratch_alloc(reinterpret_cast<void**>(&work), (C_COUNT * h->fsz + 1) * sizeof(double), h->stream);
+    const cudaError_t e =
+        scratch_alloc(reinterpret_cast<void**>(&work), C_COUNT * h->fsz * sizeof(double) + sizeof(GridWords), h->stream);
     if (e == cudaSuccess) {
       h->scratch_used = true;
       SweepIO<double> io = handle_fixed_io(h, EQ_TX);
       io.in = h->zero;
       cudaError_t k = energy_coef_launch(P.G, io, work, h->fsz, h->stream);
       P.coef = work; P.f0 = h->T[h->cT]; P.f1 = h->T[h->cT ^ 1]; P.passes = n;
-      int st = IXB_ECUDA;
-      if (k == cudaSuccess) st = handle_run_passes(h, false, P, reinterpret_cast<unsigned*>(work + C_COUNT * h->fsz));
-      else h->last_cuda = k;
+      int st = IXB_ECUDA, done = 0;
+      if (k == cudaSuccess)
+        st = handle_run_passes(h, false, P, reinterpret_cast<GridWords*>(work + C_COUNT * h->fsz), &done);
+      else
+        h->last_cuda = k;
       cudaFreeAsync(work, h->stream);
-      return st;
+      n -= done;
+      if (st != IXB_OK || n == 0) return st;
+    } else {
+      cudaGetLastError();  // no room for the factors: the sweeps
     }
-    cudaGetLastError();  // no room for the factors: the sweeps
   }
   // one pass, T-y then T-x (buffer parity back to 0); kLoopUnroll of them
   // form the body of a WHILE loop, the rest run as plain launches
@@ -1541,6 +1591,13 @@ int ixb_energy_iterations(ixb_handle* h, int n) {
   if (n >= kLoopUnroll) TRY(handle_run_loop_graph(h, h->egraph_exec, n / kLoopUnroll));
   for (int k = 0; k < n % kLoopUnroll; ++k) TRY(pass());
   CK(cudaStreamSynchronize(h->stream));
+  return IXB_OK;
+}
+
+int ixb_expire_grid_wait(ixb_handle* h, int which, int from) {
+  if (!h || which < GRID_EXPIRE_NONE || which > GRID_EXPIRE_SYNC || from < 0) return IXB_EINVAL;
+  h->grid_expire = which;
+  h->grid_expire_from = from;
   return IXB_OK;
 }
 
@@ -1649,15 +1706,18 @@ bool handle_resident_passes(ixb_handle* h, PassArgs* a) {
   a->last_y = base + 3 * (size_t)h->bcstride;
   return true;
 }
-int handle_run_passes(ixb_handle* h, bool reverse, PassArgs& a, unsigned* w) {
-  a.bar = w;
-  a.abort_flag = reinterpret_cast<int*>(w + 1);
-  CK(cudaMemsetAsync(w, 0, 2 * sizeof(unsigned), h->stream));
-  CK(energy_passes_launch(reverse, a, h->stream));
-  int gave_up = 0;
-  CK(cudaMemcpyAsync(&gave_up, a.abort_flag, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+int handle_run_passes(ixb_handle* h, bool reverse, PassArgs& a, GridWords* w, int* done) {
+  *done = 0;
+  a.waits = GridWaits{w, h->grid_expire};
+  CK(cudaMemsetAsync(w, 0, sizeof(GridWords), h->stream));
+  const cudaError_t e = energy_passes_launch(reverse, a, h->grid_expire_from, h->stream);
+  if (e == cudaErrorCooperativeLaunchTooLarge) cudaGetLastError();  // as if its CTAs had not all started
+  else CK(e);
+  GridWords r{};
+  CK(cudaMemcpyAsync(&r, w, sizeof(GridWords), cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
-  return gave_up ? IXB_ETIMEOUT : IXB_OK;
+  *done = r.passes;
+  return r.gave_up == GRID_GAVE_UP ? IXB_ETIMEOUT : IXB_OK;
 }
 int handle_single_passes(ixb_handle* h, int n) {
   // every inner test met after its first pass

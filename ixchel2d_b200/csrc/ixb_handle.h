@@ -7,6 +7,7 @@
 
 #include <vector>
 
+#include "ixb_grid.h"
 #include "ixb_passes.h"
 #include "ixb_internal.h"
 
@@ -25,8 +26,8 @@ struct Ctl {
   int exit_code, status;
   long long n_simple, n_momen, n_pres, n_ener;
   double err_u, err_p, err_t, maxbo, residuo;
-  // resident loop (ixb_loop.cuh): the run is over; a bounded grid wait ran out
-  int stop, abort_flag, mon_over;
+  // resident loop (ixb_loop.cuh): the run is over
+  int stop, mon_over;
   // Nusselt monitor (ixb_simple_converge): inputs
   int mon_vertical, mon_k0, mon_k1, mon_wall;
   long long mon_max_iters;
@@ -34,8 +35,8 @@ struct Ctl {
   // Nusselt monitor: state
   long long mon_evals;
   double mon_nu[2], mon_nu_prev, mon_dnu;
-  // arrivals of the resident loop's grid barrier, on a line of its own
-  alignas(128) unsigned bar;
+  // the resident loop's waits, on a line of their own
+  alignas(128) GridWords grid;
 };
 
 // the SIMPLE loop graphs of a handle
@@ -106,6 +107,8 @@ struct ixb_handle {
   bool shape_set[ixb::EQ_COUNT] = {};  // set by the caller (ixb_set_sweep_shape): the loop keeps to the per-sweep kernels
   bool scratch_used = false;           // a gradient has grown the scratch pool
   bool coop = false;                   // the device takes cooperative launches
+  bool loop_off = false;               // the call goes on without the resident kernel (its CTAs did not all start)
+  int grid_expire = 0, grid_expire_from = 0;  // ixb_expire_grid_wait
   int nsm = 148;
   // adjoint workspace (ixb_adjoint_energy), allocated on first use
   double* xfer = nullptr;  // seven host-shaped (column-major, unpadded) state arrays: the state transfers' staging, allocated on the first transfer
@@ -145,8 +148,10 @@ int handle_sweep_to(ixb_handle* h, int eq, const SweepIO<double>& io, bool early
 // Whether the resident energy passes (ixb_passes.h) serve the handle's grid;
 // fills the fields of `a` that follow from the handle (fixed velocities).
 bool handle_resident_passes(ixb_handle* h, ixb::PassArgs* a);
-// runs them and waits; w: two words on the device (barrier, flag)
-int handle_run_passes(ixb_handle* h, bool reverse, ixb::PassArgs& a, unsigned* w);
+// Runs them and waits; w: their waits' words on the device.  Returns in *done
+// how many ran: fewer than asked for, with IXB_OK, when a launch's CTAs did
+// not all start.
+int handle_run_passes(ixb_handle* h, bool reverse, ixb::PassArgs& a, ixb::GridWords* w, int* done);
 // n outer iterations of one pass of each equation, whatever the parameters'
 // tests say; the loop counters are left alone
 int handle_single_passes(ixb_handle* h, int n);

@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(kNuThreads)
                    int in_graph, cudaGraphConditionalHandle cond) {
   __shared__ double terms[2][3][kNuThreads];
   if (mon) {
-    if (!in_graph && mon->mon_over) return;  // launched ahead of the block that ended the run
+    if (!in_graph && (mon->mon_over || mon->grid.gave_up)) return;  // launched ahead of what ended the run
     vertical = mon->mon_vertical;
     k0 = mon->mon_k0;
     k1 = mon->mon_k1;

@@ -621,6 +621,7 @@ __global__ void __launch_bounds__(NT, 1) simple_loop_kernel(const __grid_constan
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Ctl* c = A.ctl;
   if (A.part == LOOP_ALL && c->stop) return;  // an earlier launch of this run ended it
+  grid_arrive(A.waits);
   const int mi = A.G.mi, nj = A.G.nj;
   const int ly = threadIdx.x % A.s.y_lines, ky = threadIdx.x / A.s.y_lines;
   const int gid = threadIdx.x / A.s.gx, kx = threadIdx.x - gid * A.s.gx;
@@ -679,12 +680,12 @@ __global__ void __launch_bounds__(NT, 1) simple_loop_kernel(const __grid_constan
     s.err_u = c->err_u; s.err_p = c->err_p; s.err_t = c->err_t; s.maxbo = c->maxbo; s.residuo = c->residuo;
     s.go = 1; s.passes = 0;
   }
-  __syncthreads();
+  if (!grid_meet(A.waits)) return;
   unsigned target = 0;
   double* const part = A.partials;
   const int np = gridDim.x;
 #define IXB_GRID_SYNC() \
-  if (!grid_sync(A.bar, &c->abort_flag, target)) return
+  if (!grid_sync(A.waits, target)) return
   const int part_only = A.part;
   // a single-part launch leaves its norms in A.norms and ends
   auto publish = [&](int id, double v) {
@@ -755,8 +756,8 @@ __global__ void __launch_bounds__(NT, 1) simple_loop_kernel(const __grid_constan
       if (next == NEXT_ON) stage = 2;
     } else if (stage == 2) {
       loop_correct<true>();
-      IXB_GRID_SYNC();
       if (part_only) break;
+      IXB_GRID_SYNC();
       stage = 3;
     } else {
       // energy pass (main.f90:975-1156)

@@ -37,7 +37,7 @@ struct LoopArgs {
   int bcstride;
   Ctl* ctl;
   double* partials;  // [N_COUNT][grid]
-  unsigned* bar;     // grid barrier: arrivals since the launch (zero at its start)
+  GridWaits waits;
   LoopShape s;
   double* norms;     // N_COUNT, written by a single-part launch
   int max_outer;     // outer passes this launch may run

@@ -5,6 +5,7 @@
 
 #include <cstddef>
 
+#include "ixb_grid.h"
 #include "ixb_internal.h"
 
 namespace ixb {
@@ -23,8 +24,7 @@ struct PassArgs {
   const BCEntry *first_x, *last_x, *first_y, *last_y;
   double *f0, *f1;     // f0 -> f1 -> f0 in every pass
   double* grad;        // transposed passes: += the first row's values, by x-line
-  unsigned* bar;       // zeroed before every launch
-  int* abort_flag;     // set when a grid barrier's bounded wait ran out
+  GridWaits waits;
   int passes;
   int lx, cx, ly, cy;  // lines per CTA and chunks per line of either direction
   int grid;
@@ -36,7 +36,8 @@ cudaError_t energy_coef_launch(const Geo<double>& G, const SweepIO<double>& io, 
 // Whether a grid's lines, factored in both directions, fit one CTA per SM;
 // fills lx, cx, ly, cy, grid.
 bool energy_passes_fit(int mi, int nj, int nsm, PassArgs* a);
-// a.passes (T-y, T-x) passes, or their transposes (T-x first)
-cudaError_t energy_passes_launch(bool reverse, const PassArgs& a, cudaStream_t st);
+// a.passes (T-y, T-x) passes, or their transposes (T-x first); the launches
+// from number expire_from on get a.waits.expire
+cudaError_t energy_passes_launch(bool reverse, const PassArgs& a, int expire_from, cudaStream_t st);
 
 }  // namespace ixb

@@ -218,22 +218,25 @@ template <bool REV>
 __global__ void __launch_bounds__(PMAXT, 1) energy_pass_kernel(const __grid_constant__ PassArgs A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int T = blockDim.x;
+  grid_arrive(A.waits);
   double* qx = reinterpret_cast<double*>(smem_raw);
   double* qy = qx + PQ * T;
   double* ex = qy + PQ * T;
   Chunk3 hx, hy;
   factor<REV, true>(hx, A, qx, ex);
   factor<REV, false>(hy, A, qy, ex);
+  if (!grid_meet(A.waits)) return;
   unsigned target = 0;
   double grad = 0.0;
   for (int p = 0; p < A.passes; ++p) {
     if (REV) grad += pass_sweep<REV, true>(hx, A, qx, ex, A.f0, A.f1);
     else pass_sweep<REV, false>(hy, A, qy, ex, A.f0, A.f1);
-    if (!grid_sync(A.bar, A.abort_flag, target)) return;
+    if (!grid_sync(A.waits, target)) return;
     if (REV) pass_sweep<REV, false>(hy, A, qy, ex, A.f1, A.f0);
     else pass_sweep<REV, true>(hx, A, qx, ex, A.f1, A.f0);
-    if (!grid_sync(A.bar, A.abort_flag, target)) return;
+    if (!grid_sync(A.waits, target)) return;
   }
+  if (blockIdx.x == 0 && threadIdx.x == 0) A.waits.words->passes += A.passes;
   if (REV && hx.rows > 0 && hx.k == 0) A.grad[2 + blockIdx.x * A.lx + threadIdx.x / A.cx] += grad;
 }
 
@@ -268,7 +271,7 @@ cudaError_t energy_coef_launch(const Geo<double>& G, const SweepIO<double>& io, 
 }
 
 // A launch runs up to kPassesPerLaunch passes (a bounded kernel time).
-cudaError_t energy_passes_launch(bool reverse, const PassArgs& a, cudaStream_t st) {
+cudaError_t energy_passes_launch(bool reverse, const PassArgs& a, int expire_from, cudaStream_t st) {
   const int T = threads_of(a);
   const size_t smem = smem_of(T);
   const void* k = reverse ? reinterpret_cast<const void*>(energy_pass_kernel<true>)
@@ -276,9 +279,11 @@ cudaError_t energy_passes_launch(bool reverse, const PassArgs& a, cudaStream_t s
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   PassArgs q = a;
-  for (int left = a.passes; left > 0; left -= q.passes) {
+  int launch = 0;
+  for (int left = a.passes; left > 0; left -= q.passes, ++launch) {
     q.passes = std::min(left, kPassesPerLaunch);
-    if ((e = cudaMemsetAsync(q.bar, 0, sizeof(unsigned), st)) != cudaSuccess) return e;
+    q.waits.expire = launch >= expire_from ? a.waits.expire : GRID_EXPIRE_NONE;
+    if ((e = cudaMemsetAsync(q.waits.words, 0, 2 * sizeof(unsigned), st)) != cudaSuccess) return e;
     void* params[] = {&q};
     if ((e = cudaLaunchCooperativeKernel(k, dim3(q.grid), dim3(T), params, smem, st)) != cudaSuccess) return e;
   }
