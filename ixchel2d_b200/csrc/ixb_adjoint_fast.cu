@@ -136,7 +136,7 @@ template <bool X, bool FIRST, int TL, int GT, int M>
 cudaError_t adj_sweep_go(const SweepArgs& q, cudaStream_t st) {
   auto k = adj_sweep_kernel<X, FIRST, TL, GT, M>;
   const size_t smem = (size_t)9 * TL * GT * sizeof(double);
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(k);
   if (e != cudaSuccess) return e;
   k<<<(q.s.nl + 2 + TL - 1) / TL, TL * GT, smem, st>>>(q.G, q.s, q.prev, q.coef, q.fsz, q.keep, q.f, q.mu, q.grad);
   return cudaGetLastError();

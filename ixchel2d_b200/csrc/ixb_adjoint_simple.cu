@@ -322,7 +322,7 @@ cudaError_t adj_sweep_launch(const Geo<double>& G, const SweepState& s, double* 
   auto go = [&](auto k, int tl, int g, int rp, int m) -> cudaError_t {
     const size_t smem = line_smem_elems(g, m | 1) * sizeof(double) * tl;
     if (smem > 48 * 1024) {  // beyond the default limit
-      const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      const cudaError_t e = allow_smem(k);
       if (e != cudaSuccess) return e;
     }
     return launch_pdl(true, k, (s.nfull + tl - 1) / tl, tl * g * rp, smem, st, G, s, lam, aux_bar, adj, grad, m, m | 1);

@@ -46,6 +46,20 @@ inline cudaError_t launch_k(void (*k)(KArgs...), dim3 grid, dim3 block, size_t s
   return launch_pdl(false, k, grid, block, smem, st, std::forward<Args>(args)...);
 }
 
+// Dynamic shared memory of a kernel: all that the device allows beside its
+// `statics` bytes of static shared memory, whatever this launch needs.  The
+// limit belongs to the kernel and not to a launch, and other handles' threads
+// launch it with other sizes: it is only ever set to this one value.
+template <class K>
+inline cudaError_t allow_smem(K* k, int statics = 1024) {
+  int dev = 0, optin = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(reinterpret_cast<const void*>(k), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              optin - statics);
+}
+
 enum NormId { N_DV = 0, N_DP, N_BO, N_DT, N_RES, N_COUNT };
 
 // Loop control carried by a kernel of the graph-driven SIMPLE loop (ctl

@@ -794,7 +794,7 @@ cudaError_t loop_go(const LoopArgs& a, cudaStream_t st) {
   using S = typename SweepTypes<SOLVER, EQ_UX>::S;
   const size_t line = std::max(a.s.x_lines * a.s.gx, (a.s.y_lines * a.s.gy + 31) / 32 * 32);
   const size_t smem = loop_fixed_bytes(a.G.mi, a.G.nj) + 12 * line * sizeof(S);
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(k);
   if (e != cudaSuccess) return e;
   LoopArgs args = a;
   void* params[] = {&args};

@@ -274,9 +274,8 @@ cudaError_t energy_coef_launch(const Geo<double>& G, const SweepIO<double>& io, 
 cudaError_t energy_passes_launch(bool reverse, const PassArgs& a, int expire_from, cudaStream_t st) {
   const int T = threads_of(a);
   const size_t smem = smem_of(T);
-  const void* k = reverse ? reinterpret_cast<const void*>(energy_pass_kernel<true>)
-                          : reinterpret_cast<const void*>(energy_pass_kernel<false>);
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  auto k = reverse ? energy_pass_kernel<true> : energy_pass_kernel<false>;
+  cudaError_t e = allow_smem(k);
   if (e != cudaSuccess) return e;
   PassArgs q = a;
   int launch = 0;
@@ -285,7 +284,7 @@ cudaError_t energy_passes_launch(bool reverse, const PassArgs& a, int expire_fro
     q.waits.expire = launch >= expire_from ? a.waits.expire : GRID_EXPIRE_NONE;
     if ((e = cudaMemsetAsync(q.waits.words, 0, 2 * sizeof(unsigned), st)) != cudaSuccess) return e;
     void* params[] = {&q};
-    if ((e = cudaLaunchCooperativeKernel(k, dim3(q.grid), dim3(T), params, smem, st)) != cudaSuccess) return e;
+    if ((e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k), dim3(q.grid), dim3(T), params, smem, st)) != cudaSuccess) return e;
   }
   return cudaSuccess;
 }

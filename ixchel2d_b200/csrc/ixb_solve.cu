@@ -138,7 +138,7 @@ struct SolveSet {
 #define IXB_BCASE_(TL_, G_)                                                                                \
   if (tl == TL_ && g == G_) {                                                                              \
     auto k = solve_batch_kernel<S, X, DC, EXACT, TL_, G_>;                                                 \
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);       \
+    cudaError_t e = allow_smem(k);                                                                         \
     if (e != cudaSuccess) return e;                                                                        \
     int per_sm = 0, dev = 0, nsm = 0;                                                                      \
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, TL_ * G_, smem)) != cudaSuccess)    \

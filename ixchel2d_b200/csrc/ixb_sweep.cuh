@@ -484,19 +484,12 @@ __global__ void __launch_bounds__(TL * G, TL * G > 256                          
 template <auto K>
 cudaError_t fused_go(const SweepShape& s, const Geo<double>& G, const SweepIO<double>& io, const SolveIO& so,
                      cudaStream_t st) {
-  // the limit is a per-device attribute of the kernel: raised once per device
-  // (0: the default, 48 KB less the kernel's static shared memory)
   constexpr int kMaxDev = 64;
-  static size_t limit[kMaxDev] = {};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev < 0 || dev >= kMaxDev) return cudaErrorInvalidDevice;
-  if (s.smem > (limit[dev] ? limit[dev] : 48 * 1024 - 1024)) {
-    e = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
-    if (e != cudaSuccess) return e;
-    limit[dev] = s.smem;
-  }
+  if (s.smem > 48 * 1024 - 1024 && (e = allow_smem(K)) != cudaSuccess) return e;  // beyond the default limit
   if (carveout_enabled()) {
     // shared-memory carveout: just what the CTAs of one wave need per SM (one
     // y-line CTA, three x-line CTAs, two of 512 threads), the rest of the SM's
@@ -572,7 +565,7 @@ cudaError_t fused_batch_launch(int tl, int g, size_t smem, const FusedInst* inst
                                const int* active, const BatchNorm& bn_asm, const BatchNorm& bn_sol,
                                cudaStream_t st) {
   auto go = [&](auto k, int nt) -> cudaError_t {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(k);
     if (e != cudaSuccess) return e;
     int per_sm = 0, dev = 0, nsm = 0;
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, nt, smem)) != cudaSuccess) return e;

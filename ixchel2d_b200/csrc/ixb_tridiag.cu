@@ -356,7 +356,7 @@ cudaError_t stream_launch(const R* a, const R* b, const R* c, const R* d, R* x, 
   auto k = ragged ? tri_stream_kernel<R, T, M, true> : tri_stream_kernel<R, T, M, false>;
   constexpr size_t smem = stream_smem_bytes<R, T, M>();
   if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_smem(k, 0);
     if (e != cudaSuccess) return e;
   }
   // about one wave: by shared memory (227 KB per SM, 1 KB reserved per CTA)
@@ -1142,7 +1142,7 @@ cudaError_t strided_launch(const R* a, const R* b, const R* c, const R* d, R* x,
     return cudaErrorInvalidValue;
   auto k = tri_strided_kernel<R, SEG, ROWS>;
   const size_t smem = strided_smem_bytes<R, SEG, ROWS>();
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(k, 0);
   if (e != cudaSuccess) return e;
   if (Q > 8 && (e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess)
     return e;
@@ -1205,7 +1205,7 @@ template <class R, int SOLVER, int TL>
 static cudaError_t contig_tl(const R* a, const R* b, const R* c, const R* d, R* x, int n, int nsys, int m, int mp,
                              size_t smem, cudaStream_t st) {
   auto k = tri_contig_kernel<R, SOLVER, TL, 256 / TL>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(k, 0);
   if (e != cudaSuccess) return e;
   const int grid = (nsys + TL - 1) / TL;
   k<<<grid, 256, smem, st>>>(a, b, c, d, x, n, nsys, m, mp);
