@@ -165,6 +165,11 @@ int ixb_download_wait(ixb_handle* h);
  * no counterpart in the reference. */
 int ixb_host_alloc(size_t bytes, void** out);
 int ixb_host_free(void* p);
+/* 1 if the device can reach the whole host array (page-locked and mapped, all
+ * within one allocation or registration), else 0.  ixb_upload_state and
+ * ixb_download_state read and write such arrays directly when they are 16 MB
+ * together at most, and copy otherwise. */
+int ixb_host_reachable(const void* p, size_t bytes);
 /* Work arrays after the last iteration: au, av, b_o, Resu, corr_pres. */
 int ixb_download_aux(ixb_handle* h, double* au, double* av, double* b_o, double* resu, double* corr_pres);
 

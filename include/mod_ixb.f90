@@ -131,6 +131,12 @@ module ixb
        type(c_ptr) :: p
      end function ixb_host_alloc
 
+     integer(c_int) function ixb_host_reachable(p, bytes) bind(C, name="ixb_host_reachable")
+       import :: c_int, c_ptr, c_size_t
+       type(c_ptr), value :: p
+       integer(c_size_t), value :: bytes
+     end function ixb_host_reachable
+
      integer(c_int) function ixb_host_free(p) bind(C, name="ixb_host_free")
        import :: c_int, c_ptr
        type(c_ptr), value :: p

@@ -50,6 +50,7 @@ SIGNATURES = [
     ("ixb_download_state_async", C.c_int, [_vp, _dp, _dp, _dp, _dp, _dp, _dp, _dp]),
     ("ixb_download_wait", C.c_int, [_vp]),
     ("ixb_host_alloc", C.c_int, [C.c_size_t, C.POINTER(_vp)]),
+    ("ixb_host_reachable", C.c_int, [_vp, C.c_size_t]),
     ("ixb_host_free", C.c_int, [_vp]),
     ("ixb_download_aux", C.c_int, [_vp, _dp, _dp, _dp, _dp, _dp]),
     ("ixb_simple_iterations", C.c_int, [_vp, C.c_int, C.POINTER(Report)]),

@@ -21,6 +21,8 @@
 #include <new>
 #include <vector>
 
+#include <cuda.h>
+
 #include "ixb_ctl.cuh"
 #include "ixb_handle.h"
 #include "ixb_loop.h"
@@ -817,9 +819,38 @@ XferSet make_xfer_set(const ixb_handle* h, const std::array<double*, 7>& pad, co
   return s;
 }
 
+// The device's pointer to a host array if it can reach all of it: page-locked
+// and mapped, and within one allocation or registration (that its first and
+// last bytes are reachable says nothing of what lies between); else null.
+void* host_on_device(const void* p, size_t bytes) {
+  using AttrFn = CUresult (*)(void*, CUpointer_attribute, CUdeviceptr);
+  static const AttrFn attr = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuPointerGetAttribute", &f, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      f = nullptr;
+    }
+    return reinterpret_cast<AttrFn>(f);
+  }();
+  cudaPointerAttributes a{};
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  if (!attr || a.type != cudaMemoryTypeHost || !a.devicePointer) return nullptr;
+  const CUdeviceptr d = reinterpret_cast<CUdeviceptr>(a.devicePointer);
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  if (attr(&base, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, d) != CUDA_SUCCESS ||
+      attr(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, d) != CUDA_SUCCESS)
+    return nullptr;
+  return d >= base && d - base <= size && bytes <= size - (d - base) ? a.devicePointer : nullptr;
+}
+
 // Points the set at the host arrays themselves if the device can reach every
-// one of them (page-locked and mapped, first to last element): the kernel
-// then crosses the bus, without a copy per array before or after it.  Up and
+// one of them: the kernel then crosses the bus, without a copy per array before or after it.  Up and
 // down, copies -> this: 64x64 62 / 55 -> 35 / 36 us, 256x256 122 / 118 -> 103
 // / 100, 701x301 (12 MB) 271 / 262 -> 261 / 257; at 900x700 (35 MB) the copies
 // are 2 % faster, so larger sets keep them.
@@ -828,16 +859,8 @@ bool xfer_direct(XferSet& s, const std::array<double*, 7>& host) {
   if ((s.off[s.n - 1] + (size_t)s.rows[s.n - 1] * s.cols[s.n - 1]) * sizeof(double) > kMost) return false;
   for (int k = 0, q = 0; k < 7; ++k) {
     if (!host[k]) continue;
-    const size_t last = (size_t)s.rows[q] * s.cols[q] - 1;
-    cudaPointerAttributes a{}, z{};
-    if (cudaPointerGetAttributes(&a, host[k]) != cudaSuccess ||
-        cudaPointerGetAttributes(&z, host[k] + last) != cudaSuccess) {
-      cudaGetLastError();
-      return false;
-    }
-    if (a.type != cudaMemoryTypeHost || z.type != cudaMemoryTypeHost || !a.devicePointer) return false;
-    s.flat[q] = static_cast<double*>(a.devicePointer);
-    if (static_cast<double*>(z.devicePointer) != s.flat[q] + last) return false;
+    s.flat[q] = static_cast<double*>(host_on_device(host[k], (size_t)s.rows[q] * s.cols[q] * sizeof(double)));
+    if (!s.flat[q]) return false;
     ++q;
   }
   return true;
@@ -1209,6 +1232,8 @@ int ixb_host_alloc(size_t bytes, void** out) {
   }
   return IXB_OK;
 }
+
+int ixb_host_reachable(const void* p, size_t bytes) { return p && bytes > 0 && host_on_device(p, bytes) != nullptr; }
 
 int ixb_host_free(void* p) {
   if (p && cudaFreeHost(p) != cudaSuccess) return IXB_ECUDA;
