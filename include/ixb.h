@@ -283,6 +283,12 @@ int ixb_tridiag_f64(const double* a, const double* b, const double* c, const dou
                     int nsys, int layout, int solver, void* stream);
 int ixb_tridiag_f32(const float* a, const float* b, const float* c, const float* d, float* x, int n,
                     int nsys, int layout, int solver, void* stream);
+/* Gives the library's idle scratch memory on the current device back, after
+ * waiting for all work on it.  Line solves keep up to 32 MB mapped between
+ * calls, the gradients and energy passes of all handles up to 256 MB, which
+ * goes back when a handle that has run one is destroyed.  No counterpart in
+ * the reference. */
+int ixb_release_scratch(void);
 /* The hybrid solves above run their copies through the tensor/bulk-copy
  * engine and wait on them for a bounded time; a wait that expires leaves the
  * affected systems unwritten and is recorded on the device.  This call waits

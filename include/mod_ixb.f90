@@ -373,6 +373,10 @@ module ixb
        integer(c_int), value :: n, nsys, layout, solver
      end function ixb_tridiag_f64_noalloc
 
+     integer(c_int) function ixb_release_scratch() bind(C, name="ixb_release_scratch")
+       import :: c_int
+     end function ixb_release_scratch
+
      integer(c_int) function ixb_tridiag_status() bind(C, name="ixb_tridiag_status")
        import :: c_int
      end function ixb_tridiag_status

@@ -88,6 +88,7 @@ SIGNATURES = [
      [C.c_int, C.c_int, C.c_int, C.c_double]),
     ("ixb_read_state_files", C.c_int, [C.c_char_p, C.c_char_p, C.c_char_p, C.c_int, C.c_int] + [_vp] * 8 +
      [C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_double)]),
+    ("ixb_release_scratch", C.c_int, []),
     ("ixb_tridiag_status", C.c_int, []),
     ("ixb_tridiag_set_first_wait_limit", C.c_int, [C.c_int]),
     ("ixb_expire_grid_wait", C.c_int, [_vp, C.c_int, C.c_int]),

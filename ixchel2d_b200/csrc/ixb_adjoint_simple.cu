@@ -461,7 +461,7 @@ struct SimpleAdjoint {
     G = handle_geo(h);
     const size_t nadj = F_COUNT + 4, ngd = (size_t)h->nj + 2;
     const size_t total = ((size_t)(C + 1) * S_COUNT + (size_t)segments * 4 + nadj) * fsz + ngd;
-    const cudaError_t e = scratch_alloc(reinterpret_cast<void**>(&pool), total * sizeof(double), h->stream);
+    const cudaError_t e = scratch_alloc(SCRATCH_HANDLES, reinterpret_cast<void**>(&pool), total * sizeof(double), h->stream);
     if (e != cudaSuccess) {
       cudaGetLastError();
       pool = nullptr;

@@ -1046,7 +1046,7 @@ int ixb_destroy(ixb_handle* h) {
   const bool trim = h->scratch_used;
   free_all(h);
   delete h;
-  if (trim) scratch_trim();
+  if (trim) scratch_trim(SCRATCH_HANDLES);
   return IXB_OK;
 }
 
@@ -1584,7 +1584,8 @@ int ixb_energy_iterations(ixb_handle* h, int n) {
   if (n >= 4 && !own_shape && solver_form(h) == IXB_SOLVER_HYBRID && handle_resident_passes(h, &P)) {
     double* work = nullptr;
     const cudaError_t e =
-        scratch_alloc(reinterpret_cast<void**>(&work), C_COUNT * h->fsz * sizeof(double) + sizeof(GridWords), h->stream);
+        scratch_alloc(SCRATCH_HANDLES, reinterpret_cast<void**>(&work),
+                      C_COUNT * h->fsz * sizeof(double) + sizeof(GridWords), h->stream);
     if (e == cudaSuccess) {
       h->scratch_used = true;
       SweepIO<double> io = handle_fixed_io(h, EQ_TX);

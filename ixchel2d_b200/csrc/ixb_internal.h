@@ -315,9 +315,10 @@ cudaError_t tridiag_f32(const float* a, const float* b, const float* c, const fl
                         int nsys, int layout, int solver, cudaStream_t st);
 // stream-ordered device memory from a bounded pool of the library's own
 // (free with cudaFreeAsync)
-cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t st);
+enum ScratchKind { SCRATCH_LINES = 0, SCRATCH_HANDLES, SCRATCH_KINDS };
+cudaError_t scratch_alloc(ScratchKind kind, void** p, size_t bytes, cudaStream_t st);
 // gives the pool's idle memory on the current device back
-void scratch_trim();
+cudaError_t scratch_trim(ScratchKind kind);
 // reads and clears the flag set when a line-solve kernel's bounded wait on
 // its copies expired (synchronous)
 cudaError_t tridiag_take_timeout(int* flag);

@@ -734,25 +734,31 @@ cudaError_t block_solve(const R* a, const R* b, const R* c, const R* d, R* x, in
   return cudaGetLastError();
 }
 
-// Stream-ordered scratch from a pool of the library's own (one per device
-// context), so that memory freed after a call is still mapped at the next
-// one: with the device's default pool every synchronisation unmapped it, and
-// a 0.2 ms solve that the host waits for took 4.2 ms.  The pool keeps at most
-// kPoolKeep bytes mapped across synchronisations (a 128x128 gradient of the
-// coupled iteration with a checkpoint every 10 holds 21 MB: as thirty
-// cudaMalloc / cudaFree pairs its workspace cost 2 to 10 ms per call); a
-// handle that has used it for a gradient gives the idle memory back when it
-// is destroyed.  While `st` is captured, or if the pool cannot be had, the
-// default allocator serves.
-constexpr unsigned long long kPoolKeep = 256ull << 20;
+// Stream-ordered scratch from pools of the library's own (one of each kind per
+// device context), so that memory freed after a call is still mapped at the
+// next one: with the device's default pool every synchronisation unmapped it,
+// and a 0.2 ms solve that the host waits for took 4.2 ms.  What a pool keeps
+// mapped across synchronisations is bounded:
+//  * line solves 32 MB (the block kernel's scratch takes 8.4 MB at 4095x4095
+//    binary64); larger requests, those of the exact interleaved solve, go to
+//    the default pool and back to the device at the next synchronisation;
+//  * a handle's gradients and energy passes 256 MB (a 128x128 gradient of the
+//    coupled iteration with a checkpoint every 10 holds 21 MB: as thirty
+//    cudaMalloc / cudaFree pairs its workspace cost 2 to 10 ms per call), given
+//    back when the handle is destroyed.
+// ixb_release_scratch gives back what is idle of both.  While `st` is captured,
+// or if the pool cannot be had, the default allocator serves.
+constexpr unsigned long long kPoolKeep[SCRATCH_KINDS] = {32ull << 20, 256ull << 20};
 constexpr int kPoolDevices = 64;
 
 // the pool of the current device's context; made on first use with `make`,
 // else null if there is none
-cudaMemPool_t scratch_pool(int dev, bool make) {
+cudaMemPool_t scratch_pool(ScratchKind kind, int dev, bool make) {
   static std::mutex mu;
-  static cudaMemPool_t pool[kPoolDevices] = {};
-  static unsigned long long owner[kPoolDevices] = {};  // context the pool belongs to (0: none)
+  static cudaMemPool_t pools[SCRATCH_KINDS][kPoolDevices] = {};
+  static unsigned long long owners[SCRATCH_KINDS][kPoolDevices] = {};  // context the pool belongs to (0: none)
+  cudaMemPool_t* const pool = pools[kind];
+  unsigned long long* const owner = owners[kind];
   using CtxIdFn = CUresult (*)(CUcontext, unsigned long long*);
   static CtxIdFn ctx_id = nullptr;
   if (dev < 0 || dev >= kPoolDevices) return nullptr;
@@ -772,7 +778,7 @@ cudaMemPool_t scratch_pool(int dev, bool make) {
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = dev;
     cudaMemPool_t made = nullptr;
-    unsigned long long keep = kPoolKeep;
+    unsigned long long keep = kPoolKeep[kind];
     if (cudaMemPoolCreate(&made, &props) == cudaSuccess &&
         cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess) {
       pool[dev] = made;
@@ -785,20 +791,23 @@ cudaMemPool_t scratch_pool(int dev, bool make) {
 }
 }  // namespace
 
-cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t st) {
+cudaError_t scratch_alloc(ScratchKind kind, void** p, size_t bytes, cudaStream_t st) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if ((e = cudaStreamIsCapturing(st, &cap)) != cudaSuccess) return e;
-  cudaMemPool_t use = cap == cudaStreamCaptureStatusNone ? scratch_pool(dev, true) : nullptr;
+  const bool own = cap == cudaStreamCaptureStatusNone && (kind != SCRATCH_LINES || bytes <= kPoolKeep[kind]);
+  cudaMemPool_t use = own ? scratch_pool(kind, dev, true) : nullptr;
   return use ? cudaMallocFromPoolAsync(p, bytes, use, st) : cudaMallocAsync(p, bytes, st);
 }
 
-void scratch_trim() {
+cudaError_t scratch_trim(ScratchKind kind) {
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return;
-  if (cudaMemPool_t pool = scratch_pool(dev, false)) cudaMemPoolTrimTo(pool, 0);
+  const cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  cudaMemPool_t pool = scratch_pool(kind, dev, false);
+  return pool ? cudaMemPoolTrimTo(pool, 0) : cudaSuccess;
 }
 
 // ---------------------------------------------------------------------------
@@ -1259,7 +1268,7 @@ static cudaError_t tridiag_inter(const R* a, const R* b, const R* c, const R* d,
   // a few very long systems: the block ends, padded to whole groups, can
   // exceed the fixed array, which always holds the sequential solve's scratch
   const bool sequential = SOLVER == IXB_SOLVER_EXACT || (fixed && bytes > fixed_bytes);
-  if (!fixed && (e = scratch_alloc(&work, bytes, st)) != cudaSuccess) return e;
+  if (!fixed && (e = scratch_alloc(SCRATCH_LINES, &work, bytes, st)) != cudaSuccess) return e;
   if (!sequential) {
     e = block_solve(a, b, c, d, x, n, nsys, nsm, plan, work, st);
   } else {
@@ -1389,6 +1398,14 @@ extern "C" int ixb_tridiag_f64_noalloc(const double* a, const double* b, const d
   }
   if (e == cudaErrorInvalidValue) return IXB_EINVAL;
   return e == cudaSuccess ? IXB_OK : IXB_ECUDA;
+}
+
+// The memory of work still in flight is not idle, hence the wait.
+extern "C" int ixb_release_scratch(void) {
+  if (cudaDeviceSynchronize() != cudaSuccess) return IXB_ECUDA;
+  for (int k = 0; k < ixb::SCRATCH_KINDS; ++k)
+    if (ixb::scratch_trim((ixb::ScratchKind)k) != cudaSuccess) return IXB_ECUDA;
+  return IXB_OK;
 }
 
 // Failure-detection hook (no counterpart in the reference): the poll limit of
