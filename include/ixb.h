@@ -299,7 +299,8 @@ int ixb_release_scratch(void);
 int ixb_tridiag_status(void);
 /* Failure-detection hook, no counterpart in the reference: the number of
  * polls the first copy wait of every CTA of the streamed contiguous solve
- * (hybrid solver, layout 0) may take before it counts as expired; polls < 0
+ * (hybrid solver, layout 0) and of the interleaved solve in thread-block
+ * clusters (layout 1) may take before it counts as expired; polls < 0
  * restores the default (2^22 polls, at most about two seconds).  With 0 the
  * first wait expires at once: each CTA records the timeout, waits at the
  * default bound for its copies already in flight, and returns without

@@ -132,8 +132,8 @@ namespace {
 
 constexpr int kSpinLimit = 1 << 22;  // bounded mbarrier polls (a hang guard)
 __device__ int g_tri_timeout = 0;
-// Poll limit of the streamed kernel's first wait of every CTA (its other
-// waits, and the drain after a timeout, keep kSpinLimit); lowered only by
+// Poll limit of the first wait of every CTA of the streamed and the cluster
+// kernel (their other waits, and the drain after a timeout, keep kSpinLimit); lowered only by
 // ixb_tridiag_set_first_wait_limit, for failure-detection tests.
 __device__ int g_tri_first_wait_polls = kSpinLimit;
 
@@ -969,14 +969,16 @@ __global__ void __launch_bounds__(StridedCfg<R, SEG, ROWS>::T, 1)
   }
   cluster.sync();  // every CTA of the cluster runs and its mbarriers are set up
   if (tid == 0 && cl < ngroups) issue(cl);
-  unsigned parity = 0, xpar = 0;
-  bool failed = false;
-  for (int g = cl; g < ngroups; g += nclusters, xpar ^= 1) {
+  const int first_limit = *(volatile int*)&g_tri_first_wait_polls;
+  // phase of each mbarrier that is waited for next (a wait that ran out leaves it), tiles on their way
+  unsigned parity = 0, rpar = 0, xpar = 0;
+  bool loading = cl < ngroups, failed = false;
+  for (int g = cl; g < ngroups; g += nclusters) {
     const int sys = g * W + w;
     const bool live = sys < nsys;
-    if (!failed) {
-      const bool ok = mbar_wait_bounded(bar, parity);
-      failed = __syncthreads_or(!ok);
+    {
+      const bool ok = mbar_wait_bounded(bar, parity, g == cl ? first_limit : kSpinLimit);
+      if (__syncthreads_or(!ok)) { failed = true; break; }
       parity ^= 1;
     }
     // own rows into registers; row 0 has no a, row n-1 no c, and rows or
@@ -1012,7 +1014,8 @@ __global__ void __launch_bounds__(StridedCfg<R, SEG, ROWS>::T, 1)
       }
     }
     __syncthreads();  // the tiles are free: start loading the cluster's next group
-    if (tid == 0 && !failed && g + nclusters < ngroups) issue(g + nclusters);
+    loading = g + nclusters < ngroups;
+    if (tid == 0 && loading) issue(g + nclusters);
     // modified Thomas on the own rows (as in the contiguous kernels)
     R inv = fast_rcp(rb[1]);
     R ap = ra[1] * inv, cp = rc[1] * inv, dp = rd[1] * inv;
@@ -1042,12 +1045,13 @@ __global__ void __launch_bounds__(StridedCfg<R, SEG, ROWS>::T, 1)
     my_rows[2 * CH] = P2{eD, dp};
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic accesses -> copy engine
     __syncthreads();
-    if (tid < W && !failed)
+    if (tid < W)
       bulk_send(cluster_smem_addr(red + ((tid / Q) * Q + rank) * SC::RUN, tid % Q), outr + tid * SC::RUN,
                 (unsigned)(SC::RUN * sizeof(R)), cluster_smem_addr(rbar, tid % Q));
-    if (!failed) {
-      const bool ok = mbar_wait_bounded(rbar, xpar);
-      failed = __syncthreads_or(!ok);
+    {
+      const bool ok = mbar_wait_bounded(rbar, rpar);
+      if (__syncthreads_or(!ok)) { failed = true; break; }
+      rpar ^= 1;
     }
     {
       const P2 A = my_red[0], C = my_red[CH], D = my_red[2 * CH];
@@ -1063,13 +1067,14 @@ __global__ void __launch_bounds__(StridedCfg<R, SEG, ROWS>::T, 1)
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic accesses -> copy engine
     __syncthreads();
-    if (tid < W && !failed)  // owned system tid / Q, the chunks of rank tid % Q
+    if (tid < W)  // owned system tid / Q, the chunks of rank tid % Q
       bulk_send(cluster_smem_addr(xs + ((tid / Q) * Q + rank) * 2 * CH, tid % Q),
                 outx + 2 * ((tid / Q) * G + (tid % Q) * CH), (unsigned)(2 * CH * sizeof(R)),
                 cluster_smem_addr(xbar, tid % Q));
-    if (!failed) {
+    {
       const bool ok = mbar_wait_bounded(xbar, xpar);
-      failed = __syncthreads_or(!ok);
+      if (__syncthreads_or(!ok)) { failed = true; break; }
+      xpar ^= 1;
     }
     if (tid == 0) mbar_expect_tx(xbar, xs_bytes);  // the next ones come only after the rows sent below
     const P2 sol = reinterpret_cast<const P2*>(xs)[w * CH + k];
@@ -1084,22 +1089,25 @@ __global__ void __launch_bounds__(StridedCfg<R, SEG, ROWS>::T, 1)
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic writes -> tensor engine
     __syncthreads();
     // rows past n and systems past nsys fall outside the map and are not written
-    if (tid == 0 && !failed && stores) {
+    if (tid == 0 && stores) {
 #pragma unroll
       for (int bx = 0; bx < SC::BOXES; ++bx)
         if (rank * ROWS + bx * kStrBox < n) tile_store_2d(&mapX, g * W, rank * ROWS + bx * kStrBox, xt + bx * kStrBox * W);
     }
   }
+  cluster.sync();  // no CTA of the cluster sends any more
   if (tid == 0) {
     if (failed) {
       atomicExch(&g_tri_timeout, 1);
-      mbar_wait_bounded(bar, parity);  // copies still in flight land before the CTA leaves
-      mbar_wait_bounded(rbar, xpar);
+      // copies still in flight land before the CTA leaves (the last two waits
+      // run out if nothing more was sent)
+      if (loading) mbar_wait_bounded(bar, parity);
+      mbar_wait_bounded(rbar, rpar);
       mbar_wait_bounded(xbar, xpar);
     }
     bulk_store_wait_all();
   }
-  cluster.sync();  // no CTA leaves while another may still read its shared memory
+  cluster.sync();  // no CTA leaves while the copy engine may still read its shared memory
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no
@@ -1409,7 +1417,8 @@ extern "C" int ixb_release_scratch(void) {
 }
 
 // Failure-detection hook (no counterpart in the reference): the poll limit of
-// the first copy wait of every CTA of the streamed contiguous solve.
+// the first copy wait of every CTA of the streamed contiguous solve and of the
+// interleaved solve in clusters.
 extern "C" int ixb_tridiag_set_first_wait_limit(int polls) {
   return ixb::tridiag_set_first_wait_polls(polls) == cudaSuccess ? IXB_OK : IXB_ECUDA;
 }

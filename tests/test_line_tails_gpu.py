@@ -52,7 +52,7 @@ def _solve(a, b, c, d, layout, dtype):
 # every kernel of the two layouts: streamed lines (aligned, ragged), one staged line per CTA, whole systems in
 # registers, both cluster configurations, blocks of rows
 LINES = [(0, 96, 8), (0, 301, 9), (0, 701, 8), (0, 1024, 6), (0, 4096, 4), (0, 4863, 3), (0, 6001, 2), (1, 63, 8),
-         (1, 302, 33), (1, 512, 4800), (1, 1000, 9), (1, 1024, 2368), (1, 2048, 16), (1, 1153, 7), (1, 4100, 8)]
+         (1, 302, 33), (1, 512, 4800), (1, 1000, 9), (1, 1024, 4800), (1, 520, 9600), (1, 2048, 16), (1, 1153, 7), (1, 4100, 8)]
 
 
 @pytest.mark.parametrize("dtype", ["f64", "f32"])
