@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(T) tri_stream_kernel(const R* a, const R* b, c
   }
   if (tid == 0) mbar_init(bar);
   __syncthreads();
-  auto issue = [&](int s) {
+  auto issue = [&](unsigned s) {
     const size_t off = (size_t)s * n;
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // earlier reads of buf precede the copies
     unsigned bytes = 0;
@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(T) tri_stream_kernel(const R* a, const R* b, c
     }
   };
   // this thread's edge element of system s: its slot in buf (or -1) and value
-  auto edge_load = [&](int s, R& v) -> int {
+  auto edge_load = [&](unsigned s, R& v) -> int {
     if (!RAG || tid >= 8 * E) return -1;
     const int q = tid / (2 * E);
     const R* p = row_of(q) + (size_t)s * n;
@@ -272,7 +272,9 @@ __global__ void __launch_bounds__(T) tri_stream_kernel(const R* a, const R* b, c
     v = p[r];
     return q * NS + gr.shift + r;
   };
-  if (blockIdx.x < nsys) {
+  // systems are counted in unsigned: one past the last of 2^31 - 1 by a grid still fits
+  const unsigned systems = (unsigned)nsys;
+  if (blockIdx.x < systems) {
     if (tid == 0) issue(blockIdx.x);
     R v;
     const int slot = edge_load(blockIdx.x, v);
@@ -281,8 +283,8 @@ __global__ void __launch_bounds__(T) tri_stream_kernel(const R* a, const R* b, c
   const int first_limit = *(volatile int*)&g_tri_first_wait_polls;
   unsigned parity = 0;
   bool failed = false;
-  for (int s = blockIdx.x; s < nsys; s += gridDim.x) {
-    const bool ok = mbar_wait_bounded(bar, parity, s == (int)blockIdx.x ? first_limit : kSpinLimit);
+  for (unsigned s = blockIdx.x; s < systems; s += gridDim.x) {
+    const bool ok = mbar_wait_bounded(bar, parity, s == blockIdx.x ? first_limit : kSpinLimit);
     if (__syncthreads_or(!ok)) { failed = true; break; }
     parity ^= 1;
     // own rows into registers (row 0 has no a, row n-1 no c; identity rows past n)
@@ -311,10 +313,10 @@ __global__ void __launch_bounds__(T) tri_stream_kernel(const R* a, const R* b, c
       }
     }
     __syncthreads();  // the row buffers are free: start loading the next system
-    const int next = s + (int)gridDim.x;
+    const unsigned next = s + gridDim.x;
     R ev = R(0);
     int eslot = -1;
-    if (next < nsys) {
+    if (next < systems) {
       if (tid == 0) issue(next);
       eslot = edge_load(next, ev);
     }
