@@ -52,7 +52,7 @@ Geo<double> make_geo(const ixb_handle* h) {
   G.gm = h->prm.gamma_momen; G.ge = h->prm.gamma_energ; G.Ri = h->prm.Ri; G.Riy = h->prm.Riy;
   G.dt = h->prm.dt; G.rel_vel = h->prm.rel_vel; G.rel_pres = h->prm.rel_pres; G.rel_ener = h->prm.rel_ener;
   G.p_update = h->prm.p_update;
-  G.inv_gm = 1.0 / G.gm; G.inv_dt = 1.0 / G.dt; G.inv_rel_vel = 1.0 / G.rel_vel;
+  G.inv_dt = 1.0 / G.dt; G.inv_rel_vel = 1.0 / G.rel_vel;
   G.inv_rel_pres = 1.0 / G.rel_pres; G.inv_rel_ener = 1.0 / G.rel_ener;
   return G;
 }

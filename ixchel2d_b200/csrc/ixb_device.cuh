@@ -28,10 +28,9 @@ namespace ixb {
 
 // metric arrays inside one device buffer, each `mstride` long, 1-based.
 // M_HXU/M_HYV are the energy equation's face diffusivities
-// hmean(ge,ge,fexu(k)) / hmean(ge,ge,feyv(k)), M_RHXU/M_RHYV their
-// reciprocals (fast form), filled by the table kernel.  The fast form also
-// forms the diffusive conductances gamma*delta/d of the 2-D tables below
-// from 1-D factors (a uniform gamma makes them separable): M_GRDXP =
+// hmean(ge,ge,fexu(k)) / hmean(ge,ge,feyv(k)), filled by the table kernel.  The
+// fast form forms the diffusive conductances gamma*delta/d of the 2-D tables
+// below from 1-D factors (a uniform gamma makes them separable): M_GRDXP =
 // gamma_momen/dxp, M_GRDYV = gamma_momen/dyv, M_GRDXU = gamma_momen/dxu,
 // M_GRDYP = gamma_momen/dyp, M_HRDXU = M_HXU/dxu, M_HRDYV = M_HYV/dyv.  M_PE*
 // are the factors of |velocity| in 0.1|Peclet| (0.1 * spacing / diffusivity):
@@ -39,7 +38,7 @@ namespace ixb {
 // M_PHYV).
 enum Metric {
   M_DXP = 0, M_DYP, M_DXU, M_DYU, M_DXV, M_DYV, M_FEXP, M_FEYP, M_FEXU, M_FEYV,
-  M_HXU, M_HYV, M_RHXU, M_RHYV, M_GRDXP, M_GRDYV, M_GRDXU, M_GRDYP, M_HRDXU, M_HRDYV,
+  M_HXU, M_HYV, M_GRDXP, M_GRDYV, M_GRDXU, M_GRDYP, M_HRDXU, M_HRDYV,
   M_PEXP, M_PEYV, M_PEXU, M_PEYP, M_PHXU, M_PHYV, M_COUNT
 };
 
@@ -57,8 +56,8 @@ enum Metric {
 //   T_CV2(ii,jj)  v: gammas*deltaxv/ds; BN conductance = T_CV2(ii,jj+1)
 //   T_CT1(ii,jj)  T: gammai*deltayp/di; AD conductance = T_CT1(ii+1,jj)
 //   T_CT2(ii,jj)  T: gamman*deltaxp/dn; BS conductance = T_CT2(ii,jj-1)
-//   (the fast form divides the Peclet numbers of u and v by multiplying with
-//   the scalar 1/gamma_momen: the face diffusivities of a uniform gamma)
+//   (the fast form takes its Peclet numbers from the M_PE* factors: the face
+//   diffusivities of a uniform gamma are gamma itself up to rounding)
 enum Table { T_GU = 0, T_CU1, T_CU2, T_GV, T_CV1, T_CV2, T_CT1, T_CT2, T_COUNT };
 
 // sweeps: the eight line-solve phases of main.f90
@@ -104,7 +103,7 @@ struct Geo {
   const R* m;      // M_COUNT 1-D arrays
   const R* tab;    // T_COUNT 2-D tables
   R gm, ge, Ri, Riy, dt, rel_vel, rel_pres, rel_ener, p_update;
-  R inv_gm, inv_dt, inv_rel_vel, inv_rel_pres, inv_rel_ener;  // fast form
+  R inv_dt, inv_rel_vel, inv_rel_pres, inv_rel_ener;  // fast form
   __device__ __forceinline__ R met(int which, int k) const { return __ldg(m + which * mstride + k); }
   __device__ __forceinline__ int at(int ii, int jj) const { return (jj - 1) * LD + (ii - 1); }
   __device__ __forceinline__ R t(int which, int ii, int jj) const { return __ldg(tab + which * tstride + at(ii, jj)); }
@@ -185,7 +184,9 @@ __device__ __forceinline__ R plaw(R pe) {
 template <class R>
 __device__ __forceinline__ R dmax0(R x) { return fmaxT(R(0), x); }
 // max(0, x) by the sign bit (three integer operations; the binary64 maximum
-// takes the binary64 pipe, which the fast rows keep busy).  NaN stays NaN.
+// takes the binary64 pipe, which the fast rows keep busy).  NaN gives +0 or NaN,
+// by its own sign bit (fmax: +0): a row with a velocity that is not a number
+// carries it through the field values of its right-hand side.
 __device__ __forceinline__ double pos(double x) {
   const int hi = __double2hiint(x), keep = ~(hi >> 31);
   return __hiloint2double(hi & keep, __double2loint(x) & keep);

@@ -29,14 +29,12 @@ __global__ void table1d_kernel(Geo<R> G, R* met) {
   if (k >= 1 && k <= G.mi) {
     const R h = hmean(ge, ge, G.met(M_FEXU, k));
     met[M_HXU * G.mstride + k] = h;
-    met[M_RHXU * G.mstride + k] = R(1) / h;
     met[M_HRDXU * G.mstride + k] = ratio(h, G.met(M_DXU, k));
     met[M_PHXU * G.mstride + k] = R(0.1) * G.met(M_DXU, k) / h;
   }
   if (k >= 1 && k <= G.nj) {
     const R h = hmean(ge, ge, G.met(M_FEYV, k));
     met[M_HYV * G.mstride + k] = h;
-    met[M_RHYV * G.mstride + k] = R(1) / h;
     met[M_HRDYV * G.mstride + k] = ratio(h, G.met(M_DYV, k));
     met[M_PHYV * G.mstride + k] = R(0.1) * G.met(M_DYV, k) / h;
   }

@@ -1151,7 +1151,7 @@ bool strided_map(CUtensorMap* map, const R* p, int n, int nsys, int W) {
 template <class R, int SEG, int ROWS>
 cudaError_t strided_launch(const R* a, const R* b, const R* c, const R* d, R* x, int n, int nsys, cudaStream_t st) {
   using SC = StridedCfg<R, SEG, ROWS>;
-  int Q = 4;  // CTAs per cluster: a power of two >= 4 (W / Q systems of 32 lane chunks on each owner)
+  int Q = 4;  // CTAs per cluster: a power of two >= 4; each owns W / Q systems of a group
   while (Q * ROWS < n) Q <<= 1;
   if (Q > SC::QMAX) return cudaErrorInvalidValue;
   CUtensorMap maps[5];
