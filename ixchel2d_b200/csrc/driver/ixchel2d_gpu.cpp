@@ -261,7 +261,8 @@ void parse_args(int argc, char** argv, Options* o) {
           "                    [--cuerpo sincu|trian|cuadr|chime] [--no-autotune] [--mkdir] [--check] [--quiet]\n"
           "Runs the Ixchel2D case in CASE_DIR (default: the current folder) on the GPU.\n"
           "--check reads every input, prints what it found and exits without using the GPU.\n"
-          "The launch shapes of the line sweeps are autotuned on the initial state (--no-autotune: defaults).\n");
+          "Grids too large for the resident loop run one launch per line sweep; their launch shapes are\n"
+          "autotuned on the initial state (--no-autotune: defaults).\n");
       std::exit(0);
     } else if (!a.empty() && a[0] == '-') die(2, "unknown option " + a);
     else o->dir = a;
@@ -482,7 +483,9 @@ int main(int argc, char** argv) {
   }
   ck(ixb_upload_state(h, u.data(), v.data(), p.data(), T.data(), u_ant.data(), v_ant.data(), T_ant.data()),
      "ixb_upload_state");
-  if (opt.autotune) ck(ixb_autotune(h, 3, 0, nullptr, nullptr), "ixb_autotune");
+  int launches = 0;  // per outer iteration; 0: the resident kernel, whose shape is its own
+  ck(ixb_iteration_launches(h, &launches), "ixb_iteration_launches");
+  if (opt.autotune && launches > 0) ck(ixb_autotune(h, 3, 0, nullptr, nullptr), "ixb_autotune");
 
   if (say) {
     std::printf(" IXCHEL2D: Doble : kind=  8, Precision= 15 Rango= 307\n  \n");
