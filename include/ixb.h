@@ -52,7 +52,8 @@ extern "C" {
 #define IXB_PREC_FP32_REFINED 1
 
 /* line solvers */
-#define IXB_SOLVER_HYBRID 0 /* warp Thomas-PCR hybrid (default, fast) */
+#define IXB_SOLVER_HYBRID 0 /* Thomas-PCR hybrid (default, fast): chunks of rows eliminated without
+                               pivoting, for diagonally dominant rows */
 #define IXB_SOLVER_EXACT 1  /* sequential Thomas, bit-identical to
                                source/mod_solucionador.f90:25-47 */
 
@@ -195,9 +196,10 @@ typedef struct {
   double tol_maxbo;     /* stop when maxbo < tol_maxbo (0: never) */
 } ixb_nu_monitor;
 /* Outer SIMPLE iterations (ixb_simple_iterations' passes, no outer exit
- * test) until the monitored Nusselt number settles: one CUDA graph launch,
- * the Nusselt numbers and the stopping test run on the device between
- * blocks of `every` iterations, with no host round trip.  Derived from the
+ * test) until the monitored Nusselt number settles: the Nusselt numbers and
+ * the stopping test run on the device between blocks of `every` iterations,
+ * in one CUDA graph launch or between launches of the resident loop that are
+ * queued ahead.  Derived from the
  * reference's periodic Nusselt evaluation (main.f90:1226-1247,
  * nusselt_promedio_y of mod_postproceso.f90:100-215), which runs on the
  * host every 1000 time steps and stops nothing.  nu[2] (may be NULL): both

@@ -17,7 +17,7 @@
 // that neither lambda nor the transposed rows pass through memory: 2
 // launches and 6 loads per row and pass where staging, solving and
 // scattering took 6 launches (256 x 256, 200 passes with the forward run:
-// 7.8 ms then; with the passes resident, ixb_passes_fast.cu, 3.2 ms).
+// 7.8 ms then; with the passes resident, ixb_passes_fast.cu, 3.5 ms).
 // Built with FMA contraction, like the fast forward assembly, whose
 // coefficients it re-evaluates.  ixb_adjoint_energy_coupled extends this to
 // K outer SIMPLE iterations of a flow that evolves but does not depend on

@@ -28,7 +28,7 @@
 // them transposed in shared memory, solves, and scatters.  As row, transpose,
 // line-solve and scatter kernels it was 44 launches per reversed iteration
 // instead of 9, and bound by them up to 256x256 (128x128, 30 iterations, a
-// checkpoint every 10: 20.3 ms per gradient then, 4.6 now).  The recomputed sweeps and
+// checkpoint every 10: 20.3 ms per gradient then, 4.7 now).  The recomputed sweeps and
 // the reversed ones are launched with programmatic serialisation: each is a
 // few microseconds of latency, and the next one's launch overlaps it.
 //

@@ -26,13 +26,14 @@
 //    the loop.
 // The arithmetic is that of the fused sweep kernels.
 //
-// Measured per outer iteration, graph of fused sweeps -> this kernel (binary64
-// / refined): 64x64 52.7 / 55.7 -> 42.9 / 42.8 us, 161x97 58.7 / 59.3 -> 47.4 /
-// 48.3 us, 701x301 87.7 / 95.3 -> 79.8 / 82.8 us; with several passes per inner
-// loop the graph pays a conditional body each, this kernel nothing.  At
-// 701x301 a sweep takes 4.7 us of assembly (L1 and its latency), 2.7 us of
-// line solve and, with the wait for the CTA that has a line more, 2.1 us at
-// the barrier.
+// Measured per outer iteration of a developed field, graph of fused sweeps ->
+// this kernel (binary64 / refined): 64x64 54.2 / 54.3 -> 44.0 / 45.4 us, 161x97
+// 58.8 / 58.3 -> 49.3 / 51.3 us, 256x256 69.8 / 68.7 -> 57.4 / 59.8 us; at
+// 701x301 level, 84.5 / 88.9 -> 85.8 / 88.4 us, but with several passes per
+// inner loop the graph pays a conditional body each, this kernel nothing.
+// Bound by latencies: at 701x301 a warp's issue waits for barriers (the steps
+// of the reduced systems, the grid barrier) 9.7 cycles of some 15, for loads
+// 2.6, with 30 % of the issue slots and 0.6 % of the DRAM rate in use.
 #pragma once
 #include "ixb_grid.cuh"
 #include "ixb_loop.h"

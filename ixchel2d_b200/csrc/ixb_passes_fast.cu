@@ -12,7 +12,7 @@
 // A sweep then loads nine values (transposed five) per thread, moves one word
 // per thread and PCR step instead of three, divides nothing, and ends with a
 // grid barrier.  The fields ping-pong through L2.
-// Bound by latency: loads, PCR steps, the barrier (about 3 us per sweep).
+// Bound by latency: loads, PCR steps, the barrier (about 3.4 us per sweep at 256 x 256).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -247,9 +247,9 @@ size_t smem_of(int threads) { return (size_t)(2 * PQ + 4) * threads * sizeof(dou
 
 // One CTA per SM holds the lines of both directions: up to 256 chunks per
 // line and 448 threads (the factors of more do not fit in shared memory),
-// 445 x 445 on 148 SMs.  Per pass against two launches: 256 x 256 6.1 against
-// 9.8 us forward and 6.9 against 11.0 transposed, 64 x 64 5.4 against 7.8 and
-// 6.2 against 10.1; factoring costs about a pass, so the forward run takes it
+// 445 x 445 on 148 SMs.  Per pass against two launches: 256 x 256 6.8 against
+// 10.1 us forward and 6.7 against 10.1 transposed, 64 x 64 5.6 against 7.8 and
+// 5.2 against 8.6; factoring costs about a pass, so the forward run takes it
 // from four passes on.
 bool energy_passes_fit(int mi, int nj, int nsm, PassArgs* a) {
   PassArgs p{};

@@ -111,9 +111,9 @@ __global__ void __launch_bounds__(128) tri_inter_kernel(const R* __restrict__ a,
 // t*M+M-1 (M odd, so the threads of a warp reading their own row j hit
 // different banks); it eliminates them in registers (Chunk), the reduced rows
 // go through reduced_pcr, and each thread back-substitutes its rows.
-// Long lines are bound by HBM (4096 x 4096 binary64: 6.17 TB/s, 94 % of the
-// measured copy rate; 135.2 us before the reduced system's shared-memory
-// traffic was cut, 108.8 us since), short ones by the latency of one system.
+// Long lines are bound by HBM (4096 x 4096 binary64: 105 us, 6.4 TB/s, 98 % of
+// the measured copy rate; 135.2 us before the reduced system's shared-memory
+// traffic was cut), short ones by the latency of one system.
 //
 // Bulk copies move whole 16-byte granules.  A system that starts or ends
 // inside one (odd n, or an array that is not 16-byte aligned) keeps its
@@ -122,7 +122,8 @@ __global__ void __launch_bounds__(128) tri_inter_kernel(const R* __restrict__ a,
 // go by ordinary loads and stores, so nothing outside the system is touched.
 // (701-row systems, 302 of them, binary64: 22.5 us by the staged kernel
 // before, 9.8 us here.)  RAG picks that form; where every system fills whole
-// granules the fixed addresses save 5 % at 4096 x 4096 (113.0 against 107.3 us).
+// granules the fixed addresses save 5 % at 4096 x 4096 (113.0 against 107.3 us, both before this solve
+// reached 105).
 //
 // Every wait on the copy engine is bounded: on a timeout the CTA records it
 // in g_tri_timeout, waits (bounded) for its copies still in flight and
@@ -453,7 +454,7 @@ __global__ void __launch_bounds__(512) tri_cols_kernel(const R* a, const R* b, c
 // running CTAs hold, and the wait is bounded (g_tri_timeout).  Bound by the
 // latency of an item (64 KB in registers, two items per SM): 4095 x 4095
 // binary64 307 us (2.19 TB/s), against 5057 us for one thread per system;
-// where the cluster kernel applies it is faster (4096 x 4096: 154 against
+// where the cluster kernel applies it is faster (4096 x 4096: 156 against
 // 305 us).
 template <class R>
 struct BlockCfg {
@@ -838,7 +839,7 @@ cudaError_t scratch_trim(ScratchKind kind) {
 // (g_tri_timeout, as above).  (SEG, ROWS) = (128, 256) for lines of up to
 // 1024 rows; (64, 512) above, which halves W and so the cluster size that
 // holds a group (4096 rows: 8 instead of 16 CTAs; more clusters fit the GPU).
-// 4096 x 4096 binary64: 153 us, 4.4 TB/s on the 120 SMs that clusters of 8
+// 4096 x 4096 binary64: 156 us, 4.3 TB/s on the 120 SMs that clusters of 8
 // fill; with each owned system on one warp and the solutions read across the
 // cluster between two barriers 213 us (2048 x 2048: 43.8 against 55.8).
 // ---------------------------------------------------------------------------
