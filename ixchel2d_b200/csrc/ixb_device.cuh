@@ -590,30 +590,32 @@ __device__ __forceinline__ void pcr_row(R& A, R& C, R& D, R lA, R lC, R lD, R hA
 // The textbook form (rows re-read every step) moved 24 words.
 //
 // Each step squares the couplings (they are below one in diagonally dominant
-// rows), and the loop ends after a step whose neighbours added nothing to any
-// row of the line that can be seen next to that row's own right-hand side
-// (pcr_more).  The row's own: then no component is off by more than that part
-// of itself, however small it is beside the others, because the solution x of
-// the rows D = x + A x_lo + C x_hi differs from D by at most a part e / (1 - e)
-// where |A D_lo| + |C D_hi| <= e |D| in every row.  (A line that decays from its
-// boundary value goes on until its last chunks have theirs; a test of the
-// couplings alone, one step shorter, left them at zero.)  The test rides on
-// the barrier that publishes the next rows.  Lines of a developed field end a
-// step or two early; 701x301, per outer iteration, against all steps: 84.1
-// against 88.9 us binary64, 88.7 against 96.3 us refined.
+// rows), and the loop ends after a step whose neighbours added no more to any
+// row of the line than a part t of that row's own right-hand side (pcr_more),
+// t^2 being far below rounding.  Then nothing more can be seen in any
+// component, however small it is beside the others.  For let |A D_lo| + |C D_hi|
+// <= t |D| in every row of x + K x = D, K the couplings.  With the |D| as weights
+// K has the maximum norm t at most, so |x| <= |D| / (1 - t).  The step gives
+// x + K' x = D' where K' is K^2 without its diagonal, over 1 - that diagonal, and
+// |D'| >= |D| (1 - t) / (1 + t^2); hence |x - D'| <= t^2 |D'| up to terms of t^3:
+// dropping the steps that would follow costs a part t^2 of each component.
+// (A line that decays from its boundary value goes on until its last chunks
+// have theirs; a test of the couplings' size alone left them at zero.  A row of
+// zeros has to get exact zeros.)  The test rides on the barrier that publishes
+// the next rows.
 //
 // N elements per array in `red` (9N used with HALF, else 12N); the rows of
 // neighbouring chunks are TS elements apart.  All threads of the line(s)
 // call `sync(q)`, which orders shared memory between them and returns
 // whether q holds in any of them; `active` false: barriers only.
 //
-// Whether the neighbours' rows still count in x + A x_lo + C x_hi = D (not a
-// number counts: it has to reach the whole line).  2^-58 of binary64, 2^-44 of
-// binary32: far enough below rounding that the last bits are those of all steps.
+// Whether more steps are needed after the one of x + A x_lo + C x_hi = D (not a
+// number: yes, it has to reach the whole line).  t^2 is 2^-58 in binary64, 2^-44
+// in binary32: the last bits are those of all steps.
 template <class R>
 __device__ __forceinline__ bool pcr_more(R A, R C, R D, R lD, R hD) {
-  const R e = sizeof(R) == 8 ? R(3.5e-18) : R(5.7e-14);
-  return !(fabsT(A * lD) + fabsT(C * hD) <= e * fabsT(D));
+  const R t = sizeof(R) == 8 ? R(1.862645149230957e-9) : R(2.384185791015625e-7);  // 2^-29, 2^-22
+  return !(fabsT(A * lD) + fabsT(C * hD) <= t * fabsT(D));
 }
 
 template <class R, bool HALF, class Sync>
