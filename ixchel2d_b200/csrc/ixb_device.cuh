@@ -602,7 +602,8 @@ __device__ __forceinline__ void pcr_row(R& A, R& C, R& D, R lA, R lC, R lD, R hA
 // (A line that decays from its boundary value goes on until its last chunks
 // have theirs; a test of the couplings' size alone left them at zero.  A row of
 // zeros has to get exact zeros.)  The test rides on the barrier that publishes
-// the next rows.
+// the next rows.  701x301, per outer iteration, against all steps: 82.2 against
+// 88.9 us binary64, 84.6 against 96.3 us refined.
 //
 // N elements per array in `red` (9N used with HALF, else 12N); the rows of
 // neighbouring chunks are TS elements apart.  All threads of the line(s)

@@ -27,13 +27,13 @@
 // The arithmetic is that of the fused sweep kernels.
 //
 // Measured per outer iteration of a developed field, graph of fused sweeps ->
-// this kernel (binary64 / refined): 64x64 54.2 / 54.3 -> 44.0 / 45.4 us, 161x97
-// 58.8 / 58.3 -> 49.3 / 51.3 us, 256x256 69.8 / 68.7 -> 57.4 / 59.8 us; at
-// 701x301 level, 84.5 / 88.9 -> 85.8 / 88.4 us, but with several passes per
-// inner loop the graph pays a conditional body each, this kernel nothing.
+// this kernel (binary64 / refined): 64x64 53.1 / 53.9 -> 42.9 / 43.8 us, 161x97
+// 58.0 / 57.9 -> 47.0 / 48.7 us, 256x256 67.5 / 68.0 -> 55.2 / 57.4 us, 701x301
+// 83.3 / 87.8 -> 82.2 / 84.6 us (and with several passes per inner loop the
+// graph pays a conditional body each, this kernel nothing).
 // Bound by latencies: at 701x301 a warp's issue waits for barriers (the steps
-// of the reduced systems, the grid barrier) 9.7 cycles of some 15, for loads
-// 2.6, with 30 % of the issue slots and 0.6 % of the DRAM rate in use.
+// of the reduced systems, the grid barrier) 9.8 cycles of some 15, for loads
+// 2.7, with 30 % of the issue slots and 0.6 % of the DRAM rate in use.
 #pragma once
 #include "ixb_grid.cuh"
 #include "ixb_loop.h"

@@ -248,8 +248,8 @@ size_t smem_of(int threads) { return (size_t)(2 * PQ + 4) * threads * sizeof(dou
 // One CTA per SM holds the lines of both directions: up to 256 chunks per
 // line and 448 threads (the factors of more do not fit in shared memory),
 // 445 x 445 on 148 SMs.  Per pass against two launches: 256 x 256 6.8 against
-// 10.1 us forward and 6.7 against 10.1 transposed, 64 x 64 5.6 against 7.8 and
-// 5.2 against 8.6; factoring costs about a pass, so the forward run takes it
+// 9.8 us forward and 6.7 against 10.4 transposed, 64 x 64 5.6 against 7.6 and
+// 5.2 against 8.4; factoring costs about a pass, so the forward run takes it
 // from four passes on.
 bool energy_passes_fit(int mi, int nj, int nsm, PassArgs* a) {
   PassArgs p{};

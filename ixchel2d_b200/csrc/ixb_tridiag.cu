@@ -839,7 +839,7 @@ cudaError_t scratch_trim(ScratchKind kind) {
 // (g_tri_timeout, as above).  (SEG, ROWS) = (128, 256) for lines of up to
 // 1024 rows; (64, 512) above, which halves W and so the cluster size that
 // holds a group (4096 rows: 8 instead of 16 CTAs; more clusters fit the GPU).
-// 4096 x 4096 binary64: 156 us, 4.3 TB/s on the 120 SMs that clusters of 8
+// 4096 x 4096 binary64: 154 us, 4.4 TB/s on the 120 SMs that clusters of 8
 // fill; with each owned system on one warp and the solutions read across the
 // cluster between two barriers 213 us (2048 x 2048: 43.8 against 55.8).
 // ---------------------------------------------------------------------------
